@@ -2,7 +2,7 @@
 
     python nanogpt-120a_b200/build.py [--force] [--verbose]
 
-The quantizer translation unit is compiled with -fmad=false: its arithmetic must round
+The quantizer translation units are compiled with -fmad=false: their arithmetic must round
 exactly like the reference's device code (no multiply-add contraction).
 """
 from __future__ import annotations
@@ -23,6 +23,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relax
 UNITS = [
     # (source, extra flags)
     ("quant_kernels.cu", ["-fmad=false"]),
+    ("ms_eden_tile.cu", ["-fmad=false"]),
     ("gemm_tcgen05.cu", []),
     ("api.cu", []),
     ("tensor_amax_static.cu", []),

@@ -10,7 +10,6 @@
 // 16-group (four-six) or 32-chunk (MS-EDEN) in registers, loads it with 128-bit
 // transactions and writes nibbles as 8/16-byte words.  The reduction trees are evaluated
 // in the same order as the reference's xor butterflies, so the bytes are identical.
-#include <cuda_fp16.h>
 
 #include <cstdlib>
 #include <atomic>
@@ -18,6 +17,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "ms_eden.cuh"
 
 namespace nvfp4 {
 
@@ -214,11 +214,6 @@ __global__ void __launch_bounds__(256) amax_from_chunks_kernel(const float* __re
 }
 
 // out[0] = MS-EDEN global scale of amax[0] (single thread).
-// utils/quartet.rs:1-12: global scale of an MS-EDEN operand from the amax of its source.
-__device__ __forceinline__ float ms_eden_scale_of_amax(float a) {
-  const float so = (17.0f / 16.0f) * 0.93f;
-  return (a == 0.0f) ? 1.0f : a * so / (256.0f * 6.0f);
-}
 __global__ void ms_eden_scale_from_amax_kernel(const float* __restrict__ amax, float* __restrict__ out) {
   out[0] = ms_eden_scale_of_amax(amax[0]);
 }
@@ -668,271 +663,6 @@ __global__ void __launch_bounds__(256) packed_scale_pad_kernel(uint8_t* __restri
 // MS-EDEN
 // ============================================================================
 
-// nz(decode(encode_e4m3(v))) for v >= 0: the value of the nearest E4M3 code (ties to the even
-// code, saturating at 448), with zero mapped to one.  Inside the normal range [2^-6, 448) this is
-// a round-to-nearest-even of the f32 mantissa at bit 20 and never zero (checked against the CPU
-// restatement for every seventh f32 in the range); outside it the conversions are used.
-__device__ __forceinline__ float e4m3_rounded_value_nz(float v) {
-  const uint32_t bits = __float_as_uint(v);
-  if (bits - 0x3c800000u < 0x43e00000u - 0x3c800000u)
-    return __uint_as_float((bits + 0x0007ffffu + ((bits >> 20) & 1u)) & 0xfff00000u);
-  return nz(e4m3_value(cvt_e4m3(v)));
-}
-
-// pack/scale.rs:7-30 of utils/nvfp4/quant/kernels/ms_eden.
-__device__ __forceinline__ uint32_t stochastic_e4m3_scale(float value, uint32_t seed, uint32_t group) {
-  // Values inside the normal E4M3 range [2^-6, 448) -- every block scale of a tensor whose groups
-  // are within 2^14 of its amax -- need no conversions at all: the lower neighbour keeps the top
-  // three mantissa bits, its code is (exponent, those bits) rebased, the upper neighbour is the
-  // next code, and p = (value - down) / (up - down) is exactly the low 20 mantissa bits / 2^20.
-  // The draw is 24 hash bits / 2^24, so `draw < p` is an integer comparison.  Identical to the
-  // general path below for every value in the range (checked against the CPU restatement over
-  // 7.7 million values including every grid point and its neighbours).
-  const uint32_t vbits = __float_as_uint(value);
-  if (vbits - 0x3c800000u < 0x43e00000u - 0x3c800000u) {
-    const uint32_t draw = hash_u32(seed ^ group) & 0x00ffffffu;
-    return (vbits >> 20) - 960u + (draw < ((vbits & 0x000fffffu) << 4) ? 1u : 0u);
-  }
-  const uint32_t cb = cvt_e4m3(value);
-  const float cur = e4m3_value(cb);
-  const bool above = cur > value;
-  // Only the neighbour on the far side of `value` is needed: the code below when the nearest
-  // code lies above the value, the code above otherwise (clamped like the reference's prev / next).
-  const uint32_t ob = above ? (cb == 0 ? 0u : cb - 1u) : (cb == 255u ? 255u : cb + 1u);
-  const float other = e4m3_value(ob);
-  const float up = above ? cur : other;
-  const float down = above ? other : cur;
-  const uint32_t up_bits = above ? cb : ob;
-  const uint32_t down_bits = above ? ob : cb;
-  // p = (value - down) / (up - down).  Two E4M3 codes one step apart differ by +-2^e with
-  // -9 <= e <= 5 unless one of them is the NaN code or the step was clamped, so the difference is
-  // a power of two, zero or NaN.  For a power of two the quotient equals the product with the
-  // exact reciprocal (both round the same real number); for zero the reference takes p = 0 and
-  // for NaN the quotient is NaN: either way the draw is not below p and the lower code is kept.
-  const uint32_t dbits = __float_as_uint(up - down);
-  const uint32_t mag = dbits & 0x7fffffffu;
-  const bool pow2 = (mag & 0x007fffffu) == 0u && mag - 0x00800000u <= 0x7e000000u - 0x00800000u;
-  const float p = (value - down) * __uint_as_float((0x7f000000u - mag) | (dbits & 0x80000000u));
-  return (pow2 && random_unit_f32(seed, group) < p) ? up_bits : down_bits;
-}
-
-// a / b by the IEEE division instruction, issued unconditionally (the compiler would otherwise
-// wrap it in a branch where its result is selected away, and a branch per group costs more
-// than the quotient).
-__device__ __forceinline__ float div_rn_always(float a, float b) {
-  float r;
-  asm volatile("div.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
-
-// In-register 32-point Walsh-Hadamard butterfly in the reference's order
-// (pack/hadamard.rs:6-19): stride 1,2,4,8,16; low lane a+b, high lane a-b; then * 1/sqrt(32).
-// The chunk is held as 16 packed pairs P[i] = (u[i], u[i+16]): strides 1..8 act between
-// registers on both halves at once (packed add / sub), stride 16 inside each register.
-__device__ __forceinline__ void hadamard32_x2(f32x2_t (&P)[16]) {
-#pragma unroll
-  for (int stride = 1; stride < 16; stride <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      if ((i & stride) == 0) {
-        const f32x2_t a = P[i], b = P[i | stride];
-        P[i] = add2(a, b);
-        P[i | stride] = sub2(a, b);
-      }
-    }
-  }
-  const f32x2_t c = pack2(0.17677669f, 0.17677669f);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    float lo, hi;
-    unpack2(P[i], lo, hi);
-    P[i] = mul2(pack2(lo + hi, lo - hi), c);  // after this: low lane = group 0, high lane = group 1
-  }
-}
-
-// Two rotated 16-groups at once, one per packed lane (they may belong to one chunk or to two
-// different chunks): block scale, RTN nibbles, EDEN correction and the stochastic scale byte
-// of each (pack/payload.rs:15-69).  H points at the 16 packed values.  Returns the two scale
-// bytes (low lane in bits 0..7) and the 8 nibble bytes of each lane.
-__device__ __forceinline__ uint32_t ms_eden_group_lanes(const f32x2_t* H, float safe_gs, float so, float inv6,
-                                                        uint32_t scale_seed, uint32_t group_lo, uint32_t group_hi,
-                                                        uint2& nib_lo, uint2& nib_hi) {
-  float ga0 = 0.0f, ga1 = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 16; i += 2) {
-    float a0, a1, b0, b1;
-    unpack2(H[i], a0, a1);
-    unpack2(H[i + 1], b0, b1);
-    ga0 = max3_abs(ga0, a0, b0);
-    ga1 = max3_abs(ga1, a1, b1);
-  }
-  const float s0a = e4m3_rounded_value_nz(ga0 * so * inv6);
-  const float s0b = e4m3_rounded_value_nz(ga1 * so * inv6);
-  const f32x2_t inv = pack2(inv_scale(s0a, safe_gs), inv_scale(s0b, safe_gs));
-  f32x2_t x[16];
-  float xa[16], xb[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    x[i] = mul2(H[i], inv);
-    unpack2(x[i], xa[i], xb[i]);
-  }
-  nib_lo = make_uint2(cvt_e2m1x8(xa[0], xa[1], xa[2], xa[3], xa[4], xa[5], xa[6], xa[7]),
-                      cvt_e2m1x8(xa[8], xa[9], xa[10], xa[11], xa[12], xa[13], xa[14], xa[15]));
-  nib_hi = make_uint2(cvt_e2m1x8(xb[0], xb[1], xb[2], xb[3], xb[4], xb[5], xb[6], xb[7]),
-                      cvt_e2m1x8(xb[8], xb[9], xb[10], xb[11], xb[12], xb[13], xb[14], xb[15]));
-  float qa0[8], qa1[8], qb0[8], qb1[8];  // decoded nibbles: lane a / b, elements 0..7 / 8..15
-  e2m1x8_values(nib_lo.x, qa0);
-  e2m1x8_values(nib_lo.y, qa1);
-  e2m1x8_values(nib_hi.x, qb0);
-  e2m1x8_values(nib_hi.y, qb1);
-  // first level of the xor-8 butterfly sums formed on the spot: entry i = e[i] + e[i + 8]
-  f32x2_t num8[8], den8[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    num8[i] = add2(mul2_rounded(x[i], x[i]), mul2_rounded(x[i + 8], x[i + 8]));
-    den8[i] = add2(mul2_rounded(x[i], pack2(qa0[i], qb0[i])), mul2_rounded(x[i + 8], pack2(qa1[i], qb1[i])));
-  }
-  float num_a, num_b, den_a, den_b;
-  unpack2(add2(add2(add2(num8[0], num8[4]), add2(num8[2], num8[6])), add2(add2(num8[1], num8[5]), add2(num8[3], num8[7]))),
-          num_a, num_b);
-  unpack2(add2(add2(add2(den8[0], den8[4]), add2(den8[2], den8[6])), add2(add2(den8[1], den8[5]), add2(den8[3], den8[7]))),
-          den_a, den_b);
-  const float qa = div_rn_always(num_a, den_a), qb = div_rn_always(num_b, den_b);
-  const float sa = nz(s0a * (den_a == 0.0f ? 1.0f : qa));
-  const float sb = nz(s0b * (den_b == 0.0f ? 1.0f : qb));
-  return stochastic_e4m3_scale(sa, scale_seed, group_lo) | (stochastic_e4m3_scale(sb, scale_seed, group_hi) << 8);
-}
-
-// Both 16-groups of one rotated chunk (low lane = group 0, high lane = group 1).
-__device__ __forceinline__ uint32_t ms_eden_groups_x2(const f32x2_t (&H)[16], float safe_gs, float so, float inv6,
-                                                      uint32_t scale_seed, uint32_t group0, uint4& packed) {
-  uint2 lo, hi;
-  const uint32_t sb = ms_eden_group_lanes(&H[0], safe_gs, so, inv6, scale_seed, group0, group0 + 1, lo, hi);
-  packed = make_uint4(lo.x, lo.y, hi.x, hi.y);
-  return sb;
-}
-
-// Where one orientation of an MS-EDEN result goes.
-struct MsEdenOut {
-  uint8_t* fp4;
-  uint8_t* scales;
-  float* global_scales;
-  float* chunk_amax;      // optional
-  uint32_t rows;          // valid output rows
-  uint32_t dst_row_len;   // output K (multiple of 32)
-  uint32_t scale_seed;
-  uint32_t group_offset;  // added to the flat group id of the scale RNG
-  uint32_t group_row_stride;  // 16-groups per row in the scale RNG's index space (dst_row_len / 16 unless sharded)
-  uint32_t sign_offset;   // added to the K index of the sign hash
-  int packed;             // scale bytes in the packed tile layout
-};
-
-struct MsEdenParams {
-  const void* x;
-  const uint8_t* src_bytes;
-  const uint8_t* src_scales;
-  const float* src_global;
-  int src_packed;  // NVFP4 sources: scale bytes in the packed tile layout
-  uint32_t a;      // F32_ROWS: src_row_len; transposed kinds: source_rows
-  uint32_t b;      // transposed kinds: source_cols
-  const float* global_scale_dev;
-  float global_scale_host;
-  int use_host_scale;
-  float scale_override;
-  uint32_t sign_seed;
-  MsEdenOut out;
-};
-
-// Finishes one chunk whose signed inputs are in P (P[i] = (u[i], u[i+16])): rotation, two
-// groups, stores.
-__device__ __forceinline__ void ms_eden_emit_chunk(f32x2_t (&P)[16], const MsEdenOut& o, float gs, float so,
-                                                   uint32_t row, uint32_t chunk_in_row) {
-  const uint64_t chunk = static_cast<uint64_t>(row) * (o.dst_row_len >> 5) + chunk_in_row;
-  hadamard32_x2(P);
-  if (o.chunk_amax) {
-    float m = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float lo, hi;
-      unpack2(P[i], lo, hi);
-      m = max3_abs(m, lo, hi);
-    }
-    o.chunk_amax[chunk] = m;
-  }
-  const float safe_gs = nz(gs);
-  const float inv6 = inv_scale(6.0f, safe_gs);
-  const uint32_t group0 = row * o.group_row_stride + chunk_in_row * 2u + o.group_offset;
-  uint4 nibbles;
-  const uint32_t sb = ms_eden_groups_x2(P, safe_gs, so, inv6, o.scale_seed, group0, nibbles);
-  *reinterpret_cast<uint4*>(o.fp4 + chunk * 16) = nibbles;
-  // two consecutive k-groups of one k-atom: adjacent bytes in either layout, 2-byte aligned
-  const size_t off = o.packed ? packed_scale_offset(row, chunk_in_row * 2, o.dst_row_len >> 6) : chunk * 2;
-  *reinterpret_cast<uint16_t*>(o.scales + off) = static_cast<uint16_t>(sb);
-  if (chunk_in_row == 0) o.global_scales[row] = gs;
-}
-
-// Two chunks at once, one per packed lane (low lane = chunk of row_lo, high lane = chunk of
-// row_hi, both at chunk_in_row): P[k] holds the signed inputs of K position k of both, so all
-// five butterfly strides act between registers.
-__device__ __forceinline__ void ms_eden_emit_chunk_lanes(f32x2_t (&P)[32], const MsEdenOut& o, float gs, float so,
-                                                         uint32_t row_lo, uint32_t row_hi, uint32_t chunk_in_row) {
-  const uint32_t chunks_per_row = o.dst_row_len >> 5;
-  const uint64_t chunk_lo = static_cast<uint64_t>(row_lo) * chunks_per_row + chunk_in_row;
-  const uint64_t chunk_hi = static_cast<uint64_t>(row_hi) * chunks_per_row + chunk_in_row;
-#pragma unroll
-  for (int stride = 1; stride < 32; stride <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      if ((i & stride) == 0) {
-        const f32x2_t a = P[i], b = P[i | stride];
-        P[i] = add2(a, b);
-        P[i | stride] = sub2(a, b);
-      }
-    }
-  }
-  const f32x2_t c = pack2(0.17677669f, 0.17677669f);
-#pragma unroll
-  for (int i = 0; i < 32; ++i) P[i] = mul2(P[i], c);
-  if (o.chunk_amax) {
-    float m_lo = 0.0f, m_hi = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-      float a0, a1, b0, b1;
-      unpack2(P[i], a0, a1);
-      unpack2(P[i + 1], b0, b1);
-      m_lo = max3_abs(m_lo, a0, b0);
-      m_hi = max3_abs(m_hi, a1, b1);
-    }
-    o.chunk_amax[chunk_lo] = m_lo;
-    o.chunk_amax[chunk_hi] = m_hi;
-  }
-  const float safe_gs = nz(gs);
-  const float inv6 = inv_scale(6.0f, safe_gs);
-  const uint32_t g_lo = row_lo * o.group_row_stride + chunk_in_row * 2u + o.group_offset;
-  const uint32_t g_hi = row_hi * o.group_row_stride + chunk_in_row * 2u + o.group_offset;
-  uint2 lo0, hi0, lo1, hi1;
-  const uint32_t sb0 = ms_eden_group_lanes(&P[0], safe_gs, so, inv6, o.scale_seed, g_lo, g_hi, lo0, hi0);
-  const uint32_t sb1 = ms_eden_group_lanes(&P[16], safe_gs, so, inv6, o.scale_seed, g_lo + 1, g_hi + 1, lo1, hi1);
-  *reinterpret_cast<uint4*>(o.fp4 + chunk_lo * 16) = make_uint4(lo0.x, lo0.y, lo1.x, lo1.y);
-  *reinterpret_cast<uint4*>(o.fp4 + chunk_hi * 16) = make_uint4(hi0.x, hi0.y, hi1.x, hi1.y);
-  const uint32_t k_atoms = o.dst_row_len >> 6;
-  const size_t off_lo = o.packed ? packed_scale_offset(row_lo, chunk_in_row * 2, k_atoms) : chunk_lo * 2;
-  const size_t off_hi = o.packed ? packed_scale_offset(row_hi, chunk_in_row * 2, k_atoms) : chunk_hi * 2;
-  *reinterpret_cast<uint16_t*>(o.scales + off_lo) = static_cast<uint16_t>((sb0 & 0xffu) | ((sb1 & 0xffu) << 8));
-  *reinterpret_cast<uint16_t*>(o.scales + off_hi) = static_cast<uint16_t>(((sb0 >> 8) & 0xffu) | (sb1 & 0xff00u));
-  if (chunk_in_row == 0) {
-    o.global_scales[row_lo] = gs;
-    o.global_scales[row_hi] = gs;
-  }
-}
-
-// Signed input pair (u[i], u[i+16]) from two values and the chunk's 32 sign bits.
-__device__ __forceinline__ f32x2_t signed_pair(float lo, float hi, uint32_t neg_mask, int i) {
-  const uint32_t a = __float_as_uint(lo) ^ ((neg_mask << (31 - i)) & 0x80000000u);
-  const uint32_t b = __float_as_uint(hi) ^ ((neg_mask << (15 - i)) & 0x80000000u);
-  return pack2(__uint_as_float(a), __uint_as_float(b));
-}
-
 // Generic one-thread-per-chunk kernel (row sources, and the fallback for odd transposed
 // shapes).  Input gathers follow utils/nvfp4/quant/kernels/ms_eden/input/padded.rs:9-96.
 template <int kKind, typename T>
@@ -1002,27 +732,6 @@ __global__ void __launch_bounds__(128) ms_eden_kernel(const MsEdenParams p) {
 // source is read from memory once for both orientations, where the reference reads it twice
 // and gathers the transposed half with a row-pitch stride
 // (utils/nvfp4/quant/kernels/ms_eden/fp32_pair/dispatch.rs:13-43, input/padded.rs:9-96).
-struct MsEdenTileParams {
-  const void* x;
-  const uint8_t* src_bytes;
-  const uint8_t* src_scales;
-  const float* src_global;
-  int src_packed;
-  uint32_t src_rows, src_cols;
-  const float* global_scale_dev;
-  float global_scale_host;
-  int use_host_scale;
-  float scale_override;
-  uint32_t sign_seed;
-  MsEdenOut t;  // transposed operand: rows = src_cols, K = src_rows (padded)
-  MsEdenOut r;  // row operand (pair mode): rows = src_rows, K = src_cols (padded)
-  float* col_sum_partials;  // pair mode, optional: [row tiles][src_cols] column sums of each tile
-  // whole-tile pair kernel, optional: take the global scale from the source amax (every thread
-  // evaluates the same two operations) and publish it, instead of a one-thread kernel in between
-  const float* amax_in;
-  float* gs_out;
-};
-
 constexpr int kTileRows = 128, kTileCols = 64, kTileLd = kTileCols + 1;
 
 template <int kSrc, typename T, bool kPair>
@@ -1148,273 +857,6 @@ __global__ void __launch_bounds__(256) ms_eden_tile_kernel(const MsEdenTileParam
       ms_eden_emit_chunk(P, p.r, gs, p.scale_override, out_row, k0 >> 5);
     }
   }
-}
-
-// Pair kernel for sources whose extents are whole tiles (rows % 128 == 0, cols % 64 == 0):
-// the same outputs as ms_eden_tile_kernel<0, T, true>, organised for instruction count.
-//  * Persistent CTAs walk the tiles; the next tile's 128 x 128-byte rows arrive through
-//    cp.async into the other shared-memory stage while the current one is being quantized.
-//    The tile stays bf16; the 144-byte row pitch makes all three access patterns conflict-free.
-//  * Every thread quantizes TWO chunks at once, one per f32x2 lane, chosen so that both lanes
-//    share their K positions: warps 0-3 take two adjacent source columns down 32 rows (the
-//    transposed operand), warps 4-7 take rows r and r+32 along 32 columns (the row operand).
-//    One 32-bit shared load then feeds both lanes, the random signs are one xor on the raw
-//    bf16 pair, and all five Hadamard strides are packed register-to-register operations.
-constexpr int kPairPitch = 144;                          // bytes per staged row
-constexpr int kPairStageBytes = kTileRows * kPairPitch;  // 18432
-
-__device__ __forceinline__ void cp_async_16(uint32_t smem_addr, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-
-// f32 sources use the same kernel with a [128 x 64] f32 tile (272-byte pitch, dynamic shared
-// memory): a 64-bit load is the two lanes of the transposed role, two 32-bit values of rows r and
-// r + 32 those of the row role, and the signs are xors on the f32 sign bits.
-template <typename T>
-struct PairTile {
-  static constexpr bool kBf16 = sizeof(T) == 2;
-  static constexpr int kPitch = kBf16 ? kPairPitch : kTileCols * 4 + 16;  // bytes per staged row
-  static constexpr int kStageBytes = kTileRows * kPitch;
-  static constexpr int kPiecesPerRow = kTileCols * static_cast<int>(sizeof(T)) / 16;
-  static constexpr int kPiecesPerThread = kTileRows * kPiecesPerRow / 256;
-};
-
-template <typename T>
-__global__ void __launch_bounds__(256, 2) ms_eden_pair_kernel(const MsEdenTileParams p, uint32_t tiles_x,
-                                                               uint32_t tile_count) {
-  using PT = PairTile<T>;
-  constexpr bool kBf16 = PT::kBf16;
-  extern __shared__ __align__(16) uint8_t pair_stage[];       // [2][PT::kStageBytes]
-  __shared__ __align__(16) uint32_t flip_row[kTileRows];      // sign-bit mask of the row (both bf16 halves)
-  __shared__ __align__(16) uint32_t flip_col[kTileCols];      // bf16: per column pair; f32: per column
-  __shared__ __align__(16) float2 unflip_row[kTileRows];      // (-1, -1) where the row's sign is negative, else (1, 1)
-  __shared__ __align__(8) float quarter_sum[4][kTileCols];
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const T* x = static_cast<const T*>(p.x);
-  float gs;
-  if (p.amax_in) {
-    gs = ms_eden_scale_of_amax(p.amax_in[0]);
-    if (blockIdx.x == 0 && tid == 0) p.gs_out[0] = gs;
-  } else {
-    gs = p.use_host_scale ? p.global_scale_host : p.global_scale_dev[0];
-  }
-  const uint32_t stage_base = static_cast<uint32_t>(__cvta_generic_to_shared(pair_stage));
-
-  // 16-byte pieces of the tile, row-major, PT::kPiecesPerThread per thread
-  auto issue_tile = [&](uint32_t tile, uint32_t buf) {
-    const uint32_t r0 = (tile / tiles_x) * kTileRows, c0 = (tile % tiles_x) * kTileCols;
-#pragma unroll
-    for (int k = 0; k < PT::kPiecesPerThread; ++k) {
-      const uint32_t i = tid + 256 * k, row = i / PT::kPiecesPerRow, piece = i % PT::kPiecesPerRow;
-      cp_async_16(stage_base + buf * PT::kStageBytes + row * PT::kPitch + piece * 16,
-                  x + static_cast<size_t>(r0 + row) * p.src_cols + c0 + piece * (16 / sizeof(T)));
-    }
-  };
-
-  uint32_t tile = blockIdx.x, buf = 0;
-  if (tile < tile_count) issue_tile(tile, 0);
-  cp_async_commit();
-  for (; tile < tile_count; tile += gridDim.x, buf ^= 1) {
-    const uint32_t next = tile + gridDim.x;
-    if (next < tile_count) issue_tile(next, buf ^ 1);
-    cp_async_commit();
-    const uint32_t ty = tile / tiles_x, r0 = ty * kTileRows, c0 = (tile % tiles_x) * kTileCols;
-    if (tid < kTileRows) {
-      const bool neg = random_sign_negative(p.sign_seed, r0 + tid + p.t.sign_offset);
-      flip_row[tid] = neg ? (kBf16 ? 0x80008000u : 0x80000000u) : 0u;
-      unflip_row[tid] = neg ? make_float2(-1.0f, -1.0f) : make_float2(1.0f, 1.0f);
-    } else if (kBf16 && tid < kTileRows + kTileCols / 2) {
-      const uint32_t col = c0 + 2 * (tid - kTileRows) + p.r.sign_offset;
-      flip_col[tid - kTileRows] = (random_sign_negative(p.sign_seed, col) ? 0x00008000u : 0u) |
-                                  (random_sign_negative(p.sign_seed, col + 1) ? 0x80000000u : 0u);
-    } else if (!kBf16 && tid < kTileRows + kTileCols) {
-      const uint32_t col = c0 + (tid - kTileRows) + p.r.sign_offset;
-      flip_col[tid - kTileRows] = random_sign_negative(p.sign_seed, col) ? 0x80000000u : 0u;
-    }
-    cp_async_wait_all_but_one();
-    __syncthreads();
-    const uint8_t* t = pair_stage + buf * PT::kStageBytes;
-
-    f32x2_t P[32];
-    uint32_t row_lo, row_hi, chunk_in_row;
-    if (warp < 4) {
-      // transposed operand: source columns c0 + 2*lane (+1), K = source rows r0 + 32*warp ..
-      const uint8_t* src = t + warp * 32 * PT::kPitch + lane * 2 * sizeof(T);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const uint32_t f = flip_row[warp * 32 + i];
-        if (kBf16) {
-          const uint32_t w = *reinterpret_cast<const uint32_t*>(src + i * PT::kPitch) ^ f;
-          P[i] = pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-        } else {
-          const uint2 w = *reinterpret_cast<const uint2*>(src + i * PT::kPitch);
-          P[i] = pack2(__uint_as_float(w.x ^ f), __uint_as_float(w.y ^ f));
-        }
-      }
-      if (p.col_sum_partials) {
-        // Column sums of this tile (dbias partials) in their fixed order -- per column four
-        // sequential 32-row sums, combined below as ((q0 + q1) + q2) + q3 -- from the values this
-        // thread already holds: x = P * (+-1) exactly, so acc + x is one fused multiply-add.
-        f32x2_t acc = pack2(0.0f, 0.0f);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float2 u = unflip_row[warp * 32 + i];
-          acc = fma2(P[i], pack2(u.x, u.y), acc);
-        }
-        float a0, a1;
-        unpack2(acc, a0, a1);
-        *reinterpret_cast<float2*>(&quarter_sum[warp][2 * lane]) = make_float2(a0, a1);
-      }
-      row_lo = c0 + 2 * lane;
-      row_hi = row_lo + 1;
-      chunk_in_row = (r0 >> 5) + warp;
-    } else {
-      // row operand: rows r0 + base + lane and + 32 more, K = source columns c0 + 32*chunk ..
-      const uint32_t chunk = warp & 1, row = ((warp - 4) >> 1) * 64 + lane;
-      const uint8_t* src_lo = t + row * PT::kPitch + chunk * 32 * sizeof(T);
-      const uint8_t* src_hi = src_lo + 32 * PT::kPitch;
-      if (kBf16) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint4 a = *reinterpret_cast<const uint4*>(src_lo + 16 * j);
-          const uint4 b = *reinterpret_cast<const uint4*>(src_hi + 16 * j);
-          const uint4 f = *reinterpret_cast<const uint4*>(&flip_col[chunk * 16 + 4 * j]);
-          const uint32_t wa[4] = {a.x ^ f.x, a.y ^ f.y, a.z ^ f.z, a.w ^ f.w};
-          const uint32_t wb[4] = {b.x ^ f.x, b.y ^ f.y, b.z ^ f.z, b.w ^ f.w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            P[8 * j + 2 * k] = pack2(__uint_as_float(wa[k] << 16), __uint_as_float(wb[k] << 16));
-            P[8 * j + 2 * k + 1] = pack2(__uint_as_float(wa[k] & 0xffff0000u), __uint_as_float(wb[k] & 0xffff0000u));
-          }
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint4 a = *reinterpret_cast<const uint4*>(src_lo + 16 * j);
-          const uint4 b = *reinterpret_cast<const uint4*>(src_hi + 16 * j);
-          const uint4 f = *reinterpret_cast<const uint4*>(&flip_col[chunk * 32 + 4 * j]);
-          P[4 * j] = pack2(__uint_as_float(a.x ^ f.x), __uint_as_float(b.x ^ f.x));
-          P[4 * j + 1] = pack2(__uint_as_float(a.y ^ f.y), __uint_as_float(b.y ^ f.y));
-          P[4 * j + 2] = pack2(__uint_as_float(a.z ^ f.z), __uint_as_float(b.z ^ f.z));
-          P[4 * j + 3] = pack2(__uint_as_float(a.w ^ f.w), __uint_as_float(b.w ^ f.w));
-        }
-      }
-      row_lo = r0 + row;
-      row_hi = row_lo + 32;
-      chunk_in_row = (c0 >> 5) + chunk;
-    }
-    // one copy of the quantizer body for both roles (the role is warp-uniform)
-    ms_eden_emit_chunk_lanes(P, warp < 4 ? p.t : p.r, gs, p.scale_override, row_lo, row_hi, chunk_in_row);
-    __syncthreads();
-    if (p.col_sum_partials && tid < kTileCols)
-      p.col_sum_partials[static_cast<size_t>(ty) * p.src_cols + c0 + tid] =
-          ((quarter_sum[0][tid] + quarter_sum[1][tid]) + quarter_sum[2][tid]) + quarter_sum[3][tid];
-  }
-}
-
-// Transposer for NVFP4 sources whose extents are whole 128 x 128 tiles and whose scale bytes are
-// in the packed layout: the same outputs as ms_eden_tile_kernel<2 | 3, float, false>, organised
-// like the pair kernel above.  One nibble byte holds two adjacent source columns of one row,
-// which are exactly the two f32x2 lanes of a thread (two output rows, the same K position):
-// per K position a thread does one byte load, one E2M1x2 decode and two packed multiplies,
-// (q * scale) * global_scale as utils/nvfp4/tensor.rs:48-57 decodes.  The random sign of the K
-// position (the source row) is folded into that row's global scale, (q*s) * (-g) == -((q*s) * g).
-constexpr int kNvTileCols = 128;                          // source columns per tile
-constexpr int kNvBytePitch = kNvTileCols / 2 + 16;        // staged bytes per source row
-constexpr int kNvStageBytes = kTileRows * kNvBytePitch;   // 10240
-
-// Register budget of three CTAs per SM (80 registers, a few spilled words, same speed as the
-// unconstrained 113), launched two per SM: the free third of the register file lets the
-// bandwidth-bound dY amax kernel of the same backward call run beside it on another stream.
-template <bool kRowwise>
-__global__ void __launch_bounds__(256, 3) ms_eden_nvfp4_transpose_kernel(const MsEdenTileParams p, uint32_t tiles_x,
-                                                                          uint32_t tile_count) {
-  __shared__ __align__(16) uint8_t stage[2][kNvStageBytes];
-  __shared__ __align__(16) float2 scale2[kTileRows][kNvTileCols / 16];  // block scale of (row, group), duplicated
-  __shared__ __align__(16) float2 sgs2[kTileRows];                      // signed global scale of the row, duplicated
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float gs;
-  if (p.amax_in) {
-    // the global scale from the amax of the decoded source (every thread evaluates the same two operations),
-    // published for the GEMM that follows: no one-thread kernel in between
-    gs = ms_eden_scale_of_amax(p.amax_in[0]);
-    if (blockIdx.x == 0 && tid == 0) p.gs_out[0] = gs;
-  } else {
-    gs = p.use_host_scale ? p.global_scale_host : p.global_scale_dev[0];
-  }
-  const uint32_t stage_base = static_cast<uint32_t>(__cvta_generic_to_shared(&stage[0][0]));
-  const uint32_t k_atoms = p.src_cols >> 6;
-
-  // 512 16-byte pieces per tile, two per thread: piece i = row i/4, 16-byte column i%4
-  auto issue_tile = [&](uint32_t tile, uint32_t buf) {
-    const uint32_t r0 = (tile / tiles_x) * kTileRows, c0 = (tile % tiles_x) * kNvTileCols;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const uint32_t i = tid + 256 * k, row = i >> 2, piece = i & 3;
-      cp_async_16(stage_base + buf * kNvStageBytes + row * kNvBytePitch + piece * 16,
-                  p.src_bytes + ((static_cast<size_t>(r0 + row) * p.src_cols + c0) >> 1) + piece * 16);
-    }
-  };
-  // The tile's 1024 scale bytes are two adjacent 512-byte blocks of the packed plane; thread t
-  // takes word t: block t/128, and inside it the four groups of row (w%4)*32 + w/4, w = t%128.
-  auto scale_word = [&](uint32_t tile) {
-    const uint32_t rb = tile / tiles_x, atom0 = (tile % tiles_x) * 2;
-    return __ldg(reinterpret_cast<const uint32_t*>(p.src_scales + (static_cast<size_t>(rb) * k_atoms + atom0) * 512u) + tid);
-  };
-
-  uint32_t tile = blockIdx.x, buf = 0;
-  uint32_t sw = 0;
-  if (tile < tile_count) {
-    issue_tile(tile, 0);
-    sw = scale_word(tile);
-  }
-  cp_async_commit();
-  for (; tile < tile_count; tile += gridDim.x, buf ^= 1) {
-    const uint32_t next = tile + gridDim.x;
-    uint32_t sw_next = 0;
-    if (next < tile_count) {
-      issue_tile(next, buf ^ 1);
-      sw_next = scale_word(next);
-    }
-    cp_async_commit();
-    const uint32_t r0 = (tile / tiles_x) * kTileRows, c0 = (tile % tiles_x) * kNvTileCols;
-    {
-      const uint32_t w = tid & 127, row = (w & 3) * 32 + (w >> 2), g0 = (tid >> 7) * 4;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float sc = e4m3_value((sw >> (8 * j)) & 0xffu);
-        scale2[row][g0 + j] = make_float2(sc, sc);
-      }
-    }
-    if (tid < kTileRows) {
-      const float g = kRowwise ? p.src_global[r0 + tid] : p.src_global[0];
-      const float sg = random_sign_negative(p.sign_seed, r0 + tid + p.t.sign_offset) ? -g : g;
-      sgs2[tid] = make_float2(sg, sg);
-    }
-    cp_async_wait_all_but_one();
-    __syncthreads();
-
-    // thread: source columns c0 + 2*cp (+1), K = source rows r0 + 32*q ..
-    const uint32_t cp = tid & 63, q = tid >> 6;
-    const uint8_t* src = stage[buf] + q * 32 * kNvBytePitch + cp;
-    f32x2_t P[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float2 qv = e2m1x2_values(src[i * kNvBytePitch]);
-      const float2 sc = scale2[q * 32 + i][cp >> 3];
-      const float2 sg = sgs2[q * 32 + i];
-      // the last product feeds the butterfly's packed adds: it has to be the rounded form
-      P[i] = mul2_rounded(mul2(pack2(qv.x, qv.y), pack2(sc.x, sc.y)), pack2(sg.x, sg.y));
-    }
-    const uint32_t out_row = c0 + 2 * cp;
-    ms_eden_emit_chunk_lanes(P, p.t, gs, p.scale_override, out_row, out_row + 1, (r0 >> 5) + q);
-    __syncthreads();
-    sw = sw_next;
-  }
-  (void)lane;
-  (void)warp;
 }
 
 // ReLU^2 backward between the two MLP linears (gpt/mlp/kernels.rs:72-104):
@@ -1904,15 +1346,13 @@ static bool tile_covers(uint32_t src_rows, uint32_t dst_row_len) {
 
 int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a_in, const float* amax_in, float* gs_out) {
   nvfp4_ms_eden_args a = a_in;
+  const bool nv_kind = a.src_kind == NVFP4_SRC_NVFP4_TRANSPOSED || a.src_kind == NVFP4_SRC_ROWWISE_NVFP4_TRANSPOSED;
+  const bool nv_tiles = nv_kind && a.rows != 0 && a.cols != 0 && tile_covers(a.rows, a.dst_row_len) &&
+                        ms_eden_nvfp4_has_tile_form(a.src_bytes, a.src_scales, a.cols);
   if (amax_in) {
-    // the whole-tile NVFP4 transposers derive the scale from the amax themselves; every other kernel gets it
-    // from a one-thread kernel first
-    const bool nv_kind = a.src_kind == NVFP4_SRC_NVFP4_TRANSPOSED || a.src_kind == NVFP4_SRC_ROWWISE_NVFP4_TRANSPOSED;
-    const bool whole = nv_kind && a.src_scale_layout == NVFP4_SCALES_PACKED && a.rows % kTileRows == 0 &&
-                       a.cols % kNvTileCols == 0 && a.dst_row_len == a.rows &&
-                       (reinterpret_cast<uintptr_t>(a.src_bytes) & 15u) == 0 &&
-                       (reinterpret_cast<uintptr_t>(a.src_scales) & 3u) == 0 && a.rows != 0 && a.cols != 0;
-    if (!whole) {
+    // the tiled NVFP4 transposer derives the scale from the amax itself; every other kernel gets it from a
+    // one-thread kernel first
+    if (!nv_tiles) {
       const int rc = launch_ms_eden_scale_from_amax(s, amax_in, gs_out);
       if (rc) return rc;
       amax_in = nullptr;
@@ -1945,26 +1385,17 @@ int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a_in, const float* 
     p.col_sum_partials = nullptr;
     p.amax_in = amax_in;
     p.gs_out = gs_out;
-    const bool nv_whole_tiles = p.src_packed && a.rows % kTileRows == 0 && a.cols % kNvTileCols == 0 &&
-                                a.dst_row_len == a.rows && (reinterpret_cast<uintptr_t>(a.src_bytes) & 15u) == 0 &&
-                                (reinterpret_cast<uintptr_t>(a.src_scales) & 3u) == 0;
-    const uint32_t nv_tiles_x = a.cols / kNvTileCols, nv_tiles = nv_tiles_x * (a.rows / kTileRows);
+    if (nv_tiles) return launch_ms_eden_nvfp4_tiles(s, p, a.src_kind == NVFP4_SRC_ROWWISE_NVFP4_TRANSPOSED);
     switch (a.src_kind) {
       case NVFP4_SRC_F32_TRANSPOSED:
         if (bf16) launch_tile<0, __nv_bfloat16, false>(s, p);
         else launch_tile<0, float, false>(s, p);
         break;
       case NVFP4_SRC_NVFP4_TRANSPOSED:
-        if (nv_whole_tiles)
-          ms_eden_nvfp4_transpose_kernel<false><<<min(nv_tiles, 148u * 2u), 256, 0, s>>>(p, nv_tiles_x, nv_tiles);
-        else
-          launch_tile<2, float, false>(s, p);
+        launch_tile<2, float, false>(s, p);
         break;
       case NVFP4_SRC_ROWWISE_NVFP4_TRANSPOSED:
-        if (nv_whole_tiles)
-          ms_eden_nvfp4_transpose_kernel<true><<<min(nv_tiles, 148u * 2u), 256, 0, s>>>(p, nv_tiles_x, nv_tiles);
-        else
-          launch_tile<3, float, false>(s, p);
+        launch_tile<3, float, false>(s, p);
         break;
       default:
         return 1;
@@ -2027,13 +1458,8 @@ int launch_col_sum_reduce(cudaStream_t s, const float* partials, float* dbias, u
   NVFP4_RETURN_LAST();
 }
 
-static bool pair_whole_tiles(const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_args& t) {
-  return r.rows % kTileRows == 0 && r.cols % kTileCols == 0 && t.dst_row_len == r.rows && r.dst_row_len == r.cols &&
-         (reinterpret_cast<uintptr_t>(r.x) & 15u) == 0;
-}
-
 bool ms_eden_pair_takes_amax(const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_args& t) {
-  return ms_eden_pair_is_tiled(r, t) && pair_whole_tiles(r, t);
+  return ms_eden_pair_is_tiled(r, t) && ms_eden_pair_has_tile_form(r.x, r.src_dtype, r.cols);
 }
 
 int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_args& t,
@@ -2062,29 +1488,8 @@ int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& r, const nvfp4
   p.col_sum_partials = col_sum_partials;
   p.amax_in = amax_in;
   p.gs_out = gs_out;
-  const bool whole_tiles = pair_whole_tiles(r, t);
-  if (whole_tiles) {
-    const uint32_t tiles_x = cols / kTileCols, tile_count = tiles_x * (rows / kTileRows);
-    const uint32_t grid = min(tile_count, 148u * 2u);
-    if (r.src_dtype == NVFP4_DTYPE_BF16) {
-      ms_eden_pair_kernel<__nv_bfloat16>
-          <<<grid, 256, 2 * PairTile<__nv_bfloat16>::kStageBytes, s>>>(p, tiles_x, tile_count);
-    } else {
-      // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
-      static std::atomic<int> attr_state[64];  // per device ordinal: 0 = not set, 1 = set, -(error) = failed
-      int dev = 0;
-      if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return static_cast<int>(cudaErrorInvalidDevice);
-      int st = attr_state[dev].load(std::memory_order_acquire);
-      if (st == 0) {
-        const cudaError_t e = cudaFuncSetAttribute(ms_eden_pair_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   2 * PairTile<float>::kStageBytes);
-        st = e == cudaSuccess ? 1 : -static_cast<int>(e);
-        attr_state[dev].store(st, std::memory_order_release);
-      }
-      if (st < 0) return -st;
-      ms_eden_pair_kernel<float><<<grid, 256, 2 * PairTile<float>::kStageBytes, s>>>(p, tiles_x, tile_count);
-    }
-  } else if (r.src_dtype == NVFP4_DTYPE_BF16) {
+  if (ms_eden_pair_has_tile_form(r.x, r.src_dtype, cols)) return launch_ms_eden_pair_tiles(s, p, r.src_dtype);
+  if (r.src_dtype == NVFP4_DTYPE_BF16) {
     launch_tile<0, __nv_bfloat16, true>(s, p);
   } else {
     launch_tile<0, float, true>(s, p);

@@ -1,0 +1,77 @@
+"""Tiled quantizer kernels of the linear backward at the sizes where tiling can go wrong: one row, a row either side of
+a 128-row tile, column counts inside and beyond a 64-column tile and a 128-row scale block, and the values that leave
+the straight-line path.  Bit-exact against the oracle, and against the generic one-thread-per-chunk kernel on a tensor
+large enough for a single wrong rounding in a few million block scales to show."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import bf16_normal
+
+pytestmark = pytest.mark.gpu
+SIGN, SCALE = 0x12345678, 0x9ABCDEF0
+
+
+def cpu(t):
+    return t.detach().cpu().numpy()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,in_dim,out_dim", [(1, 64, 64), (127, 64, 72), (128, 192, 136), (129, 128, 200),
+                                                   (257, 320, 64), (130, 64, 1000)])
+def test_backward_operands_ragged_tiles(pkg, oracle, dev, tokens, in_dim, out_dim, dtype):
+    q, bwd = pkg.Nvfp4QuantModule(), pkg.LinearBackwardModule()
+    x, w = bf16_normal(701, (tokens, in_dim)), bf16_normal(702, (out_dim, in_dim), 0.02)
+    dy = bf16_normal(703, (tokens, out_dim), 1e-3)
+    dy[tokens // 2] = 0.0                     # zero groups, negative zeros, sub-normal block scales, one outlier
+    dy[:, out_dim // 3] = -0.0
+    dy[: max(1, tokens // 4)] *= 2.0 ** -20
+    dy[-1, -1] = 3.0e4
+    x[tokens // 3] = 0.0
+    w[:, in_dim // 2] = 0.0
+    w[out_dim // 2] *= 2.0 ** -14
+    xq = q.quantize_four_six(x.to(dev), rowwise=True, packed=True, decoded_amax=True)
+    wq = q.quantize_four_six(w.to(dev), rowwise=False, packed=True)
+    sc = pkg.LinearBackwardScratch(tokens, in_dim, out_dim, dev)
+    e = dy.to(dev) if dtype == torch.bfloat16 else dy.float().to(dev)
+    _, _, db = bwd.backward_ms_eden(e=e, weight=wq, input=xq, scratch=sc, sign_seed=SIGN, scale_seed=SCALE)
+    torch.cuda.synchronize()
+    assert pkg.read_device_status() == 0
+    xf, wf, ef = x.float().numpy(), w.float().numpy(), dy.float().numpy()
+    oxq, owq = oracle.four_six(xf, oracle.row_amax(xf), True), oracle.four_six(wf, oracle.tensor_amax(wf)[1], False)
+    ok, tk = oracle.padded_k(out_dim), oracle.padded_k(tokens)
+    gs_e = oracle.ms_eden_global_scale(float(np.abs(ef).max()))
+    gs_w = oracle.ms_eden_global_scale(float(oracle.nvfp4_amax(*owq, out_dim, in_dim, False)[1][0]))
+    gs_x = oracle.ms_eden_global_scale(float(oracle.nvfp4_amax(*oxq, tokens, in_dim, True)[1][0]))
+    want = {
+        "e_h": (oracle.ms_eden(0, ef, tokens, ok, gs_e, SIGN, SCALE, want_chunk_amax=False), tokens, ok),
+        "e_t_h": (oracle.ms_eden(1, ef, out_dim, tk, gs_e, SIGN, SCALE ^ 0x85EBCA6B, want_chunk_amax=False), out_dim, tk),
+        "weight_t_h": (oracle.ms_eden(2, (*owq, out_dim, in_dim), in_dim, ok, gs_w, SIGN, SCALE ^ 0x9E3779B9,
+                                      want_chunk_amax=False), in_dim, ok),
+        "input_t_h": (oracle.ms_eden(3, (*oxq, tokens, in_dim), in_dim, tk, gs_x, SIGN, SCALE ^ 0xC2B2AE35,
+                                     want_chunk_amax=False), in_dim, tk),
+    }
+    for name, (ref, rows, k) in want.items():
+        op = getattr(sc, name)
+        assert np.array_equal(cpu(op["bytes"]), ref[0]), name
+        assert np.array_equal(cpu(op["scales_packed"]), oracle.scale_pack(ref[1], rows, k)), name
+        assert np.array_equal(cpu(op["global_scales"]), ref[2]), name
+    assert np.array_equal(cpu(db), oracle.bias_grad_tiled(ef))
+
+
+def test_pair_rows_equal_generic_kernel_large(pkg, dev):
+    """16.4 million block scales of dY rows: the pair kernel against the generic kernel, every byte."""
+    q, bwd = pkg.Nvfp4QuantModule(), pkg.LinearBackwardModule()
+    tokens, in_dim, out_dim = 8192, 64, 32000
+    g = torch.Generator(device=dev).manual_seed(11)
+    e = (torch.randn((tokens, out_dim), generator=g, device=dev) * 1e-3).to(torch.bfloat16)
+    x = torch.randn((tokens, in_dim), generator=g, device=dev).to(torch.bfloat16)
+    w = (torch.randn((out_dim, in_dim), generator=g, device=dev) * 0.02).to(torch.bfloat16)
+    xq = q.quantize_four_six(x, rowwise=True, packed=True, decoded_amax=True)
+    wq = q.quantize_four_six(w, rowwise=False, packed=True)
+    sc = pkg.LinearBackwardScratch(tokens, in_dim, out_dim, dev)
+    bwd.backward_ms_eden(e=e, weight=wq, input=xq, scratch=sc, sign_seed=SIGN, scale_seed=SCALE)
+    ref, _ = q.ms_eden_quantize(src_kind=pkg.SRC_F32_ROWS, x=e, rows=tokens, cols=out_dim, dst_row_len=out_dim,
+                                global_scale=sc.e_h["global_scale"], sign_seed=SIGN, scale_seed=SCALE, packed=True)
+    assert torch.equal(sc.e_h["bytes"], ref.bytes)
+    assert torch.equal(sc.e_h["scales_packed"], ref.scales)

@@ -142,6 +142,13 @@ int nvfp4_quantize_four_six(void* stream, const void* x, int dtype, const float*
                             uint32_t rows, uint32_t cols, uint8_t* out_fp4, uint8_t* out_scales,
                             int scale_layout, float* out_global_scale);
 
+/* Tensor amax and tensor-scale four-six of one matrix: nvfp4_tensor_amax_* followed by nvfp4_quantize_four_six with
+ * rowwise = 0, without the amax leaving the library (the reduction's partial maxima go straight to the quantizer: two
+ * launches instead of three).  partials: f32[nvfp4_tensor_amax_partials()] scratch. */
+uint32_t nvfp4_tensor_amax_partials(void);
+int nvfp4_quantize_four_six_tensor(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols, float* partials,
+                                   uint8_t* out_fp4, uint8_t* out_scales, int scale_layout, float* out_global_scale);
+
 /* Row amax and rowwise four-six in one pass over the input (the caller pattern
  * RowwiseNvfp4Scratch::quantize_row_amax, crates/gpt2-nvfp4/src/types/nvfp4_scratch/scratch.rs:35-52,
  * issues row_amax_f32 then fp32_to_nvfp4_four_six_rowwise).  Same bytes as those two calls.
@@ -200,6 +207,11 @@ int nvfp4_materialize_schedule_free_matrix(void* stream, const float* z_master, 
                                            float* chunk_amax, float* amax, uint8_t* bytes, uint8_t* scales,
                                            int scale_layout, float* global_scale, float beta, uint32_t rows,
                                            uint32_t cols);
+/* The same through scratch for the reduction's partial maxima (f32[nvfp4_tensor_amax_partials()]) instead of a chunk
+ * list: two launches instead of three, no chunk maxima. */
+int nvfp4_materialize_schedule_free_partials(void* stream, const float* z_master, const float* x_master, float* partials,
+                                             float* amax, uint8_t* bytes, uint8_t* scales, int scale_layout,
+                                             float* global_scale, float beta, uint32_t rows, uint32_t cols);
 
 /* MS-EDEN quantizer (random-sign Hadamard-32 rotation, RTN nibbles, EDEN-corrected block
  * scale rounded stochastically with a counter RNG) ---------------------------------------- */

@@ -135,6 +135,7 @@ _SIGNATURES = {
     "nvfp4_fp32_to_nvfp4_four_six_padded": [_P, _P, _P, _P, _P, _P, _U, _U, _U, _U],
     "nvfp4_fp32_transpose_to_nvfp4_four_six_padded": [_P, _P, _P, _P, _P, _P, _U, _U, _U, _U],
     "nvfp4_quantize_four_six": [_P, _P, c_int, _P, c_int, _U, _U, _P, _P, c_int, _P],
+    "nvfp4_quantize_four_six_tensor": [_P, _P, c_int, _U, _U, _P, _P, _P, c_int, _P],
     "nvfp4_quantize_four_six_rowwise_fused": [_P, _P, c_int, _U, _U, _P, _P, c_int, _P, _P, _P],
     "nvfp4_quantize_relu2_four_six_rowwise": [_P, _P, c_int, _U, _U, _P, _P, _P, c_int, _P, _P, _P],
     "nvfp4_tc_matmul_ms_eden": [_P, _P, _P, _P, POINTER(MsEdenOperand), _F, POINTER(MsEdenOperand), _F, _U, _U, _U, _U, _U],
@@ -144,6 +145,7 @@ _SIGNATURES = {
     "nvfp4_relu2_backward_amax": [_P, _P, c_int, _P, _P, c_int, ctypes.c_uint64, _P, _U, POINTER(c_uint32)],
     "nvfp4_materialize_schedule_free": [_P, _P, _P, _P, _P, _P, _P, _P, _F, _U],
     "nvfp4_materialize_schedule_free_matrix": [_P, _P, _P, _P, _P, _P, _P, c_int, _P, _F, _U, _U],
+    "nvfp4_materialize_schedule_free_partials": [_P, _P, _P, _P, _P, _P, _P, c_int, _P, _F, _U, _U],
     "nvfp4_ms_eden_quantize": [_P, POINTER(MsEdenArgs)],
     "nvfp4_fp32_to_nvfp4_ms_eden": [_P, _P, _P, _P, _P, _P, _U, _U, _U, _F, _F, _U, _U],
     "nvfp4_fp32_to_nvfp4_ms_eden_device_scale": [_P, _P, _P, _P, _P, _P, _P, _U, _U, _U, _F, _U, _U],
@@ -217,6 +219,7 @@ _SPECIAL = {
     "nvfp4_get_deterministic_reductions": (c_int, []),
     "nvfp4_launch_count": (ctypes.c_uint64, []),
     "nvfp4_last_error": (c_char_p, []),
+    "nvfp4_tensor_amax_partials": (c_uint32, []),
     "nvfp4_padded_k": (c_uint32, [_U]),
     "nvfp4_scale_padded_mn_extent": (c_uint32, [_U]),
     "nvfp4_scale_packed_len": (c_size_t, [_U, _U]),

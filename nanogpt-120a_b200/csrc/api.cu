@@ -111,6 +111,23 @@ int nvfp4_quantize_four_six(void* stream, const void* x, int dtype, const float*
                          scale_layout == NVFP4_SCALES_PACKED, out_gs);
 }
 
+uint32_t nvfp4_tensor_amax_partials(void) { return kAmaxPartials; }
+int nvfp4_quantize_four_six_tensor(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols, float* partials,
+                                   uint8_t* out_fp4, uint8_t* out_scales, int scale_layout, float* out_gs) {
+  if (cols % 16 != 0) return invalid("quantize_four_six_tensor: cols must be a multiple of 16");
+  if (scale_layout == NVFP4_SCALES_PACKED && cols % 64 != 0)
+    return invalid("quantize_four_six_tensor: the packed scale layout needs cols % 64 == 0");
+  if (dtype != NVFP4_DTYPE_F32 && dtype != NVFP4_DTYPE_BF16) return invalid("quantize_four_six_tensor: unknown dtype");
+  if (reinterpret_cast<uintptr_t>(x) & 15u) return invalid("quantize_four_six_tensor: input must be 16-byte aligned");
+  if (!partials) return invalid("quantize_four_six_tensor: null partials");
+  const uint64_t n = static_cast<uint64_t>(rows) * cols;
+  if (n == 0) return 0;
+  const int rc = launch_tensor_amax(S(stream), x, dtype, nullptr, nullptr, n, partials);
+  if (rc) return rc;
+  return launch_four_six(S(stream), x, dtype, partials, 0, rows, cols, out_fp4, out_scales,
+                         scale_layout == NVFP4_SCALES_PACKED, out_gs, 0, nullptr, tensor_amax_partials(n));
+}
+
 int nvfp4_quantize_four_six_rowwise_fused(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols,
                                           uint8_t* out_fp4, uint8_t* out_scales, int scale_layout,
                                           float* out_global_scale, float* out_row_amax,
@@ -217,6 +234,20 @@ int nvfp4_materialize_schedule_free_matrix(void* stream, const float* z_master, 
     return invalid("materialize_schedule_free_matrix: the masters must be 16-byte aligned");
   return launch_schedule_free_materialize(S(stream), z_master, x_master, beta, chunk_amax, amax, bytes, scales,
                                           scale_layout == NVFP4_SCALES_PACKED, global_scale, rows, cols);
+}
+
+int nvfp4_materialize_schedule_free_partials(void* stream, const float* z_master, const float* x_master, float* partials,
+                                             float* amax, uint8_t* bytes, uint8_t* scales, int scale_layout,
+                                             float* global_scale, float beta, uint32_t rows, uint32_t cols) {
+  if (cols % 16 != 0) return invalid("materialize_schedule_free_partials: cols must be a multiple of 16");
+  if (scale_layout == NVFP4_SCALES_PACKED && cols % 64 != 0)
+    return invalid("materialize_schedule_free_partials: the packed scale layout needs cols % 64 == 0");
+  if (!partials || !amax || !bytes || !scales || !global_scale || (rows && cols && (!z_master || !x_master)))
+    return invalid("materialize_schedule_free_partials: null pointer");
+  if ((reinterpret_cast<uintptr_t>(z_master) | reinterpret_cast<uintptr_t>(x_master)) & 15u)
+    return invalid("materialize_schedule_free_partials: the masters must be 16-byte aligned");
+  return launch_schedule_free_materialize(S(stream), z_master, x_master, beta, nullptr, amax, bytes, scales,
+                                          scale_layout == NVFP4_SCALES_PACKED, global_scale, rows, cols, partials);
 }
 
 // ---- MS-EDEN ----------------------------------------------------------------------------

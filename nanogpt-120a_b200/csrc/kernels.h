@@ -10,7 +10,12 @@ namespace nvfp4 {
 
 // quant_kernels.cu --------------------------------------------------------------------------
 int launch_row_amax(cudaStream_t s, const void* x, int dtype, float* out, uint32_t rows, uint32_t row_len);
-int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_amax, float* out, uint64_t n);
+// partials (optional, kAmaxPartials floats): every CTA leaves its maximum there -- tensor_amax_partials(n) of them -- for
+// a consumer that reduces them, and `out` is not touched (no zeroing launch, no atomics).
+constexpr uint32_t kAmaxPartials = 148u * 4u;
+uint32_t tensor_amax_partials(uint64_t n);
+int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_amax, float* out, uint64_t n,
+                       float* partials = nullptr);
 int launch_nvfp4_amax(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, const float* gscales, uint32_t rows,
                       uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out);
 // transform 0: out[0] = max(chunks); 1: out[0] = MS-EDEN global scale of that max
@@ -19,7 +24,7 @@ int launch_ms_eden_scale_from_amax(cudaStream_t s, const float* amax, float* out
 // relu2: quantize relu(x)^2 computed on load; decoded_amax (optional f32[1]): max |decoded value| of the result
 int launch_four_six(cudaStream_t s, const void* x, int dtype, const float* amax, int rowwise, uint32_t rows,
                     uint32_t cols, uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, int relu2 = 0,
-                    float* decoded_amax = nullptr);
+                    float* decoded_amax = nullptr, uint32_t amax_count = 1);
 int launch_four_six_rowwise_fused(cudaStream_t s, const void* x, int dtype, uint32_t rows, uint32_t cols,
                                   uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, float* out_amax,
                                   float* decoded_amax, int relu2 = 0);
@@ -30,7 +35,7 @@ int launch_packed_scale_pad(cudaStream_t s, uint8_t* packed, uint32_t rows, uint
 // y = z + beta * (x - z) -> tensor amax -> four-six (tensor scale); chunk_amax optional
 int launch_schedule_free_materialize(cudaStream_t s, const float* z, const float* x, float beta, float* chunk_amax,
                                      float* amax, uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs,
-                                     uint32_t rows, uint32_t cols);
+                                     uint32_t rows, uint32_t cols, float* partials = nullptr);
 // amax_in / gs_out (optional): the global scale is the MS-EDEN scale of amax_in[0] (derived inside the kernel
 // where the kernel supports it, by a one-thread kernel otherwise) and is written to gs_out[0]; a.global_scale
 // and a.host_global_scale are then not read.

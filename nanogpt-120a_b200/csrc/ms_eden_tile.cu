@@ -92,18 +92,6 @@ __device__ __forceinline__ float widen_f16_lo(uint32_t x) {
   return r;
 }
 
-// a / b, correctly rounded, for b and a / b well inside the normal range: a reciprocal refined once, the quotient
-// corrected by its exact remainder (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990).  No range check and no branch; compared with the division operator over 2^34 operand pairs of
-// the range this file uses it on (tests/test_gpu_parity.py repeats a sample).
-__device__ __forceinline__ float div_in_range(float a, float b) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-  y = __fmaf_rn(y, __fmaf_rn(-b, y, 1.0f), y);
-  const float q = __fmul_rn(a, y);
-  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-}
-
 // Stochastic E4M3 code of a value in [2^-6, 448): lower neighbour plus one with probability (low 20 mantissa bits) /
 // 2^20, drawn as 24 hash bits < low bits * 16 (ms_eden.cuh: stochastic_e4m3_scale, same comparison shifted up by 8).
 __device__ __forceinline__ uint32_t stochastic_code(uint32_t value_bits, uint32_t seed, uint32_t group) {
@@ -122,22 +110,6 @@ __device__ __forceinline__ void first_stage_hi(uint32_t a, uint32_t b, uint32_t 
   const float ua = __uint_as_float((a ^ sa) & 0xffff0000u), ub = __uint_as_float((b ^ sb) & 0xffff0000u);
   sum = __fadd_rn(ua, ub);
   diff = __fsub_rn(ua, ub);
-}
-
-// Eight E2M1 codes, byte selects inside the conversions.  `opaque_zero` is 0 and unknown to the compiler: without an
-// operation between packing the codes and unpacking them the assembler forwards the unmasked 8-bit temporaries and the
-// values come out wrong (common.cuh: e2m1x8_values spends a byte extract per conversion on it instead).
-__device__ __forceinline__ void e2m1x8_unpacked(uint32_t word, uint32_t opaque_zero, float (&q)[8]) {
-  word ^= opaque_zero;
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t.reg .b32 h0, h1, h2, h3;\n\t.reg .b16 l0, l1, l2, l3, u0, u1, u2, u3;\n\t"
-      "mov.b32 {b0, b1, b2, b3}, %8;\n\t"
-      "cvt.rn.f16x2.e2m1x2 h0, b0;\n\tcvt.rn.f16x2.e2m1x2 h1, b1;\n\t"
-      "cvt.rn.f16x2.e2m1x2 h2, b2;\n\tcvt.rn.f16x2.e2m1x2 h3, b3;\n\t"
-      "mov.b32 {l0, u0}, h0;\n\tmov.b32 {l1, u1}, h1;\n\tmov.b32 {l2, u2}, h2;\n\tmov.b32 {l3, u3}, h3;\n\t"
-      "add.rn.f32.f16 %0, l0, %9;\n\tcvt.f32.f16 %1, u0;\n\tadd.rn.f32.f16 %2, l1, %9;\n\tcvt.f32.f16 %3, u1;\n\t"
-      "add.rn.f32.f16 %4, l2, %9;\n\tcvt.f32.f16 %5, u2;\n\tadd.rn.f32.f16 %6, l3, %9;\n\tcvt.f32.f16 %7, u3;\n\t}"
-      : "=f"(q[0]), "=f"(q[1]), "=f"(q[2]), "=f"(q[3]), "=f"(q[4]), "=f"(q[5]), "=f"(q[6]), "=f"(q[7])
-      : "r"(word), "f"(-0.0f));
 }
 
 // Two chunks of one thread, one per packed lane.

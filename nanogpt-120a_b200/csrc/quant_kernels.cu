@@ -99,6 +99,26 @@ __device__ __forceinline__ void cta_atomic_max(float warp_value, float* out) {
   }
 }
 
+// The CTA's maximum to its slot of `partials` where the consumer reduces them (no zeroing launch, no atomics), else one
+// atomic max into out[0].
+__device__ __forceinline__ void cta_publish_max(float warp_value, float* out, float* partials) {
+  if (!partials) {
+    cta_atomic_max(warp_value, out);
+    return;
+  }
+  __shared__ float partial[8];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float m = warp_max(warp_value);
+  if (lane == 0) partial[w] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float r = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r = max_f32(r, partial[i]);
+    partials[blockIdx.x] = r;
+  }
+}
+
 // amax of one full, 16-byte aligned 1024-value chunk, 32 lanes cooperating (result in every lane).
 // bf16: the maximum is taken on packed bf16 pairs (exact -- a maximum rounds nothing -- and NaN
 // operands are dropped like max.f32 drops them), four instructions per eight values.
@@ -130,7 +150,8 @@ __device__ __forceinline__ float chunk_amax_1024<__nv_bfloat16>(const __nv_bfloa
 // utils/nvfp4/quant/kernels/row_amax.rs:67-101.
 template <typename T>
 __global__ void __launch_bounds__(256) tensor_amax_kernel(const T* __restrict__ x, float* __restrict__ chunk_amax,
-                                                           float* __restrict__ out, uint64_t n) {
+                                                           float* __restrict__ out, float* __restrict__ partials,
+                                                           uint64_t n) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t warps = static_cast<uint64_t>(gridDim.x) * 8;
   const uint64_t chunks = (n + 1023) / 1024;
@@ -149,7 +170,7 @@ __global__ void __launch_bounds__(256) tensor_amax_kernel(const T* __restrict__ 
     if (lane == 0 && chunk_amax) chunk_amax[chunk] = m;
     running = max_f32(running, m);
   }
-  cta_atomic_max(running, out);
+  cta_publish_max(running, out, partials);
 }
 
 // amax of a decoded NVFP4 tensor [n/cols][cols], warps striding over 1024-value chunks.
@@ -221,60 +242,101 @@ __global__ void ms_eden_scale_from_amax_kernel(const float* __restrict__ amax, f
 // ============================================================================
 // four-six
 // ============================================================================
+//
+// Bound by instruction dispatch like the MS-EDEN kernels (ms_eden_tile.cu has the measured costs): per 16-group two
+// candidate scales, two sets of nibbles and two error sums.  The scalar side of a group -- two quotients by the global
+// scale, two reciprocals, two E4M3 conversions -- is straight-line code for global scales inside [2^-80, 2^80]
+// (four IEEE divisions with their range checks and branches cost a third of the group before); other global scales,
+// NaN included, take the generic code per group.
 
 __device__ __forceinline__ float four_six_global_scale(float amax) {
   // utils/nvfp4/quant/kernels/four_six/helpers.rs:33-39 with scale_override = 1.0
   return nz(amax == 0.0f ? 1.0f : amax * 1.0f / (256.0f * 6.0f));
 }
 
-// Squared quantization error of the group for the 6-anchored (low lane) and the 4-anchored
-// (high lane) candidate scale at once: sum of (v - q(v*inv) * (s*gs))^2 in butterfly order
-// (utils/nvfp4/quant/kernels/convert.rs:27-35), each lane with its own inv / dequant scale.
-// The nibble bytes of both candidates come back too: the winner's bytes are the output.
-__device__ __forceinline__ f32x2_t candidate_errors16(const float (&v)[16], float s6, float s4, float gs, uint2& nib6,
-                                                      uint2& nib4, float& inv6, float& inv4) {
-  inv6 = inv_scale(s6, gs);
-  inv4 = inv_scale(s4, gs);
-  const f32x2_t inv = pack2(inv6, inv4);
-  const f32x2_t dq = pack2(s6 * gs, s4 * gs);
-  float x6[16], x4[16];
+// What the groups of one global scale share.
+struct FourSixScale {
+  float gs;        // global scale
+  float d6, y6;    // 6 gs + eps and its reciprocal
+  float d4, y4;
+  float limit;     // groups with a larger amax (the caller's amax was not theirs) take the generic code
+  bool plain;      // gs inside the range of the straight-line code
+  __device__ __forceinline__ explicit FourSixScale(float amax) {
+    // amax / 1536 correctly rounded (the remainder form, exact for every amax the straight-line code accepts)
+    const float quick = div_by_rcp(amax, 1536.0f, 1.0f / 1536.0f);
+    plain = quick >= 0x1p-80f && quick <= 0x1p80f;
+    gs = plain ? quick : four_six_global_scale(amax);
+    d6 = 6.0f * gs + kDenomEps;
+    d4 = 4.0f * gs + kDenomEps;
+    y6 = rcp_in_range(d6);
+    y4 = rcp_in_range(d4);
+    limit = plain ? gs * 0x1p20f : -1.0f;
+  }
+};
+
+// Squared quantization error of the group for one candidate scale: sum of (v - q(v * inv) * dq)^2 in butterfly order
+// (utils/nvfp4/quant/kernels/convert.rs:27-35).  V[i] = (v[i], v[i + 8]).  The nibble bytes come back too: the
+// winner's bytes are the output.
+__device__ __forceinline__ float candidate_error16(const f32x2_t (&V)[8], float inv, float dq, uint32_t opaque_zero, uint2& nib) {
+  const f32x2_t inv2 = pack2(inv, inv), dq2 = pack2(dq, dq);
+  float lo[8], hi[8];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) unpack2(mul2(pack2(v[i], v[i]), inv), x6[i], x4[i]);
-  nib6 = make_uint2(cvt_e2m1x8(x6[0], x6[1], x6[2], x6[3], x6[4], x6[5], x6[6], x6[7]),
-                    cvt_e2m1x8(x6[8], x6[9], x6[10], x6[11], x6[12], x6[13], x6[14], x6[15]));
-  nib4 = make_uint2(cvt_e2m1x8(x4[0], x4[1], x4[2], x4[3], x4[4], x4[5], x4[6], x4[7]),
-                    cvt_e2m1x8(x4[8], x4[9], x4[10], x4[11], x4[12], x4[13], x4[14], x4[15]));
-  float q6a[8], q6b[8], q4a[8], q4b[8];
-  e2m1x8_values(nib6.x, q6a);
-  e2m1x8_values(nib6.y, q6b);
-  e2m1x8_values(nib4.x, q4a);
-  e2m1x8_values(nib4.y, q4b);
-  f32x2_t a8[8];  // first butterfly level: a8[i] = e[i] + e[i + 8]
+  for (int i = 0; i < 8; ++i) unpack2(mul2(V[i], inv2), lo[i], hi[i]);
+  nib = make_uint2(cvt_e2m1x8(lo[0], lo[1], lo[2], lo[3], lo[4], lo[5], lo[6], lo[7]),
+                   cvt_e2m1x8(hi[0], hi[1], hi[2], hi[3], hi[4], hi[5], hi[6], hi[7]));
+  float qa[8], qb[8];
+  e2m1x8_unpacked(nib.x, opaque_zero, qa);
+  e2m1x8_unpacked(nib.y, opaque_zero, qb);
+  float a8[8];  // first butterfly level: e[i] + e[i + 8]
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const f32x2_t d0 = sub2(pack2(v[i], v[i]), mul2_rounded(pack2(q6a[i], q4a[i]), dq));
-    const f32x2_t d8 = sub2(pack2(v[i + 8], v[i + 8]), mul2_rounded(pack2(q6b[i], q4b[i]), dq));
-    a8[i] = add2(mul2_rounded(d0, d0), mul2_rounded(d8, d8));
+    const f32x2_t d = sub2(V[i], mul2_rounded(pack2(qa[i], qb[i]), dq2));
+    float e0, e1;
+    unpack2(mul2(d, d), e0, e1);
+    a8[i] = e0 + e1;  // scalar: never contracted with the product
   }
-  return add2(add2(add2(a8[0], a8[4]), add2(a8[2], a8[6])), add2(add2(a8[1], a8[5]), add2(a8[3], a8[7])));
+  return ((a8[0] + a8[4]) + (a8[2] + a8[6])) + ((a8[1] + a8[5]) + (a8[3] + a8[7]));
 }
 
-// v: one 16-group.  Returns the scale byte and writes the 8 nibble bytes into `packed`.
-// helpers.rs:42-76 and four_six.rs:309-344 of utils/nvfp4/quant/kernels.  The output nibbles
-// are cvt(v * inv) with the chosen candidate's inv, i.e. exactly that candidate's trial bytes.
-__device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float gs, uint2& packed,
-                                                   float* decoded_amax = nullptr) {
-  float ga = 0.0f;
+// The scale byte of one candidate pair and everything that follows from it, any values.
+__device__ __noinline__ void four_six_scales_any(float ga, float gs, uint32_t& codes, float& inv6, float& inv4) {
+  const uint32_t b6 = cvt_e4m3(ga * 1.0f / (6.0f * gs + kDenomEps));
+  const uint32_t b4 = cvt_e4m3(ga * 1.0f / (4.0f * gs + kDenomEps));
+  codes = b6 | (b4 << 8);
+  inv6 = inv_scale(e4m3_value(b6), gs);
+  inv4 = inv_scale(e4m3_value(b4), gs);
+}
+
+// v: one 16-group, ga its amax.  Returns the scale byte and writes the 8 nibble bytes into `packed`.
+// helpers.rs:42-76 and four_six.rs:309-344 of utils/nvfp4/quant/kernels.  The output nibbles are cvt(v * inv) with the
+// chosen candidate's inv, i.e. exactly that candidate's trial bytes.
+__device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float ga, const FourSixScale& sc, uint32_t opaque_zero,
+                                                   uint2& packed, float* decoded_amax = nullptr) {
+  uint32_t codes;
+  float inv6, inv4;
+  {
+    uint16_t c;
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;"
+        : "=h"(c)
+        : "f"(div_by_rcp(ga, sc.d4, sc.y4)), "f"(div_by_rcp(ga, sc.d6, sc.y6)));
+    codes = c;
+  }
+  const bool plain = ga <= sc.limit;
+  if (!plain) four_six_scales_any(ga, sc.gs, codes, inv6, inv4);
+  uint32_t h2;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"(static_cast<uint16_t>(codes)));
+  const float2 s = __half22float2(*reinterpret_cast<__half2*>(&h2));
+  const float dq6 = s.x * sc.gs, dq4 = s.y * sc.gs;
+  if (plain) {
+    inv6 = rcp_in_range((s.x == 0.0f ? sc.gs : dq6) + kDenomEps);
+    inv4 = rcp_in_range((s.y == 0.0f ? sc.gs : dq4) + kDenomEps);
+  }
+  f32x2_t V[8];
 #pragma unroll
-  for (int i = 0; i < 16; i += 2) ga = max3_abs(ga, v[i], v[i + 1]);
-  const float gsn = nz(gs);
-  const uint32_t b6 = cvt_e4m3(ga * 1.0f / (6.0f * gsn + kDenomEps));
-  const uint32_t b4 = cvt_e4m3(ga * 1.0f / (4.0f * gsn + kDenomEps));
-  const float s6 = e4m3_value(b6);
-  const float s4 = e4m3_value(b4);
-  float err6, err4, inv6, inv4;
+  for (int i = 0; i < 8; ++i) V[i] = pack2(v[i], v[i + 8]);
   uint2 nib6, nib4;
-  unpack2(candidate_errors16(v, s6, s4, gsn, nib6, nib4, inv6, inv4), err6, err4);
+  const float err6 = candidate_error16(V, inv6, dq6, opaque_zero, nib6);
+  const float err4 = candidate_error16(V, inv4, dq4, opaque_zero, nib4);
   const bool six = err6 <= err4;
   packed = six ? nib6 : nib4;
   if (decoded_amax) {
@@ -282,127 +344,145 @@ __device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float g
     // evaluates it (utils/nvfp4/quant/kernels/ms_eden/amax.rs:23-64): rounding to E2M1 is monotonic
     // in |x|, so the largest nibble is the one of the element with the largest magnitude, ga.
     const float q = e2m1x2_values(cvt_e2m1x2(0.0f, ga * (six ? inv6 : inv4))).x;
-    *decoded_amax = fabsf(q * (six ? s6 : s4) * gs);
+    *decoded_amax = fabsf(q * (six ? s.x : s.y) * sc.gs);
   }
-  return six ? b6 : b4;
+  return six ? codes & 0xffu : codes >> 8;
 }
 
-// relu(x)^2 of the values a quantizer has just loaded (the MLP activation computed on load from the stored
-// pre-activation): max(x, 0) drops NaN like the reference's max_f32, the square is one rounded multiply.
-__device__ __forceinline__ void relu2_inplace16(float (&v)[16]) {
+__device__ __forceinline__ float group_amax16(const float (&v)[16]) {
+  float ga = 0.0f;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float r = max_f32(v[i], 0.0f);
-    v[i] = r * r;
-  }
+  for (int i = 0; i < 16; i += 2) ga = max3_abs(ga, v[i], v[i + 1]);
+  return ga;
 }
 
-// One thread per 16-group of a [rows][cols] tensor.  kRelu2: the tensor quantized is relu(x)^2.
+// What a quantizer reads: a group of 16 values of a stored tensor, relu(x)^2 of it (the MLP activation computed on load
+// from the stored pre-activation: max(x, 0) drops NaN like the reference's max_f32, the square is one rounded multiply),
+// or the schedule-free weight y = z + beta (x - z) of two f32 masters, which is never written out in f32
+// (gpt/optimizer/schedule_free/{value,amax,four_six}.rs).
+template <typename T, bool kRelu2>
+struct TensorSource {
+  const T* x;
+  __device__ __forceinline__ void load16(size_t group, float (&v)[16]) const {
+    Load16<T>::run(x + group * 16, v);
+    if (kRelu2) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float r = max_f32(v[i], 0.0f);
+        v[i] = r * r;
+      }
+    }
+  }
+};
+__device__ __forceinline__ float schedule_free_value(float z, float x, float beta) { return z + beta * (x - z); }
+struct ScheduleFreeSource {
+  const float* z;
+  const float* x;
+  float beta;
+  __device__ __forceinline__ void load16(size_t group, float (&v)[16]) const {
+    float zv[16], xv[16];
+    Load16<float>::run(z + group * 16, zv);
+    Load16<float>::run(x + group * 16, xv);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = schedule_free_value(zv[i], xv[i], beta);
+  }
+};
+
+// n / d for n < 2^32 by a multiplication (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", 1994, figure 4.1): a 64-bit division per group cost a quarter of the quantizer.
+struct FastDiv {
+  uint32_t d, m, s1, s2;
+  explicit FastDiv(uint32_t divisor) : d(divisor) {
+    uint32_t l = 0;
+    while (l < 32 && (1ull << l) < divisor) ++l;
+    m = static_cast<uint32_t>(((1ull << 32) * ((1ull << l) - divisor)) / divisor + 1);
+    s1 = l < 1 ? l : 1;
+    s2 = l < 1 ? 0 : l - 1;
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const {
+    const uint32_t t = __umulhi(m, n);
+    return (t + ((n - t) >> s1)) >> s2;
+  }
+};
+
+// Scale bytes of four neighbouring lanes (one k-atom of a row) as one 32-bit store; every lane of the warp calls it.
+__device__ __forceinline__ void store_scale_quad(uint8_t* dst, uint32_t byte, bool first_of_four) {
+  uint32_t word = byte | (__shfl_down_sync(0xffffffffu, byte, 1) << 8);
+  word |= __shfl_down_sync(0xffffffffu, word, 2) << 16;
+  if (first_of_four) *reinterpret_cast<uint32_t*>(dst) = word;
+}
+
+// Max over `count` non-negative partial maxima, by the whole CTA (256 threads).
+__device__ __forceinline__ float cta_max_of(const float* partials, uint32_t count) {
+  if (count == 1) return partials[0];
+  __shared__ uint32_t bits;
+  if (threadIdx.x == 0) bits = 0u;
+  __syncthreads();
+  float m = 0.0f;
+  for (uint32_t i = threadIdx.x; i < count; i += 256) m = max_f32(m, partials[i]);
+  const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+  if ((threadIdx.x & 31u) == 0) atomicMax(&bits, w);
+  __syncthreads();
+  return __uint_as_float(bits);
+}
+
+// One thread per 16-group and step over a [rows][cols] tensor; `groups` counts those of the pad rows too where the
+// scales are packed (pad rows of the plane hold 1.0, the nibbles have none).  Rowwise: amax holds one value per row;
+// otherwise `amax_count` partial maxima whose maximum is the tensor's, published in out_amax when asked for.
 // decoded_amax (optional, zeroed by the launcher): max |decoded value| of the quantized tensor.
-template <typename T, bool kRowwise, bool kPacked, bool kRelu2>
-__global__ void __launch_bounds__(256) four_six_kernel(const T* __restrict__ x, const float* __restrict__ amax,
-                                                        uint8_t* __restrict__ out_fp4, uint8_t* __restrict__ out_scales,
-                                                        float* __restrict__ out_gs, float* __restrict__ decoded_amax,
-                                                        uint64_t group_count, uint32_t groups_per_row) {
-  const uint64_t g = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x;
+// Measured, 8192 x 768 bf16 with a tensor scale: 8.5 -> 5.4 us (HBM allows 2.5).
+template <typename Source, bool kRowwise, bool kPacked, bool kQuads>
+__global__ void __launch_bounds__(256, 4)
+    four_six_kernel(const Source src, const float* __restrict__ amax, uint32_t amax_count, float* __restrict__ out_amax,
+                    uint8_t* __restrict__ out_fp4, uint8_t* __restrict__ out_scales, float* __restrict__ out_gs,
+                    float* __restrict__ decoded_amax, uint32_t rows, uint32_t groups, const FastDiv groups_per_row,
+                    uint32_t opaque_zero) {
   float dec = 0.0f;
-  if (g < group_count) {
-    const uint32_t row = static_cast<uint32_t>(g / groups_per_row);
-    const uint32_t kg = static_cast<uint32_t>(g - static_cast<uint64_t>(row) * groups_per_row);
-    const float gs = four_six_global_scale(amax[kRowwise ? row : 0]);
-    float v[16];
-    Load16<T>::run(x + g * 16, v);
-    if (kRelu2) relu2_inplace16(v);
-    uint2 packed;
-    const uint32_t b = four_six_group(v, gs, packed, decoded_amax ? &dec : nullptr);
-    *reinterpret_cast<uint2*>(out_fp4 + g * 8) = packed;
-    if (kPacked)
-      out_scales[packed_scale_offset(row, kg, groups_per_row >> 2)] = static_cast<uint8_t>(b);
-    else
-      out_scales[g] = static_cast<uint8_t>(b);
-    if (kRowwise ? (kg == 0) : (g == 0)) out_gs[kRowwise ? row : 0] = gs;
+  float tensor_amax = 0.0f;
+  if (!kRowwise) {
+    tensor_amax = cta_max_of(amax, amax_count);
+    if (out_amax && blockIdx.x == 0 && threadIdx.x == 0) out_amax[0] = tensor_amax;
+  }
+  const FourSixScale tensor_scale(tensor_amax);
+  const uint32_t step = gridDim.x * 256u;
+  // whole warps walk together: the scale bytes of neighbouring lanes leave in one store
+  for (uint32_t g0 = blockIdx.x * 256u + (threadIdx.x & ~31u); g0 < groups; g0 += step) {
+    const uint32_t g = g0 + (threadIdx.x & 31u);
+    const uint32_t row = groups_per_row.div(g), kg = g - row * groups_per_row.d;
+    const bool in_plane = g < groups;
+    uint32_t b = 0x38u;
+    if (in_plane && row < rows) {
+      float v[16];
+      src.load16(g, v);
+      const FourSixScale sc = kRowwise ? FourSixScale(amax[row]) : tensor_scale;
+      uint2 packed;
+      float d;
+      b = four_six_group(v, group_amax16(v), sc, opaque_zero, packed, decoded_amax ? &d : nullptr);
+      if (decoded_amax) dec = max_f32(dec, d);
+      *reinterpret_cast<uint2*>(out_fp4 + static_cast<size_t>(g) * 8) = packed;
+      if (kRowwise ? (kg == 0) : (g == 0)) out_gs[kRowwise ? row : 0] = sc.gs;
+    }
+    uint8_t* const dst = out_scales + (kPacked ? packed_scale_offset(row, kg, groups_per_row.d >> 2) : static_cast<size_t>(g));
+    if (kQuads)
+      store_scale_quad(dst, b, in_plane && (kg & 3u) == 0);
+    else if (in_plane)
+      *dst = static_cast<uint8_t>(b);
+    if (g0 + step < g0) break;  // the index space ends below 2^32
   }
   if (decoded_amax) cta_atomic_max(warp_max(dec), decoded_amax);  // uniform across the CTA
 }
 
-// Row amax and rowwise four-six in ONE pass over the input: a CTA owns whole rows (one thread
-// per 16-group), the row amax is the shared-memory max of the group amaxes the quantizer needs
-// anyway, and the groups are quantized from registers.  Same bytes as row_amax followed by the
-// rowwise kernel (crates/gpt2-nvfp4/src/types/nvfp4_scratch/scratch.rs:35-52 issues those two).
-// decoded_amax (optional, zeroed by the launcher): max |decoded value| of the whole quantized
-// tensor, i.e. what utils/nvfp4/quant/kernels/ms_eden/amax.rs:23-64 computes from the stored
-// tensor before the backward transposer -- handed over so that pass can be skipped.
-template <typename T, bool kPacked, bool kRelu2>
-__global__ void __launch_bounds__(256) four_six_rowwise_fused_kernel(const T* __restrict__ x,
-                                                                      uint8_t* __restrict__ out_fp4,
-                                                                      uint8_t* __restrict__ out_scales,
-                                                                      float* __restrict__ out_gs,
-                                                                      float* __restrict__ out_amax,
-                                                                      float* __restrict__ decoded_amax, uint32_t rows,
-                                                                      uint32_t groups_per_row, uint32_t rows_per_cta) {
-  extern __shared__ unsigned int row_amax_bits[];  // [rows_per_cta] row amax, then one word for the CTA's decoded amax
-  const uint32_t t = threadIdx.x;
-  for (uint32_t i = t; i <= rows_per_cta; i += blockDim.x) row_amax_bits[i] = 0u;
-  __syncthreads();
-  const uint32_t local_row = t / groups_per_row;
-  const uint32_t kg = t - local_row * groups_per_row;
-  const uint32_t row = blockIdx.x * rows_per_cta + local_row;
-  const bool active = local_row < rows_per_cta && row < rows;
-  float v[16];
-  float ga = 0.0f;
-  if (active) {
-    Load16<T>::run(x + (static_cast<size_t>(row) * groups_per_row + kg) * 16, v);
-    if (kRelu2) relu2_inplace16(v);
-#pragma unroll
-    for (int i = 0; i < 16; i += 2) ga = max3_abs(ga, v[i], v[i + 1]);
-  }
-  // Row max: non-negative floats order like their bit patterns.  With at least 32 groups per row a
-  // warp touches at most two rows, so two warp-wide integer maxima and two shared-memory atomics
-  // replace up to 32 atomics on the same word.
-  const uint32_t ga_bits = active ? __float_as_uint(ga) : 0u;
-  if (groups_per_row >= 32) {
-    const uint32_t first_row = __shfl_sync(0xffffffffu, local_row, 0);
-    const bool in_first = local_row == first_row;
-    const uint32_t m_first = __reduce_max_sync(0xffffffffu, in_first ? ga_bits : 0u);
-    const uint32_t m_other = __reduce_max_sync(0xffffffffu, in_first ? 0u : ga_bits);
-    const uint32_t other_lanes = __ballot_sync(0xffffffffu, !in_first && active);
-    const uint32_t lane_id = t & 31u;
-    if (lane_id == 0 && active) atomicMax(&row_amax_bits[local_row], m_first);
-    if (other_lanes != 0u && lane_id == static_cast<uint32_t>(__ffs(other_lanes) - 1))
-      atomicMax(&row_amax_bits[local_row], m_other);
-  } else if (active) {
-    atomicMax(&row_amax_bits[local_row], ga_bits);
-  }
-  __syncthreads();
-  uint32_t dec_bits = 0u;
-  if (active) {
-    const float amax = __uint_as_float(row_amax_bits[local_row]);
-    const float gs = four_six_global_scale(amax);
-    uint2 packed;
-    float dec = 0.0f;
-    const uint32_t b = four_six_group(v, gs, packed, decoded_amax ? &dec : nullptr);
-    const size_t g = static_cast<size_t>(row) * groups_per_row + kg;
-    *reinterpret_cast<uint2*>(out_fp4 + g * 8) = packed;
-    if (kPacked)
-      out_scales[packed_scale_offset(row, kg, groups_per_row >> 2)] = static_cast<uint8_t>(b);
-    else
-      out_scales[g] = static_cast<uint8_t>(b);
-    if (kg == 0) {
-      out_gs[row] = gs;
-      if (out_amax) out_amax[row] = amax;
-    }
-    dec_bits = __float_as_uint(dec);
-  }
-  if (decoded_amax) {  // uniform across the CTA
-    dec_bits = __reduce_max_sync(0xffffffffu, dec_bits);
-    if ((t & 31) == 0) atomicMax(&row_amax_bits[rows_per_cta], dec_bits);
-    __syncthreads();
-    if (t == 0) atomicMax(reinterpret_cast<unsigned int*>(decoded_amax), row_amax_bits[rows_per_cta]);
-  }
-}
-
-// Raw 16-element group as loaded (two or four 128-bit words) and its widening to f32: kept apart so that
-// the next group's words can be in flight while the current one is quantized.
+// Row amax and rowwise four-six in ONE pass over the input: a CTA owns whole rows (one thread per 16-group), the row
+// amax is the shared-memory max of the group amaxes the quantizer needs anyway, and the groups are quantized from
+// registers.  Same bytes as row_amax followed by the rowwise kernel
+// (crates/gpt2-nvfp4/src/types/nvfp4_scratch/scratch.rs:35-52 issues those two).  CTAs walk row blocks blockIdx.x,
+// blockIdx.x + gridDim.x, ... with the raw words of the next block in flight while the current one is quantized: one
+// CTA-wide barrier per row block, the per-row maxima rotate through three shared-memory buffers so that clearing a
+// buffer is always separated from its next use by a barrier.  Row blocks run on to the pad rows of a packed scale
+// plane, which are written with 1.0.
+// decoded_amax (optional, zeroed by the launcher): max |decoded value| of the whole quantized tensor, i.e. what
+// utils/nvfp4/quant/kernels/ms_eden/amax.rs:23-64 computes from the stored tensor before the backward transposer --
+// handed over so that pass can be skipped.
 template <typename T>
 struct RawGroup;
 template <>
@@ -442,29 +522,22 @@ struct RawGroup<__nv_bfloat16> {
   }
 };
 
-// The same outputs as four_six_rowwise_fused_kernel from persistent CTAs: a CTA walks row blocks
-// blockIdx.x, blockIdx.x + gridDim.x, ... and every thread has the raw words of its next group in flight
-// while it quantizes the current one, so global-load latency no longer sits in front of the row-amax
-// barrier (one CTA-wide barrier per row block; the per-row maxima rotate through three shared-memory
-// buffers so that clearing a buffer is always separated from its next use by a barrier).
 constexpr int kStreamMaxRowsPerCta = 256;
 template <typename T, bool kPacked, bool kRelu2>
-__global__ void __launch_bounds__(256) four_six_rowwise_stream_kernel(const T* __restrict__ x,
-                                                                       uint8_t* __restrict__ out_fp4,
-                                                                       uint8_t* __restrict__ out_scales,
-                                                                       float* __restrict__ out_gs,
-                                                                       float* __restrict__ out_amax,
-                                                                       float* __restrict__ decoded_amax, uint32_t rows,
-                                                                       uint32_t groups_per_row, uint32_t rows_per_cta,
-                                                                       uint32_t row_blocks) {
+__global__ void __launch_bounds__(256, 3)
+    four_six_rowwise_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_fp4, uint8_t* __restrict__ out_scales,
+                            float* __restrict__ out_gs, float* __restrict__ out_amax, float* __restrict__ decoded_amax,
+                            uint32_t rows, uint32_t padded_rows, uint32_t groups_per_row, uint32_t rows_per_cta,
+                            uint32_t row_blocks, uint32_t opaque_zero) {
   __shared__ unsigned int row_amax_bits[3][kStreamMaxRowsPerCta];
   const uint32_t t = threadIdx.x, lane_id = t & 31u;
-  for (uint32_t i = t; i < 3 * kStreamMaxRowsPerCta; i += blockDim.x) (&row_amax_bits[0][0])[i] = 0u;
+  for (uint32_t i = t; i < 3 * rows_per_cta; i += blockDim.x) row_amax_bits[i / rows_per_cta][i % rows_per_cta] = 0u;
   __syncthreads();
   const uint32_t local_row = t / groups_per_row;
   const uint32_t kg = t - local_row * groups_per_row;
   const bool in_use = local_row < rows_per_cta;
-  const bool quads = (groups_per_row & 3u) == 0;  // four neighbouring lanes hold four neighbouring scale bytes
+  // four neighbouring lanes hold four neighbouring scale bytes of one aligned word
+  const bool quads = (groups_per_row & 3u) == 0 && (reinterpret_cast<uintptr_t>(out_scales) & 3u) == 0;
   RawGroup<T> raw;
   uint32_t blk = blockIdx.x;
   {
@@ -480,9 +553,14 @@ __global__ void __launch_bounds__(256) four_six_rowwise_stream_kernel(const T* _
     float ga = 0.0f;
     if (active) {
       raw.widen(v);
-      if (kRelu2) relu2_inplace16(v);
+      if (kRelu2) {
 #pragma unroll
-      for (int i = 0; i < 16; i += 2) ga = max3_abs(ga, v[i], v[i + 1]);
+        for (int i = 0; i < 16; ++i) {
+          const float r = max_f32(v[i], 0.0f);
+          v[i] = r * r;
+        }
+      }
+      ga = group_amax16(v);
     }
     {
       // the next row block's words: in flight across the barrier and the whole quantization below
@@ -509,37 +587,27 @@ __global__ void __launch_bounds__(256) four_six_rowwise_stream_kernel(const T* _
     // every thread is past its reads of the buffer of the previous row block: clear it for the block after next
     const uint32_t stale = buf == 0 ? 2u : buf - 1u;
     if (t < rows_per_cta) row_amax_bits[stale][t] = 0u;
-    uint32_t b = 0;
+    uint32_t b = 0x38u;
     if (active) {
       const float amax = __uint_as_float(row_amax_bits[buf][local_row]);
-      const float gs = four_six_global_scale(amax);
+      const FourSixScale sc(amax);
       uint2 packed;
-      float dec = 0.0f;
-      b = four_six_group(v, gs, packed, decoded_amax ? &dec : nullptr);
-      const size_t g = static_cast<size_t>(row) * groups_per_row + kg;
-      *reinterpret_cast<uint2*>(out_fp4 + g * 8) = packed;
-      if (!quads) {
-        if (kPacked)
-          out_scales[packed_scale_offset(row, kg, groups_per_row >> 2)] = static_cast<uint8_t>(b);
-        else
-          out_scales[g] = static_cast<uint8_t>(b);
-      }
+      float dec;
+      b = four_six_group(v, ga, sc, opaque_zero, packed, decoded_amax ? &dec : nullptr);
+      *reinterpret_cast<uint2*>(out_fp4 + (static_cast<size_t>(row) * groups_per_row + kg) * 8) = packed;
       if (kg == 0) {
-        out_gs[row] = gs;
+        out_gs[row] = sc.gs;
         if (out_amax) out_amax[row] = amax;
       }
-      dec_running = max_f32(dec_running, dec);
+      if (decoded_amax) dec_running = max_f32(dec_running, dec);
     }
-    if (quads) {
-      // lanes 4j .. 4j+3 hold k-groups 4i .. 4i+3 of one row (one k-atom): one 32-bit store instead of four bytes
-      uint32_t word = b | (__shfl_down_sync(0xffffffffu, b, 1) << 8);
-      word |= __shfl_down_sync(0xffffffffu, word, 2) << 16;
-      if (active && (kg & 3u) == 0) {
-        const size_t off = kPacked ? packed_scale_offset(row, kg, groups_per_row >> 2)
-                                   : static_cast<size_t>(row) * groups_per_row + kg;
-        *reinterpret_cast<uint32_t*>(out_scales + off) = word;
-      }
-    }
+    const bool in_plane = in_use && row < (kPacked ? padded_rows : rows);
+    uint8_t* const dst = out_scales + (kPacked ? packed_scale_offset(row, kg, groups_per_row >> 2)
+                                               : static_cast<size_t>(row) * groups_per_row + kg);
+    if (quads)
+      store_scale_quad(dst, b, in_plane && (kg & 3u) == 0);
+    else if (in_plane)
+      *dst = static_cast<uint8_t>(b);
     buf = buf == 2 ? 0u : buf + 1u;
   }
   if (decoded_amax) {  // uniform across the CTA; the CTA may have fewer than eight warps
@@ -553,16 +621,11 @@ __global__ void __launch_bounds__(256) four_six_rowwise_stream_kernel(const T* _
   }
 }
 
-// Schedule-free weight materialisation (gpt/optimizer/schedule_free/{value,amax,four_six}.rs):
-// the weight quantized every step is y = z + beta * (x - z) of the two f32 masters; it is never
-// written out in f32.  Kernel 1: tensor amax of y (1024-value chunks per warp, chunk amax kept for
-// callers that want it); kernel 2: four-six of y with the tensor scale, one thread per 16-group.
-__device__ __forceinline__ float schedule_free_value(float z, float x, float beta) { return z + beta * (x - z); }
-
+// Tensor amax of the schedule-free weight, 1024-value chunks per warp.
 __global__ void __launch_bounds__(256) schedule_free_amax_kernel(const float* __restrict__ z,
                                                                   const float* __restrict__ x,
-                                                                  float* __restrict__ chunk_amax,
-                                                                  float* __restrict__ out, float beta, uint64_t n) {
+                                                                  float* __restrict__ chunk_amax, float* __restrict__ out,
+                                                                  float* __restrict__ partials, float beta, uint64_t n) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t warps = static_cast<uint64_t>(gridDim.x) * 8;
   const uint64_t chunks = (n + 1023) / 1024;
@@ -587,36 +650,7 @@ __global__ void __launch_bounds__(256) schedule_free_amax_kernel(const float* __
     if (lane == 0 && chunk_amax) chunk_amax[chunk] = m;
     running = max_f32(running, m);
   }
-  cta_atomic_max(running, out);
-}
-
-template <bool kPacked>
-__global__ void __launch_bounds__(256) schedule_free_four_six_kernel(const float* __restrict__ z,
-                                                                      const float* __restrict__ x,
-                                                                      const float* __restrict__ amax,
-                                                                      uint8_t* __restrict__ out_fp4,
-                                                                      uint8_t* __restrict__ out_scales,
-                                                                      float* __restrict__ out_gs, float beta,
-                                                                      uint64_t group_count, uint32_t groups_per_row) {
-  const uint64_t g = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x;
-  if (g >= group_count) return;
-  const float gs = four_six_global_scale(amax[0]);
-  float zv[16], xv[16], v[16];
-  Load16<float>::run(z + g * 16, zv);
-  Load16<float>::run(x + g * 16, xv);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = schedule_free_value(zv[i], xv[i], beta);
-  uint2 packed;
-  const uint32_t b = four_six_group(v, gs, packed);
-  *reinterpret_cast<uint2*>(out_fp4 + g * 8) = packed;
-  if (kPacked) {
-    const uint32_t row = static_cast<uint32_t>(g / groups_per_row);
-    const uint32_t kg = static_cast<uint32_t>(g - static_cast<uint64_t>(row) * groups_per_row);
-    out_scales[packed_scale_offset(row, kg, groups_per_row >> 2)] = static_cast<uint8_t>(b);
-  } else {
-    out_scales[g] = static_cast<uint8_t>(b);
-  }
-  if (g == 0) out_gs[0] = gs;
+  cta_publish_max(running, out, partials);
 }
 
 // Padded / transposed-padded variants: generic gather, zero outside the source extent.
@@ -625,10 +659,10 @@ template <bool kTransposed>
 __global__ void __launch_bounds__(256)
     four_six_padded_kernel(const float* __restrict__ x, const float* __restrict__ amax, uint8_t* __restrict__ out_fp4,
                            uint8_t* __restrict__ out_scales, float* __restrict__ out_gs, uint32_t rows, uint32_t cols,
-                           uint32_t padded_cols, uint64_t group_count) {
+                           uint32_t padded_cols, uint64_t group_count, uint32_t opaque_zero) {
   const uint64_t g = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x;
   if (g >= group_count) return;
-  const float gs = four_six_global_scale(amax[0]);
+  const FourSixScale sc(amax[0]);
   float v[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
@@ -641,10 +675,10 @@ __global__ void __launch_bounds__(256)
       v[i] = (r < cols && c < rows) ? x[static_cast<size_t>(c) * cols + r] : 0.0f;
   }
   uint2 packed;
-  const uint32_t b = four_six_group(v, gs, packed);
+  const uint32_t b = four_six_group(v, group_amax16(v), sc, opaque_zero, packed);
   *reinterpret_cast<uint2*>(out_fp4 + g * 8) = packed;
   out_scales[g] = static_cast<uint8_t>(b);
-  if (g == 0) out_gs[0] = gs;
+  if (g == 0) out_gs[0] = sc.gs;
 }
 
 // Fills the pad rows [rows, padded_rows) of a packed scale plane with 0x38 (= 1.0).
@@ -981,6 +1015,69 @@ __global__ void __launch_bounds__(256) decode_kernel(const uint8_t* __restrict__
   out[transpose ? static_cast<size_t>(c) * rows + r : idx] = v;
 }
 
+// Row-major decode, eight elements (one 32-byte store) per thread and step, four steps in flight: one element per thread
+// spent its time on index arithmetic and four-byte accesses (8192 x 768: 23 us; this form 5.5 us, HBM allows 4.4).
+__global__ void __launch_bounds__(256) decode_rows_kernel(const uint8_t* __restrict__ bytes, const uint8_t* __restrict__ scales,
+                                                           const float* __restrict__ gscales, float* __restrict__ out,
+                                                           uint32_t octets, const FastDiv octets_per_row, int rowwise) {
+  const float tensor_gs = rowwise ? 0.0f : gscales[0];
+  for (uint32_t i0 = blockIdx.x * 1024u + threadIdx.x; i0 < octets; i0 += gridDim.x * 1024u) {
+    uint32_t word[4], sc[4];
+    float gs[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t i = i0 + 256u * k;
+      if (i < octets && i >= i0) {
+        word[k] = __ldg(reinterpret_cast<const uint32_t*>(bytes) + i);
+        sc[k] = __ldg(scales + (i >> 1));
+        gs[k] = rowwise ? __ldg(gscales + octets_per_row.div(i)) : tensor_gs;
+      }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t i = i0 + 256u * k;
+      if (i < octets && i >= i0) {
+        float q[8];
+        e2m1x8_values(word[k], q);
+        const float s = e4m3_value(sc[k]);
+        uint32_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = __float_as_uint(q[j] * s * gs[k]);
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + static_cast<size_t>(i) * 8),
+                     "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+      }
+    }
+    if (i0 + gridDim.x * 1024u < i0) break;
+  }
+}
+
+// One [128 rows x 16 k-atoms] block of a logical scale plane into its sixteen packed 512-byte tiles, through shared
+// memory: 64-byte row segments in, whole tiles out (a byte per thread gathered one byte per 4-byte access and wrote
+// single bytes 16 apart: 8192 x 8192 8.9 us; this form 3.1 us).
+__global__ void __launch_bounds__(256) scale_pack_tiles_kernel(const uint8_t* __restrict__ logical, uint8_t* __restrict__ packed,
+                                                                uint32_t mn, uint32_t k_atoms) {
+  __shared__ uint32_t words[128][17];
+  const uint32_t atom0 = blockIdx.x * 16u, row0 = blockIdx.y * 128u;
+  const uint32_t atoms = min(16u, k_atoms - atom0);
+  const uint32_t w = threadIdx.x & 15u;
+#pragma unroll
+  for (uint32_t k = 0; k < 8; ++k) {
+    const uint32_t r = (threadIdx.x >> 4) + 16u * k;
+    if (w < atoms)
+      words[r][w] = row0 + r < mn ? __ldg(reinterpret_cast<const uint32_t*>(logical) + static_cast<size_t>(row0 + r) * k_atoms + atom0 + w)
+                                  : 0x38383838u;
+  }
+  __syncthreads();
+#pragma unroll
+  for (uint32_t k = 0; k < 2; ++k) {
+    const uint32_t i = threadIdx.x + 256u * k, atom = i >> 5, l = i & 31u;
+    if (atom < atoms)
+      reinterpret_cast<uint4*>(packed)[(static_cast<size_t>(blockIdx.y) * k_atoms + atom0 + atom) * 32u + l] =
+          make_uint4(words[l][atom], words[l + 32][atom], words[l + 64][atom], words[l + 96][atom]);
+  }
+}
+
 // utils/nvfp4_tma_matmul/scale_pack.rs:14-40
 __global__ void __launch_bounds__(256) scale_pack_kernel(const uint8_t* __restrict__ logical,
                                                           uint8_t* __restrict__ packed, uint32_t mn, uint32_t padded_mn,
@@ -1137,15 +1234,19 @@ int launch_row_amax(cudaStream_t s, const void* x, int dtype, float* out, uint32
   NVFP4_RETURN_LAST();
 }
 
-int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_amax, float* out, uint64_t n) {
-  cudaError_t err = cudaMemsetAsync(out, 0, sizeof(float), s);
-  if (err != cudaSuccess) return static_cast<int>(err);
-  if (n == 0) return 0;
-  const uint32_t grid = blocks_for((n + 1023) / 1024, 8, 148 * 8);
+uint32_t tensor_amax_partials(uint64_t n) { return blocks_for((n + 1023) / 1024, 8, kAmaxPartials); }
+
+int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_amax, float* out, uint64_t n, float* partials) {
+  if (!partials) {
+    const cudaError_t err = cudaMemsetAsync(out, 0, sizeof(float), s);
+    if (err != cudaSuccess) return static_cast<int>(err);
+    if (n == 0) return 0;
+  }
+  const uint32_t grid = partials ? tensor_amax_partials(n) : blocks_for((n + 1023) / 1024, 8, 148 * 8);
   if (dtype == 0)
-    tensor_amax_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float*>(x), chunk_amax, out, n);
+    tensor_amax_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float*>(x), chunk_amax, out, partials, n);
   else
-    tensor_amax_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), chunk_amax, out, n);
+    tensor_amax_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), chunk_amax, out, partials, n);
   NVFP4_RETURN_LAST();
 }
 
@@ -1170,47 +1271,76 @@ int launch_ms_eden_scale_from_amax(cudaStream_t s, const float* amax, float* out
   NVFP4_RETURN_LAST();
 }
 
-template <typename T, bool kRelu2>
-static int launch_four_six_t(cudaStream_t s, const T* x, const float* amax, int rowwise, uint32_t rows, uint32_t cols,
-                             uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, float* decoded_amax) {
+// Groups of one launch stay below 2^32 (32-bit index space): larger tensors go in slabs of whole 128-row blocks.
+template <typename Source>
+static Source advance(const Source& s, size_t elements);
+template <>
+TensorSource<float, false> advance(const TensorSource<float, false>& s, size_t n) { return {s.x + n}; }
+template <>
+TensorSource<float, true> advance(const TensorSource<float, true>& s, size_t n) { return {s.x + n}; }
+template <>
+TensorSource<__nv_bfloat16, false> advance(const TensorSource<__nv_bfloat16, false>& s, size_t n) { return {s.x + n}; }
+template <>
+TensorSource<__nv_bfloat16, true> advance(const TensorSource<__nv_bfloat16, true>& s, size_t n) { return {s.x + n}; }
+template <>
+ScheduleFreeSource advance(const ScheduleFreeSource& s, size_t n) { return {s.z + n, s.x + n, s.beta}; }
+
+template <typename Source>
+static int launch_four_six_source(cudaStream_t s, const Source& src, const float* amax, uint32_t amax_count, float* out_amax,
+                                  int rowwise, uint32_t rows, uint32_t cols, uint8_t* out_fp4, uint8_t* out_scales, int packed,
+                                  float* out_gs, float* decoded_amax) {
   const uint32_t gpr = cols / 16;
-  const uint64_t groups = static_cast<uint64_t>(rows) * gpr;
-  const uint32_t grid = blocks_for(groups, 256);
-#define NVFP4_LAUNCH_FS(R, P) \
-  four_six_kernel<T, R, P, kRelu2><<<grid, 256, 0, s>>>(x, amax, out_fp4, out_scales, out_gs, decoded_amax, groups, gpr)
+  const uint64_t limit = 0xfff00000ull;
+  const uint64_t slab_rows = limit / gpr >= 128 ? limit / gpr / 128 * 128 : limit / gpr;
+  if (rows > slab_rows) {
+    if (packed && slab_rows < 128) return static_cast<int>(cudaErrorInvalidValue);  // 2^36 elements: beyond the memory
+    for (uint64_t r = 0; r < rows; r += slab_rows) {
+      const uint32_t n = static_cast<uint32_t>(rows - r < slab_rows ? rows - r : slab_rows);
+      const size_t g = static_cast<size_t>(r) * gpr;
+      const int rc = launch_four_six_source(s, advance(src, g * 16), rowwise ? amax + r : amax, amax_count, out_amax, rowwise, n,
+                                            cols, out_fp4 + g * 8, out_scales + g, packed, rowwise ? out_gs + r : out_gs, decoded_amax);
+      if (rc) return rc;
+    }
+    return 0;
+  }
+  // few but very long rows: the plane's pad rows alone would leave the index space, they get their own launch
+  const uint64_t plane_rows = packed ? (rows + 127u) / 128u * 128u : rows;
+  const bool pad_apart = plane_rows * gpr > limit;
+  const uint32_t groups = static_cast<uint32_t>((pad_apart ? rows : plane_rows) * gpr);
+  // one wave of resident CTAs where the prologue reduces partial maxima or the tensor is large; each thread then walks
+  const uint32_t grid = blocks_for(groups, 256, 148u * 4u);
+  const bool quads = gpr % 4 == 0 && (reinterpret_cast<uintptr_t>(out_scales) & 3u) == 0;
+  const FastDiv div(gpr);
+#define NVFP4_LAUNCH_FS(R, P, Q)                                                                                          \
+  four_six_kernel<Source, R, P, Q><<<grid, 256, 0, s>>>(src, amax, amax_count, out_amax, out_fp4, out_scales, out_gs,      \
+                                                        decoded_amax, rows, groups, div, 0u)
   if (rowwise) {
-    if (packed) NVFP4_LAUNCH_FS(true, true);
-    else NVFP4_LAUNCH_FS(true, false);
+    if (packed) { if (quads) NVFP4_LAUNCH_FS(true, true, true); else NVFP4_LAUNCH_FS(true, true, false); }
+    else { if (quads) NVFP4_LAUNCH_FS(true, false, true); else NVFP4_LAUNCH_FS(true, false, false); }
   } else {
-    if (packed) NVFP4_LAUNCH_FS(false, true);
-    else NVFP4_LAUNCH_FS(false, false);
+    if (packed) { if (quads) NVFP4_LAUNCH_FS(false, true, true); else NVFP4_LAUNCH_FS(false, true, false); }
+    else { if (quads) NVFP4_LAUNCH_FS(false, false, true); else NVFP4_LAUNCH_FS(false, false, false); }
   }
 #undef NVFP4_LAUNCH_FS
   count_launch();
-  return static_cast<int>(cudaGetLastError());
+  const int rc = static_cast<int>(cudaGetLastError());
+  return rc == 0 && pad_apart ? launch_packed_scale_pad(s, out_scales, rows, cols) : rc;
 }
 
 int launch_four_six(cudaStream_t s, const void* x, int dtype, const float* amax, int rowwise, uint32_t rows,
                     uint32_t cols, uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, int relu2,
-                    float* decoded_amax) {
+                    float* decoded_amax, uint32_t amax_count) {
   if (decoded_amax) {
     const cudaError_t err = cudaMemsetAsync(decoded_amax, 0, sizeof(float), s);
     if (err != cudaSuccess) return static_cast<int>(err);
   }
   if (rows == 0 || cols == 0) return 0;
-  int rc;
-  if (dtype == 0) {
-    const float* xf = static_cast<const float*>(x);
-    rc = relu2 ? launch_four_six_t<float, true>(s, xf, amax, rowwise, rows, cols, out_fp4, out_scales, packed, out_gs, decoded_amax)
-               : launch_four_six_t<float, false>(s, xf, amax, rowwise, rows, cols, out_fp4, out_scales, packed, out_gs, decoded_amax);
-  } else {
-    const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
-    rc = relu2 ? launch_four_six_t<__nv_bfloat16, true>(s, xb, amax, rowwise, rows, cols, out_fp4, out_scales, packed, out_gs, decoded_amax)
-               : launch_four_six_t<__nv_bfloat16, false>(s, xb, amax, rowwise, rows, cols, out_fp4, out_scales, packed, out_gs, decoded_amax);
-  }
-  if (rc) return rc;
-  if (packed) return launch_packed_scale_pad(s, out_scales, rows, cols);
-  return 0;
+#define NVFP4_FS_SOURCE(T, R)                                                                                              \
+  launch_four_six_source(s, TensorSource<T, R>{static_cast<const T*>(x)}, amax, amax_count, nullptr, rowwise, rows, cols,   \
+                         out_fp4, out_scales, packed, out_gs, decoded_amax)
+  if (dtype == NVFP4_DTYPE_F32) return relu2 ? NVFP4_FS_SOURCE(float, true) : NVFP4_FS_SOURCE(float, false);
+  return relu2 ? NVFP4_FS_SOURCE(__nv_bfloat16, true) : NVFP4_FS_SOURCE(__nv_bfloat16, false);
+#undef NVFP4_FS_SOURCE
 }
 
 // Fused row amax + rowwise four-six.  Returns -1 when the row is too long for one CTA (the
@@ -1227,27 +1357,16 @@ int launch_four_six_rowwise_fused(cudaStream_t s, const void* x, int dtype, uint
   if (rows == 0) return 0;
   const uint32_t rpc = 256 / gpr;
   const uint32_t threads = (rpc * gpr + 31) / 32 * 32;
-  const uint32_t row_blocks = (rows + rpc - 1) / rpc;
-  const size_t smem = (rpc + 1) * sizeof(unsigned int);
-  // Persistent CTAs (three fit an SM) once there are more row blocks than resident CTAs and a CTA holds several
-  // rows (measured on B200 at 65536 rows: 768 columns 62 against 67 us; rows of 3072 columns, one per CTA,
-  // are faster with one CTA per row: 207 against 228 us); the grid is sized so that every CTA walks the same
-  // number of row blocks.
-  const uint32_t resident = 148u * 3u;  // 80 registers x 256 threads: three CTAs per SM
-  const bool stream = row_blocks > resident && gpr <= 64 && ((reinterpret_cast<uintptr_t>(out_scales) & 3u) == 0);
+  const uint32_t padded_rows = packed ? (rows + 127u) / 128u * 128u : rows;
+  const uint32_t row_blocks = (padded_rows + rpc - 1) / rpc;
+  // one wave of resident CTAs (80 registers: 768 threads per SM), every one with the same number of row blocks
+  const uint32_t resident = 148u * (768u / threads);
   const uint32_t per_cta = (row_blocks + resident - 1) / resident;
-  const uint32_t grid = stream ? (row_blocks + per_cta - 1) / per_cta : row_blocks;
+  const uint32_t grid = (row_blocks + per_cta - 1) / per_cta;
 #define NVFP4_LAUNCH_FUSED(T, P, R)                                                                                   \
-  do {                                                                                                                \
-    if (stream)                                                                                                       \
-      four_six_rowwise_stream_kernel<T, P, R><<<grid, threads, 0, s>>>(static_cast<const T*>(x), out_fp4, out_scales, \
-                                                                       out_gs, out_amax, decoded_amax, rows, gpr, rpc, \
-                                                                       row_blocks);                                   \
-    else                                                                                                              \
-      four_six_rowwise_fused_kernel<T, P, R><<<grid, threads, smem, s>>>(static_cast<const T*>(x), out_fp4,           \
-                                                                         out_scales, out_gs, out_amax, decoded_amax,  \
-                                                                         rows, gpr, rpc);                             \
-  } while (0)
+  four_six_rowwise_kernel<T, P, R><<<grid, threads, 0, s>>>(static_cast<const T*>(x), out_fp4, out_scales, out_gs,     \
+                                                            out_amax, decoded_amax, rows, padded_rows, gpr, rpc,       \
+                                                            row_blocks, 0u)
 #define NVFP4_LAUNCH_FUSED_R(T, P)       \
   do {                                   \
     if (relu2) NVFP4_LAUNCH_FUSED(T, P, true); \
@@ -1262,35 +1381,25 @@ int launch_four_six_rowwise_fused(cudaStream_t s, const void* x, int dtype, uint
   }
 #undef NVFP4_LAUNCH_FUSED_R
 #undef NVFP4_LAUNCH_FUSED
-  count_launch();
-  int rc = static_cast<int>(cudaGetLastError());
-  if (rc) return rc;
-  if (packed) return launch_packed_scale_pad(s, out_scales, rows, cols);
-  return 0;
+  NVFP4_RETURN_LAST();
 }
 
 int launch_schedule_free_materialize(cudaStream_t s, const float* z, const float* x, float beta, float* chunk_amax,
                                      float* amax, uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs,
-                                     uint32_t rows, uint32_t cols) {
+                                     uint32_t rows, uint32_t cols, float* partials) {
   const uint64_t n = static_cast<uint64_t>(rows) * cols;
-  cudaError_t err = cudaMemsetAsync(amax, 0, sizeof(float), s);
-  if (err != cudaSuccess) return static_cast<int>(err);
-  if (n == 0) return 0;
-  schedule_free_amax_kernel<<<blocks_for((n + 1023) / 1024, 8, 148 * 8), 256, 0, s>>>(z, x, chunk_amax, amax, beta, n);
+  if (!partials || n == 0) {
+    const cudaError_t err = cudaMemsetAsync(amax, 0, sizeof(float), s);
+    if (err != cudaSuccess) return static_cast<int>(err);
+    if (n == 0) return 0;
+  }
+  const uint32_t grid = partials ? tensor_amax_partials(n) : blocks_for((n + 1023) / 1024, 8, 148 * 8);
+  schedule_free_amax_kernel<<<grid, 256, 0, s>>>(z, x, chunk_amax, amax, partials, beta, n);
   count_launch();
-  const uint64_t groups = n / 16;
-  const uint32_t gpr = cols / 16;
-  if (packed)
-    schedule_free_four_six_kernel<true><<<blocks_for(groups, 256), 256, 0, s>>>(z, x, amax, out_fp4, out_scales, out_gs,
-                                                                               beta, groups, gpr);
-  else
-    schedule_free_four_six_kernel<false><<<blocks_for(groups, 256), 256, 0, s>>>(z, x, amax, out_fp4, out_scales, out_gs,
-                                                                                beta, groups, gpr);
-  count_launch();
-  int rc = static_cast<int>(cudaGetLastError());
+  const int rc = static_cast<int>(cudaGetLastError());
   if (rc) return rc;
-  if (packed) return launch_packed_scale_pad(s, out_scales, rows, cols);
-  return 0;
+  return launch_four_six_source(s, ScheduleFreeSource{z, x, beta}, partials ? partials : amax, partials ? grid : 1u,
+                                partials ? amax : nullptr, 0, rows, cols, out_fp4, out_scales, packed, out_gs, nullptr);
 }
 
 int launch_packed_scale_pad(cudaStream_t s, uint8_t* packed, uint32_t rows, uint32_t k_dim) {
@@ -1309,10 +1418,10 @@ int launch_four_six_padded(cudaStream_t s, const float* x, const float* amax, ui
   if (groups == 0) return 0;
   if (transposed)
     four_six_padded_kernel<true>
-        <<<blocks_for(groups, 256), 256, 0, s>>>(x, amax, out_fp4, out_scales, out_gs, rows, cols, padded_cols, groups);
+        <<<blocks_for(groups, 256), 256, 0, s>>>(x, amax, out_fp4, out_scales, out_gs, rows, cols, padded_cols, groups, 0u);
   else
     four_six_padded_kernel<false>
-        <<<blocks_for(groups, 256), 256, 0, s>>>(x, amax, out_fp4, out_scales, out_gs, rows, cols, padded_cols, groups);
+        <<<blocks_for(groups, 256), 256, 0, s>>>(x, amax, out_fp4, out_scales, out_gs, rows, cols, padded_cols, groups, 0u);
   NVFP4_RETURN_LAST();
 }
 
@@ -1536,7 +1645,15 @@ int launch_decode(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, c
                   int transpose, float* out, uint32_t rows, uint32_t cols) {
   const uint64_t n = static_cast<uint64_t>(rows) * cols;
   if (n == 0) return 0;
-  decode_kernel<<<blocks_for(n, 256), 256, 0, s>>>(bytes, scales, gscales, out, rows, cols, rowwise, transpose);
+  // the wide form needs whole 16-groups per row, aligned words and a 32-bit index space
+  if (!transpose && cols % 16 == 0 && n / 8 < 0xff000000ull && (reinterpret_cast<uintptr_t>(bytes) & 3u) == 0 &&
+      (reinterpret_cast<uintptr_t>(out) & 31u) == 0) {
+    const uint32_t octets = static_cast<uint32_t>(n / 8);
+    decode_rows_kernel<<<blocks_for(octets, 1024, 148u * 8u), 256, 0, s>>>(bytes, scales, gscales, out, octets, FastDiv(cols / 8),
+                                                                          rowwise);
+  } else {
+    decode_kernel<<<blocks_for(n, 256), 256, 0, s>>>(bytes, scales, gscales, out, rows, cols, rowwise, transpose);
+  }
   NVFP4_RETURN_LAST();
 }
 
@@ -1544,7 +1661,11 @@ int launch_scale_pack(cudaStream_t s, const uint8_t* logical, uint8_t* packed, u
   const uint32_t padded = (mn + 127u) / 128u * 128u, kg = k_dim / 16;
   const uint64_t total = static_cast<uint64_t>(padded) * kg;
   if (total == 0) return 0;
-  scale_pack_kernel<<<blocks_for(total, 256, 148 * 16), 256, 0, s>>>(logical, packed, mn, padded, kg);
+  const uint32_t row_blocks = padded / 128u, k_atoms = kg / 4u;
+  if ((reinterpret_cast<uintptr_t>(logical) & 3u) == 0 && (reinterpret_cast<uintptr_t>(packed) & 15u) == 0 && row_blocks <= 65535u)
+    scale_pack_tiles_kernel<<<dim3((k_atoms + 15u) / 16u, row_blocks), 256, 0, s>>>(logical, packed, mn, k_atoms);
+  else
+    scale_pack_kernel<<<blocks_for(total, 256, 148 * 16), 256, 0, s>>>(logical, packed, mn, padded, kg);
   NVFP4_RETURN_LAST();
 }
 

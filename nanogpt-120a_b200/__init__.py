@@ -14,6 +14,7 @@ library is missing or no CUDA device is present.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_size_t, c_uint8, c_uint32, c_void_p
 from dataclasses import dataclass
@@ -252,6 +253,25 @@ def library() -> ctypes.CDLL:
     return _lib
 
 
+BINDING_PATH = os.path.join(_HERE, "_nvfp4_binding.so")
+_binding = None
+
+
+def _native():
+    """The compiled binding of the hot entry points (host/binding.cpp); raises if it is missing."""
+    global _binding
+    if _binding is None:
+        if not os.path.exists(BINDING_PATH):
+            raise RuntimeError(f"{BINDING_PATH} is missing: build it with `python nanogpt-120a_b200/build.py`")
+        library()
+        spec = importlib.util.spec_from_file_location("_nvfp4_binding", BINDING_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.set_error_type(Nvfp4Error)
+        _binding = module
+    return _binding
+
+
 def _call(name: str, *args) -> None:
     lib = library()
     rc = getattr(lib, name)(*args)
@@ -259,9 +279,15 @@ def _call(name: str, *args) -> None:
         raise Nvfp4Error(rc, lib.nvfp4_last_error().decode())
 
 
+_cuda_seen = False
+
+
 def _require_cuda() -> None:
-    if not torch.cuda.is_available():
-        raise RuntimeError("the NVFP4 projection path needs a CUDA device (sm_100a); no fallback exists")
+    global _cuda_seen
+    if not _cuda_seen:
+        if not torch.cuda.is_available():
+            raise RuntimeError("the NVFP4 projection path needs a CUDA device (sm_100a); no fallback exists")
+        _cuda_seen = True  # a device does not go away again within a process
 
 
 def _stream() -> c_void_p:
@@ -383,12 +409,7 @@ class Nvfp4QuantModule:
     # ---- amax ---------------------------------------------------------------------------
     def row_amax(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         _require_cuda()
-        rows, cols = x.shape
-        out = torch.empty(rows, dtype=torch.float32, device=x.device) if out is None else out
-        name = "nvfp4_row_amax_f32" if x.dtype == torch.float32 else "nvfp4_row_amax_bf16"
-        _dtype_code(x)
-        _call(name, _stream(), _ptr(x), _ptr(out), rows, cols)
-        return out
+        return _native().row_amax(x, out)
 
     row_amax_f32 = row_amax
 
@@ -436,13 +457,7 @@ class Nvfp4QuantModule:
     def fp32_to_nvfp4_four_six_rowwise(self, x: torch.Tensor, amax: torch.Tensor) -> Nvfp4Tensor:
         _require_cuda()
         assert x.dtype == torch.float32
-        rows, cols = x.shape
-        n = rows * cols
-        t = Nvfp4Tensor(_empty_u8(n // 2, x.device), _empty_u8(n // 16, x.device),
-                        torch.empty(rows, dtype=torch.float32, device=x.device), rows, cols, rowwise=True)
-        _call("nvfp4_fp32_to_nvfp4_four_six_rowwise", _stream(), _ptr(x), _ptr(amax), _ptr(t.bytes), _ptr(t.scales),
-              _ptr(t.global_scales), n // 16, cols)
-        return t
+        return Nvfp4Tensor(*_native().four_six_rowwise_f32(x, amax), x.shape[0], x.shape[1], rowwise=True)
 
     def fp32_to_nvfp4_four_six_padded(self, x, amax, padded_rows, padded_cols, transposed=False) -> Nvfp4Tensor:
         _require_cuda()
@@ -466,29 +481,17 @@ class Nvfp4QuantModule:
         decoded_amax (fused rowwise path only): also emit max |decoded value| of the result, which
         LinearBackwardModule.backward_ms_eden then uses instead of a pass over the saved tensor."""
         _require_cuda()
-        rows, cols = x.shape
         fused = amax is None and rowwise
-        if amax is None and not rowwise:
-            amax = self.tensor_amax(x)[1]
         if out is None:
-            n = rows * cols
-            nsc = scale_packed_len(rows, cols) if packed else n // 16
-            out = Nvfp4Tensor(_empty_u8(n // 2, x.device), _empty_u8(nsc, x.device),
-                              torch.empty(rows if rowwise else 1, dtype=torch.float32, device=x.device), rows, cols,
-                              packed=packed, rowwise=rowwise)
+            b, sc, g, dec = _native().quantize_new(x, amax, rowwise, packed, fused and decoded_amax)
+            return Nvfp4Tensor(b, sc, g, x.shape[0], x.shape[1], packed, rowwise, dec)
         if fused:  # row amax and quantization in one pass over x
-            row_amax = torch.empty(rows, dtype=torch.float32, device=x.device) if cols > 4096 else None
             if decoded_amax and out.decoded_amax is None:
                 out.decoded_amax = torch.empty(1, dtype=torch.float32, device=x.device)
             elif not decoded_amax:
                 out.decoded_amax = None
-            _call("nvfp4_quantize_four_six_rowwise_fused", _stream(), _ptr(x), _dtype_code(x), rows, cols,
-                  _ptr(out.bytes), _ptr(out.scales), SCALES_PACKED if packed else SCALES_LOGICAL,
-                  _ptr(out.global_scales), _ptr(row_amax), _ptr(out.decoded_amax))
-            return out
-        _call("nvfp4_quantize_four_six", _stream(), _ptr(x), _dtype_code(x), _ptr(amax), 1 if rowwise else 0, rows,
-              cols, _ptr(out.bytes), _ptr(out.scales), SCALES_PACKED if packed else SCALES_LOGICAL,
-              _ptr(out.global_scales))
+        _native().quantize_into(x, amax, rowwise, packed, out.decoded_amax if fused else None, out.bytes, out.scales,
+                                out.global_scales)
         return out
 
     def quantize_relu2_four_six_rowwise(self, pre_activation: torch.Tensor, row_amax: Optional[torch.Tensor] = None,
@@ -673,15 +676,13 @@ class MlpModule:
             pre_activation = torch.empty((input.rows, weight.rows), dtype=out_dtype, device=dev)
         if store_activation and out is None:
             out = torch.empty((input.rows, weight.rows), dtype=pre_activation.dtype, device=dev)
-        a, keep = _projection_args(input, weight, bias, out if store_activation else None, pre_activation, relu2_row_amax)
-        _call("nvfp4_mlp_up_relu2", _stream(), ctypes.byref(a))
+        _projection(_UP_RELU2, input, weight, bias, out if store_activation else None, pre_activation, relu2_row_amax)
         return pre_activation, (out if store_activation else None)
 
     def down_residual(self, input: Nvfp4Tensor, weight: Nvfp4Tensor, bias: Nvfp4Tensor, residual: torch.Tensor):
         """gpt/mlp/launcher.rs:60-66: residual (f32, in place) += X . W^T + b."""
         _require_cuda()
-        a, keep = _projection_args(input, weight, bias, residual)
-        _call("nvfp4_mlp_down_residual", _stream(), ctypes.byref(a))
+        _projection(_DOWN_RESIDUAL, input, weight, bias, residual)
         return residual
 
     def relu2_backward(self, pre_activation: torch.Tensor, d_out: torch.Tensor,
@@ -733,11 +734,10 @@ class OptimizerModule:
         _require_cuda()
         assert z_master.dtype == torch.float32 and x_master.dtype == torch.float32 and z_master.shape == x_master.shape
         rows, cols = z_master.shape
-        dev, n = z_master.device, rows * cols
         if out is None:
-            nsc = scale_packed_len(rows, cols) if packed else n // 16
-            out = Nvfp4Tensor(_empty_u8(n // 2, dev), _empty_u8(nsc, dev),
-                              torch.empty(1, dtype=torch.float32, device=dev), rows, cols, packed=packed, rowwise=False)
+            b, sc, g, amax = _native().materialize(z_master, x_master, beta, packed)
+            return Nvfp4Tensor(b, sc, g, rows, cols, packed), amax
+        dev, n = z_master.device, rows * cols
         amax = torch.empty(1, dtype=torch.float32, device=dev)
         chunk = torch.empty(max(1, tensor_amax_chunks(n)), dtype=torch.float32, device=dev)
         if packed:
@@ -755,15 +755,7 @@ class Nvfp4DecodeModule:
     def decode(self, t: Nvfp4Tensor, transpose: bool = False) -> torch.Tensor:
         _require_cuda()
         assert not t.packed, "decode reads the logical scale layout"
-        shape = (t.cols, t.rows) if transpose else (t.rows, t.cols)
-        out = torch.empty(shape, dtype=torch.float32, device=t.bytes.device)
-        if transpose:
-            name = "nvfp4_decode_rowwise_transpose_f32" if t.rowwise else "nvfp4_decode_transpose_f32"
-            _call(name, _stream(), _ptr(t.bytes), _ptr(t.scales), _ptr(t.global_scales), _ptr(out), t.rows, t.cols)
-        else:
-            _call("nvfp4_decode_f32", _stream(), _ptr(t.bytes), _ptr(t.scales), _ptr(t.global_scales),
-                  1 if t.rowwise else 0, _ptr(out), t.rows, t.cols)
-        return out
+        return _native().decode(t.bytes, t.scales, t.global_scales, t.rows, t.cols, t.rowwise, transpose)
 
     def decode_transpose_f32(self, t: Nvfp4Tensor) -> torch.Tensor:
         return self.decode(t, transpose=True)
@@ -857,13 +849,20 @@ class Nvfp4GemmModule:
             mode = GS_ROWWISE_A if a.rowwise else GS_TENSOR
         if out is None:
             out = torch.empty((m, ldo), dtype=out_dtype, device=a.bytes.device)
-        g, keep = self._args(a, b, out, aux, bias, mode, epilogue, weight_global_scale, n, ldo, relu2_row_amax)
         if plan_only:
+            g, keep = self._args(a, b, out, aux, bias, mode, epilogue, weight_global_scale, n, ldo, relu2_row_amax)
             plan = GemmPlan()
             _call("nvfp4_gemm_plan_query", ctypes.byref(g), ctypes.byref(plan))
             return plan
-        _call("nvfp4_gemm", _stream(), ctypes.byref(g))
-        del keep
+        # (possibly temporary) packed planes: referenced until the launch is enqueued
+        a_scales, b_scales = _packed_scales(a), _packed_scales(b)
+        if isinstance(bias, Nvfp4Tensor):  # NVFP4-encoded bias, decoded in the epilogue
+            assert not bias.packed and not bias.rowwise, "an NVFP4 bias carries logical scales and one global scale"
+            plain, bb, bs, bg = None, bias.bytes, bias.scales, bias.global_scales
+        else:
+            plain, bb, bs, bg = bias, None, None, None
+        _native().gemm(a.bytes, a_scales, a.global_scales, b.bytes, b_scales, b.global_scales, out, aux, plain, bb, bs, bg,
+                       m, n, a.cols, ldo, mode, weight_global_scale, epilogue, relu2_row_amax)
         return out
 
     def plan(self, a: Nvfp4Tensor, b: Nvfp4Tensor, **kw) -> "GemmPlan":
@@ -898,31 +897,21 @@ class Nvfp4GemmModule:
         return self._named("nvfp4_gemm_tma_nvfp4_rowwise_a_scale_padded_output", a, b, extra_dims=(output_dim,))
 
 
-def _projection_args(input: Nvfp4Tensor, weight: Nvfp4Tensor, bias: Optional[Nvfp4Tensor], out, pre_activation=None,
-                     relu2_row_amax=None):
+# entry numbers of the binding's `projection`
+_QKV, _C_PROJ, _UP_RELU2, _DOWN_RESIDUAL, _LOGITS, _LOGITS_TMA, _NEXTLAT = range(7)
+
+
+def _projection(entry: int, input: Nvfp4Tensor, weight: Nvfp4Tensor, bias: Optional[Nvfp4Tensor], out, pre_activation=None,
+                relu2_row_amax=None) -> None:
     assert input.rowwise and not weight.rowwise and input.cols == weight.cols
-    a = ProjectionArgs()
-    dev = input.bytes.device
-    keep = []
-    a.input_bytes, a.input_scales, a.input_global_scales = _ptr(input.bytes), _ptr(input.scales), _ptr(input.global_scales)
-    a.input_scale_layout = SCALES_PACKED if input.packed else SCALES_LOGICAL
-    a.weight_bytes, a.weight_scales, a.weight_global_scale = _ptr(weight.bytes), _ptr(weight.scales), _ptr(weight.global_scales)
-    a.weight_scale_layout = SCALES_PACKED if weight.packed else SCALES_LOGICAL
-    if not input.packed:
-        keep.append(_empty_u8(scale_packed_len(input.rows, input.cols), dev))
-        a.input_scales_packed_scratch = _ptr(keep[-1])
-    if not weight.packed:
-        keep.append(_empty_u8(scale_packed_len(weight.rows, weight.cols), dev))
-        a.weight_scales_packed_scratch = _ptr(keep[-1])
-    if bias is not None:
+    if bias is None:
+        bb = bs = bg = None
+    else:
         assert not bias.packed and not bias.rowwise
-        a.bias_bytes, a.bias_scales, a.bias_global_scale = _ptr(bias.bytes), _ptr(bias.scales), _ptr(bias.global_scales)
-    ref = out if out is not None else pre_activation
-    a.out, a.pre_activation = _ptr(out), _ptr(pre_activation)
-    a.out_dtype = _dtype_code(ref)
-    a.relu2_row_amax = _ptr(relu2_row_amax)
-    a.token_count, a.input_dim, a.output_dim = input.rows, input.cols, weight.rows
-    return a, keep
+        bb, bs, bg = bias.bytes, bias.scales, bias.global_scales
+    _native().projection(entry, input.bytes, input.scales, input.packed, input.global_scales, weight.bytes, weight.scales,
+                         weight.packed, weight.global_scales, bb, bs, bg, out, pre_activation, relu2_row_amax, input.rows,
+                         input.cols, weight.rows)
 
 
 class AttentionModule:
@@ -932,15 +921,13 @@ class AttentionModule:
                        out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
         _require_cuda()
         out = torch.empty((input.rows, weight.rows), dtype=out_dtype, device=input.bytes.device) if out is None else out
-        a, keep = _projection_args(input, weight, bias, out)
-        _call("nvfp4_qkv_projection", _stream(), ctypes.byref(a))
+        _projection(_QKV, input, weight, bias, out)
         return out
 
     def c_proj(self, input: Nvfp4Tensor, weight: Nvfp4Tensor, bias: Nvfp4Tensor, residual: torch.Tensor) -> torch.Tensor:
         """residual (f32, in place) = fma(1, X . W^T + b, residual)."""
         _require_cuda()
-        a, keep = _projection_args(input, weight, bias, residual)
-        _call("nvfp4_c_proj", _stream(), ctypes.byref(a))
+        _projection(_C_PROJ, input, weight, bias, residual)
         return residual
 
 
@@ -951,8 +938,7 @@ class LmHeadModule:
                tma: bool = False) -> torch.Tensor:
         _require_cuda()
         logits = torch.empty((input.rows, weight.rows), dtype=out_dtype, device=input.bytes.device) if logits is None else logits
-        a, keep = _projection_args(input, weight, None, logits)
-        _call("nvfp4_lm_head_logits_tma" if tma else "nvfp4_lm_head_logits", _stream(), ctypes.byref(a))
+        _projection(_LOGITS_TMA if tma else _LOGITS, input, weight, None, logits)
         return logits
 
     def logits_tma(self, input, weight, logits=None, out_dtype: torch.dtype = torch.float32):
@@ -966,8 +952,7 @@ class NextLatModule:
                    out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
         _require_cuda()
         out = torch.empty((input.rows, weight.rows), dtype=out_dtype, device=input.bytes.device) if out is None else out
-        a, keep = _projection_args(input, weight, bias, out)
-        _call("nvfp4_nextlat_projection", _stream(), ctypes.byref(a))
+        _projection(_NEXTLAT, input, weight, bias, out)
         return out
 
 
@@ -1041,6 +1026,9 @@ class SideStream:
             self.fork.record(self.stream)
             self.join.record(self.stream)
 
+    def numbers(self):
+        return self.stream.cuda_stream, self.fork.cuda_event, self.join.cuda_event
+
     def handles(self):
         return (c_void_p(self.stream.cuda_stream), c_void_p(self.fork.cuda_event), c_void_p(self.join.cuda_event))
 
@@ -1089,37 +1077,16 @@ class LinearBackwardModule:
         in_dim = weight.cols
         assert weight.rows == out_dim and input.rows == tokens and input.cols == in_dim
         assert scratch.dims == (tokens, in_dim, out_dim)
-        dev = e.device
-        dinput = torch.empty((tokens, in_dim), dtype=grad_dtype, device=dev) if dinput is None else dinput
-        dweight = torch.empty((out_dim, in_dim), dtype=grad_dtype, device=dev) if dweight is None else dweight
-        if want_dbias and dbias is None:
-            dbias = torch.empty(out_dim, dtype=torch.float32, device=dev)
-        a = LinearBackwardArgs()
-        a.e, a.e_dtype = _ptr(e), _dtype_code(e)
-        a.w_bytes, a.w_scales, a.w_global = _ptr(weight.bytes), _ptr(weight.scales), _ptr(weight.global_scales)
-        a.w_scale_layout = SCALES_PACKED if weight.packed else SCALES_LOGICAL
-        a.x_bytes, a.x_scales, a.x_globals = _ptr(input.bytes), _ptr(input.scales), _ptr(input.global_scales)
-        a.x_scale_layout = SCALES_PACKED if input.packed else SCALES_LOGICAL
-        a.e_h, a.e_t_h = scratch._c(scratch.e_h), scratch._c(scratch.e_t_h)
-        a.weight_t_h, a.input_t_h = scratch._c(scratch.weight_t_h), scratch._c(scratch.input_t_h)
-        a.dinput, a.dinput_dtype = _ptr(dinput), _dtype_code(dinput)
-        a.dweight, a.dweight_dtype = _ptr(dweight), _dtype_code(dweight)
-        a.dbias = _ptr(dbias if want_dbias else None)
-        a.token_count, a.input_dim, a.output_dim = tokens, in_dim, out_dim
-        a.sign_seed, a.scale_seed = sign_seed & 0xFFFFFFFF, scale_seed & 0xFFFFFFFF
-        a.precomputed_e_amax_chunks = precomputed_e_amax_chunks
-        a.token_offset = token_offset
-        a.e_global_scale_override = _ptr(e_global_scale)
-        a.x_decoded_amax = _ptr(x_decoded_amax if x_decoded_amax is not None else input.decoded_amax)
-        a.total_token_count = total_token_count
-        a.weight_t_prepared = 1 if weight_t_prepared else 0
-        if prepare_weight_t_only:  # the W^T step alone (it reads only the weight and the seeds)
-            _call("nvfp4_linear_backward_prepare_weight_t", _stream(), ctypes.byref(a))
-            return None
-        if side is not None:
-            a.side_stream, a.fork_event, a.join_event = side.handles()
-        _call("nvfp4_linear_backward_ms_eden", _stream(), ctypes.byref(a))
-        return dinput, dweight, (dbias if want_dbias else None)
+        if grad_dtype not in (torch.float32, torch.bfloat16):
+            raise TypeError(f"unsupported dtype {grad_dtype}; the path takes float32 or bfloat16")
+        side_stream, fork, join = side.numbers() if side is not None and not prepare_weight_t_only else (0, 0, 0)
+        return _native().linear_backward(
+            prepare_weight_t_only, e, weight.bytes, weight.scales, weight.packed, weight.global_scales, input.bytes,
+            input.scales, input.packed, input.global_scales, scratch.e_h, scratch.e_t_h, scratch.weight_t_h,
+            scratch.input_t_h, dinput, dweight, dbias, want_dbias, DTYPE_F32 if grad_dtype == torch.float32 else DTYPE_BF16,
+            tokens, in_dim, out_dim, sign_seed, scale_seed, precomputed_e_amax_chunks, token_offset, e_global_scale,
+            x_decoded_amax if x_decoded_amax is not None else input.decoded_amax, side_stream, fork, join,
+            total_token_count, weight_t_prepared)
 
 
 # =============================================================================================
@@ -1212,9 +1179,13 @@ def projection_forward(x: torch.Tensor, weight: Nvfp4Tensor, bias: Optional[torc
                        rowwise: bool = True, out: Optional[torch.Tensor] = None, keep_logical: bool = False):
     """Y = X.W^T + b: quantize X (four-six, rowwise or tensor scale) then the block-scaled GEMM
     with the fused epilogue.  Returns (Y, quantized X) so the caller can keep X for backward."""
-    q = Nvfp4QuantModule()
-    xq = q.quantize_four_six(x, rowwise=rowwise, packed=not keep_logical)
+    _require_cuda()
     if epilogue is None:
         epilogue = EPI_BIAS if bias is not None else EPI_NONE
-    y = Nvfp4GemmModule().gemm(xq, weight, bias=bias, epilogue=epilogue, out_dtype=out_dtype, out=out)
-    return y, xq
+    if not weight.packed or isinstance(bias, Nvfp4Tensor) or out_dtype not in (torch.float32, torch.bfloat16):
+        xq = Nvfp4QuantModule().quantize_four_six(x, rowwise=rowwise, packed=not keep_logical)
+        return Nvfp4GemmModule().gemm(xq, weight, bias=bias, epilogue=epilogue, out_dtype=out_dtype, out=out), xq
+    y, b, sc, g = _native().projection_forward(x, rowwise, not keep_logical, weight.bytes, weight.scales,
+                                               weight.global_scales, weight.rows, weight.cols, bias, epilogue,
+                                               DTYPE_F32 if out_dtype == torch.float32 else DTYPE_BF16, out)
+    return y, Nvfp4Tensor(b, sc, g, x.shape[0], x.shape[1], not keep_logical, rowwise)

@@ -88,6 +88,32 @@ def build_step_library(force: bool = False) -> str:
     return STEP_LIB
 
 
+BINDING = os.path.join(HERE, "_nvfp4_binding.so")
+
+
+def build_binding(force: bool = False) -> str:
+    """Compiles the CPython binding of the hot entry points (host/binding.cpp) against the installed torch."""
+    import sysconfig
+
+    import torch
+
+    src = os.path.join(HERE, "host", "binding.cpp")
+    include = os.path.abspath(os.path.join(HERE, "..", "include"))
+    if force or _stale(BINDING, [src, build(), os.path.join(include, "nvfp4_b200.h")]):
+        troot = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(_nvcc()))
+        tmp = BINDING + ".tmp"
+        subprocess.check_call(
+            ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             "-I", include, "-I", sysconfig.get_paths()["include"], "-isystem", os.path.join(troot, "include"),
+             "-isystem", os.path.join(troot, "include", "torch", "csrc", "api", "include"),
+             "-isystem", os.path.join(cuda, "include"), src, "-o", tmp, "-L", HERE, "-lnvfp4_b200",
+             "-L", os.path.join(troot, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda",
+             "-Wl,-rpath,$ORIGIN", "-Wl,--no-as-needed"])
+        os.replace(tmp, BINDING)
+    return BINDING
+
+
 def build_cpp_driver(force: bool = False) -> str:
     """Compiles tests/cpp/mlp_layer_driver.cpp (a C++ caller of include/nvfp4_b200.hpp that walks one MLP
     block forward and backward) against the in-tree library; returns the binary's path."""
@@ -107,4 +133,5 @@ def build_cpp_driver(force: bool = False) -> str:
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
     print(build_step_library(force="--force" in sys.argv))
+    print(build_binding(force="--force" in sys.argv))
     print(build_cpp_driver(force="--force" in sys.argv))

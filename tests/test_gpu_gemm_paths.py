@@ -569,3 +569,44 @@ def test_bounded_wait_runs_out_and_kernel_returns(pkg, oracle, dev):
         assert rel_fro(cpu(out), oracle.gemm(a, b, m, k, n, 2)) <= GEMM_TOL
     pkg.set_gemm_tile_override(0)
     no_timeouts(pkg)
+
+
+@pytest.mark.parametrize("bias_kind", ["f32", "nvfp4"])
+@pytest.mark.parametrize("m,n,k,ldo", [(1, 4, 64, 4), (127, 192, 256, 192), (129, 132, 320, 136), (257, 260, 1088, 260),
+                                       (130, 100, 4160, 100), (64, 33, 128, 33)])
+def test_residual_add_reduction_and_direct(pkg, oracle, dev, m, n, k, ldo, bias_kind):
+    """The f32 residual stream leaves as a TMA reduce-add where the output can be described by a tensor map and through
+    direct stores where it cannot (a row pitch that is no multiple of 16 bytes); either way every element is added to
+    exactly once, columns beyond n are left alone, infinities and NaNs of the stream stay, and two runs agree bit for bit."""
+    gemm = pkg.Nvfp4GemmModule()
+    rng = np.random.default_rng(m * 7 + n)
+    a, b = rand_nvfp4(rng, m, k, True), rand_nvfp4(rng, n, k, False)
+    A, B = to_dev(pkg, dev, a, m, k, True), to_dev(pkg, dev, b, n, k, False)
+    if bias_kind == "nvfp4":
+        if n % 16:
+            pytest.skip("an NVFP4 bias holds whole groups of 16")
+        q = pkg.Nvfp4QuantModule()
+        bias_d = q.quantize_four_six(torch.from_numpy(rng.normal(0, 50.0, (1, n)).astype(np.float32)).to(dev), rowwise=False,
+                                     packed=False)
+        bias = cpu(pkg.Nvfp4DecodeModule().decode(bias_d))[0]
+    else:
+        bias = rng.normal(0, 50.0, n).astype(np.float32)
+        bias_d = torch.from_numpy(bias).to(dev)
+    res = rng.normal(0, 100.0, (m, ldo)).astype(np.float32)
+    res[m // 2, n // 2] = np.inf
+    res[m - 1, 0] = np.nan
+    want = oracle.gemm(a, b, m, k, n, 2, bias=bias, epi=1).astype(np.float64) + res[:, :n]
+    runs = []
+    for _ in range(2):
+        out = torch.from_numpy(res).to(dev).clone()
+        plan = gemm.plan(A, B, bias=bias_d, epilogue=pkg.EPI_RESIDUAL, out=out, ldo=ldo)
+        gemm.gemm(A, B, bias=bias_d, epilogue=pkg.EPI_RESIDUAL, out=out, ldo=ldo)
+        runs.append(cpu(out))
+    assert plan.tma_store == (1 if ldo % 4 == 0 else 0) and plan.k_splits == 1
+    got = runs[0]
+    assert got.tobytes() == runs[1].tobytes()
+    assert np.array_equal(got[:, n:], res[:, n:])
+    assert np.array_equal(np.isnan(got[:, :n]), np.isnan(want)) and np.array_equal(np.isinf(got[:, :n]), np.isinf(want))
+    ok = np.isfinite(want)
+    assert rel_fro(got[:, :n][ok], want[ok]) <= GEMM_TOL
+    no_timeouts(pkg)

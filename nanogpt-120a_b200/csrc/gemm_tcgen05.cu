@@ -10,7 +10,7 @@
 //               scale-factor tiles with bulk copies into a shared-memory ring,
 //   warp 1      issues tcgen05.mma.kind::mxf4nvf4.block_scale (128 x BLOCK_N x 64 per
 //               instruction), FP32 accumulators in tensor memory,
-//   warp 2      owns the tensor-memory allocation,
+//   warps 2, 3  issue the TMA stores of the two epilogue groups; warp 2 owns the tensor-memory allocation,
 //   warps 4..7 and 12..15  two epilogue groups: drain accumulators (tcgen05.ld), apply global
 //               scales / bias / ReLU^2 / residual, cast and store; the groups take alternate
 //               128-byte column sub-tiles of a tile (a warp reaches the tensor-memory lanes of
@@ -225,22 +225,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 // one named barrier per epilogue warp group (ids 1 and 2), 128 threads each
 __device__ __forceinline__ void epilogue_barrier(uint32_t group) {
   asm volatile("bar.sync %0, 128;" ::"r"(group + 1u) : "memory");
-}
-
-// Named barrier of one epilogue group that also ANDs a predicate over its 128 threads: the decision to
-// go on with a tile or to leave for the teardown is then the same in every thread of the group, so no
-// thread can be left alone in a later bar.sync.
-__device__ __forceinline__ bool epilogue_all(uint32_t group, bool pred) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %2, 0;\n\t"
-      "bar.red.and.pred q, %1, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"(group + 1u), "r"(static_cast<uint32_t>(pred))
-      : "memory");
-  return r != 0;
 }
 
 __device__ __forceinline__ bool elect_one() {
@@ -470,7 +454,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t smem_store = smem_sfb + b_slots * C::kSfbStageBytes;  // staging ring, 16 KB buffers, 1024-byte aligned
   const uint32_t smem_bar = smem_store + C::kStoreBufs * kStoreStageBytes;
   // barrier block: full[8], empty[8], tmem_full[2], tmem_empty[2], b_full, b_empty, sf_full[4], sf_empty[4],
-  // tmem base, abort flag
+  // mma_drain, staged[4], stored[4], tmem base, abort flag
   const uint32_t smem_bias = smem_bar + 512;  // kBlockN floats per epilogue group
   const uint32_t bar_full = smem_bar;
   const uint32_t bar_empty = bar_full + 8 * kMaxStages;
@@ -481,8 +465,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t bar_sf_full = bar_b_empty + 8;
   const uint32_t bar_sf_empty = bar_sf_full + 8 * C::kSfSets;
   const uint32_t bar_mma_drain = bar_sf_empty + 8 * C::kSfSets;  // abort path only: issued MMAs have retired
-  uint32_t* tmem_base_ptr =
-      reinterpret_cast<uint32_t*>(smem_gen + (smem_bar - smem_base) + 8 * (2 * kMaxStages + 7 + 2 * C::kSfSets));
+  const uint32_t bar_staged = bar_mma_drain + 8;                 // one per staging buffer: a sub-tile is in it
+  const uint32_t bar_stored = bar_staged + 8 * C::kStoreBufs;    // one per staging buffer: its TMA store has read it
+  uint32_t* tmem_base_ptr = reinterpret_cast<uint32_t*>(
+      smem_gen + (smem_bar - smem_base) + 8 * (2 * kMaxStages + 7 + 2 * C::kSfSets + 2 * C::kStoreBufs));
   volatile uint32_t* abort_flag = tmem_base_ptr + 1;
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -512,6 +498,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(bar_b_full, 1);
     mbar_init(bar_b_empty, 1);
     mbar_init(bar_mma_drain, 1);
+    for (int b = 0; b < C::kStoreBufs; ++b) {
+      mbar_init(bar_staged + 8 * b, 4);  // the four warps of the epilogue group
+      mbar_init(bar_stored + 8 * b, 1);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -531,13 +521,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   // contiguous range of tiles ordered column block major, so its B panel changes at most a
   // couple of times.
   const uint32_t tiles_mn = p.num_m_blocks * p.num_n_blocks;
-  uint32_t w_begin, w_end, w_step;
+  uint32_t w_begin, w_end, w_step, band_n = 0;
   if (p.b_resident && p.resident_cpn) {
     // Column block c / cpn, row blocks j, j + cpn, j + 2 cpn, ...: at any moment the CTAs of all
     // column blocks work on the same band of cpn row blocks, so whole output rows are written at
     // about the same time (full DRAM pages when L2 writes them back).
     const bool has_work = blockIdx.x < p.resident_cpn * p.num_n_blocks;
-    w_begin = blockIdx.x % p.resident_cpn;
+    band_n = blockIdx.x / p.resident_cpn;
+    w_begin = blockIdx.x - band_n * p.resident_cpn;
     w_end = has_work ? p.num_m_blocks : 0;
     w_step = p.resident_cpn;
   } else if (p.b_resident) {
@@ -551,7 +542,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   auto decode = [&](uint32_t w, uint32_t& m_blk, uint32_t& n_blk, uint32_t& split) {
     if (p.b_resident && p.resident_cpn) {
-      n_blk = blockIdx.x / p.resident_cpn;
+      n_blk = band_n;
       m_blk = w;
       split = 0;
     } else if (p.b_resident) {
@@ -565,6 +556,26 @@ __global__ void __launch_bounds__(kThreads, 1)
       n_blk = tile - m_blk * p.num_n_blocks;
     }
   };
+
+  // Sub-tiles of 128 rows x 128 bytes leave through shared memory with TMA stores.  The items of a tile -- (row half,
+  // column sub-tile) -- alternate between the two epilogue groups; with an odd number of items per tile (192 bf16
+  // columns = 3) the group that takes two alternates from tile to tile, which the double-buffered accumulator evens out.
+  constexpr int kSub = SubTile<OutT>::kCols;
+  constexpr int kNumSub = kBlockN / kSub;
+  constexpr int kItems = kMHalves * kNumSub;
+  constexpr uint32_t kRing = C::kStoreBufs / 2;  // staging buffers per group
+  auto first_item_of = [&](uint32_t group, uint32_t tile_iter) {
+    return static_cast<int>((kItems & 1) ? (group ^ (tile_iter & 1u)) : group);
+  };
+  auto item_valid = [&](int item, uint32_t m_blk, uint32_t n_blk) {  // not wholly outside the matrix
+    const uint32_t h = static_cast<uint32_t>(item / kNumSub), sub = static_cast<uint32_t>(item % kNumSub);
+    return n_blk * kBlockN + sub * kSub < p.n && m_blk * kBlockM + h * kRowBlock < p.m;
+  };
+  // epilogue and store warps wait on what the MMA warp feeds them: their limit is the longer one, so that the status
+  // word names the role whose input failed to come
+  const uint64_t downstream_timeout_ns = 2 * p.wait_timeout_ns;
+  // a ReLU^2 with its pre-activation kept stores every item twice: the pre-activation, then the activation
+  const int item_passes = (p.epilogue == NVFP4_EPI_RELU2 && p.aux) ? 2 : 1;
 
   if (warp == 0) {
     // ===================== TMA producer =====================
@@ -869,26 +880,70 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     }
+  } else if (warp == 2 || warp == 3) {
+    // ===================== store warps (one per epilogue group) =====================
+    // Issuing a TMA store takes about 400 cycles and its read of the staging buffer as long again.  This thread waits for
+    // both, so that between two sub-tiles the epilogue warps have only the next sub-tile to do.  Measured against one
+    // epilogue thread issuing the stores between two barriers of its group: 65536 x 2304 and x 3072 bf16 at K = 768,
+    // 87.3 -> 83.0 us and 116.9 -> 111.3 us, 3.6 TB/s of output where a plain fill reaches 3.8.  A third or fourth buffer
+    // in place of an A stage gains nothing: at these sizes HBM takes the writes no faster.
+    if (kTmaStore && lane == 0) {
+      const uint32_t eg = warp - 2u;
+      uint32_t buf = 0, phase = 0, tile_iter = 0, issued = 0;
+      bool ok = true;
+      for (uint32_t w = w_begin; w < w_end && ok; w += w_step, ++tile_iter) {
+        uint32_t m_blk, n_blk, split;
+        decode(w, m_blk, n_blk, split);
+        for (int item = first_item_of(eg, tile_iter); item < kItems && ok; item += 2) {
+          if (!item_valid(item, m_blk, n_blk)) continue;
+          const int32_t x = static_cast<int32_t>(n_blk * kBlockN + (item % kNumSub) * kSub);
+          const int32_t y = static_cast<int32_t>(m_blk * kBlockM + (item / kNumSub) * kRowBlock);
+          for (int pass = 0; pass < item_passes; ++pass) {
+            const uint32_t slot = eg * kRing + buf;
+            if (!mbar_wait(bar_staged + 8 * slot, phase, abort_flag, kStatusEpilogueTimeout, downstream_timeout_ns)) {
+              ok = false;
+              break;
+            }
+            const CUtensorMap* map = item_passes == 2 && pass == 0 ? &tmap_aux : &tmap_out;
+            if (p.reduce_out)
+              tma_reduce_add_2d(map, smem_store + slot * kStoreStageBytes, x, y);
+            else
+              tma_store_2d(map, smem_store + slot * kStoreStageBytes, x, y);
+            bulk_commit_group();
+            // the buffer the epilogue needs next is handed back as soon as its store has read it: this one with a
+            // single buffer, the previous one with two
+            bulk_wait_group_read<static_cast<int>(kRing) - 1>();
+            if (kRing == 1)
+              mbar_arrive(bar_stored + 8 * slot);
+            else if (issued > 0)
+              mbar_arrive(bar_stored + 8 * (eg * kRing + (buf ^ 1u)));
+            ++issued;
+            if (++buf == kRing) {
+              buf = 0;
+              phase ^= 1u;
+            }
+          }
+        }
+      }
+      bulk_wait_group0();  // stores complete before the CTA exits
+    }
   } else if (warp >= 4) {
     // ===================== epilogue (two groups of four warps) =====================
     const uint32_t ew = warp & 3u;               // lane quadrant of tensor memory this warp reaches
     const uint32_t eg = warp >= 12 ? 1u : 0u;    // epilogue group
     const uint32_t gtid = ew * 32 + lane;        // thread index inside the group, also the tile row
-    const bool elected = gtid == 0;
-    constexpr uint32_t kRing = C::kStoreBufs / 2;  // staging buffers per group
+    [[maybe_unused]] const bool elected = gtid == 0;
     OutT* out = static_cast<OutT*>(p.out);
     OutT* aux = static_cast<OutT*>(p.aux);
-    uint32_t acc = 0, acc_phase = 0, store_buf = 0, tile_iter = 0;
+    uint32_t acc = 0, acc_phase = 0, store_buf = 0, store_phase = 1, tile_iter = 0;
+    bool ok = true;  // warp uniform; false: some wait ran out, the rest of the list is walked without work
     const uint32_t my_bias = smem_bias + eg * kBlockN * 4;
     const float* my_bias_gen = reinterpret_cast<const float*>(smem_gen + (my_bias - smem_base));
-    const uint32_t my_store = smem_store + eg * kRing * kStoreStageBytes;
     const float gb = p.mode == NVFP4_GS_NONE ? 1.0f : __ldg(p.b_global);
     const float ga_scalar = p.mode == NVFP4_GS_TENSOR ? __ldg(p.a_global) : 1.0f;
     // the rows' global scales of a tile are fetched one tile ahead: their load latency would
     // otherwise sit between the accumulator becoming ready and the first store
-    auto row_scale = [&](uint32_t w, uint32_t h) {
-      uint32_t mb, nb, sp;
-      decode(w, mb, nb, sp);
+    auto row_scale = [&](uint32_t mb, uint32_t h) {
       const uint32_t r = mb * kBlockM + h * kRowBlock + gtid;
       return (p.mode == NVFP4_GS_ROWWISE_A && r < p.m) ? __ldg(p.a_global + r) : 0.0f;
     };
@@ -897,9 +952,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // column block for many tiles).
     float bias_next[C::kBiasSlots];
     uint32_t staged_bias_blk = 0xffffffffu;
-    auto fetch_bias = [&](uint32_t w) {
-      uint32_t mb, nb, sp;
-      decode(w, mb, nb, sp);
+    auto fetch_bias = [&](uint32_t nb) {
 #pragma unroll
       for (int j = 0; j < C::kBiasSlots; ++j) {
         const uint32_t in_tile = gtid + 128 * j;
@@ -909,24 +962,29 @@ __global__ void __launch_bounds__(kThreads, 1)
                            : 0.0f;
       }
     };
-    if (w_begin < w_end) fetch_bias(w_begin);
-    float ga_next[kMHalves];
+    float ga_next[kMHalves] = {};
+    uint32_t m_next = 0, n_next = 0, split_next = 0;
+    if (w_begin < w_end) {
+      decode(w_begin, m_next, n_next, split_next);
+      fetch_bias(n_next);
 #pragma unroll
-    for (int h = 0; h < kMHalves; ++h) ga_next[h] = w_begin < w_end ? row_scale(w_begin, h) : 0.0f;
+      for (int h = 0; h < kMHalves; ++h) ga_next[h] = row_scale(m_next, h);
+    }
     for (uint32_t w = w_begin; w < w_end; w += w_step, ++tile_iter) {
-      uint32_t m_blk, n_blk, split;
-      decode(w, m_blk, n_blk, split);
+      const uint32_t m_blk = m_next, n_blk = n_next, split = split_next;
       float ga_row[kMHalves];
 #pragma unroll
-      for (int h = 0; h < kMHalves; ++h) {
-        ga_row[h] = ga_next[h];
-        if (w + w_step < w_end) ga_next[h] = row_scale(w + w_step, h);
+      for (int h = 0; h < kMHalves; ++h) ga_row[h] = ga_next[h];
+      if (w + w_step < w_end) {
+        decode(w + w_step, m_next, n_next, split_next);
+#pragma unroll
+        for (int h = 0; h < kMHalves; ++h) ga_next[h] = row_scale(m_next, h);
       }
-      // the tile's bias slice goes through shared memory once (every row then reads it broadcast); it is
-      // fetched before the wait for the accumulator so that its latency hides behind the main loop.  The
-      // group's last barrier of the previous tile comes after that tile's last read of the slice.
+      // the tile's bias slice goes through shared memory once (every row then reads it broadcast), staged before the
+      // wait for the accumulator so that this hides behind the main loop
       const bool add_bias = kTmaStore && p.epilogue != NVFP4_EPI_NONE && (p.k_splits == 1 || split == 0);
       if (add_bias && n_blk != staged_bias_blk) {  // uniform across the group
+        epilogue_barrier(eg);  // every warp has read the slice staged before
 #pragma unroll
         for (int j = 0; j < C::kBiasSlots; ++j)
           if (gtid + 128 * j < static_cast<uint32_t>(kBlockN))
@@ -934,13 +992,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         epilogue_barrier(eg);
         staged_bias_blk = n_blk;
       }
-      if (w + w_step < w_end) fetch_bias(w + w_step);
-      // go on only if every thread of the group saw the accumulator arrive (no thread may be left in a
-      // later barrier of the group when another one gives up)
+      if (n_next != n_blk) fetch_bias(n_next);
+      // Once a wait has run out a warp walks the rest of its tiles without work instead of leaving: the group's
+      // barriers (a bias slice per change of column block) then always see all four warps.
       GEMM_TRACE(3 + eg, 30, elected);
-      if (!epilogue_all(eg, mbar_wait(bar_tmem_full + 8 * acc, acc_phase, abort_flag, kStatusEpilogueTimeout,
-                                      p.wait_timeout_ns)))
-        break;
+      ok = ok && mbar_wait(bar_tmem_full + 8 * acc, acc_phase, abort_flag, kStatusEpilogueTimeout, downstream_timeout_ns);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) continue;
       GEMM_TRACE(3 + eg, 31, elected);
       tcgen05_fence_after();
       // reference order: (weight * a_scale) * b_scale, then acc * scale
@@ -958,24 +1016,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) mbar_arrive(bar_tmem_empty + 8 * acc);
       };
       if (kTmaStore) {
-        // Sub-tiles of 128 rows x 128 bytes go through the group's shared-memory ring and leave
-        // with TMA stores (TMA reduce-add for split-K partial sums); rows / columns outside the
-        // matrix are clipped by the tensor map.  The items of a tile -- (row half, column sub-tile) --
-        // alternate between the two groups; with an odd number of items per tile (192 bf16 columns = 3)
-        // the group that takes two alternates from tile to tile, which the double-buffered accumulator
-        // evens out.
-        constexpr int kSub = SubTile<OutT>::kCols;
-        constexpr int kNumSub = kBlockN / kSub;
-        constexpr int kItems = kMHalves * kNumSub;
-        const int first_item = static_cast<int>((kItems & 1) ? (eg ^ (tile_iter & 1u)) : eg);
-        auto item_valid = [&](int item) {  // uniform across the group
-          const uint32_t h = static_cast<uint32_t>(item / kNumSub), sub = static_cast<uint32_t>(item % kNumSub);
-          return n_blk * kBlockN + sub * kSub < p.n && m_blk * kBlockM + h * kRowBlock < p.m;
-        };
+        // the group's sub-tiles go through its shared-memory ring to the store warp; rows / columns outside the matrix
+        // are clipped by the tensor map
+        const int first_item = first_item_of(eg, tile_iter);
         int last_item = -1;
 #pragma unroll
         for (int item = first_item; item < kItems; item += 2)
-          if (item_valid(item)) last_item = item;
+          if (item_valid(item, m_blk, n_blk)) last_item = item;
         if (last_item < 0) release_accumulator();  // nothing of this tile is for this group to read
         float row_max = -INFINITY;  // largest value this thread stores for its row in the current row half
         uint32_t max_h = 0;
@@ -994,11 +1041,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         };
 #pragma unroll 1
         for (int item = first_item; item < kItems; item += 2) {
-          if (!item_valid(item)) continue;
+          if (!item_valid(item, m_blk, n_blk)) continue;
           const uint32_t h = static_cast<uint32_t>(item / kNumSub);
           const int c = (item % kNumSub) * kSub;
           const uint32_t col0 = n_blk * kBlockN + c;
-          const uint32_t row0 = m_blk * kBlockM + h * kRowBlock;
           if (h != max_h) {
             flush_row_max();
             max_h = h;
@@ -1049,9 +1095,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (static_cast<uint32_t>(i) < valid) row_max = fmaxf(row_max, v[i]);
             }
           }
-          const int passes = (p.epilogue == NVFP4_EPI_RELU2 && p.aux) ? 2 : 1;
-          for (int pass = 0; pass < passes; ++pass) {
-            const bool is_pre = passes == 2 && pass == 0;
+          for (int pass = 0; pass < item_passes; ++pass) {
+            const bool is_pre = item_passes == 2 && pass == 0;
             if (p.epilogue == NVFP4_EPI_RELU2 && !is_pre) {
 #pragma unroll
               for (int i = 0; i < kSub; i += 2) {
@@ -1060,30 +1105,21 @@ __global__ void __launch_bounds__(kThreads, 1)
                 square_f32x2(v[i], v[i + 1]);
               }
             }
-            const uint32_t buf = my_store + store_buf * kStoreStageBytes;
-            if (kRing == 1) {
-              // single staging buffer: the previous store must have read it before it is rewritten
-              if (elected) bulk_wait_group_read<0>();
-              epilogue_barrier(eg);
-            }
+            const uint32_t slot = eg * kRing + store_buf;
+            ok = ok && mbar_wait(bar_stored + 8 * slot, store_phase, abort_flag, kStatusEpilogueTimeout, downstream_timeout_ns);
+            ok = __all_sync(0xffffffffu, ok);
             GEMM_TRACE(3 + eg, 36, elected);
-            SubTile<OutT>::stage(buf + gtid * 128, gtid, v);
-            fence_proxy_async_smem();
-            GEMM_TRACE(3 + eg, 33, elected);
-            // deeper rings: the buffer written next was last used kRing - 1 stores ago
-            if (kRing > 1 && elected) bulk_wait_group_read<(kRing > 1 ? kRing - 2 : 0)>();
-            epilogue_barrier(eg);
-            GEMM_TRACE(3 + eg, 34, elected);
-            if (elected) {
-              const CUtensorMap* map = is_pre ? &tmap_aux : &tmap_out;
-              if (p.reduce_out)
-                tma_reduce_add_2d(map, buf, static_cast<int32_t>(col0), static_cast<int32_t>(row0));
-              else
-                tma_store_2d(map, buf, static_cast<int32_t>(col0), static_cast<int32_t>(row0));
-              bulk_commit_group();
+            if (ok) {
+              SubTile<OutT>::stage(smem_store + slot * kStoreStageBytes + gtid * 128, gtid, v);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar_staged + 8 * slot);
             }
-            GEMM_TRACE(3 + eg, 35, elected);
-            store_buf = (store_buf + 1) % kRing;
+            GEMM_TRACE(3 + eg, 33, elected);
+            if (++store_buf == kRing) {
+              store_buf = 0;
+              store_phase ^= 1u;
+            }
           }
         }
         flush_row_max();
@@ -1144,7 +1180,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         acc_phase ^= 1u;
       }
     }
-    if (kTmaStore && elected) bulk_wait_group0();  // stores complete before the CTA exits
   }
 
   // ===================== teardown =====================
@@ -1518,7 +1553,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   // and row pitch); odd layouts use direct stores.  The f32 residual stream leaves as a TMA reduce-add: one rounded
   // addition per element, as the fused multiply-add by one of the direct path, done in L2 instead of through a
   // register round trip whose lanes read a row each (like every f32 reduction in global memory it treats subnormals as
-  // zero): 4096 x 2048 x K 8192, 100 us with direct stores, 55 us with the reduction.  A bf16 residual stays on the
+  // zero): 4096 x 2048 x K 8192, 100 us with direct stores, 55 us with the reduction, 44 us once store warps
+  // issued it.  A bf16 residual stays on the
   // direct path, which adds in f32 and rounds once.
   pl.tma_store = (pl.vec_store && (a.epilogue != NVFP4_EPI_RESIDUAL || a.out_dtype == NVFP4_DTYPE_F32)) ? 1 : 0;
 

@@ -333,6 +333,7 @@ struct PairTile {
 template <typename T, bool kColSum, bool kEdge>
 __global__ void __launch_bounds__(256, 2)
     ms_eden_pair_kernel(const __grid_constant__ MsEdenTileParams p, uint32_t tiles_x, uint32_t tile_count) {
+  allow_next_kernel();
   using PT = PairTile<T>;
   constexpr bool kBf16 = PT::kBf16;
   constexpr uint32_t kSize = sizeof(T);
@@ -558,6 +559,7 @@ constexpr int kNvPitch = kTileCols * 4 + 16;
 template <bool kRowwise, bool kEdge>
 __global__ void __launch_bounds__(128, 4)
     ms_eden_nvfp4_transpose_kernel(const __grid_constant__ MsEdenTileParams p, uint32_t tiles_x, uint32_t tile_count) {
+  allow_next_kernel();
   __shared__ __align__(16) uint8_t nv_stage[kTileRows * kNvPitch];
   __shared__ float2 inv_table[kScaleCodes];
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);

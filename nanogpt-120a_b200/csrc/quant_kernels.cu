@@ -437,6 +437,7 @@ __global__ void __launch_bounds__(256, 4)
                     uint8_t* __restrict__ out_fp4, uint8_t* __restrict__ out_scales, float* __restrict__ out_gs,
                     float* __restrict__ decoded_amax, uint32_t rows, uint32_t groups, const FastDiv groups_per_row,
                     uint32_t opaque_zero) {
+  allow_next_kernel();
   float dec = 0.0f;
   float tensor_amax = 0.0f;
   if (!kRowwise) {
@@ -529,6 +530,7 @@ __global__ void __launch_bounds__(256, 3)
                             float* __restrict__ out_gs, float* __restrict__ out_amax, float* __restrict__ decoded_amax,
                             uint32_t rows, uint32_t padded_rows, uint32_t groups_per_row, uint32_t rows_per_cta,
                             uint32_t row_blocks, uint32_t opaque_zero) {
+  allow_next_kernel();
   __shared__ unsigned int row_amax_bits[3][kStreamMaxRowsPerCta];
   const uint32_t t = threadIdx.x, lane_id = t & 31u;
   for (uint32_t i = t; i < 3 * rows_per_cta; i += blockDim.x) row_amax_bits[i / rows_per_cta][i % rows_per_cta] = 0u;
@@ -770,6 +772,7 @@ constexpr int kTileRows = 128, kTileCols = 64, kTileLd = kTileCols + 1;
 
 template <int kSrc, typename T, bool kPair>
 __global__ void __launch_bounds__(256) ms_eden_tile_kernel(const MsEdenTileParams p) {
+  allow_next_kernel();
   __shared__ float tile[kTileRows * kTileLd];
   __shared__ uint32_t neg_r[kTileRows / 32];  // sign bits of the tile's rows (K of the transposed operand)
   __shared__ uint32_t neg_c[kTileCols / 32];  // sign bits of the tile's columns (K of the row operand)
@@ -1057,6 +1060,7 @@ __global__ void __launch_bounds__(256) decode_rows_kernel(const uint8_t* __restr
 // single bytes 16 apart: 8192 x 8192 8.9 us; this form 3.1 us).
 __global__ void __launch_bounds__(256) scale_pack_tiles_kernel(const uint8_t* __restrict__ logical, uint8_t* __restrict__ packed,
                                                                 uint32_t mn, uint32_t k_atoms) {
+  allow_next_kernel();
   __shared__ uint32_t words[128][17];
   const uint32_t atom0 = blockIdx.x * 16u, row0 = blockIdx.y * 128u;
   const uint32_t atoms = min(16u, k_atoms - atom0);
@@ -1182,6 +1186,7 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const T* __restrict__ e,
 // column each add tiles lane, lane+8, ... in sequence, then the lane sums are added 0..7.
 __global__ void __launch_bounds__(256) col_sum_reduce_kernel(const float* __restrict__ partials,
                                                               float* __restrict__ dbias, uint32_t tiles, uint32_t n) {
+  allow_next_kernel();
   __shared__ float sums[256];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t c = blockIdx.x * 32 + lane;

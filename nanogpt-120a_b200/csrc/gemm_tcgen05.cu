@@ -326,19 +326,32 @@ __device__ __forceinline__ constexpr uint32_t make_idesc() {
          (static_cast<uint32_t>(kRowBlock >> 4) << 24);
 }
 
+// Loads of values that the kernel before this one may have written.  Volatile and through the coherent path: a read-only
+// load counts as movable, and must not move above the wait for that kernel.
+__device__ __forceinline__ float load_prior(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t load_prior(const uint8_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Bias of one output column: an f32 vector, or an NVFP4-encoded one decoded as the reference's post-op
 // kernels decode it, (e2m1 * e4m3) * global_scale (utils/nvfp4/tensor.rs:48-57, gpt/projection_postop.rs:97-115).
 __device__ __forceinline__ float bias_value(const GemmParams& p, uint32_t col) {
-  if (p.bias) return __ldg(p.bias + col);
-  const uint32_t byte = __ldg(p.bias_bytes + (col >> 1));
+  if (p.bias) return load_prior(p.bias + col);
+  const uint32_t byte = load_prior(p.bias_bytes + (col >> 1));
   const uint32_t nib = (col & 1u) ? (byte >> 4) : (byte & 0xfu);
   uint32_t h2;
   asm("{ .reg .b8 t; cvt.u8.u32 t, %1; cvt.rn.f16x2.e2m1x2 %0, t; }" : "=r"(h2) : "r"(nib));
   const float q = __low2float(*reinterpret_cast<__half2*>(&h2));
   uint32_t s2;
-  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(s2) : "h"(static_cast<uint16_t>(__ldg(p.bias_scales + (col >> 4)))));
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(s2) : "h"(static_cast<uint16_t>(load_prior(p.bias_scales + (col >> 4)))));
   const float sc = __low2float(*reinterpret_cast<__half2*>(&s2));
-  return __fmul_rn(__fmul_rn(q, sc), __ldg(p.bias_global));
+  return __fmul_rn(__fmul_rn(q, sc), load_prior(p.bias_global));
 }
 
 // ---- epilogue stores ------------------------------------------------------------------------
@@ -943,13 +956,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = true;  // warp uniform; false: some wait ran out, the rest of the list is walked without work
     const uint32_t my_bias = smem_bias + eg * kBlockN * 4;
     const float* my_bias_gen = reinterpret_cast<const float*>(smem_gen + (my_bias - smem_base));
-    const float gb = p.mode == NVFP4_GS_NONE ? 1.0f : __ldg(p.b_global);
-    const float ga_scalar = p.mode == NVFP4_GS_TENSOR ? __ldg(p.a_global) : 1.0f;
+    const float gb = p.mode == NVFP4_GS_NONE ? 1.0f : load_prior(p.b_global);
+    const float ga_scalar = p.mode == NVFP4_GS_TENSOR ? load_prior(p.a_global) : 1.0f;
     // the rows' global scales of a tile are fetched one tile ahead: their load latency would
     // otherwise sit between the accumulator becoming ready and the first store
     auto row_scale = [&](uint32_t mb, uint32_t h) {
       const uint32_t r = mb * kBlockM + h * kRowBlock + gtid;
-      return (p.mode == NVFP4_GS_ROWWISE_A && r < p.m) ? __ldg(p.a_global + r) : 0.0f;
+      return (p.mode == NVFP4_GS_ROWWISE_A && r < p.m) ? load_prior(p.a_global + r) : 0.0f;
     };
     // The bias slice of a tile travels the same way: its values are fetched into registers one tile ahead
     // and reach shared memory only when the column block changes (a banded schedule keeps a CTA on one

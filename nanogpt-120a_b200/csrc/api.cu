@@ -631,12 +631,23 @@ static int projection(void* stream, const nvfp4_projection_args* a, ProjectionKi
   if (kind == kProjResidual && a->out_dtype != NVFP4_DTYPE_F32) return invalid("projection: the residual stream is f32");
   if (kind == kProjRelu2 ? (!a->pre_activation && !a->out) : !a->out) return invalid("projection: null output");
   const uint8_t *xs = nullptr, *ws = nullptr;
-  int rc = packed_plane(stream, a->input_scales, a->input_scale_layout, a->input_scales_packed_scratch, a->token_count,
-                        a->input_dim, &xs, "projection: logical input scales need input_scales_packed_scratch");
-  if (rc) return rc;
-  rc = packed_plane(stream, a->weight_scales, a->weight_scale_layout, a->weight_scales_packed_scratch, a->output_dim,
-                    a->input_dim, &ws, "projection: logical weight scales need weight_scales_packed_scratch");
-  if (rc) return rc;
+  int rc;
+  if (a->input_scale_layout == NVFP4_SCALES_LOGICAL && a->weight_scale_layout == NVFP4_SCALES_LOGICAL &&
+      a->input_scales_packed_scratch && a->weight_scales_packed_scratch) {  // both planes in one launch
+    xs = a->input_scales_packed_scratch;
+    ws = a->weight_scales_packed_scratch;
+    rc = launch_scale_pack_pair(S(stream), {a->input_scales, a->weight_scales},
+                                {a->input_scales_packed_scratch, a->weight_scales_packed_scratch},
+                                {a->token_count, a->output_dim}, a->input_dim);
+    if (rc) return rc;
+  } else {
+    rc = packed_plane(stream, a->input_scales, a->input_scale_layout, a->input_scales_packed_scratch, a->token_count,
+                      a->input_dim, &xs, "projection: logical input scales need input_scales_packed_scratch");
+    if (rc) return rc;
+    rc = packed_plane(stream, a->weight_scales, a->weight_scale_layout, a->weight_scales_packed_scratch, a->output_dim,
+                      a->input_dim, &ws, "projection: logical weight scales need weight_scales_packed_scratch");
+    if (rc) return rc;
+  }
   nvfp4_gemm_args g;
   std::memset(&g, 0, sizeof(g));
   g.a_bytes = a->input_bytes;

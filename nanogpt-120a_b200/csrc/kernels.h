@@ -53,6 +53,9 @@ int launch_col_sum_reduce(cudaStream_t s, const float* partials, float* dbias, u
 int launch_decode(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, const float* gscales, int rowwise,
                   int transpose, float* out, uint32_t rows, uint32_t cols);
 int launch_scale_pack(cudaStream_t s, const uint8_t* logical, uint8_t* packed, uint32_t mn, uint32_t k_dim);
+// two planes of one k_dim (the operands of a GEMM), in one launch where both allow the tiled kernel
+int launch_scale_pack_pair(cudaStream_t s, const uint8_t* const (&logical)[2], uint8_t* const (&packed)[2],
+                           const uint32_t (&mn)[2], uint32_t k_dim);
 int launch_pad_u4_rows(cudaStream_t s, const uint8_t* src, uint8_t* dst, uint32_t rows, uint32_t padded_rows,
                        uint32_t cols);
 int launch_pad_f32(cudaStream_t s, const float* src, float* dst, uint32_t rows, uint32_t cols, uint32_t padded_rows,

@@ -610,3 +610,27 @@ def test_residual_add_reduction_and_direct(pkg, oracle, dev, m, n, k, ldo, bias_
     ok = np.isfinite(want)
     assert rel_fro(got[:, :n][ok], want[ok]) <= GEMM_TOL
     no_timeouts(pkg)
+
+
+@pytest.mark.parametrize("tokens,in_dim,out_dim", [(1, 64, 16), (128, 64, 128), (129, 1088, 144), (300, 2048, 400)])
+def test_projection_packs_both_scale_planes(pkg, oracle, dev, tokens, in_dim, out_dim):
+    """Logical scales on both operands are packed in one launch, row blocks of the weight behind those of the input:
+    the result is the one of operands packed apart, bit for bit (row blocks with pad rows, k-atom blocks with tails)."""
+    rng = np.random.default_rng(tokens + in_dim)
+    a, b = rand_nvfp4(rng, tokens, in_dim, True), rand_nvfp4(rng, out_dim, in_dim, False)
+    q = pkg.Nvfp4QuantModule()
+    bias = q.quantize_four_six(torch.from_numpy(rng.normal(0, 5.0, (1, out_dim)).astype(np.float32)).to(dev), rowwise=False,
+                               packed=False)
+    outs = []
+    for packed in (False, True):
+        x, w = q.quantize_four_six(torch.ones(tokens, in_dim, device=dev), rowwise=True, packed=packed), \
+            q.quantize_four_six(torch.ones(out_dim, in_dim, device=dev), rowwise=False, packed=packed)
+        for t, src, rows in ((x, a, tokens), (w, b, out_dim)):
+            t.bytes.copy_(torch.from_numpy(src[0]))
+            t.scales.copy_(torch.from_numpy(oracle.scale_pack(src[1], rows, in_dim) if packed else src[1]))
+            t.global_scales.copy_(torch.from_numpy(src[2]))
+        outs.append(pkg.NextLatModule().projection(x, w, bias))
+    assert torch.equal(outs[0], outs[1])
+    assert rel_fro(cpu(outs[0]), oracle.gemm(a, b, tokens, in_dim, out_dim, 2, bias=cpu(pkg.Nvfp4DecodeModule().decode(bias))[0],
+                                             epi=1)) <= GEMM_TOL
+    no_timeouts(pkg)

@@ -634,3 +634,54 @@ def test_projection_packs_both_scale_planes(pkg, oracle, dev, tokens, in_dim, ou
     assert rel_fro(cpu(outs[0]), oracle.gemm(a, b, tokens, in_dim, out_dim, 2, bias=cpu(pkg.Nvfp4DecodeModule().decode(bias))[0],
                                              epi=1)) <= GEMM_TOL
     no_timeouts(pkg)
+
+
+@pytest.mark.parametrize("tokens,in_dim,out_dim", [(16, 64, 128), (2048, 768, 768), (8192, 1024, 256)])
+def test_gemm_set_up_early_waits_for_its_operands(pkg, dev, tokens, in_dim, out_dim):
+    """The GEMM is set up while the quantizer before it drains: with the inputs changing from call to call and nothing
+    synchronised in between (default stream, another stream, a captured graph), every result is the one of a call that ran
+    alone."""
+    q, gemm = pkg.Nvfp4QuantModule(), pkg.Nvfp4GemmModule()
+    gen = torch.Generator(device=dev).manual_seed(tokens)
+    xs = [torch.randn(tokens, in_dim, generator=gen, device=dev).to(torch.bfloat16) * (1 + i) for i in range(3)]
+    w = q.quantize_four_six(torch.randn(out_dim, in_dim, generator=gen, device=dev), rowwise=False, packed=True)
+    xq = q.quantize_four_six(xs[0], rowwise=True, packed=True)
+    outs = [torch.empty(tokens, out_dim, device=dev) for _ in xs]
+
+    def step(i):
+        q.quantize_four_six(xs[i], rowwise=True, packed=True, out=xq)  # overwrites what the GEMM before it has read
+        gemm.gemm(xq, w, out=outs[i])
+
+    want = []
+    for i in range(3):
+        step(i)
+        torch.cuda.synchronize()
+        want.append(outs[i].clone())
+    assert not torch.equal(want[0], want[1])
+
+    def check():
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, e) for o, e in zip(outs, want))
+        for o in outs:
+            o.zero_()
+
+    for _ in range(8):
+        for i in range(3):
+            step(i)
+    check()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        for _ in range(8):
+            for i in range(3):
+                step(i)
+        side.synchronize()
+    check()
+    with torch.cuda.graph(graph):
+        for i in range(3):
+            step(i)
+    for _ in range(4):
+        graph.replay()
+    check()
+    no_timeouts(pkg)

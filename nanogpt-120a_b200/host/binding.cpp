@@ -78,6 +78,7 @@ struct NoGil {
   PyThreadState* s = PyEval_SaveThread();
   ~NoGil() { PyEval_RestoreThread(s); }
 };
+// Runs without the GIL: `f` may use pointers and at::Tensors taken before, no PyObject.
 template <typename F>
 void call(F&& f) {
   int rc;
@@ -174,11 +175,12 @@ PyObject* quantize_into(Args a) {
 // x f32 [rows, cols], row amax -> (bytes, logical scales, global_scales)
 PyObject* four_six_rowwise_f32(Args a) {
   const at::Tensor& x = tensor(a[0]);
+  const float* amax = ptr<float>(a[1]);
   uint32_t rows, cols;
   matrix_shape(x, rows, cols);
   const Fp4 q = new_fp4(rows, cols, false, rows, x.device());
   call([&] {
-    return nvfp4_fp32_to_nvfp4_four_six_rowwise(stream(), ptr<float>(x), ptr<float>(a[1]), ptr<uint8_t>(q.bytes),
+    return nvfp4_fp32_to_nvfp4_four_six_rowwise(stream(), ptr<float>(x), amax, ptr<uint8_t>(q.bytes),
                                                 ptr<uint8_t>(q.scales), ptr<float>(q.globals),
                                                 static_cast<uint32_t>(static_cast<uint64_t>(rows) * cols / 16), cols);
   });

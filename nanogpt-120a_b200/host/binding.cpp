@@ -63,7 +63,16 @@ float f32(PyObject* o) {
   if (v == -1.0 && PyErr_Occurred()) throw Raised{};
   return static_cast<float>(v);
 }
-bool flag(PyObject* o) { return PyObject_IsTrue(o) == 1; }
+bool flag(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw Raised{};
+  return v != 0;
+}
+void* handle(PyObject* o) {
+  void* p = PyLong_AsVoidPtr(o);
+  if (!p && PyErr_Occurred()) throw Raised{};
+  return p;
+}
 
 int dtype_code(const at::Tensor& t) {
   if (t.scalar_type() == at::kFloat) return NVFP4_DTYPE_F32;
@@ -368,7 +377,7 @@ PyObject* linear_backward(Args a) {
   b.token_count = static_cast<uint32_t>(tokens), b.input_dim = static_cast<uint32_t>(in_dim), b.output_dim = static_cast<uint32_t>(out_dim);
   b.sign_seed = u32(a[22]), b.scale_seed = u32(a[23]), b.precomputed_e_amax_chunks = u32(a[24]), b.token_offset = u32(a[25]);
   b.e_global_scale_override = ptr<float>(a[26]), b.x_decoded_amax = ptr<float>(a[27]);
-  b.side_stream = PyLong_AsVoidPtr(a[28]), b.fork_event = PyLong_AsVoidPtr(a[29]), b.join_event = PyLong_AsVoidPtr(a[30]);
+  b.side_stream = handle(a[28]), b.fork_event = handle(a[29]), b.join_event = handle(a[30]);
   b.total_token_count = u32(a[31]), b.weight_t_prepared = flag(a[32]);
   call([&] { return prepare_only ? nvfp4_linear_backward_prepare_weight_t(stream(), &b) : nvfp4_linear_backward_ms_eden(stream(), &b); });
   if (prepare_only) return none();

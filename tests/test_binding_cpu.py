@@ -37,3 +37,9 @@ def test_four_six_rowwise_amax_error():
     """The amax is unwrapped, and refused, before the GIL is released."""
     calls = ["native.four_six_rowwise_f32(x, %s)" % amax for amax in ("cpu", "strided", "7")]
     assert errors(calls) == ["AssertionError", "AssertionError", "TypeError"]
+
+
+def test_truth_value_error():
+    """A flag without a truth value is an error, not a false."""
+    calls = ["native.quantize_new(x, None, np.zeros(2), True, False)", "native.quantize_new(x, None, True, np.zeros(2), False)"]
+    assert errors(calls) == ["ValueError", "ValueError"]

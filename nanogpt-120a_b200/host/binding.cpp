@@ -236,6 +236,9 @@ PyObject* materialize(Args a) {
   const bool packed = flag(a[3]);
   const Fp4 q = new_fp4(rows, cols, packed, 1, z.device());
   const at::Tensor amax = floats(1, z.device()), partials = floats(nvfp4_tensor_amax_partials(), z.device());
+  // With logical scales the 16-groups run over the flat tensor: its rows need not be whole groups.
+  const uint64_t n = static_cast<uint64_t>(rows) * cols;
+  if (!packed && cols % 16 != 0 && n <= UINT32_MAX) rows = 1, cols = static_cast<uint32_t>(n);
   call([&] {
     return nvfp4_materialize_schedule_free_partials(stream(), ptr<float>(z), ptr<float>(x), ptr<float>(partials), ptr<float>(amax),
                                                     ptr<uint8_t>(q.bytes), ptr<uint8_t>(q.scales),

@@ -9,7 +9,7 @@
 //  * a bf16 source is widened, sign-flipped and taken through the first butterfly stage by mixed-precision FMAs,
 //    x * (+-1) + u (exact product, one rounding), or for the upper half of a word by one logic instruction;
 //  * the lower E2M1 code of a byte is widened with add.f32.f16 instead of cvt.f32.f16;
-//  * the reciprocal of a block scale, 1 / (s * gs + eps), depends on the 128 possible s only: a table per CTA;
+//  * the reciprocal of a block scale, 1 / (s * gs + eps), depends on the scale byte only: a table per CTA;
 //  * every range check of a chunk (corrected scale inside the normal E4M3 range, finite quotients) is folded into one
 //    predicate at the end; a chunk that fails it is quantized again by the generic code behind the tile's barrier.
 //    The common path is one straight line, so the chains of the 16-groups overlap; with a branch per check they did not;
@@ -26,7 +26,7 @@ namespace {
 
 constexpr int kTileRows = 128, kTileCols = 64;
 
-constexpr uint32_t kScaleCodes = 128;  // non-negative E4M3 codes
+constexpr uint32_t kScaleCodes = 256;  // every E4M3 byte: a negative global scale or scale override gives negative codes
 
 __device__ __forceinline__ void cp_async_16(uint32_t smem_addr, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gmem) : "memory");
@@ -137,7 +137,7 @@ __device__ __forceinline__ uint32_t ms_eden_group(const f32x2_t* H, uint32_t inv
   // block scale code: nearest E4M3 value, ties to even, saturating at 448
   uint16_t codes;
   asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(codes) : "f"(ga_hi * so * inv6), "f"(ga_lo * so * inv6));
-  const uint2 t0 = lds_64(inv_table + (codes & 0x7fu) * 8), t1 = lds_64(inv_table + (static_cast<uint32_t>(codes) >> 8) * 8);
+  const uint2 t0 = lds_64(inv_table + (codes & 0xffu) * 8), t1 = lds_64(inv_table + (static_cast<uint32_t>(codes) >> 8) * 8);
   const f32x2_t inv = pack2(__uint_as_float(t0.x), __uint_as_float(t1.x));
   f32x2_t x[16];
   float xa[16], xb[16];

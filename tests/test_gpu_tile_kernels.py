@@ -75,3 +75,57 @@ def test_pair_rows_equal_generic_kernel_large(pkg, dev):
                                 global_scale=sc.e_h["global_scale"], sign_seed=SIGN, scale_seed=SCALE, packed=True)
     assert torch.equal(sc.e_h["bytes"], ref.bytes)
     assert torch.equal(sc.e_h["scales_packed"], ref.scales)
+
+
+# factors on the global scale the tensor's amax gives, and scale overrides: signs, block scales that all saturate or all
+# round to zero, quotients that overflow
+SCALES = [(-1.0, None), (1.0, -0.988125), (-1.0, -0.988125), (1e-30, None), (1e30, None), (1.0, 1e-20), (1.0, 0.03), (1.0, 30.0),
+          (1.0, 1e20)]
+
+
+@pytest.mark.parametrize("factor,override", SCALES)
+@pytest.mark.parametrize("rows,cols", [(128, 64), (130, 96)])
+@pytest.mark.parametrize("rowwise", [False, True])
+def test_nvfp4_transpose_any_scale(pkg, oracle, dev, rows, cols, rowwise, factor, override):
+    """A caller's global scale and scale override may have any sign and size: bytes of the oracle."""
+    q = pkg.Nvfp4QuantModule()
+    x = bf16_normal(711, (rows, cols)).float().numpy()
+    x[3], x[:, 5] = 0.0, -0.0
+    src = oracle.four_six(x, oracle.row_amax(x) if rowwise else oracle.tensor_amax(x)[1], rowwise)
+    gs = float(np.float32(factor * oracle.ms_eden_global_scale(float(oracle.nvfp4_amax(*src, rows, cols, rowwise)[1][0]))))
+    so = pkg.QUARTET_MS_EDEN_SCALE_OVERRIDE if override is None else override
+    k = oracle.padded_k(rows)
+    want = oracle.ms_eden(3 if rowwise else 2, (*src, rows, cols), cols, k, gs, SIGN, SCALE, so=so, want_chunk_amax=False)
+    t = pkg.Nvfp4Tensor(*(torch.from_numpy(a).to(dev) for a in src), rows, cols, packed=False, rowwise=rowwise)
+    got, _ = q.ms_eden_quantize(src_kind=pkg.SRC_ROWWISE_NVFP4_TRANSPOSED if rowwise else pkg.SRC_NVFP4_TRANSPOSED, src=t,
+                                rows=rows, cols=cols, dst_row_len=k, global_scale=gs, sign_seed=SIGN, scale_seed=SCALE,
+                                scale_override=so)
+    assert np.array_equal(cpu(got.bytes), want[0])
+    assert np.array_equal(cpu(got.scales), want[1])
+    assert np.array_equal(cpu(got.global_scales), want[2])
+
+
+@pytest.mark.parametrize("factor", [-1.0, 1e-30, 1e30])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,out_dim", [(128, 128), (129, 72)])
+def test_pair_any_scale(pkg, oracle, dev, tokens, out_dim, dtype, factor):
+    """The same for dY in both orientations, whose scale a caller may give."""
+    q, bwd, in_dim = pkg.Nvfp4QuantModule(), pkg.LinearBackwardModule(), 64
+    dy = bf16_normal(712, (tokens, out_dim), 1e-3)
+    dy[7], dy[:, 9] = 0.0, -0.0
+    ef = dy.float().numpy()
+    gs = np.float32(factor * oracle.ms_eden_global_scale(float(np.abs(ef).max())))
+    xq = q.quantize_four_six(bf16_normal(713, (tokens, in_dim)).to(dev), rowwise=True, packed=True, decoded_amax=True)
+    wq = q.quantize_four_six(bf16_normal(714, (out_dim, in_dim), 0.02).to(dev), rowwise=False, packed=True)
+    sc = pkg.LinearBackwardScratch(tokens, in_dim, out_dim, dev)
+    bwd.backward_ms_eden(e=dy.to(dev).to(dtype), weight=wq, input=xq, scratch=sc, sign_seed=SIGN, scale_seed=SCALE,
+                         e_global_scale=torch.tensor([gs], device=dev))
+    ok, tk = oracle.padded_k(out_dim), oracle.padded_k(tokens)
+    for name, kind, rows, k, seed in (("e_h", 0, tokens, ok, SCALE), ("e_t_h", 1, out_dim, tk, SCALE ^ 0x85EBCA6B)):
+        ref = oracle.ms_eden(kind, ef, rows, k, float(gs), SIGN, seed, want_chunk_amax=False)
+        op = getattr(sc, name)
+        assert np.array_equal(cpu(op["bytes"]), ref[0]), name
+        assert np.array_equal(cpu(op["scales_packed"]), oracle.scale_pack(ref[1], rows, k)), name
+        assert np.array_equal(cpu(op["global_scales"]), ref[2]), name
+    torch.cuda.synchronize()
+    assert pkg.read_device_status() == 0

@@ -167,9 +167,10 @@ __device__ __forceinline__ uint32_t ms_eden_group(const f32x2_t* H, uint32_t inv
           num_a, num_b);
   unpack2(add2(add2(add2(den8[0], den8[4]), add2(den8[2], den8[6])), add2(add2(den8[1], den8[5]), add2(den8[3], den8[7]))),
           den_a, den_b);
-  // A scale of at least 2^-9 leaves the group's largest |x| at 4 or more: both sums are at least 16, and the quotient
-  // needs no range check.  With the scale's code 0 (it stands for 1 then) den may be 0 and the result NaN, which the
-  // range check of the product catches like every product outside [2^-6, 448).
+  // The quotient needs no range check of its own, whatever the global scale and the scale override make of x: an E2M1
+  // value is 0 up to |x| = 1/4 and at least 1/2 beyond, so den is 0 or at least 1/8, and where the sums stay finite den is
+  // below 2^71, its reciprocal far inside the normal range.  den = 0 and infinite sums end as NaN, which the range check
+  // of the product catches like every product outside [2^-6, 448).
   const uint32_t s0 = __float_as_uint(__uint_as_float(t0.y) * div_in_range(num_a, den_a));
   const uint32_t s1 = __float_as_uint(__uint_as_float(t1.y) * div_in_range(num_b, den_b));
   ok = ok && s0 - 0x3c800000u < 0x43e00000u - 0x3c800000u && s1 - 0x3c800000u < 0x43e00000u - 0x3c800000u;

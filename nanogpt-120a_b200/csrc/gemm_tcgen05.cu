@@ -117,7 +117,6 @@ struct GemmParams {
   int b_resident;   // the B panel of a column block stays in shared memory (short K)
   uint32_t resident_cpn;  // resident mode: CTAs per column block (0 = contiguous tile ranges instead)
   int mode, epilogue, vec_store, tma_store;
-  int reduce_out;  // TMA stores add to `out` instead of replacing it: split-K partial sums, the f32 residual stream
   float weight;
   uint64_t wait_timeout_ns;  // limit of every mbarrier wait
   uint32_t debug_flags;      // bit 0: CTA 0 never loads its first k-tile (exercises the bounded waits)
@@ -171,6 +170,12 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
+__device__ __forceinline__ uint32_t clock32() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+  return t;
+}
+
 // Bounded wait.  Returns false when the CTA is aborting (this waiter timed out, or another
 // role already did); the caller then leaves its loop and goes to the common teardown.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
@@ -196,6 +201,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
       : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int32_t x, int32_t y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y)
+               : "memory");
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -420,6 +429,19 @@ struct SubTile<float> {
     }
   }
 };
+// v += the row of an f32 sub-tile that a TMA load has left in the staging buffer, laid out as `stage` writes it
+__device__ __forceinline__ void add_staged_row(uint32_t row_addr, uint32_t row, float* v) {
+#pragma unroll
+  for (uint32_t c = 0; c < 8; ++c) {
+    float r[4];
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3])
+                 : "r"(row_addr + ((c ^ (row & 7u)) << 4))
+                 : "memory");
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) v[4 * c + j] = __fadd_rn(v[4 * c + j], r[j]);
+  }
+}
 template <>
 struct SubTile<__nv_bfloat16> {
   static constexpr int kCols = 64;
@@ -593,6 +615,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint64_t downstream_timeout_ns = 2 * p.wait_timeout_ns;
   // a ReLU^2 with its pre-activation kept stores every item twice: the pre-activation, then the activation
   const int item_passes = (p.epilogue == NVFP4_EPI_RELU2 && p.aux) ? 2 : 1;
+  // The f32 residual stream: an item's old values arrive in the staging buffer the item will leave from, `stored` of a
+  // buffer then means that they are there, and the epilogue adds to them in place.
+  const bool residual = kTmaStore && sizeof(OutT) == 4 && p.epilogue == NVFP4_EPI_RESIDUAL;
 
   if (warp == 0) {
     // ===================== TMA producer =====================
@@ -908,13 +933,52 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t eg = warp - 2u;
       uint32_t buf = 0, phase = 0, tile_iter = 0, issued = 0;
       bool ok = true;
+      auto item_x = [&](int item, uint32_t n_blk) { return static_cast<int32_t>(n_blk * kBlockN + (item % kNumSub) * kSub); };
+      auto item_y = [&](int item, uint32_t m_blk) { return static_cast<int32_t>(m_blk * kBlockM + (item / kNumSub) * kRowBlock); };
+      // residual stream: a second walk over the group's items, one ring ahead, loads what they will be added to
+      uint32_t load_w = w_begin, load_tile = 0, load_m = 0, load_n = 0, load_split = 0, loads = 0;
+      int load_item = kItems;  // next item of the tile (load_m, load_n); kItems: on to the tile of load_w
+      auto load_next = [&](uint32_t slot) {
+        while (true) {
+          if (load_item >= kItems) {
+            if (load_w >= w_end) return;
+            decode(load_w, load_m, load_n, load_split);
+            load_item = first_item_of(eg, load_tile++);
+            load_w += w_step;
+          }
+          const int item = load_item;
+          load_item += 2;
+          if (!item_valid(item, load_m, load_n)) continue;
+          mbar_expect_tx(bar_stored + 8 * slot, kStoreStageBytes);  // parts outside the matrix arrive as zeros
+          tma_load_2d(smem_store + slot * kStoreStageBytes, &tmap_out, bar_stored + 8 * slot, item_x(item, load_n),
+                      item_y(item, load_m));
+          ++loads;
+          return;
+        }
+      };
+      if (residual)
+        for (uint32_t b = 0; b < kRing; ++b) load_next(eg * kRing + b);
       for (uint32_t w = w_begin; w < w_end && ok; w += w_step, ++tile_iter) {
         uint32_t m_blk, n_blk, split;
         decode(w, m_blk, n_blk, split);
+        if (residual) {
+          // The items of this tile that no buffer is free for yet go to L2 during its main loop, spread over it: all at
+          // once they would stand before the operands in the queue to HBM.  8192 x 768 x K 3072 from HBM: 27.2 us without,
+          // 27.5 all at once, 23.4 spread; from L2 20.2.
+          const uint32_t t0 = clock32(), pace = p.num_k_tiles * 700u / (kItems / 2);
+          uint32_t due = 0;
+          for (int item = first_item_of(eg, tile_iter) + 2 * static_cast<int>(kRing); item < kItems; item += 2) {
+            if (!item_valid(item, m_blk, n_blk)) continue;
+            due += pace;
+            bool staged = false;
+            while (!staged && clock32() - t0 < due) staged = mbar_try_wait(bar_staged + 8 * (eg * kRing + buf), phase);
+            if (staged) break;
+            tma_prefetch_2d(&tmap_out, item_x(item, n_blk), item_y(item, m_blk));
+          }
+        }
         for (int item = first_item_of(eg, tile_iter); item < kItems && ok; item += 2) {
           if (!item_valid(item, m_blk, n_blk)) continue;
-          const int32_t x = static_cast<int32_t>(n_blk * kBlockN + (item % kNumSub) * kSub);
-          const int32_t y = static_cast<int32_t>(m_blk * kBlockM + (item / kNumSub) * kRowBlock);
+          const int32_t x = item_x(item, n_blk), y = item_y(item, m_blk);
           for (int pass = 0; pass < item_passes; ++pass) {
             const uint32_t slot = eg * kRing + buf;
             if (!mbar_wait(bar_staged + 8 * slot, phase, abort_flag, kStatusEpilogueTimeout, downstream_timeout_ns)) {
@@ -922,18 +986,23 @@ __global__ void __launch_bounds__(kThreads, 1)
               break;
             }
             const CUtensorMap* map = item_passes == 2 && pass == 0 ? &tmap_aux : &tmap_out;
-            if (p.reduce_out)
+            if (p.k_splits > 1)
               tma_reduce_add_2d(map, smem_store + slot * kStoreStageBytes, x, y);
             else
               tma_store_2d(map, smem_store + slot * kStoreStageBytes, x, y);
             bulk_commit_group();
             // the buffer the epilogue needs next is handed back as soon as its store has read it: this one with a
-            // single buffer, the previous one with two
-            bulk_wait_group_read<static_cast<int>(kRing) - 1>();
-            if (kRing == 1)
-              mbar_arrive(bar_stored + 8 * slot);
-            else if (issued > 0)
-              mbar_arrive(bar_stored + 8 * (eg * kRing + (buf ^ 1u)));
+            // single buffer, the previous one with two; with a load to come into it, this one at once
+            if (residual) {
+              bulk_wait_group_read<0>();
+              load_next(slot);
+            } else {
+              bulk_wait_group_read<static_cast<int>(kRing) - 1>();
+              if (kRing == 1)
+                mbar_arrive(bar_stored + 8 * slot);
+              else if (issued > 0)
+                mbar_arrive(bar_stored + 8 * (eg * kRing + (buf ^ 1u)));
+            }
             ++issued;
             if (++buf == kRing) {
               buf = 0;
@@ -943,6 +1012,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       bulk_wait_group0();  // stores complete before the CTA exits
+      if (!ok && residual) {
+        // aborting: give loads already in flight a bounded chance to land; load j is phase j / kRing of its buffer
+        for (uint32_t j = loads > kRing ? loads - kRing : 0; j < loads; ++j)
+          for (int spin = 0; spin < 4096 && !mbar_try_wait(bar_stored + 8 * (eg * kRing + j % kRing), (j / kRing) & 1u); ++spin) {
+          }
+      }
     }
   } else if (warp >= 4) {
     // ===================== epilogue (two groups of four warps) =====================
@@ -952,7 +1027,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     [[maybe_unused]] const bool elected = gtid == 0;
     OutT* out = static_cast<OutT*>(p.out);
     OutT* aux = static_cast<OutT*>(p.aux);
-    uint32_t acc = 0, acc_phase = 0, store_buf = 0, store_phase = 1, tile_iter = 0;
+    uint32_t acc = 0, acc_phase = 0, store_buf = 0, store_phase = residual ? 0u : 1u, tile_iter = 0;
     bool ok = true;  // warp uniform; false: some wait ran out, the rest of the list is walked without work
     const uint32_t my_bias = smem_bias + eg * kBlockN * 4;
     const float* my_bias_gen = reinterpret_cast<const float*>(smem_gen + (my_bias - smem_base));
@@ -1076,7 +1151,17 @@ __global__ void __launch_bounds__(kThreads, 1)
             tcgen05_wait_ld();
             GEMM_TRACE(3 + eg, 32, elected);
             if (item == last_item) release_accumulator();  // the group's last read of this tile
-            if (add_bias) {
+            if (residual) {
+              // the roundings of the direct path: the product, the sum with the bias, then the one with the stream
+#pragma unroll
+              for (int i = 0; i < kSub; i += 4) {
+                const float4 b = *reinterpret_cast<const float4*>(my_bias_gen + c + i);
+                mul_f32x2(v[i], v[i + 1], __uint_as_float(r[i / 32][i % 32]), __uint_as_float(r[i / 32][i % 32 + 1]), scale2);
+                mul_f32x2(v[i + 2], v[i + 3], __uint_as_float(r[i / 32][i % 32 + 2]), __uint_as_float(r[i / 32][i % 32 + 3]), scale2);
+                v[i] = __fadd_rn(v[i], b.x), v[i + 1] = __fadd_rn(v[i + 1], b.y);
+                v[i + 2] = __fadd_rn(v[i + 2], b.z), v[i + 3] = __fadd_rn(v[i + 3], b.w);
+              }
+            } else if (add_bias) {
               // acc * scale + bias in one rounding (the reference rounds the product first; the
               // difference is below the f32 ulp and far inside the GEMM tolerance)
 #pragma unroll
@@ -1127,6 +1212,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             ok = __all_sync(0xffffffffu, ok);
             GEMM_TRACE(3 + eg, 36, elected);
             if (ok) {
+              if constexpr (sizeof(OutT) == 4) {
+                if (residual) add_staged_row(smem_store + slot * kStoreStageBytes + gtid * 128, gtid, v);
+              }
               SubTile<OutT>::stage(smem_store + slot * kStoreStageBytes + gtid * 128, gtid, v);
               fence_proxy_async_smem();
               __syncwarp();
@@ -1496,6 +1584,12 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   // streamed long-K GEMMs; 128 x 128 remains for everything else.
   const bool can_split = a.out_dtype == NVFP4_DTYPE_F32 &&
                          (a.epilogue == NVFP4_EPI_NONE || a.epilogue == NVFP4_EPI_BIAS) && num_k_tiles >= 16;
+  //
+  // The f32 residual stream is loaded into the staging buffers its sums leave from.  Two buffers per group (128 x 128)
+  // keep a load in flight beside a store; one (the wider tiles) has them take turns, which a main loop of up to eight
+  // k-tiles does not hide: 65536 x 768 x K 768 82 us at 128 x 128, 98 to 100 at the others, K 1536 96 against 106 to 110;
+  // 8192 x 768 x K 3072 25 against 24.  Beyond, the estimate carries what the turns add to a tile.
+  const bool f32_residual = a.epilogue == NVFP4_EPI_RESIDUAL && a.out_dtype == NVFP4_DTYPE_F32;
   // Work items, waves and an estimated duration (SM cycles) of a candidate shape.  The constants are fits to
   // B200 measurements of the training step's shapes: a streamed k-tile costs what its operand bytes take
   // through the SM's L2 port (about 47 bytes per cycle: 128 x 128 700, 128 x 192 980, 128 x 256 1150,
@@ -1509,7 +1603,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   auto evaluate = [&](uint32_t bm, uint32_t bn) {
     const uint32_t tiles = tiles_of(bm, bn);
     const uint64_t ck = bm == 256 ? 1360 : bn == 256 ? 1150 : bn == 192 ? 980 : 700;
-    const uint64_t ce = bm == 256 ? 5000 : bn == 256 ? 3500 : bn == 192 ? 2000 : 1500;
+    const uint64_t ce = (bm == 256 ? 5000 : bn == 256 ? 3500 : bn == 192 ? 2000 : 1500) +
+                        (!f32_residual ? 0 : bm == 256 ? 11000 : bn == 256 ? 6000 : bn == 192 ? 1000 : 0);
     Candidate best{1, ~0ull};
     uint32_t max_splits = 1;
     if (can_split && tiles < 2 * usms) {
@@ -1532,7 +1627,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   if (forced) {
     block_m = static_cast<uint32_t>(forced) >> 16;
     block_n = static_cast<uint32_t>(forced) & 0xffffu;
-  } else {
+  } else if (!f32_residual || num_k_tiles > 8) {
     const uint32_t tiles192 = tiles_of(128, 192), tiles256 = tiles_of(128, 256);
     // columns of the last 192-wide block that lie outside the matrix, as a share of all columns computed
     const uint32_t cols192 = (a.n + 191) / 192 * 192;
@@ -1581,12 +1676,10 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
                      ? 1
                      : 0;
   // TMA-store epilogue whenever the output satisfies the tensor-map rules (16-byte aligned base
-  // and row pitch); odd layouts use direct stores.  The f32 residual stream leaves as a TMA reduce-add: one rounded
-  // addition per element, as the fused multiply-add by one of the direct path, done in L2 instead of through a
-  // register round trip whose lanes read a row each (like every f32 reduction in global memory it treats subnormals as
-  // zero): 4096 x 2048 x K 8192, 100 us with direct stores, 55 us with the reduction, 44 us once store warps
-  // issued it.  A bf16 residual stays on the
-  // direct path, which adds in f32 and rounds once.
+  // and row pitch); odd layouts use direct stores.  The f32 residual stream goes through the staging buffers as well, where
+  // its lanes would read and write a row each: 4096 x 2048 x K 8192 100 us with direct stores, 54 us.  A TMA reduction into
+  // the stream took 48 us, but every f32 reduction in global memory takes subnormals for zero.  A bf16 residual stays on
+  // the direct path, which adds in f32 and rounds once.
   pl.tma_store = (pl.vec_store && (a.epilogue != NVFP4_EPI_RESIDUAL || a.out_dtype == NVFP4_DTYPE_F32)) ? 1 : 0;
 
   const uint32_t work = tiles * pl.k_splits;
@@ -1767,7 +1860,6 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a) {
   p.resident_cpn = pl.resident_cpn;
   p.vec_store = static_cast<int>(pl.vec_store);
   p.tma_store = static_cast<int>(pl.tma_store);
-  p.reduce_out = pl.k_splits > 1 || a.epilogue == NVFP4_EPI_RESIDUAL;
   p.wait_timeout_ns = g_wait_timeout_ns.load(std::memory_order_relaxed);
   p.debug_flags = g_debug_flags.load(std::memory_order_relaxed);
 #ifdef NVFP4_GEMM_TRACE

@@ -575,9 +575,9 @@ def test_bounded_wait_runs_out_and_kernel_returns(pkg, oracle, dev):
 @pytest.mark.parametrize("m,n,k,ldo", [(1, 4, 64, 4), (127, 192, 256, 192), (129, 132, 320, 136), (257, 260, 1088, 260),
                                        (130, 100, 4160, 100), (64, 33, 128, 33)])
 def test_residual_add_reduction_and_direct(pkg, oracle, dev, m, n, k, ldo, bias_kind):
-    """The f32 residual stream leaves as a TMA reduce-add where the output can be described by a tensor map and through
-    direct stores where it cannot (a row pitch that is no multiple of 16 bytes); either way every element is added to
-    exactly once, columns beyond n are left alone, infinities and NaNs of the stream stay, and two runs agree bit for bit."""
+    """The f32 residual stream goes through the staging buffers where the output can be described by a tensor map and
+    through direct stores where it cannot (a row pitch that is no multiple of 16 bytes); either way every element is added
+    to exactly once, columns beyond n are left alone, infinities and NaNs of the stream stay, and two runs agree bit for bit."""
     gemm = pkg.Nvfp4GemmModule()
     rng = np.random.default_rng(m * 7 + n)
     a, b = rand_nvfp4(rng, m, k, True), rand_nvfp4(rng, n, k, False)
@@ -684,4 +684,59 @@ def test_gemm_set_up_early_waits_for_its_operands(pkg, dev, tokens, in_dim, out_
     for _ in range(4):
         graph.replay()
     check()
+    no_timeouts(pkg)
+
+
+@pytest.mark.parametrize("tile", [(128, 128), (192, 128), (256, 128), (192, 256), None])
+@pytest.mark.parametrize("m,n,k", [(1, 4, 64), (257, 260, 1088), (4096, 1060, 128), (16384, 776, 64)])
+def test_residual_routes_agree_bit_for_bit(pkg, dev, m, n, k, tile):
+    """The f32 residual stream adds in place in the staging buffers (aligned row pitch) or in registers (any other): the
+    same three roundings -- product, bias, residual -- and no value of the stream is lost, subnormal ones included.  One to
+    many items per epilogue group, tiles over the edge in both directions, streamed and resident B panels."""
+    gemm, q = pkg.Nvfp4GemmModule(), pkg.Nvfp4QuantModule()
+    gen = torch.Generator(device=dev).manual_seed(m + n)
+    a = torch.randn((m, k), generator=gen, device=dev)
+    a[::2] = 0.0  # rows whose product is zero: what comes out is the stream itself
+    A = q.quantize_four_six(a, rowwise=True, packed=True)
+    B = q.quantize_four_six(torch.randn((n, k), generator=gen, device=dev), rowwise=False, packed=True)
+    bias = torch.randn((n,), generator=gen, device=dev)
+    bias[::2] = 0.0
+    res = torch.randn((m, n), generator=gen, device=dev)
+    res[:, ::4] *= 2.0 ** -128  # subnormal
+    res[-1, -1] = -0.0
+    wide = torch.zeros((m, n + 1), device=dev)  # a row pitch no tensor map describes
+    wide[:, :n] = res
+    out, direct = res.clone(), wide.clone()
+    if tile:
+        pkg.set_gemm_tile_override(tile[0], tile[1])
+    try:
+        assert gemm.plan(A, B, bias=bias, epilogue=pkg.EPI_RESIDUAL, out=out).tma_store == 1
+        gemm.gemm(A, B, bias=bias, epilogue=pkg.EPI_RESIDUAL, out=out)
+        gemm.gemm(A, B, bias=bias, epilogue=pkg.EPI_RESIDUAL, out=direct, ldo=n + 1)
+    finally:
+        pkg.set_gemm_tile_override(0)
+    assert torch.equal(out.view(torch.int32), direct[:, :n].contiguous().view(torch.int32))
+    assert torch.equal(direct[:, n], wide[:, n])
+    kept = out[::2, ::4]
+    assert torch.equal(kept, res[::2, ::4]) and bool((kept != 0).any())
+    no_timeouts(pkg)
+
+
+def test_residual_wait_runs_out(pkg, dev):
+    """A CTA whose operands never come gives up with loads of the stream in its staging buffers; the next call is whole."""
+    gemm, q = pkg.Nvfp4GemmModule(), pkg.Nvfp4QuantModule()
+    a, w = torch.randn(512, 1024, device=dev), torch.randn(512, 1024, device=dev)
+    A, B = q.quantize_four_six(a, rowwise=True, packed=True), q.quantize_four_six(w, rowwise=False, packed=True)
+    bias, res = torch.randn(512, device=dev), torch.randn(512, 512, device=dev)
+    want = gemm.gemm(A, B, bias=bias, epilogue=pkg.EPI_RESIDUAL, out=res.clone())
+    pkg.set_gemm_wait_timeout_ns(2_000_000)
+    pkg.set_gemm_debug_flags(1)
+    try:
+        gemm.gemm(A, B, bias=bias, epilogue=pkg.EPI_RESIDUAL, out=res.clone())
+        torch.cuda.synchronize()
+        assert pkg.read_device_status() != 0
+    finally:
+        pkg.set_gemm_debug_flags(0)
+        pkg.set_gemm_wait_timeout_ns(0)
+    assert torch.equal(gemm.gemm(A, B, bias=bias, epilogue=pkg.EPI_RESIDUAL, out=res.clone()), want)
     no_timeouts(pkg)

@@ -1077,7 +1077,7 @@ class LinearBackwardModule:
         in_dim = weight.cols
         assert weight.rows == out_dim and input.rows == tokens and input.cols == in_dim
         assert scratch.dims == (tokens, in_dim, out_dim)
-        if grad_dtype not in (torch.float32, torch.bfloat16):
+        if (dinput is None or dweight is None) and grad_dtype not in (torch.float32, torch.bfloat16):
             raise TypeError(f"unsupported dtype {grad_dtype}; the path takes float32 or bfloat16")
         side_stream, fork, join = side.numbers() if side is not None and not prepare_weight_t_only else (0, 0, 0)
         return _native().linear_backward(

@@ -23,3 +23,19 @@ def test_materialize_rows_of_partial_groups(pkg, oracle, dev, shape):
     ob, os_, og = oracle.four_six(y, want, False)
     assert cpu(amax).tobytes() == want.tobytes() and (t.rows, t.cols) == shape
     assert np.array_equal(cpu(t.bytes), ob) and np.array_equal(cpu(t.scales), os_) and np.array_equal(cpu(t.global_scales), og)
+
+
+def test_backward_outputs_decide_their_dtype(pkg, dev):
+    """`grad_dtype` is the type of the gradients the call allocates; with both given it is not looked at."""
+    t, i, o = 64, 64, 128
+    q, bwd, sc = pkg.Nvfp4QuantModule(), pkg.LinearBackwardModule(), pkg.LinearBackwardScratch(64, 64, 128, dev)
+    xq = q.quantize_four_six(torch.randn(t, i, device=dev), rowwise=True, packed=True)
+    wq = q.quantize_four_six(torch.randn(o, i, device=dev), rowwise=False, packed=True)
+    args = dict(e=torch.randn(t, o, device=dev), weight=wq, input=xq, scratch=sc, sign_seed=1, scale_seed=2)
+    want = bwd.backward_ms_eden(**args)
+    dx, dw = torch.empty(t, i, device=dev), torch.empty(o, i, device=dev)
+    got = bwd.backward_ms_eden(**args, grad_dtype=torch.float16, dinput=dx, dweight=dw)
+    assert got[0] is dx and got[1] is dw and torch.equal(dx, want[0]) and torch.equal(dw, want[1])
+    for given in (dict(), dict(dinput=dx), dict(dweight=dw)):
+        with pytest.raises(TypeError):
+            bwd.backward_ms_eden(**args, grad_dtype=torch.float16, **given)

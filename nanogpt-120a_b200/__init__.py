@@ -16,6 +16,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import sysconfig
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_size_t, c_uint8, c_uint32, c_void_p
 from dataclasses import dataclass
 from typing import Optional
@@ -253,7 +254,8 @@ def library() -> ctypes.CDLL:
     return _lib
 
 
-BINDING_PATH = os.path.join(_HERE, "_nvfp4_binding.so")
+# bound to the C++ ABI of one torch and the C ABI of one Python: both are in its name
+BINDING_PATH = os.path.join(_HERE, f"_nvfp4_binding.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
 _binding = None
 
 

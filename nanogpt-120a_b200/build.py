@@ -11,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -88,21 +89,24 @@ def build_step_library(force: bool = False) -> str:
     return STEP_LIB
 
 
-BINDING = os.path.join(HERE, "_nvfp4_binding.so")
+def binding_path() -> str:
+    """The binding of this Python and this torch (the package loads no other): a new one of either is a new file."""
+    import torch
+
+    return os.path.join(HERE, f"_nvfp4_binding.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
 
 
 def build_binding(force: bool = False) -> str:
     """Compiles the CPython binding of the hot entry points (host/binding.cpp) against the installed torch."""
-    import sysconfig
-
     import torch
 
+    target = binding_path()
     src = os.path.join(HERE, "host", "binding.cpp")
     include = os.path.abspath(os.path.join(HERE, "..", "include"))
-    if force or _stale(BINDING, [src, build(), os.path.join(include, "nvfp4_b200.h")]):
+    if force or _stale(target, [src, build(), os.path.join(include, "nvfp4_b200.h")]):
         troot = os.path.dirname(torch.__file__)
         cuda = os.path.dirname(os.path.dirname(_nvcc()))
-        tmp = BINDING + ".tmp"
+        tmp = target + ".tmp"
         subprocess.check_call(
             ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
              "-I", include, "-I", sysconfig.get_paths()["include"], "-isystem", os.path.join(troot, "include"),
@@ -110,8 +114,8 @@ def build_binding(force: bool = False) -> str:
              "-isystem", os.path.join(cuda, "include"), src, "-o", tmp, "-L", HERE, "-lnvfp4_b200",
              "-L", os.path.join(troot, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda",
              "-Wl,-rpath,$ORIGIN", "-Wl,--no-as-needed"])
-        os.replace(tmp, BINDING)
-    return BINDING
+        os.replace(tmp, target)
+    return target
 
 
 def build_cpp_driver(force: bool = False) -> str:

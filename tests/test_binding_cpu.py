@@ -43,3 +43,21 @@ def test_truth_value_error():
     """A flag without a truth value is an error, not a false."""
     calls = ["native.quantize_new(x, None, np.zeros(2), True, False)", "native.quantize_new(x, None, True, np.zeros(2), False)"]
     assert errors(calls) == ["ValueError", "ValueError"]
+
+
+def test_binding_of_another_torch_or_python_is_another_file(pkg, monkeypatch):
+    """The file the package loads is the one the build makes, and neither is taken over from another torch or Python."""
+    import sysconfig
+
+    import torch
+
+    import __graft_entry__ as entry
+
+    script = entry._load_build_script()
+    assert script.binding_path() == pkg.BINDING_PATH
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "0.0.1")
+        assert script.binding_path() != pkg.BINDING_PATH
+    with monkeypatch.context() as m:
+        m.setattr(sysconfig, "get_config_var", lambda name: "cpython-00")
+        assert script.binding_path() != pkg.BINDING_PATH

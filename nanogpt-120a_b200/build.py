@@ -134,8 +134,21 @@ def build_cpp_driver(force: bool = False) -> str:
     return exe
 
 
+def build_exact_math(force: bool = False) -> str:
+    """Compiles tests/cpp/exact_math.cu (the quantizers' divisions against the operators) as the quantizers are compiled."""
+    root = os.path.abspath(os.path.join(HERE, ".."))
+    src = os.path.join(root, "tests", "cpp", "exact_math.cu")
+    out_dir = os.path.join(root, "tests", "cpp", "build")
+    exe = os.path.join(out_dir, "exact_math")
+    if force or _stale(exe, [src, os.path.join(CSRC, "common.cuh")]):
+        os.makedirs(out_dir, exist_ok=True)
+        subprocess.check_call([_nvcc(), *ARCH, *COMMON, "-fmad=false", "-I", CSRC, src, "-o", exe])
+    return exe
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
     print(build_step_library(force="--force" in sys.argv))
     print(build_binding(force="--force" in sys.argv))
     print(build_cpp_driver(force="--force" in sys.argv))
+    print(build_exact_math(force="--force" in sys.argv))

@@ -388,23 +388,6 @@ struct ScheduleFreeSource {
   }
 };
 
-// n / d for n < 2^32 by a multiplication (Granlund and Montgomery, "Division by invariant integers using
-// multiplication", 1994, figure 4.1): a 64-bit division per group cost a quarter of the quantizer.
-struct FastDiv {
-  uint32_t d, m, s1, s2;
-  explicit FastDiv(uint32_t divisor) : d(divisor) {
-    uint32_t l = 0;
-    while (l < 32 && (1ull << l) < divisor) ++l;
-    m = static_cast<uint32_t>(((1ull << 32) * ((1ull << l) - divisor)) / divisor + 1);
-    s1 = l < 1 ? l : 1;
-    s2 = l < 1 ? 0 : l - 1;
-  }
-  __device__ __forceinline__ uint32_t div(uint32_t n) const {
-    const uint32_t t = __umulhi(m, n);
-    return (t + ((n - t) >> s1)) >> s2;
-  }
-};
-
 // Scale bytes of four neighbouring lanes (one k-atom of a row) as one 32-bit store; every lane of the warp calls it.
 __device__ __forceinline__ void store_scale_quad(uint8_t* dst, uint32_t byte, bool first_of_four) {
   uint32_t word = byte | (__shfl_down_sync(0xffffffffu, byte, 1) << 8);

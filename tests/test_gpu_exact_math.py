@@ -1,0 +1,78 @@
+"""The quantizers' arithmetic at the ends of its straight-line range, and their index space beyond 2^32 groups."""
+import importlib.util
+import os
+import subprocess
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import ROOT
+from helpers import bf16_normal
+
+pytestmark = pytest.mark.gpu
+
+
+def cpu(t):
+    return t.detach().cpu().numpy()
+
+
+def test_divisions_equal_the_operators():
+    """Reciprocals of every float of the range, 3.4e10 quotients, every amax, index divisions: no bit differs."""
+    spec = importlib.util.spec_from_file_location("nvfp4_build_script", os.path.join(ROOT, "nanogpt-120a_b200", "build.py"))
+    script = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(script)
+    r = subprocess.run([script.build_exact_math()], capture_output=True, text=True, timeout=300)
+    lines = {k: (int(n), int(bad)) for k, n, bad in (line.split() for line in r.stdout.splitlines())}
+    assert set(lines) == {"reciprocals", "quotients", "amax_quotients", "index_quotients"}, (r.returncode, r.stderr)
+    assert r.returncode == 0 and all(bad == 0 for _, bad in lines.values()), lines
+    assert lines["reciprocals"][0] == 157 << 23 and lines["quotients"][0] == 1 << 35 and lines["amax_quotients"][0] > 160 << 23
+
+
+# 2^-80 and 2^80 times 1536, a step inside and outside, and amaxes far outside down to subnormal and up to the largest
+AMAX = [f * 1536.0 * s for s in (2.0 ** -80, 2.0 ** 80) for f in (1 - 2 ** -24, 1.0, 1 + 2 ** -23, 0.5, 1.37, 2.0)]
+AMAX += [2.0 ** -149, 2.0 ** -130, 1e-37, 1e-30, 1e25, 1e30, 3.0e38]
+
+
+@pytest.mark.parametrize("given", [False, True])
+@pytest.mark.parametrize("rowwise", [False, True])
+def test_four_six_at_the_ends_of_the_range(pkg, oracle, dev, rowwise, given):
+    q = pkg.Nvfp4QuantModule()
+    base = bf16_normal(721, (len(AMAX), 128)).float().numpy()
+    base /= np.abs(base).max(axis=1, keepdims=True)
+    with np.errstate(over="ignore", under="ignore"):
+        x = (base.astype(np.float64) * np.array(AMAX)[:, None]).astype(np.float32)
+    rows = [x] if rowwise else [r[None] for r in x]
+    for part in rows:
+        amax = oracle.row_amax(part) if rowwise else oracle.tensor_amax(part)[1]
+        t = q.quantize_four_six(torch.from_numpy(part).to(dev), torch.from_numpy(amax).to(dev) if given else None, rowwise=rowwise,
+                                packed=False)
+        ob, os_, og = oracle.four_six(part, amax, rowwise)
+        assert np.array_equal(cpu(t.bytes), ob) and np.array_equal(cpu(t.scales), os_) and np.array_equal(cpu(t.global_scales), og)
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -70, 2.0 ** 70])
+def test_four_six_amax_smaller_than_the_data(pkg, oracle, dev, scale):
+    """An amax that is not the data's: groups beyond 2^20 global scales leave the straight-line code."""
+    q = pkg.Nvfp4QuantModule()
+    x = (bf16_normal(722, (24, 64)).float().numpy() * np.float32(scale)).astype(np.float32)
+    amax = np.array([oracle.row_amax(x)[i] * 2.0 ** (4 - i) for i in range(24)], np.float32)
+    amax[0], amax[1] = 0.0, np.nan
+    t = q.quantize_four_six(torch.from_numpy(x).to(dev), torch.from_numpy(amax).to(dev), rowwise=True, packed=False)
+    ob, os_, og = oracle.four_six(x, amax, True)
+    assert np.array_equal(cpu(t.bytes), ob) and np.array_equal(cpu(t.scales), os_)
+    assert cpu(t.global_scales).tobytes() == og.tobytes() or np.array_equal(cpu(t.global_scales), og, equal_nan=True)
+
+
+def test_pad_rows_beyond_the_index_space(pkg, dev):
+    """One row so long that the groups of its 127 pad rows alone pass 2^32: the pad rows get a launch of their own."""
+    q = pkg.Nvfp4QuantModule()
+    cols = (0xFFF00000 // 128 + 4) // 4 * 64
+    x = torch.randn(1, 1 << 20, device=dev).to(torch.bfloat16).repeat(1, (cols >> 20) + 1)[:, :cols].contiguous()
+    amax = q.tensor_amax(x)[1]
+    logical = q.quantize_four_six(x, amax, packed=False)
+    packed = q.quantize_four_six(x, amax, packed=True)
+    assert torch.equal(logical.bytes, packed.bytes) and torch.equal(logical.global_scales, packed.global_scales)
+    atoms = packed.scales.view(-1, 512)
+    assert torch.equal(atoms[:, :4].reshape(-1), logical.scales)
+    assert bool((atoms[:, 4:] == 0x38).all())

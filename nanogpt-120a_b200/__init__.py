@@ -1003,11 +1003,6 @@ class LinearBackwardScratch:
         self.input_t_h = operand(input_dim, tk, token_count * input_dim)
         self.dims = (token_count, input_dim, output_dim)
 
-    @staticmethod
-    def _c(op) -> MsEdenOperand:
-        return MsEdenOperand(_ptr(op["bytes"]), _ptr(op["scales_packed"]), _ptr(op["global_scales"]),
-                             _ptr(op["global_scale"]), _ptr(op["chunk_amax"]))
-
     def as_tensor(self, name: str) -> Nvfp4Tensor:
         op = getattr(self, name)
         t, i, o = self.dims
@@ -1030,9 +1025,6 @@ class SideStream:
 
     def numbers(self):
         return self.stream.cuda_stream, self.fork.cuda_event, self.join.cuda_event
-
-    def handles(self):
-        return (c_void_p(self.stream.cuda_stream), c_void_p(self.fork.cuda_event), c_void_p(self.join.cuda_event))
 
 
 class LinearBackwardModule:

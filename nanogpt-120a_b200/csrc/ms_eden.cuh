@@ -218,61 +218,6 @@ __device__ __forceinline__ void ms_eden_emit_chunk(f32x2_t (&P)[16], const MsEde
   if (chunk_in_row == 0) o.global_scales[row] = gs;
 }
 
-// Two chunks at once, one per packed lane (low lane = chunk of row_lo, high lane = chunk of
-// row_hi, both at chunk_in_row): P[k] holds the signed inputs of K position k of both, so all
-// five butterfly strides act between registers.
-__device__ __forceinline__ void ms_eden_emit_chunk_lanes(f32x2_t (&P)[32], const MsEdenOut& o, float gs, float so,
-                                                         uint32_t row_lo, uint32_t row_hi, uint32_t chunk_in_row) {
-  const uint32_t chunks_per_row = o.dst_row_len >> 5;
-  const uint64_t chunk_lo = static_cast<uint64_t>(row_lo) * chunks_per_row + chunk_in_row;
-  const uint64_t chunk_hi = static_cast<uint64_t>(row_hi) * chunks_per_row + chunk_in_row;
-#pragma unroll
-  for (int stride = 1; stride < 32; stride <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      if ((i & stride) == 0) {
-        const f32x2_t a = P[i], b = P[i | stride];
-        P[i] = add2(a, b);
-        P[i | stride] = sub2(a, b);
-      }
-    }
-  }
-  const f32x2_t c = pack2(0.17677669f, 0.17677669f);
-#pragma unroll
-  for (int i = 0; i < 32; ++i) P[i] = mul2(P[i], c);
-  if (o.chunk_amax) {
-    float m_lo = 0.0f, m_hi = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-      float a0, a1, b0, b1;
-      unpack2(P[i], a0, a1);
-      unpack2(P[i + 1], b0, b1);
-      m_lo = max3_abs(m_lo, a0, b0);
-      m_hi = max3_abs(m_hi, a1, b1);
-    }
-    o.chunk_amax[chunk_lo] = m_lo;
-    o.chunk_amax[chunk_hi] = m_hi;
-  }
-  const float safe_gs = nz(gs);
-  const float inv6 = inv_scale(6.0f, safe_gs);
-  const uint32_t g_lo = row_lo * o.group_row_stride + chunk_in_row * 2u + o.group_offset;
-  const uint32_t g_hi = row_hi * o.group_row_stride + chunk_in_row * 2u + o.group_offset;
-  uint2 lo0, hi0, lo1, hi1;
-  const uint32_t sb0 = ms_eden_group_lanes(&P[0], safe_gs, so, inv6, o.scale_seed, g_lo, g_hi, lo0, hi0);
-  const uint32_t sb1 = ms_eden_group_lanes(&P[16], safe_gs, so, inv6, o.scale_seed, g_lo + 1, g_hi + 1, lo1, hi1);
-  *reinterpret_cast<uint4*>(o.fp4 + chunk_lo * 16) = make_uint4(lo0.x, lo0.y, lo1.x, lo1.y);
-  *reinterpret_cast<uint4*>(o.fp4 + chunk_hi * 16) = make_uint4(hi0.x, hi0.y, hi1.x, hi1.y);
-  const uint32_t k_atoms = o.dst_row_len >> 6;
-  const size_t off_lo = o.packed ? packed_scale_offset(row_lo, chunk_in_row * 2, k_atoms) : chunk_lo * 2;
-  const size_t off_hi = o.packed ? packed_scale_offset(row_hi, chunk_in_row * 2, k_atoms) : chunk_hi * 2;
-  *reinterpret_cast<uint16_t*>(o.scales + off_lo) = static_cast<uint16_t>((sb0 & 0xffu) | ((sb1 & 0xffu) << 8));
-  *reinterpret_cast<uint16_t*>(o.scales + off_hi) = static_cast<uint16_t>(((sb0 >> 8) & 0xffu) | (sb1 & 0xff00u));
-  if (chunk_in_row == 0) {
-    o.global_scales[row_lo] = gs;
-    o.global_scales[row_hi] = gs;
-  }
-}
-
 // Signed input pair (u[i], u[i+16]) from two values and the chunk's 32 sign bits.
 __device__ __forceinline__ f32x2_t signed_pair(float lo, float hi, uint32_t neg_mask, int i) {
   const uint32_t a = __float_as_uint(lo) ^ ((neg_mask << (31 - i)) & 0x80000000u);

@@ -97,6 +97,10 @@ struct Cfg {
   static_assert(kTmemSfa + kSfSets * kSfSetCols <= kTmemCols, "tensor memory overflow");
 };
 
+// How a sub-tile leaves: registers to memory (outputs a tensor map cannot describe, a bf16 residual), staging buffer and
+// TMA store, or the same added to the f32 residual stream.
+enum class StorePath { kDirect, kTma, kTmaResidual };
+
 struct GemmParams {
   const uint8_t* sfa;
   const uint8_t* sfb;
@@ -468,12 +472,14 @@ struct SubTile<__nv_bfloat16> {
 // Streaming mode: one B slot per pipeline stage.  Resident mode (short K): the whole
 // [kBlockN x K] B panel of the current column block stays in shared memory -- one slot per
 // k-tile -- while a CTA walks down the row blocks, so only A tiles stream through the ring.
-template <int kBlockM, int kBlockN, typename OutT, bool kTmaStore>
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore>
 __global__ void __launch_bounds__(kThreads, 1)
     nvfp4_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                               const __grid_constant__ CUtensorMap tmap_out,
                               const __grid_constant__ CUtensorMap tmap_aux, const GemmParams p) {
   using C = Cfg<kBlockM, kBlockN>;
+  constexpr bool kTmaStore = kStore != StorePath::kDirect, kResidual = kStore == StorePath::kTmaResidual;
+  static_assert(!kResidual || sizeof(OutT) == 4, "the residual stream of the TMA path is f32");
   constexpr int kMHalves = C::kMHalves;
   constexpr int kAStageBytes = C::kAStageBytes;
   constexpr int kSfaStageBytes = C::kSfaStageBytes;
@@ -614,10 +620,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   // word names the role whose input failed to come
   const uint64_t downstream_timeout_ns = 2 * p.wait_timeout_ns;
   // a ReLU^2 with its pre-activation kept stores every item twice: the pre-activation, then the activation
-  const int item_passes = (p.epilogue == NVFP4_EPI_RELU2 && p.aux) ? 2 : 1;
-  // The f32 residual stream: an item's old values arrive in the staging buffer the item will leave from, `stored` of a
-  // buffer then means that they are there, and the epilogue adds to them in place.
-  const bool residual = kTmaStore && sizeof(OutT) == 4 && p.epilogue == NVFP4_EPI_RESIDUAL;
+  const int item_passes = (!kResidual && p.epilogue == NVFP4_EPI_RELU2 && p.aux) ? 2 : 1;
+  // kResidual, the f32 residual stream: an item's old values arrive in the staging buffer the item will leave from,
+  // `stored` of a buffer then means that they are there, and the epilogue adds to them in place.
 
   if (warp == 0) {
     // ===================== TMA producer =====================
@@ -956,12 +961,12 @@ __global__ void __launch_bounds__(kThreads, 1)
           return;
         }
       };
-      if (residual)
+      if (kResidual)
         for (uint32_t b = 0; b < kRing; ++b) load_next(eg * kRing + b);
       for (uint32_t w = w_begin; w < w_end && ok; w += w_step, ++tile_iter) {
         uint32_t m_blk, n_blk, split;
         decode(w, m_blk, n_blk, split);
-        if (residual) {
+        if (kResidual) {
           // The items of this tile that no buffer is free for yet go to L2 during its main loop, spread over it: all at
           // once they would stand before the operands in the queue to HBM.  8192 x 768 x K 3072 from HBM: 27.2 us without,
           // 27.5 all at once, 23.4 spread; from L2 20.2.
@@ -986,14 +991,14 @@ __global__ void __launch_bounds__(kThreads, 1)
               break;
             }
             const CUtensorMap* map = item_passes == 2 && pass == 0 ? &tmap_aux : &tmap_out;
-            if (p.k_splits > 1)
+            if (!kResidual && p.k_splits > 1)
               tma_reduce_add_2d(map, smem_store + slot * kStoreStageBytes, x, y);
             else
               tma_store_2d(map, smem_store + slot * kStoreStageBytes, x, y);
             bulk_commit_group();
             // the buffer the epilogue needs next is handed back as soon as its store has read it: this one with a
             // single buffer, the previous one with two; with a load to come into it, this one at once
-            if (residual) {
+            if (kResidual) {
               bulk_wait_group_read<0>();
               load_next(slot);
             } else {
@@ -1012,7 +1017,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       bulk_wait_group0();  // stores complete before the CTA exits
-      if (!ok && residual) {
+      if (kResidual && !ok) {
         // aborting: give loads already in flight a bounded chance to land; load j is phase j / kRing of its buffer
         for (uint32_t j = loads > kRing ? loads - kRing : 0; j < loads; ++j)
           for (int spin = 0; spin < 4096 && !mbar_try_wait(bar_stored + 8 * (eg * kRing + j % kRing), (j / kRing) & 1u); ++spin) {
@@ -1027,7 +1032,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     [[maybe_unused]] const bool elected = gtid == 0;
     OutT* out = static_cast<OutT*>(p.out);
     OutT* aux = static_cast<OutT*>(p.aux);
-    uint32_t acc = 0, acc_phase = 0, store_buf = 0, store_phase = residual ? 0u : 1u, tile_iter = 0;
+    uint32_t acc = 0, acc_phase = 0, store_buf = 0, store_phase = kResidual ? 0u : 1u, tile_iter = 0;
     bool ok = true;  // warp uniform; false: some wait ran out, the rest of the list is walked without work
     const uint32_t my_bias = smem_bias + eg * kBlockN * 4;
     const float* my_bias_gen = reinterpret_cast<const float*>(smem_gen + (my_bias - smem_base));
@@ -1151,7 +1156,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             tcgen05_wait_ld();
             GEMM_TRACE(3 + eg, 32, elected);
             if (item == last_item) release_accumulator();  // the group's last read of this tile
-            if (residual) {
+            if (kResidual) {
               // the roundings of the direct path: the product, the sum with the bias, then the one with the stream
 #pragma unroll
               for (int i = 0; i < kSub; i += 4) {
@@ -1212,9 +1217,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             ok = __all_sync(0xffffffffu, ok);
             GEMM_TRACE(3 + eg, 36, elected);
             if (ok) {
-              if constexpr (sizeof(OutT) == 4) {
-                if (residual) add_staged_row(smem_store + slot * kStoreStageBytes + gtid * 128, gtid, v);
-              }
+              if constexpr (kResidual) add_staged_row(smem_store + slot * kStoreStageBytes + gtid * 128, gtid, v);
               SubTile<OutT>::stage(smem_store + slot * kStoreStageBytes + gtid * 128, gtid, v);
               fence_proxy_async_smem();
               __syncwarp();
@@ -1460,7 +1463,7 @@ TileBytes tile_bytes(uint32_t block_m, uint32_t block_n) {
   return block_n == 256 ? tile_bytes_of<128, 256>() : block_n == 192 ? tile_bytes_of<128, 192>() : tile_bytes_of<128, 128>();
 }
 
-template <int kBlockM, int kBlockN, typename OutT, bool kTmaStore>
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore>
 int launch_store_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo,
                          const CUtensorMap& mx, const GemmParams& p, const GemmPlan& pl) {
   // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
@@ -1469,7 +1472,7 @@ int launch_store_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMa
   if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
   int st = attr_state[dev].load(std::memory_order_acquire);
   if (st == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kTmaStore>,
+    const cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
     st = e == cudaSuccess ? 1 : -static_cast<int>(e);
     attr_state[dev].store(st, std::memory_order_release);
@@ -1498,21 +1501,25 @@ int launch_store_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMa
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int rc = static_cast<int>(
-      cudaLaunchKernelEx(&cfg, nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kTmaStore>, ma, mb, mo, mx, p));
+      cudaLaunchKernelEx(&cfg, nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore>, ma, mb, mo, mx, p));
   count_launch();
   if (rc == 0) rc = static_cast<int>(cudaGetLastError());
   if (rec) cudaEventRecord(rec->stop, s);
   return rc;
 }
 
-// The store path is a compile-time property of the kernel (TMA stores through the staging ring, or direct
-// stores for outputs a tensor map cannot describe and for a bf16 residual): each variant
-// carries only its own epilogue code.
+// The store path is a compile-time property of the kernel: each variant carries only its own epilogue code.  Deciding for
+// the residual stream at run time inside the f32 TMA variant cost the others their registers: 1000 tokens x 768 -> 32000,
+// f32 out, 41.0 -> 42.7 us.
 template <int kBlockM, int kBlockN, typename OutT>
 int launch_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo,
                    const CUtensorMap& mx, const GemmParams& p, const GemmPlan& pl) {
-  return p.tma_store ? launch_store_variant<kBlockM, kBlockN, OutT, true>(s, ma, mb, mo, mx, p, pl)
-                     : launch_store_variant<kBlockM, kBlockN, OutT, false>(s, ma, mb, mo, mx, p, pl);
+  if (!p.tma_store) return launch_store_variant<kBlockM, kBlockN, OutT, StorePath::kDirect>(s, ma, mb, mo, mx, p, pl);
+  if constexpr (sizeof(OutT) == 4) {
+    if (p.epilogue == NVFP4_EPI_RESIDUAL)
+      return launch_store_variant<kBlockM, kBlockN, OutT, StorePath::kTmaResidual>(s, ma, mb, mo, mx, p, pl);
+  }
+  return launch_store_variant<kBlockM, kBlockN, OutT, StorePath::kTma>(s, ma, mb, mo, mx, p, pl);
 }
 
 std::atomic<int> g_tile_override{-1};  // -1 = read NVFP4_GEMM_TILE once, 0 = automatic, else (block_m << 16) | block_n

@@ -2,10 +2,11 @@
 // read of it, and the transposed operand of an NVFP4 matrix (X^T, W^T).
 //
 // Same bytes as the generic kernels of quant_kernels.cu (one thread per 32-chunk, utils/nvfp4/quant/kernels/
-// ms_eden/**), organised for what bounds them.  On B200 these kernels are bound by instruction dispatch and
-// register-file reads, not by HBM: measured costs per warp instruction and scheduler are 1 cycle for scalar FP32 (mixed
-// f32 += bf16 * bf16 included), 2 for the packed f32x2 forms with distinct operands and for every integer, logic and
-// conversion instruction and cvt.f32.f16, and the costs of different pipes add up almost fully.  So:
+// ms_eden/**), organised for the rate at which instructions issue: the schedulers issue on 58 % of the cycles, the FMA pipe
+// is busy 52 % of them and the ALU 39 %, HBM 22 %.  Measured costs per warp instruction and scheduler are 1 cycle for scalar
+// FP32 (mixed f32 += bf16 * bf16 included), 2 for the packed f32x2 forms with distinct operands and for every integer, logic
+// and conversion instruction and cvt.f32.f16, and the costs of different pipes add up almost fully.  The counters fit that;
+// whether latency holds a part of the idle slots (16 warps per SM, a barrier per tile) is not settled.  So:
 //  * a bf16 source is widened, sign-flipped and taken through the first butterfly stage by mixed-precision FMAs,
 //    x * (+-1) + u (exact product, one rounding), or for the upper half of a word by one logic instruction;
 //  * the lower E2M1 code of a byte is widened with add.f32.f16 instead of cvt.f32.f16;

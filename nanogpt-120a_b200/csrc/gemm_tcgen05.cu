@@ -555,7 +555,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     tcgen05_fence_before();
   }
   // Programmatic dependent launch: up to here the CTA has touched only its own SM.  Whatever runs before it in the stream
-  // is complete and visible beyond this point.
+  // is complete and visible beyond this point.  The GEMM itself does not allow the next kernel to start early: its CTAs end
+  // at different times, and the first SMs that come free would take all of a small grid's CTAs.
   wait_for_prior_kernels();
   __syncthreads();
   tcgen05_fence_after();

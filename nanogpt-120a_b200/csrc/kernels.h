@@ -95,4 +95,26 @@ void set_last_error(const char* msg);
 // Host-side tally of kernel launches made by this library (read through nvfp4_launch_count).
 void count_launch();
 
+// Launches a kernel that may start while the kernel before it in the stream drains (programmatic stream serialization).
+// Only for kernels whose every thread waits for that one before its first access to memory
+// (wait_for_prior_then_allow_next): launch latency and the start of the thread blocks then cost nothing behind another
+// kernel.
+template <typename... Params, typename... Args>
+int launch_chained(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t shared_bytes, cudaStream_t s, const Args&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = shared_bytes;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t launched = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  count_launch();
+  const cudaError_t last = cudaGetLastError();
+  return static_cast<int>(launched != cudaSuccess ? launched : last);
+}
+
 }  // namespace nvfp4

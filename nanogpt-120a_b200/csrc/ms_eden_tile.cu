@@ -307,8 +307,8 @@ __device__ __forceinline__ void fill_inv_table(float2* table, float safe_gs) {
 }
 
 __device__ __forceinline__ float tile_global_scale(const MsEdenTileParams& p) {
-  if (!p.amax_in) return p.use_host_scale ? p.global_scale_host : p.global_scale_dev[0];
-  const float gs = ms_eden_scale_of_amax(p.amax_in[0]);
+  if (!p.amax_in) return p.use_host_scale ? p.global_scale_host : after_prior(p.global_scale_dev)[0];
+  const float gs = ms_eden_scale_of_amax(after_prior(p.amax_in)[0]);
   if (blockIdx.x == 0 && threadIdx.x == 0) p.gs_out[0] = gs;
   return gs;
 }
@@ -335,7 +335,7 @@ struct PairTile {
 template <typename T, bool kColSum, bool kEdge>
 __global__ void __launch_bounds__(256, 2)
     ms_eden_pair_kernel(const __grid_constant__ MsEdenTileParams p, uint32_t tiles_x, uint32_t tile_count) {
-  allow_next_kernel();
+  wait_for_prior_then_allow_next();
   using PT = PairTile<T>;
   constexpr bool kBf16 = PT::kBf16;
   constexpr uint32_t kSize = sizeof(T);
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256, 2)
   __shared__ uint32_t slow_count;      // threads of this tile whose chunks need the generic code, and which
   __shared__ uint8_t slow_list[256];
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const T* x = static_cast<const T*>(p.x);
+  const T* x = after_prior(static_cast<const T*>(p.x));
   const float gs = tile_global_scale(p), safe_gs = nz(gs);
   fill_inv_table(inv_table, safe_gs);
   const float inv6 = inv_scale(6.0f, safe_gs);
@@ -561,7 +561,10 @@ constexpr int kNvPitch = kTileCols * 4 + 16;
 template <bool kRowwise, bool kEdge>
 __global__ void __launch_bounds__(128, 4)
     ms_eden_nvfp4_transpose_kernel(const __grid_constant__ MsEdenTileParams p, uint32_t tiles_x, uint32_t tile_count) {
-  allow_next_kernel();
+  wait_for_prior_then_allow_next();
+  const uint8_t* const src_bytes = after_prior(p.src_bytes);
+  const uint8_t* const src_scales = after_prior(p.src_scales);
+  const float* const src_global = after_prior(p.src_global);
   __shared__ __align__(16) uint8_t nv_stage[kTileRows * kNvPitch];
   __shared__ float2 inv_table[kScaleCodes];
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -569,7 +572,7 @@ __global__ void __launch_bounds__(128, 4)
   fill_inv_table(inv_table, safe_gs);
   const float inv6 = inv_scale(6.0f, safe_gs);
   const uint32_t table = static_cast<uint32_t>(__cvta_generic_to_shared(inv_table));
-  const float tensor_global = kRowwise ? 0.0f : p.src_global[0];
+  const float tensor_global = kRowwise ? 0.0f : src_global[0];
   // this thread's chunks: columns 2 * lane and 2 * lane + 1, rows 32 * warp ... of the tile
   const ChunkOffsets at = chunk_offsets(p.t, 2 * lane, warp);
   const ChunkOffsets row_step = {(p.t.dst_row_len >> 5) * 16, p.t.packed ? 16u : (p.t.dst_row_len >> 5) * 2, p.t.group_row_stride};
@@ -584,15 +587,15 @@ __global__ void __launch_bounds__(128, 4)
     raw_scales = 0;
     raw_global = kRowwise ? 1.0f : tensor_global;
     if (!kEdge || r < p.src_rows) {
-      if (kRowwise) raw_global = __ldg(p.src_global + r);
+      if (kRowwise) raw_global = __ldg(src_global + r);
 #pragma unroll
       for (uint32_t h = 0; h < 2; ++h) {
         const uint32_t c = tx * kTileCols + 32 * h;
         if (!kEdge || c < p.src_cols) {  // columns come in whole 32s
           const size_t index = static_cast<size_t>(r) * p.src_cols + c;
-          raw[h] = __ldg(reinterpret_cast<const uint4*>(p.src_bytes + (index >> 1)));
+          raw[h] = __ldg(reinterpret_cast<const uint4*>(src_bytes + (index >> 1)));
           const size_t sidx = p.src_packed ? packed_scale_offset(r, c >> 4, p.src_cols >> 6) : index >> 4;
-          raw_scales |= static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(p.src_scales + sidx))) << (16 * h);
+          raw_scales |= static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(src_scales + sidx))) << (16 * h);
         }
       }
     }
@@ -699,9 +702,8 @@ int launch_pair(cudaStream_t s, const MsEdenTileParams& p) {
   const uint32_t tiles_x = (p.src_cols + kTileCols - 1) / kTileCols;
   const uint32_t tiles = tiles_x * ((p.src_rows + kTileRows - 1) / kTileRows);
   const uint32_t resident = 148u * 2u;
-  ms_eden_pair_kernel<T, kColSum, kEdge><<<tiles < resident ? tiles : resident, 256, kStage, s>>>(p, tiles_x, tiles);
-  count_launch();
-  return static_cast<int>(cudaGetLastError());
+  return launch_chained(ms_eden_pair_kernel<T, kColSum, kEdge>, tiles < resident ? tiles : resident, 256, kStage, s, p, tiles_x,
+                        tiles);
 }
 
 template <typename T>
@@ -731,10 +733,8 @@ static int launch_nvfp4(cudaStream_t s, const MsEdenTileParams& p) {
   const uint32_t tiles_x = (p.src_cols + kTileCols - 1) / kTileCols;
   const uint32_t tiles = tiles_x * ((p.src_rows + kTileRows - 1) / kTileRows);
   const uint32_t resident = 148u * 4u;
-  ms_eden_nvfp4_transpose_kernel<kRowwise, kEdge>
-      <<<tiles < resident ? tiles : resident, 128, 0, s>>>(p, tiles_x, tiles);
-  count_launch();
-  return static_cast<int>(cudaGetLastError());
+  return launch_chained(ms_eden_nvfp4_transpose_kernel<kRowwise, kEdge>, tiles < resident ? tiles : resident, 128, 0, s, p,
+                        tiles_x, tiles);
 }
 int launch_ms_eden_nvfp4_tiles(cudaStream_t s, const MsEdenTileParams& p, bool rowwise) {
   const bool edge = p.src_rows % 128 != 0 || p.src_cols % 128 != 0 || p.t.dst_row_len != p.src_rows;

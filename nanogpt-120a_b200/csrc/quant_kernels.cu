@@ -66,6 +66,8 @@ __device__ __forceinline__ float warp_max(float v) {
 template <typename T>
 __global__ void __launch_bounds__(256) row_amax_kernel(const T* __restrict__ x, float* __restrict__ out,
                                                         uint32_t rows, uint32_t row_len) {
+  wait_for_prior_then_allow_next();
+  x = after_prior(x);
   const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5);
   const uint32_t lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -152,6 +154,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) tensor_amax_kernel(const T* __restrict__ x, float* __restrict__ chunk_amax,
                                                            float* __restrict__ out, float* __restrict__ partials,
                                                            uint64_t n) {
+  wait_for_prior_then_allow_next();
+  x = after_prior(x);
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t warps = static_cast<uint64_t>(gridDim.x) * 8;
   const uint64_t chunks = (n + 1023) / 1024;
@@ -181,6 +185,10 @@ __global__ void __launch_bounds__(256) nvfp4_amax_kernel(const uint8_t* __restri
                                                           const float* __restrict__ gscales, uint64_t n, uint32_t cols,
                                                           int rowwise, int packed, float* __restrict__ chunk_amax,
                                                           float* __restrict__ out) {
+  wait_for_prior_then_allow_next();
+  bytes = after_prior(bytes);
+  scales = after_prior(scales);
+  gscales = after_prior(gscales);
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t warps = static_cast<uint64_t>(gridDim.x) * 8;
   const uint64_t chunks = (n + 1023) / 1024;
@@ -216,6 +224,8 @@ __global__ void __launch_bounds__(256) nvfp4_amax_kernel(const uint8_t* __restri
 __global__ void __launch_bounds__(256) amax_from_chunks_kernel(const float* __restrict__ chunk_amax,
                                                                 float* __restrict__ out, uint32_t chunk_count,
                                                                 int transform) {
+  wait_for_prior_then_allow_next();
+  chunk_amax = after_prior(chunk_amax);
   __shared__ float partial[8];
   float m = 0.0f;
   for (uint32_t i = threadIdx.x; i < chunk_count; i += 256) m = max_f32(m, chunk_amax[i]);
@@ -236,6 +246,8 @@ __global__ void __launch_bounds__(256) amax_from_chunks_kernel(const float* __re
 
 // out[0] = MS-EDEN global scale of amax[0] (single thread).
 __global__ void ms_eden_scale_from_amax_kernel(const float* __restrict__ amax, float* __restrict__ out) {
+  wait_for_prior_then_allow_next();
+  amax = after_prior(amax);
   out[0] = ms_eden_scale_of_amax(amax[0]);
 }
 
@@ -363,6 +375,7 @@ __device__ __forceinline__ float group_amax16(const float (&v)[16]) {
 template <typename T, bool kRelu2>
 struct TensorSource {
   const T* x;
+  __device__ __forceinline__ void pin_loads() { x = after_prior(x); }
   __device__ __forceinline__ void load16(size_t group, float (&v)[16]) const {
     Load16<T>::run(x + group * 16, v);
     if (kRelu2) {
@@ -379,6 +392,10 @@ struct ScheduleFreeSource {
   const float* z;
   const float* x;
   float beta;
+  __device__ __forceinline__ void pin_loads() {
+    z = after_prior(z);
+    x = after_prior(x);
+  }
   __device__ __forceinline__ void load16(size_t group, float (&v)[16]) const {
     float zv[16], xv[16];
     Load16<float>::run(z + group * 16, zv);
@@ -416,11 +433,13 @@ __device__ __forceinline__ float cta_max_of(const float* partials, uint32_t coun
 // Measured, 8192 x 768 bf16 with a tensor scale: 8.5 -> 5.4 us (HBM allows 2.5).
 template <typename Source, bool kRowwise, bool kPacked, bool kQuads>
 __global__ void __launch_bounds__(256, 4)
-    four_six_kernel(const Source src, const float* __restrict__ amax, uint32_t amax_count, float* __restrict__ out_amax,
+    four_six_kernel(Source src, const float* __restrict__ amax, uint32_t amax_count, float* __restrict__ out_amax,
                     uint8_t* __restrict__ out_fp4, uint8_t* __restrict__ out_scales, float* __restrict__ out_gs,
                     float* __restrict__ decoded_amax, uint32_t rows, uint32_t groups, const FastDiv groups_per_row,
                     uint32_t opaque_zero) {
-  allow_next_kernel();
+  wait_for_prior_then_allow_next();
+  src.pin_loads();
+  amax = after_prior(amax);
   float dec = 0.0f;
   float tensor_amax = 0.0f;
   if (!kRowwise) {
@@ -513,7 +532,8 @@ __global__ void __launch_bounds__(256, 3)
                             float* __restrict__ out_gs, float* __restrict__ out_amax, float* __restrict__ decoded_amax,
                             uint32_t rows, uint32_t padded_rows, uint32_t groups_per_row, uint32_t rows_per_cta,
                             uint32_t row_blocks, uint32_t opaque_zero) {
-  allow_next_kernel();
+  wait_for_prior_then_allow_next();
+  x = after_prior(x);
   __shared__ unsigned int row_amax_bits[3][kStreamMaxRowsPerCta];
   const uint32_t t = threadIdx.x, lane_id = t & 31u;
   for (uint32_t i = t; i < 3 * rows_per_cta; i += blockDim.x) row_amax_bits[i / rows_per_cta][i % rows_per_cta] = 0u;
@@ -611,6 +631,9 @@ __global__ void __launch_bounds__(256) schedule_free_amax_kernel(const float* __
                                                                   const float* __restrict__ x,
                                                                   float* __restrict__ chunk_amax, float* __restrict__ out,
                                                                   float* __restrict__ partials, float beta, uint64_t n) {
+  wait_for_prior_then_allow_next();
+  z = after_prior(z);
+  x = after_prior(x);
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t warps = static_cast<uint64_t>(gridDim.x) * 8;
   const uint64_t chunks = (n + 1023) / 1024;
@@ -755,7 +778,7 @@ constexpr int kTileRows = 128, kTileCols = 64, kTileLd = kTileCols + 1;
 
 template <int kSrc, typename T, bool kPair>
 __global__ void __launch_bounds__(256) ms_eden_tile_kernel(const MsEdenTileParams p) {
-  allow_next_kernel();
+  wait_for_prior_then_allow_next();
   __shared__ float tile[kTileRows * kTileLd];
   __shared__ uint32_t neg_r[kTileRows / 32];  // sign bits of the tile's rows (K of the transposed operand)
   __shared__ uint32_t neg_c[kTileCols / 32];  // sign bits of the tile's columns (K of the row operand)
@@ -1006,6 +1029,10 @@ __global__ void __launch_bounds__(256) decode_kernel(const uint8_t* __restrict__
 __global__ void __launch_bounds__(256) decode_rows_kernel(const uint8_t* __restrict__ bytes, const uint8_t* __restrict__ scales,
                                                            const float* __restrict__ gscales, float* __restrict__ out,
                                                            uint32_t octets, const FastDiv octets_per_row, int rowwise) {
+  wait_for_prior_then_allow_next();
+  bytes = after_prior(bytes);
+  scales = after_prior(scales);
+  gscales = after_prior(gscales);
   const float tensor_gs = rowwise ? 0.0f : gscales[0];
   for (uint32_t i0 = blockIdx.x * 1024u + threadIdx.x; i0 < octets; i0 += gridDim.x * 1024u) {
     uint32_t word[4], sc[4];
@@ -1049,10 +1076,10 @@ struct ScalePlane {
   uint32_t mn, row_blocks;
 };
 __global__ void __launch_bounds__(256) scale_pack_tiles_kernel(const ScalePlane first, const ScalePlane second, uint32_t k_atoms) {
-  allow_next_kernel();
+  wait_for_prior_then_allow_next();
   __shared__ uint32_t words[128][17];
   const bool is_first = blockIdx.y < first.row_blocks;
-  const uint8_t* const logical = is_first ? first.logical : second.logical;
+  const uint8_t* const logical = after_prior(is_first ? first.logical : second.logical);
   uint8_t* const packed = is_first ? first.packed : second.packed;
   const uint32_t mn = is_first ? first.mn : second.mn, row_block = is_first ? blockIdx.y : blockIdx.y - first.row_blocks;
   const uint32_t atom0 = blockIdx.x * 16u, row0 = row_block * 128u;
@@ -1179,7 +1206,8 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const T* __restrict__ e,
 // column each add tiles lane, lane+8, ... in sequence, then the lane sums are added 0..7.
 __global__ void __launch_bounds__(256) col_sum_reduce_kernel(const float* __restrict__ partials,
                                                               float* __restrict__ dbias, uint32_t tiles, uint32_t n) {
-  allow_next_kernel();
+  wait_for_prior_then_allow_next();
+  partials = after_prior(partials);
   __shared__ float sums[256];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t c = blockIdx.x * 32 + lane;
@@ -1225,11 +1253,9 @@ static inline uint32_t blocks_for(uint64_t n, uint32_t per_block, uint32_t cap =
 int launch_row_amax(cudaStream_t s, const void* x, int dtype, float* out, uint32_t rows, uint32_t row_len) {
   if (rows == 0) return 0;
   if (dtype == 0)
-    row_amax_kernel<float><<<blocks_for(rows, 8), 256, 0, s>>>(static_cast<const float*>(x), out, rows, row_len);
-  else
-    row_amax_kernel<__nv_bfloat16>
-        <<<blocks_for(rows, 8), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), out, rows, row_len);
-  NVFP4_RETURN_LAST();
+    return launch_chained(row_amax_kernel<float>, blocks_for(rows, 8), 256, 0, s, static_cast<const float*>(x), out, rows, row_len);
+  return launch_chained(row_amax_kernel<__nv_bfloat16>, blocks_for(rows, 8), 256, 0, s, static_cast<const __nv_bfloat16*>(x), out,
+                        rows, row_len);
 }
 
 uint32_t tensor_amax_partials(uint64_t n) { return blocks_for((n + 1023) / 1024, 8, kAmaxPartials); }
@@ -1242,10 +1268,9 @@ int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_am
   }
   const uint32_t grid = partials ? tensor_amax_partials(n) : blocks_for((n + 1023) / 1024, 8, 148 * 8);
   if (dtype == 0)
-    tensor_amax_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float*>(x), chunk_amax, out, partials, n);
-  else
-    tensor_amax_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), chunk_amax, out, partials, n);
-  NVFP4_RETURN_LAST();
+    return launch_chained(tensor_amax_kernel<float>, grid, 256, 0, s, static_cast<const float*>(x), chunk_amax, out, partials, n);
+  return launch_chained(tensor_amax_kernel<__nv_bfloat16>, grid, 256, 0, s, static_cast<const __nv_bfloat16*>(x), chunk_amax, out,
+                        partials, n);
 }
 
 int launch_nvfp4_amax(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, const float* gscales, uint32_t rows,
@@ -1254,19 +1279,16 @@ int launch_nvfp4_amax(cudaStream_t s, const uint8_t* bytes, const uint8_t* scale
   cudaError_t err = cudaMemsetAsync(out, 0, sizeof(float), s);
   if (err != cudaSuccess) return static_cast<int>(err);
   if (n == 0) return 0;
-  nvfp4_amax_kernel<<<blocks_for((n + 1023) / 1024, 8, 148 * 8), 256, 0, s>>>(bytes, scales, gscales, n, cols, rowwise, packed,
-                                                                     chunk_amax, out);
-  NVFP4_RETURN_LAST();
+  return launch_chained(nvfp4_amax_kernel, blocks_for((n + 1023) / 1024, 8, 148 * 8), 256, 0, s, bytes, scales, gscales, n, cols,
+                        rowwise, packed, chunk_amax, out);
 }
 
 int launch_amax_from_chunks(cudaStream_t s, const float* chunk_amax, float* out, uint32_t chunk_count, int transform) {
-  amax_from_chunks_kernel<<<1, 256, 0, s>>>(chunk_amax, out, chunk_count, transform);
-  NVFP4_RETURN_LAST();
+  return launch_chained(amax_from_chunks_kernel, 1, 256, 0, s, chunk_amax, out, chunk_count, transform);
 }
 
 int launch_ms_eden_scale_from_amax(cudaStream_t s, const float* amax, float* out) {
-  ms_eden_scale_from_amax_kernel<<<1, 1, 0, s>>>(amax, out);
-  NVFP4_RETURN_LAST();
+  return launch_chained(ms_eden_scale_from_amax_kernel, 1, 1, 0, s, amax, out);
 }
 
 // Groups of one launch stay below 2^32 (32-bit index space): larger tensors go in slabs of whole 128-row blocks.
@@ -1309,9 +1331,10 @@ static int launch_four_six_source(cudaStream_t s, const Source& src, const float
   const uint32_t grid = blocks_for(groups, 256, 148u * 4u);
   const bool quads = gpr % 4 == 0 && (reinterpret_cast<uintptr_t>(out_scales) & 3u) == 0;
   const FastDiv div(gpr);
+  int rc;
 #define NVFP4_LAUNCH_FS(R, P, Q)                                                                                          \
-  four_six_kernel<Source, R, P, Q><<<grid, 256, 0, s>>>(src, amax, amax_count, out_amax, out_fp4, out_scales, out_gs,      \
-                                                        decoded_amax, rows, groups, div, 0u)
+  rc = launch_chained(four_six_kernel<Source, R, P, Q>, grid, 256, 0, s, src, amax, amax_count, out_amax, out_fp4,         \
+                      out_scales, out_gs, decoded_amax, rows, groups, div, 0u)
   if (rowwise) {
     if (packed) { if (quads) NVFP4_LAUNCH_FS(true, true, true); else NVFP4_LAUNCH_FS(true, true, false); }
     else { if (quads) NVFP4_LAUNCH_FS(true, false, true); else NVFP4_LAUNCH_FS(true, false, false); }
@@ -1320,8 +1343,6 @@ static int launch_four_six_source(cudaStream_t s, const Source& src, const float
     else { if (quads) NVFP4_LAUNCH_FS(false, false, true); else NVFP4_LAUNCH_FS(false, false, false); }
   }
 #undef NVFP4_LAUNCH_FS
-  count_launch();
-  const int rc = static_cast<int>(cudaGetLastError());
   return rc == 0 && pad_apart ? launch_packed_scale_pad(s, out_scales, rows, cols) : rc;
 }
 
@@ -1362,9 +1383,8 @@ int launch_four_six_rowwise_fused(cudaStream_t s, const void* x, int dtype, uint
   const uint32_t per_cta = (row_blocks + resident - 1) / resident;
   const uint32_t grid = (row_blocks + per_cta - 1) / per_cta;
 #define NVFP4_LAUNCH_FUSED(T, P, R)                                                                                   \
-  four_six_rowwise_kernel<T, P, R><<<grid, threads, 0, s>>>(static_cast<const T*>(x), out_fp4, out_scales, out_gs,     \
-                                                            out_amax, decoded_amax, rows, padded_rows, gpr, rpc,       \
-                                                            row_blocks, 0u)
+  return launch_chained(four_six_rowwise_kernel<T, P, R>, grid, threads, 0, s, static_cast<const T*>(x), out_fp4,      \
+                        out_scales, out_gs, out_amax, decoded_amax, rows, padded_rows, gpr, rpc, row_blocks, 0u)
 #define NVFP4_LAUNCH_FUSED_R(T, P)       \
   do {                                   \
     if (relu2) NVFP4_LAUNCH_FUSED(T, P, true); \
@@ -1379,7 +1399,6 @@ int launch_four_six_rowwise_fused(cudaStream_t s, const void* x, int dtype, uint
   }
 #undef NVFP4_LAUNCH_FUSED_R
 #undef NVFP4_LAUNCH_FUSED
-  NVFP4_RETURN_LAST();
 }
 
 int launch_schedule_free_materialize(cudaStream_t s, const float* z, const float* x, float beta, float* chunk_amax,
@@ -1392,9 +1411,7 @@ int launch_schedule_free_materialize(cudaStream_t s, const float* z, const float
     if (n == 0) return 0;
   }
   const uint32_t grid = partials ? tensor_amax_partials(n) : blocks_for((n + 1023) / 1024, 8, 148 * 8);
-  schedule_free_amax_kernel<<<grid, 256, 0, s>>>(z, x, chunk_amax, amax, partials, beta, n);
-  count_launch();
-  const int rc = static_cast<int>(cudaGetLastError());
+  const int rc = launch_chained(schedule_free_amax_kernel, grid, 256, 0, s, z, x, chunk_amax, amax, partials, beta, n);
   if (rc) return rc;
   return launch_four_six_source(s, ScheduleFreeSource{z, x, beta}, partials ? partials : amax, partials ? grid : 1u,
                                 partials ? amax : nullptr, 0, rows, cols, out_fp4, out_scales, packed, out_gs, nullptr);
@@ -1561,8 +1578,7 @@ bool ms_eden_pair_is_tiled(const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_args
 
 int launch_col_sum_reduce(cudaStream_t s, const float* partials, float* dbias, uint32_t tiles, uint32_t n) {
   if (n == 0) return 0;
-  col_sum_reduce_kernel<<<blocks_for(n, 32), 256, 0, s>>>(partials, dbias, tiles, n);
-  NVFP4_RETURN_LAST();
+  return launch_chained(col_sum_reduce_kernel, blocks_for(n, 32), 256, 0, s, partials, dbias, tiles, n);
 }
 
 bool ms_eden_pair_takes_amax(const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_args& t) {
@@ -1647,11 +1663,10 @@ int launch_decode(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, c
   if (!transpose && cols % 16 == 0 && n / 8 < 0xff000000ull && (reinterpret_cast<uintptr_t>(bytes) & 3u) == 0 &&
       (reinterpret_cast<uintptr_t>(out) & 31u) == 0) {
     const uint32_t octets = static_cast<uint32_t>(n / 8);
-    decode_rows_kernel<<<blocks_for(octets, 1024, 148u * 8u), 256, 0, s>>>(bytes, scales, gscales, out, octets, FastDiv(cols / 8),
-                                                                          rowwise);
-  } else {
-    decode_kernel<<<blocks_for(n, 256), 256, 0, s>>>(bytes, scales, gscales, out, rows, cols, rowwise, transpose);
+    return launch_chained(decode_rows_kernel, blocks_for(octets, 1024, 148u * 8u), 256, 0, s, bytes, scales, gscales, out, octets,
+                          FastDiv(cols / 8), rowwise);
   }
+  decode_kernel<<<blocks_for(n, 256), 256, 0, s>>>(bytes, scales, gscales, out, rows, cols, rowwise, transpose);
   NVFP4_RETURN_LAST();
 }
 
@@ -1671,9 +1686,9 @@ int launch_scale_pack(cudaStream_t s, const uint8_t* logical, uint8_t* packed, u
   const uint32_t k_atoms = kg / 4u;
   const ScalePlane plane = scale_plane(logical, packed, mn);
   if (scale_pack_tiled(plane))
-    scale_pack_tiles_kernel<<<dim3((k_atoms + 15u) / 16u, plane.row_blocks), 256, 0, s>>>(plane, ScalePlane{}, k_atoms);
-  else
-    scale_pack_kernel<<<blocks_for(total, 256, 148 * 16), 256, 0, s>>>(logical, packed, mn, padded, kg);
+    return launch_chained(scale_pack_tiles_kernel, dim3((k_atoms + 15u) / 16u, plane.row_blocks), 256, 0, s, plane, ScalePlane{},
+                          k_atoms);
+  scale_pack_kernel<<<blocks_for(total, 256, 148 * 16), 256, 0, s>>>(logical, packed, mn, padded, kg);
   NVFP4_RETURN_LAST();
 }
 
@@ -1686,8 +1701,8 @@ int launch_scale_pack_pair(cudaStream_t s, const uint8_t* const (&logical)[2], u
     const int rc = launch_scale_pack(s, logical[0], packed[0], mn[0], k_dim);
     return rc ? rc : launch_scale_pack(s, logical[1], packed[1], mn[1], k_dim);
   }
-  scale_pack_tiles_kernel<<<dim3((k_atoms + 15u) / 16u, a.row_blocks + b.row_blocks), 256, 0, s>>>(a, b, k_atoms);
-  NVFP4_RETURN_LAST();
+  return launch_chained(scale_pack_tiles_kernel, dim3((k_atoms + 15u) / 16u, a.row_blocks + b.row_blocks), 256, 0, s, a, b,
+                        k_atoms);
 }
 
 int launch_pad_u4_rows(cudaStream_t s, const uint8_t* src, uint8_t* dst, uint32_t rows, uint32_t padded_rows,

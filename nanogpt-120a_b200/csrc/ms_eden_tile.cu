@@ -2,21 +2,24 @@
 // read of it, and the transposed operand of an NVFP4 matrix (X^T, W^T).
 //
 // Same bytes as the generic kernels of quant_kernels.cu (one thread per 32-chunk, utils/nvfp4/quant/kernels/
-// ms_eden/**), organised for the rate at which instructions issue: the schedulers issue on 58 % of the cycles, the FMA pipe
-// is busy 52 % of them and the ALU 39 %, HBM 22 %.  Measured costs per warp instruction and scheduler are 1 cycle for scalar
-// FP32 (mixed f32 += bf16 * bf16 included), 2 for the packed f32x2 forms with distinct operands and for every integer, logic
-// and conversion instruction and cvt.f32.f16, and the costs of different pipes add up almost fully.  The counters fit that;
-// whether latency holds a part of the idle slots (16 warps per SM, a barrier per tile) is not settled.  So:
+// ms_eden/**), organised for the rate at which instructions issue: in the pair kernel the schedulers issue on 67 % of the
+// cycles, the FMA pipe is busy 61 % of them and the ALU 38 %, HBM 24 %.  Measured costs per warp instruction and scheduler are
+// 1 cycle for scalar FP32 (mixed f32 += bf16 * bf16 included, either half of a word), 2 for the packed f32x2 forms, and 2 for
+// integer, logic and conversion instructions; the two pipes overlap as far as register reads allow (a butterfly stage beside
+// two conversions 5.3 cycles instead of 8, beside two three-input maxima 7.7).  So:
 //  * a bf16 source is widened, sign-flipped and taken through the first butterfly stage by mixed-precision FMAs,
-//    x * (+-1) + u (exact product, one rounding), or for the upper half of a word by one logic instruction;
-//  * the lower E2M1 code of a byte is widened with add.f32.f16 instead of cvt.f32.f16;
+//    x * (+-1) + u (exact product, one rounding), which read either half of a word;
+//  * the E2M1 codes are widened with add.f32.f16 instead of cvt.f32.f16;
 //  * the reciprocal of a block scale, 1 / (s * gs + eps), depends on the scale byte only: a table per CTA;
 //  * every range check of a chunk (corrected scale inside the normal E4M3 range, finite quotients) is folded into one
-//    predicate at the end; a chunk that fails it is quantized again by the generic code behind the tile's barrier.
+//    predicate at the end; a chunk that fails it is quantized again by the generic code, from the source.
 //    The common path is one straight line, so the chains of the 16-groups overlap; with a branch per check they did not;
-//  * output addresses are a pointer per tile plus an offset per thread; the row operand leaves in 32-byte stores.
-// Measured at 32768 x 2304 bf16, both orientations and column sums: 136 -> 114 us (instructions per chunk 581 -> 490);
-// X^T of 32768 x 768: 33 -> 25 us.  HBM would allow 36 and 4 us.
+//  * output addresses are a pointer per tile plus an offset per thread; the row operand leaves in 32-byte stores;
+//  * warps share nothing but the table, so that they drift apart and the FP32 of one runs beside the conversions of another:
+//    with a barrier per tile all began their butterflies together.
+// Measured at 32768 x 2304 bf16, both orientations and column sums: 117 -> 106 us (with a barrier per tile and the upper halves
+// masked out by logic instructions 117, without the logic instructions 115); HBM would allow 36 us.  In a long step the board's
+// power limit takes the gain back in clock rate (1927 -> 1852 MHz): there the count of operations is what is left.
 #include <atomic>
 
 #include "ms_eden.cuh"
@@ -36,14 +39,8 @@ __device__ __forceinline__ void cp_async_16(uint32_t smem_addr, const void* gmem
 __device__ __forceinline__ void cp_async_16_or_zero(uint32_t smem_addr, const void* gmem, uint32_t bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr), "l"(gmem), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
-  uint16_t v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-  return v;
-}
 __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
@@ -73,11 +70,18 @@ __device__ __forceinline__ uint4 lds_128(uint32_t addr) {
   return v;
 }
 
-// x * s + c, x and s (+-1) bf16 in the low halves of 32-bit words (the mixed-precision forms read low halves only; a
-// high half would cost a shift): the product is exact, so this is the sum's one rounding.
+// x * s + c, x and s (+-1) bf16 in the low or high halves of 32-bit words: the product is exact, so this is the sum's one
+// rounding.
 __device__ __forceinline__ float signed_bf16_lo(uint32_t x, uint32_t s, float c) {
   float r;
   asm("{ .reg .b16 a, b, u, v; mov.b32 {a, u}, %1; mov.b32 {b, v}, %2; fma.rn.f32.bf16 %0, a, b, %3; }"
+      : "=f"(r)
+      : "r"(x), "r"(s), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float signed_bf16_hi(uint32_t x, uint32_t s, float c) {
+  float r;
+  asm("{ .reg .b16 a, b, u, v; mov.b32 {a, u}, %1; mov.b32 {b, v}, %2; fma.rn.f32.bf16 %0, u, v, %3; }"
       : "=f"(r)
       : "r"(x), "r"(s), "f"(c));
   return r;
@@ -87,9 +91,19 @@ __device__ __forceinline__ float add_bf16_lo(uint32_t x, float c) {
   asm("{ .reg .b16 a, u; mov.b32 {a, u}, %1; add.rn.f32.bf16 %0, a, %2; }" : "=f"(r) : "r"(x), "f"(c));
   return r;
 }
+__device__ __forceinline__ float add_bf16_hi(uint32_t x, float c) {
+  float r;
+  asm("{ .reg .b16 a, u; mov.b32 {a, u}, %1; add.rn.f32.bf16 %0, u, %2; }" : "=f"(r) : "r"(x), "f"(c));
+  return r;
+}
 __device__ __forceinline__ float widen_f16_lo(uint32_t x) {
   float r;
   asm("{ .reg .b16 a, u; mov.b32 {a, u}, %1; add.rn.f32.f16 %0, a, %2; }" : "=f"(r) : "r"(x), "f"(-0.0f));
+  return r;
+}
+__device__ __forceinline__ float widen_f16_hi(uint32_t x) {
+  float r;
+  asm("{ .reg .b16 a, u; mov.b32 {a, u}, %1; add.rn.f32.f16 %0, u, %2; }" : "=f"(r) : "r"(x), "f"(-0.0f));
   return r;
 }
 
@@ -108,9 +122,9 @@ __device__ __forceinline__ void first_stage_lo(uint32_t a, uint32_t b, uint32_t 
 }
 // ... and high halves.
 __device__ __forceinline__ void first_stage_hi(uint32_t a, uint32_t b, uint32_t sa, uint32_t sb, float& sum, float& diff) {
-  const float ua = __uint_as_float((a ^ sa) & 0xffff0000u), ub = __uint_as_float((b ^ sb) & 0xffff0000u);
-  sum = __fadd_rn(ua, ub);
-  diff = __fsub_rn(ua, ub);
+  const float ub = signed_bf16_hi(b, sb, -0.0f);
+  sum = signed_bf16_hi(a, sa, ub);
+  diff = signed_bf16_hi(a, sa, -ub);
 }
 
 // Two chunks of one thread, one per packed lane.
@@ -211,11 +225,11 @@ __device__ __forceinline__ PairCode ms_eden_chunk_pair(f32x2_t (&P)[32], uint32_
   return r;
 }
 
-// A chunk again by the generic code, any values (zero groups, scales outside the normal range, NaN).  Reloads it from
-// the staged tile: first value at `src`, `step` bytes apart, K index k0 ...
+// A chunk again by the generic code, any values (zero groups, scales outside the normal range, NaN), from the source:
+// `valid` values `step` elements apart, zeros behind them, K index k0 ...
 template <typename T>
-__device__ __noinline__ void requantize(uint32_t src, uint32_t step, uint32_t sign_seed, uint32_t k0, const MsEdenOut* o,
-                                        float gs, float so, uint32_t row, uint32_t chunk_in_row) {
+__device__ __noinline__ void requantize(const T* src, uint32_t step, uint32_t valid, uint32_t sign_seed, uint32_t k0,
+                                        const MsEdenOut* o, float gs, float so, uint32_t row, uint32_t chunk_in_row) {
   f32x2_t P[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
@@ -223,7 +237,7 @@ __device__ __noinline__ void requantize(uint32_t src, uint32_t step, uint32_t si
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const uint32_t k = i + 16 * h;
-      v[h] = sizeof(T) == 2 ? lds_u16(src + k * step) << 16 : __float_as_uint(lds_f32(src + k * step));
+      v[h] = k < valid ? __float_as_uint(load_as_f32<T>(src, static_cast<size_t>(k) * step)) : 0u;
       v[h] ^= random_sign_negative(sign_seed, k0 + k) ? 0x80000000u : 0u;
     }
     P[i] = pack2(__uint_as_float(v[0]), __uint_as_float(v[1]));
@@ -317,61 +331,62 @@ __device__ __forceinline__ float tile_global_scale(const MsEdenTileParams& p) {
 
 // ---- dY in both orientations ------------------------------------------------------------------
 
-// A staged tile: 128 source rows of 64 values, 16 bytes of padding per row (conflict-free 16-byte reads along rows
-// and 2- or 4-byte reads down columns), and the +-1 signs of its rows and columns in the form the first butterfly
-// stage multiplies by: packed bf16 pairs, or f32.
+// What a warp stages of a tile: 32 source rows of 64 values, 16 bytes of padding per row (conflict-free 16-byte reads along
+// rows and 2- or 4-byte reads down columns).
+constexpr int kBlockRows = 32;
 template <typename T>
-struct PairTile {
+struct PairBlock {
   static constexpr bool kBf16 = sizeof(T) == 2;
   static constexpr int kPitch = kTileCols * static_cast<int>(sizeof(T)) + 16;
-  static constexpr int kStageBytes = kTileRows * kPitch;
+  static constexpr int kBytes = kBlockRows * kPitch;
   static constexpr int kPiecesPerRow = kTileCols * static_cast<int>(sizeof(T)) / 16;
-  static constexpr int kPiecesPerThread = kTileRows * kPiecesPerRow / 256;
+  static constexpr int kSignWords = kBf16 ? 32 : kTileCols;
 };
 
-// The row role reads its 32 values along a row, the transposed role down a column; `rows` and `cols` need not be
-// whole tiles in the kEdge form (zero fill on the way in, guards on the way out, pad rows of the packed scale
-// planes written with 1.0).
+// Warps 0-3: the transposed operand, columns 2 * lane and 2 * lane + 1, rows 32 * warp ... of the CTA's tile.  Warps 4-7: the
+// row operand, row 32 * (warp - 4) + lane, both of its chunks.  The roles are separate code, so that neither pays for
+// selecting the other's addresses.  Every warp stages its rows and its signs for itself, and loads the next tile's as soon as
+// it holds this one's in registers: no barrier ties the warps together (but the column sums, once per tile, those of the
+// transposed role), so that the butterfly of one, all FP32, runs beside the conversions of another.
+// `rows` and `cols` need not be whole tiles in the kEdge form (zero fill on the way in, guards on the way out, pad rows of
+// the packed scale planes written with 1.0).
 template <typename T, bool kColSum, bool kEdge>
 __global__ void __launch_bounds__(256, 2)
     ms_eden_pair_kernel(const __grid_constant__ MsEdenTileParams p, uint32_t tiles_x, uint32_t tile_count) {
   wait_for_prior_then_allow_next();
-  using PT = PairTile<T>;
-  constexpr bool kBf16 = PT::kBf16;
+  using PB = PairBlock<T>;
+  constexpr bool kBf16 = PB::kBf16;
   constexpr uint32_t kSize = sizeof(T);
-  extern __shared__ __align__(16) uint8_t pair_stage[];  // [2][PT::kStageBytes]
-  // Random signs.  bf16 sources: +-1 in bf16 for the low half of a word, the bare sign bit for its high half; the K
-  // positions of the transposed operand share one sign for both halves (two columns), those of the row operand have
-  // one each.  f32 sources: the bare sign bit.
-  __shared__ __align__(16) uint32_t sign_row[kTileRows];
-  __shared__ __align__(16) uint32_t sign_col[kBf16 ? kTileCols / 2 : kTileCols];
-  __shared__ __align__(8) float quarter_sum[4][kTileCols];
+  extern __shared__ __align__(16) uint8_t pair_stage[];  // [8][PB::kBytes]
+  // Random signs of a warp's rows (transposed role) or columns (row role).  bf16 sources: +-1 in bf16 for each half of a word;
+  // the K positions of the transposed operand share one sign for both halves (two columns), those of the row operand have one
+  // each.  f32 sources: the bare sign bit.
+  __shared__ __align__(16) uint32_t sign_words[8][PB::kSignWords];
+  __shared__ __align__(8) float quarter_sum[2][4][kTileCols];
   __shared__ float2 inv_table[kScaleCodes];
-  __shared__ uint32_t slow_count;      // threads of this tile whose chunks need the generic code, and which
-  __shared__ uint8_t slow_list[256];
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const T* x = after_prior(static_cast<const T*>(p.x));
   const float gs = tile_global_scale(p), safe_gs = nz(gs);
   fill_inv_table(inv_table, safe_gs);
   const float inv6 = inv_scale(6.0f, safe_gs);
-  const uint32_t stage_base = static_cast<uint32_t>(__cvta_generic_to_shared(pair_stage));
-  const uint32_t sign_row_base = static_cast<uint32_t>(__cvta_generic_to_shared(sign_row));
-  const uint32_t sign_col_base = static_cast<uint32_t>(__cvta_generic_to_shared(sign_col));
+  const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(pair_stage)) + warp * PB::kBytes;
+  const uint32_t signs = static_cast<uint32_t>(__cvta_generic_to_shared(sign_words[warp]));
   const uint32_t table = static_cast<uint32_t>(__cvta_generic_to_shared(inv_table));
+  const uint32_t row_in_tile = (warp & 3u) * kBlockRows;  // of the warp's first row
 
-  // 16-byte pieces, row-major over the tile, kPiecesPerThread passes of kPassRows rows
-  constexpr uint32_t kPassRows = 256 / PT::kPiecesPerRow;
-  const uint32_t piece_row = tid / PT::kPiecesPerRow, piece_col = tid % PT::kPiecesPerRow * (16 / kSize);
-  const uint32_t piece_dst = stage_base + piece_row * PT::kPitch + piece_col * kSize;
-  const size_t piece_off = static_cast<size_t>(piece_row) * p.src_cols + piece_col;
+  // 16-byte pieces, row-major over the block, kPiecesPerRow passes of kPassRows rows
+  constexpr uint32_t kPassRows = 32 / PB::kPiecesPerRow;
+  const uint32_t piece_row = lane / PB::kPiecesPerRow, piece_col = lane % PB::kPiecesPerRow * (16 / kSize);
+  const uint32_t piece_dst = stage + piece_row * PB::kPitch + piece_col * kSize;
+  const size_t piece_off = static_cast<size_t>(row_in_tile + piece_row) * p.src_cols + piece_col;
   const size_t pass_stride = static_cast<size_t>(kPassRows) * p.src_cols;
-  auto issue_tile = [&](uint32_t ty, uint32_t tx, uint32_t buf) {
+  auto issue_block = [&](uint32_t ty, uint32_t tx) {
     const T* src = x + static_cast<size_t>(ty) * kTileRows * p.src_cols + tx * kTileCols + piece_off;
 #pragma unroll
-    for (uint32_t k = 0; k < PT::kPiecesPerThread; ++k) {
-      const uint32_t dst = piece_dst + buf * PT::kStageBytes + k * kPassRows * PT::kPitch;
+    for (uint32_t k = 0; k < PB::kPiecesPerRow; ++k) {
+      const uint32_t dst = piece_dst + k * kPassRows * PB::kPitch;
       if (kEdge) {
-        const bool inside = ty * kTileRows + piece_row + k * kPassRows < p.src_rows &&
+        const bool inside = ty * kTileRows + row_in_tile + piece_row + k * kPassRows < p.src_rows &&
                             tx * kTileCols + piece_col < p.src_cols;  // columns come in whole 16-byte pieces
         cp_async_16_or_zero(dst, inside ? src + k * pass_stride : x, inside ? 16u : 0u);
       } else {
@@ -380,49 +395,42 @@ __global__ void __launch_bounds__(256, 2)
     }
   };
 
-  // Warps 0-3: the transposed operand, columns 2 * lane and 2 * lane + 1, rows 32 * warp ... of the tile.  Warps 4-7:
-  // the row operand, row 32 * (warp - 4) + lane, both of its chunks.  The roles are separate code, so that neither
-  // pays for selecting the other's addresses.
-  const uint32_t src_off = warp < 4 ? warp * 32 * PT::kPitch + lane * 2 * kSize : ((warp & 3u) * 32 + lane) * PT::kPitch;
-  const ChunkOffsets at = warp < 4 ? chunk_offsets(p.t, 2 * lane, warp) : chunk_offsets(p.r, (warp & 3u) * 32 + lane, 0);
+  const uint32_t src = stage + (warp < 4 ? lane * 2 * kSize : lane * PB::kPitch);
+  const ChunkOffsets at = warp < 4 ? chunk_offsets(p.t, 2 * lane, warp) : chunk_offsets(p.r, row_in_tile + lane, 0);
   const ChunkOffsets row_step = {(p.t.dst_row_len >> 5) * 16, p.t.packed ? 16u : (p.t.dst_row_len >> 5) * 2, p.t.group_row_stride};
   const bool wide_rows = (p.r.dst_row_len & 63u) == 0 && (reinterpret_cast<uintptr_t>(p.r.fp4) & 31u) == 0 &&
                          (reinterpret_cast<uintptr_t>(p.r.scales) & 3u) == 0;
-  if (tid == 0) slow_count = 0;
 
   TileWalk next(tiles_x);
   uint32_t buf = 0;
-  if (blockIdx.x < tile_count) issue_tile(next.ty, next.tx, 0);
-  cp_async_commit();
+  if (blockIdx.x < tile_count) issue_block(next.ty, next.tx);
+  __syncthreads();  // the table
 #pragma unroll 1
   for (uint32_t tile = blockIdx.x; tile < tile_count; tile += gridDim.x, buf ^= 1) {
     const uint32_t ty = next.ty, r0 = ty * kTileRows, c0 = next.tx * kTileCols;
     next.advance();
-    if (tile + gridDim.x < tile_count) issue_tile(next.ty, next.tx, buf ^ 1);
-    cp_async_commit();
-    if (tid < kTileRows) {
-      const bool neg = random_sign_negative(p.sign_seed, r0 + tid + p.t.sign_offset);
-      sign_row[tid] = kBf16 ? (neg ? 0x8000bf80u : 0x3f80u) : (neg ? 0x80000000u : 0u);
-      if (c0 == 0 && (!kEdge || r0 + tid < p.r.rows)) p.r.global_scales[r0 + tid] = gs;
-    } else if (tid < kTileRows + kTileCols) {
-      const uint32_t i = tid - kTileRows;
-      if (kBf16 && i < kTileCols / 2) {
-        const uint32_t col = c0 + 2 * i + p.r.sign_offset;
-        sign_col[i] = (random_sign_negative(p.sign_seed, col) ? 0xbf80u : 0x3f80u) |
-                      (random_sign_negative(p.sign_seed, col + 1) ? 0x80000000u : 0u);
-      } else if (!kBf16) {
-        sign_col[i] = random_sign_negative(p.sign_seed, c0 + i + p.r.sign_offset) ? 0x80000000u : 0u;
+    const bool more = tile + gridDim.x < tile_count;
+    if (warp < 4) {
+      const bool neg = random_sign_negative(p.sign_seed, r0 + row_in_tile + lane + p.t.sign_offset);
+      sign_words[warp][lane] = kBf16 ? (neg ? 0xbf80bf80u : 0x3f803f80u) : (neg ? 0x80000000u : 0u);
+      if (r0 == 0 && warp < 2 && (!kEdge || c0 + tid < p.t.rows)) p.t.global_scales[c0 + tid] = gs;
+    } else {
+      const uint32_t col = c0 + (kBf16 ? 2 * lane : lane) + p.r.sign_offset;
+      const bool neg0 = random_sign_negative(p.sign_seed, col), neg1 = random_sign_negative(p.sign_seed, col + (kBf16 ? 1u : 32u));
+      if (kBf16) {
+        sign_words[warp][lane] = (neg0 ? 0xbf80u : 0x3f80u) | (neg1 ? 0xbf800000u : 0x3f800000u);
+      } else {
+        sign_words[warp][lane] = neg0 ? 0x80000000u : 0u;
+        sign_words[warp][lane + PB::kSignWords - 32] = neg1 ? 0x80000000u : 0u;
       }
-      if (r0 == 0 && (!kEdge || c0 + i < p.t.rows)) p.t.global_scales[c0 + i] = gs;
+      const uint32_t row = r0 + row_in_tile + lane;
+      if (c0 == 0 && (!kEdge || row < p.r.rows)) p.r.global_scales[row] = gs;
     }
-    cp_async_wait_all_but_one();
-    __syncthreads();
-    const uint32_t t = stage_base + buf * PT::kStageBytes;
+    cp_async_wait_all();
+    __syncwarp();
 
-    bool ok;
     f32x2_t P[32];
     if (warp < 4) {
-      const uint32_t src = t + src_off, signs = sign_row_base + warp * 128;
       float sum_lo = 0.0f, sum_hi = 0.0f;
 #pragma unroll
       for (int g = 0; g < 8; ++g) {
@@ -432,7 +440,7 @@ __global__ void __launch_bounds__(256, 2)
         for (int k = 0; k < 4; k += 2) {
           const int pos = 4 * g + k;
           if (kBf16) {
-            const uint32_t wa = lds_u32(src + pos * PT::kPitch), wb = lds_u32(src + (pos + 1) * PT::kPitch);
+            const uint32_t wa = lds_u32(src + pos * PB::kPitch), wb = lds_u32(src + (pos + 1) * PB::kPitch);
             float sl, dl, sh, dh;
             first_stage_lo(wa, wb, sw[k], sw[k + 1], sl, dl);
             first_stage_hi(wa, wb, sw[k], sw[k + 1], sh, dh);
@@ -440,10 +448,10 @@ __global__ void __launch_bounds__(256, 2)
             P[pos + 1] = pack2(dl, dh);
             if (kColSum) {
               sum_lo = add_bf16_lo(wb, add_bf16_lo(wa, sum_lo));
-              sum_hi = (sum_hi + __uint_as_float(wa & 0xffff0000u)) + __uint_as_float(wb & 0xffff0000u);
+              sum_hi = add_bf16_hi(wb, add_bf16_hi(wa, sum_hi));
             }
           } else {
-            const uint2 wa = lds_64(src + pos * PT::kPitch), wb = lds_64(src + (pos + 1) * PT::kPitch);
+            const uint2 wa = lds_64(src + pos * PB::kPitch), wb = lds_64(src + (pos + 1) * PB::kPitch);
             const f32x2_t ua = pack2(__uint_as_float(wa.x ^ sw[k]), __uint_as_float(wa.y ^ sw[k]));
             const f32x2_t ub = pack2(__uint_as_float(wb.x ^ sw[k + 1]), __uint_as_float(wb.y ^ sw[k + 1]));
             P[pos] = add2(ua, ub);
@@ -455,14 +463,16 @@ __global__ void __launch_bounds__(256, 2)
           }
         }
       }
+      __syncwarp();
+      if (more) issue_block(next.ty, next.tx);
       // dbias partials: four sequential 32-row sums per column, added below in the order ((q0 + q1) + q2) + q3
-      if (kColSum) *reinterpret_cast<float2*>(&quarter_sum[warp][2 * lane]) = make_float2(sum_lo, sum_hi);
+      if (kColSum) *reinterpret_cast<float2*>(&quarter_sum[buf][warp][2 * lane]) = make_float2(sum_lo, sum_hi);
       const uint32_t group = at.group + c0 * p.t.group_row_stride + (r0 >> 4);
       const PairCode code =
           ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.t.scale_seed, p.opaque_zero, group, group + row_step.group);
+      const uint32_t row = c0 + 2 * lane, chunk_in_row = (r0 >> 5) + warp;
       bool first = true, second = true;
       if (kEdge) {
-        const uint32_t row = c0 + 2 * lane, chunk_in_row = (r0 >> 5) + warp;
         const bool k_inside = chunk_in_row * 32u < p.t.dst_row_len;
         if (p.t.packed && k_inside) {
           store_pad_scales(p.t, row, chunk_in_row, c0 + kTileCols >= p.src_cols);
@@ -471,23 +481,35 @@ __global__ void __launch_bounds__(256, 2)
         first = k_inside && row < p.t.rows;
         second = k_inside && row + 1 < p.t.rows;
       }
-      ok = code.ok || (kEdge && !first);
       store_column_pair(code, tile_nibbles(p.t, c0, r0 >> 5), tile_scales(p.t, c0, r0 >> 5), at, row_step, first, second);
+      if (!code.ok && first) {  // rare
+        const uint32_t k0 = r0 + warp * kBlockRows, valid = kEdge ? p.src_rows - min(p.src_rows, k0) : 32u;
+#pragma unroll 1
+        for (uint32_t h = 0; h < (second ? 2u : 1u); ++h)
+          requantize<T>(x + static_cast<size_t>(k0) * p.src_cols + row + h, p.src_cols, valid, p.sign_seed, k0 + p.t.sign_offset, &p.t,
+                        gs, p.scale_override, row + h, chunk_in_row);
+      }
+      if (kColSum) {
+        // two buffers: a warp that is here again has passed the barrier of the tile between, behind the sums of this one
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (warp < 2 && (!kEdge || c0 + tid < p.src_cols))
+          p.col_sum_partials[static_cast<size_t>(ty) * p.src_cols + c0 + tid] =
+              ((quarter_sum[buf][0][tid] + quarter_sum[buf][1][tid]) + quarter_sum[buf][2][tid]) + quarter_sum[buf][3][tid];
+      }
     } else {
-      const uint32_t src = t + src_off;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         constexpr int kPerLoad = 16 / static_cast<int>(kSize);
 #pragma unroll
         for (int g = 0; g < 32 / kPerLoad; ++g) {
           const uint4 v = lds_128(src + half * 32 * kSize + g * 16);
-          const uint4 s = lds_128(sign_col_base + half * (kBf16 ? 64 : 128) + g * 16);
+          const uint4 s = lds_128(signs + half * (kBf16 ? 64 : 128) + g * 16);
           const uint32_t vw[4] = {v.x, v.y, v.z, v.w}, sw[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             if (kBf16) {  // K positions 2j (low half) and 2j + 1 (high half)
               const int pos = 8 * g + 2 * k;
-              const float ub = __uint_as_float((vw[k] ^ sw[k]) & 0xffff0000u);
+              const float ub = signed_bf16_hi(vw[k], sw[k], -0.0f);
               set_lane(P[pos], half, signed_bf16_lo(vw[k], sw[k], ub));
               set_lane(P[pos + 1], half, signed_bf16_lo(vw[k], sw[k], -ub));
             } else if ((k & 1) == 0) {
@@ -498,16 +520,17 @@ __global__ void __launch_bounds__(256, 2)
           }
         }
       }
+      __syncwarp();
+      if (more) issue_block(next.ty, next.tx);
       const uint32_t group = at.group + r0 * p.r.group_row_stride + (c0 >> 4);
       const PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.r.scale_seed, p.opaque_zero, group, group + 2);
       uint8_t* const nibbles = tile_nibbles(p.r, r0, c0 >> 5) + at.nibbles;
       uint8_t* const scales = tile_scales(p.r, r0, c0 >> 5) + at.scales;
-      const uint32_t row = r0 + (warp & 3u) * 32 + lane, chunk_in_row = c0 >> 5;
-      const bool inside = !kEdge || row < p.r.rows;
-      ok = code.ok || !inside;
+      const uint32_t row = r0 + row_in_tile + lane, chunk_in_row = c0 >> 5;
+      const bool inside = !kEdge || row < p.r.rows, second = !kEdge || (chunk_in_row + 1) * 32u < p.r.dst_row_len;
       if (kEdge && p.r.packed) {
         store_pad_scales(p.r, row, chunk_in_row, false);
-        if ((chunk_in_row + 1) * 32u < p.r.dst_row_len) store_pad_scales(p.r, row, chunk_in_row + 1, false);
+        if (second) store_pad_scales(p.r, row, chunk_in_row + 1, false);
       }
       if (inside) {
         if (wide_rows) {  // 32 nibble bytes in one store, four scale bytes in one
@@ -523,29 +546,17 @@ __global__ void __launch_bounds__(256, 2)
             *reinterpret_cast<uint16_t*>(scales + 2) = static_cast<uint16_t>(code.scales >> 16);
           }
         }
-      }
-    }
-    if (!ok) slow_list[atomicAdd(&slow_count, 1u)] = static_cast<uint8_t>(tid);
-    __syncthreads();
-    if (kColSum && tid < kTileCols && (!kEdge || c0 + tid < p.src_cols))
-      p.col_sum_partials[static_cast<size_t>(ty) * p.src_cols + c0 + tid] =
-          ((quarter_sum[0][tid] + quarter_sum[1][tid]) + quarter_sum[2][tid]) + quarter_sum[3][tid];
-    if (slow_count != 0) {  // rare; uniform: every thread reads the same count behind the barrier
-      for (uint32_t i = tid; i < 2 * slow_count; i += 256) {
-        const uint32_t who = slow_list[i >> 1], w = (who >> 5) & 3u, l = who & 31u, second = i & 1u;
-        if (who < 128) {
-          const uint32_t row = c0 + 2 * l + second;
-          if (!kEdge || row < p.t.rows)
-            requantize<T>(t + w * 32 * PT::kPitch + (2 * l + second) * kSize, PT::kPitch, p.sign_seed,
-                          r0 + w * 32 + p.t.sign_offset, &p.t, gs, p.scale_override, row, (r0 >> 5) + w);
-        } else if (!kEdge || ((c0 >> 5) + second) * 32u < p.r.dst_row_len) {
-          requantize<T>(t + (w * 32 + l) * PT::kPitch + second * 32 * kSize, kSize, p.sign_seed,
-                        c0 + second * 32 + p.r.sign_offset, &p.r, gs, p.scale_override, r0 + w * 32 + l, (c0 >> 5) + second);
+        if (!code.ok) {  // rare
+#pragma unroll 1
+          for (uint32_t h = 0; h < (second ? 2u : 1u); ++h) {
+            const uint32_t k0 = c0 + 32 * h, valid = kEdge ? p.src_cols - min(p.src_cols, k0) : 32u;
+            requantize<T>(x + static_cast<size_t>(row) * p.src_cols + k0, 1, valid, p.sign_seed, k0 + p.r.sign_offset, &p.r, gs,
+                          p.scale_override, row, chunk_in_row + h);
+          }
         }
       }
-      __syncthreads();
-      if (tid == 0) slow_count = 0;  // the next barrier stands before the next use
     }
+    __syncwarp();
   }
 }
 
@@ -627,7 +638,7 @@ __global__ void __launch_bounds__(128, 4)
             asm("{ .reg .b8 t; cvt.u8.u32 t, %1; cvt.rn.f16x2.e2m1x2 %0, t; }" : "=r"(h2) : "r"(__byte_perm(words[w], 0u, 0x4440u | k)));
             const __half2 v = __hmul2(*reinterpret_cast<__half2*>(&h2), s[w >> 1]);
             u[2 * k] = __fmul_rn(widen_f16_lo(*reinterpret_cast<const uint32_t*>(&v)), g);
-            u[2 * k + 1] = __fmul_rn(__high2float(v), g);
+            u[2 * k + 1] = __fmul_rn(widen_f16_hi(*reinterpret_cast<const uint32_t*>(&v)), g);
           }
           sts_128(dst + h * 128 + w * 32, u[0], u[1], u[2], u[3]);
           sts_128(dst + h * 128 + w * 32 + 16, u[4], u[5], u[6], u[7]);
@@ -696,7 +707,7 @@ int opt_in_shared(int bytes) {
 
 template <typename T, bool kColSum, bool kEdge>
 int launch_pair(cudaStream_t s, const MsEdenTileParams& p) {
-  constexpr int kStage = 2 * PairTile<T>::kStageBytes;
+  constexpr int kStage = 8 * PairBlock<T>::kBytes;
   const int rc = opt_in_shared<ms_eden_pair_kernel<T, kColSum, kEdge>>(kStage);
   if (rc) return rc;
   const uint32_t tiles_x = (p.src_cols + kTileCols - 1) / kTileCols;

@@ -566,7 +566,8 @@ __global__ void __launch_bounds__(256, 2)
 // 32-chunks down a column pair.  Decoding is (q * s) * g as utils/nvfp4/tensor.rs:48-57 evaluates it: q * s in f16 (exact:
 // E2M1 times E4M3 has six significant bits and lies between 2^-10 and 2688), then one rounding; the random sign of a K
 // position is folded into its row's g, (q s)(-g) == -((q s) g).  Each thread's row of the next tile is in flight in
-// registers during the current one.
+// registers during the current one.  A warp decodes the 32 rows whose chunks it takes, so that no barrier ties the warps
+// together.
 constexpr int kNvPitch = kTileCols * 4 + 16;
 
 template <bool kRowwise, bool kEdge>
@@ -615,6 +616,7 @@ __global__ void __launch_bounds__(128, 4)
   const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(nv_stage));
   TileWalk next(tiles_x);
   if (blockIdx.x < tile_count) load_tile(next.ty, next.tx);
+  __syncthreads();  // the table
 #pragma unroll 1
   for (uint32_t tile = blockIdx.x; tile < tile_count; tile += gridDim.x) {
     const uint32_t r0 = next.ty * kTileRows, c0 = next.tx * kTileCols;
@@ -647,7 +649,7 @@ __global__ void __launch_bounds__(128, 4)
       if (r0 == 0 && tid < kTileCols && (!kEdge || c0 + tid < p.t.rows)) p.t.global_scales[c0 + tid] = gs;
     }
     if (tile + gridDim.x < tile_count) load_tile(next.ty, next.tx);
-    __syncthreads();
+    __syncwarp();
 
     const uint32_t src = stage + warp * 32 * kNvPitch + lane * 8;
     f32x2_t P[32];
@@ -682,7 +684,7 @@ __global__ void __launch_bounds__(128, 4)
       for (uint32_t h = 0; h < (second ? 2u : 1u); ++h)
         requantize_staged(src + h * 4, kNvPitch, &p.t, gs, p.scale_override, row + h, chunk_in_row);
     }
-    __syncthreads();
+    __syncwarp();
   }
 }
 

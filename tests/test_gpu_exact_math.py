@@ -64,6 +64,23 @@ def test_four_six_amax_smaller_than_the_data(pkg, oracle, dev, scale):
     assert cpu(t.global_scales).tobytes() == og.tobytes() or np.array_equal(cpu(t.global_scales), og, equal_nan=True)
 
 
+@pytest.mark.parametrize("rowwise", [False, True])
+@pytest.mark.parametrize("values,scale", [("normal", 1.0), ("integers", 1.0), ("integers", 0.1), ("normal", 2.0 ** -31),
+                                          ("normal", 2.0 ** 60)])
+def test_four_six_close_candidates(pkg, oracle, dev, rowwise, values, scale):
+    """Groups whose two candidate errors tie or nearly do (small integers tie often, a million normal groups hold some
+    hundreds of close ones), and amaxes on either side of where the cheap errors are trusted: bytes of the oracle."""
+    q = pkg.Nvfp4QuantModule()
+    rng = np.random.default_rng(723)
+    x = rng.normal(size=(8192, 2048)) if values == "normal" else rng.integers(-12, 13, (8192, 2048)).astype(np.float64)
+    x[5], x[7, :16], x[:, 32:48] = 0, 0, x[:, 32:48] * 2.0 ** -12
+    x = (x * scale).astype(np.float32)
+    amax = oracle.row_amax(x) if rowwise else oracle.tensor_amax(x)[1]
+    t = q.quantize_four_six(torch.from_numpy(x).to(dev), torch.from_numpy(amax).to(dev), rowwise=rowwise, packed=False)
+    ob, os_, og = oracle.four_six(x, amax, rowwise)
+    assert np.array_equal(cpu(t.bytes), ob) and np.array_equal(cpu(t.scales), os_) and np.array_equal(cpu(t.global_scales), og)
+
+
 def test_pad_rows_beyond_the_index_space(pkg, dev):
     """One row so long that the groups of its 127 pad rows alone pass 2^32: the pad rows get a launch of their own."""
     q = pkg.Nvfp4QuantModule()

@@ -273,14 +273,15 @@ static int validate_ms_eden(const nvfp4_ms_eden_args* a) {
 
 // Row operand + transposed operand of one matrix in a single pass (same scale, same signs).
 static int ms_eden_pair(void* stream, nvfp4_ms_eden_args rows, nvfp4_ms_eden_args transposed,
-                        float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr) {
+                        float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr,
+                        void* zero = nullptr, uint64_t zero_words = 0) {
   rows.src_kind = NVFP4_SRC_F32_ROWS;
   transposed.src_kind = NVFP4_SRC_F32_TRANSPOSED;
   int rc = validate_ms_eden(&rows);
   if (rc) return rc;
   rc = validate_ms_eden(&transposed);
   if (rc) return rc;
-  return launch_ms_eden_pair(S(stream), rows, transposed, col_sum_partials, amax_in, gs_out);
+  return launch_ms_eden_pair(S(stream), rows, transposed, col_sum_partials, amax_in, gs_out, zero, zero_words);
 }
 
 static nvfp4_ms_eden_args rows_args(const float* x, uint8_t* out_fp4, uint8_t* out_scales, float* out_gss,
@@ -831,12 +832,28 @@ int nvfp4_tc_matmul_ms_eden(void* stream, const float* a, const float* b_t, floa
 }
 
 // The gradient GEMMs over quantized operands: dX = e_h . weight_t_h^T, dW = e_t_h . input_t_h^T.
+// Shapes, types and output of dW = dY^T . X.
+static nvfp4_gemm_args dweight_gemm(void* dweight, int dweight_dtype, uint32_t T, uint32_t I, uint32_t O) {
+  nvfp4_gemm_args g;
+  std::memset(&g, 0, sizeof(g));
+  g.global_scale_mode = NVFP4_GS_ROWWISE_A;
+  g.weight_global_scale = 1.0f;
+  g.epilogue = NVFP4_EPI_NONE;
+  g.out = dweight;
+  g.out_dtype = dweight_dtype;
+  g.m = O;
+  g.n = I;
+  g.k = padded_k(T);
+  g.ldo = I;
+  return g;
+}
+
+// dweight_is_zero: dweight holds zeros already
 static int backward_gemms(cudaStream_t s, const uint8_t* eh_b, const uint8_t* eh_s, const float* eh_g,
                           const uint8_t* wt_b, const uint8_t* wt_s, const float* wt_g, const uint8_t* et_b,
                           const uint8_t* et_s, const float* et_g, const uint8_t* xt_b, const uint8_t* xt_s,
                           const float* xt_g, void* dinput, int dinput_dtype, void* dweight, int dweight_dtype,
-                          uint32_t T, uint32_t I, uint32_t O) {
-  const uint32_t ok = padded_k(O), tk = padded_k(T);
+                          uint32_t T, uint32_t I, uint32_t O, bool dweight_is_zero = false) {
   nvfp4_gemm_args g;
   std::memset(&g, 0, sizeof(g));
   g.global_scale_mode = NVFP4_GS_ROWWISE_A;
@@ -852,22 +869,18 @@ static int backward_gemms(cudaStream_t s, const uint8_t* eh_b, const uint8_t* eh
   g.out = dinput;
   g.m = T;
   g.n = I;
-  g.k = ok;
+  g.k = padded_k(O);
   g.ldo = I;
   int rc = launch_gemm(s, g);
   if (rc) return rc;
+  g = dweight_gemm(dweight, dweight_dtype, T, I, O);
   g.a_bytes = et_b;
   g.a_scales = et_s;
   g.a_global = et_g;
   g.b_bytes = xt_b;
   g.b_scales = xt_s;
   g.b_global = xt_g;
-  g.out = dweight;
-  g.out_dtype = dweight_dtype;
-  g.m = O;
-  g.n = I;
-  g.k = tk;
-  return launch_gemm(s, g);
+  return launch_gemm(s, g, dweight_is_zero);
 }
 
 static int backward_device_scale(void* stream, const nvfp4_linear_backward_device_scale_args* a) {
@@ -923,7 +936,8 @@ int nvfp4_linear_backward_prepare_weight_t(void* stream, const nvfp4_linear_back
 
 // Everything of nvfp4_linear_backward_ms_eden that runs between the fork onto the caller's side stream and the
 // join; `ts` is the stream the two transposers go to (the side stream, or the main one when there is none).
-static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_backward_args* a) {
+// dweight_is_zero: set where dweight was cleared along the way for a dW GEMM that adds into it.
+static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_backward_args* a, bool& dweight_is_zero) {
   const uint32_t T = a->token_count, I = a->input_dim, O = a->output_dim;
   const uint32_t ok = padded_k(O), tk = padded_k(T);
   cudaStream_t s = S(stream);
@@ -1013,8 +1027,14 @@ static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_
     if (rc) return rc;
   }
   float* partials = fuse_dbias ? static_cast<float*>(a->dinput) : nullptr;
+  // A dW GEMM that splits K adds into dW.  The pair kernel, whose stores are idle, clears it: a launch for that between the
+  // two GEMMs cost c_attn at 8192 tokens 3 us and kept the second GEMM from being set up early.
+  uint64_t zero_words = static_cast<uint64_t>(O) * I * (a->dweight_dtype == NVFP4_DTYPE_F32 ? 4 : 2);
+  dweight_is_zero = ms_eden_pair_takes_amax(q, qt) && ((reinterpret_cast<uintptr_t>(a->dweight) | zero_words) & 15u) == 0 &&
+                    gemm_adds_into_output(dweight_gemm(a->dweight, a->dweight_dtype, T, I, O));
+  zero_words = dweight_is_zero ? zero_words / 16 : 0;
   // one pass over dY for both orientations (+ column sums)
-  rc = ms_eden_pair(stream, q, qt, partials, amax_in, amax_in ? a->e_h.global_scale : nullptr);
+  rc = ms_eden_pair(stream, q, qt, partials, amax_in, amax_in ? a->e_h.global_scale : nullptr, a->dweight, zero_words);
   if (rc) return rc;
   if (fuse_dbias) rc = launch_col_sum_reduce(s, partials, a->dbias, ms_eden_pair_row_tiles(T), O);
   return rc;
@@ -1051,7 +1071,8 @@ int nvfp4_linear_backward_ms_eden(void* stream, const nvfp4_linear_backward_args
     ts = a->side_stream;
     forked = true;
   }
-  int rc = backward_ms_eden_quantize(stream, ts, a);
+  bool dweight_is_zero = false;
+  int rc = backward_ms_eden_quantize(stream, ts, a, dweight_is_zero);
   if (forked) {
     // join: the GEMMs need W^T and X^T; on an error path this leaves neither stream (nor a capture in
     // progress) dangling
@@ -1065,7 +1086,8 @@ int nvfp4_linear_backward_ms_eden(void* stream, const nvfp4_linear_backward_args
   return backward_gemms(s, a->e_h.bytes, a->e_h.scales_packed, a->e_h.global_scales, a->weight_t_h.bytes,
                         a->weight_t_h.scales_packed, a->weight_t_h.global_scale, a->e_t_h.bytes, a->e_t_h.scales_packed,
                         a->e_t_h.global_scales, a->input_t_h.bytes, a->input_t_h.scales_packed,
-                        a->input_t_h.global_scale, a->dinput, a->dinput_dtype, a->dweight, a->dweight_dtype, T, I, O);
+                        a->input_t_h.global_scale, a->dinput, a->dinput_dtype, a->dweight, a->dweight_dtype, T, I, O,
+                        dweight_is_zero);
 }
 
 }  // extern "C"

@@ -1825,7 +1825,14 @@ int gemm_prepare_operand_maps(const uint8_t* a_bytes, const uint8_t* b_bytes, ui
   return rc;
 }
 
-int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a) {
+bool gemm_adds_into_output(const nvfp4_gemm_args& a) {
+  if (a.m == 0 || a.n == 0 || a.k == 0 || a.k % 64 != 0) return false;
+  GemmPlan pl;
+  plan_gemm(a, sm_count(), pl);
+  return pl.k_splits > 1;
+}
+
+int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero) {
   if (a.m == 0 || a.n == 0) return 0;
   int rc = validate_gemm(a);
   if (rc) return rc;
@@ -1891,7 +1898,7 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a) {
   }
 
   const size_t esz = a.out_dtype == NVFP4_DTYPE_F32 ? 4 : 2;
-  if (p.k_splits > 1) {
+  if (p.k_splits > 1 && !out_is_zero) {
     cudaError_t e = cudaMemset2DAsync(a.out, static_cast<size_t>(a.ldo) * esz, 0, static_cast<size_t>(a.n) * esz, a.m, s);
     if (e != cudaSuccess) return static_cast<int>(e);
   }

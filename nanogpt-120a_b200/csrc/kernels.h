@@ -44,8 +44,10 @@ int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a, const float* ama
 // per-row-tile column sums [ms_eden_pair_row_tiles(rows)][cols] for launch_col_sum_reduce.
 // amax_in / gs_out (only when ms_eden_pair_takes_amax): the kernel derives the global scale from amax_in[0]
 // itself and writes it to gs_out[0]; rows.global_scale / transposed.global_scale are then not read.
+// zero (likewise only when ms_eden_pair_takes_amax): zero_words 16-byte words that the kernel clears beside its work.
 int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed,
-                        float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr);
+                        float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr,
+                        void* zero = nullptr, uint64_t zero_words = 0);
 bool ms_eden_pair_takes_amax(const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed);
 bool ms_eden_pair_is_tiled(const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed);
 uint32_t ms_eden_pair_row_tiles(uint32_t rows);
@@ -71,7 +73,10 @@ int launch_relu2_backward(cudaStream_t s, const void* pre, int pre_kind, const v
 uint32_t relu2_backward_grid(uint64_t n);
 
 // gemm_tcgen05.cu ---------------------------------------------------------------------------
-int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a);
+// out_is_zero: the output holds zeros already (it is cleared first where gemm_adds_into_output otherwise)
+int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero = false);
+// Whether launch_gemm splits K and sums the partial tiles in the output.
+bool gemm_adds_into_output(const nvfp4_gemm_args& a);
 // What launch_gemm would choose for these arguments on the current device (no launch).
 int gemm_plan_query(const nvfp4_gemm_args& a, nvfp4_gemm_plan* out);
 // Encodes (and keeps in the calling thread's cache) the operand tensor maps of a GEMM ahead of its launch.

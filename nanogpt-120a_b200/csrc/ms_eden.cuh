@@ -245,6 +245,8 @@ struct MsEdenTileParams {
   // evaluates the same two operations) and publish it, instead of a one-thread kernel in between
   const float* amax_in;
   float* gs_out;
+  uint4* zero = nullptr;  // pair kernel, optional: words to clear
+  uint64_t zero_words = 0;
   uint32_t opaque_zero = 0;  // always 0; keeps the assembler from seeing through a pack / unpack pair (ms_eden_tile.cu)
 };
 

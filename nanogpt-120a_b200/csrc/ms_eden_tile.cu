@@ -401,6 +401,8 @@ __global__ void __launch_bounds__(256, 2)
   const bool wide_rows = (p.r.dst_row_len & 63u) == 0 && (reinterpret_cast<uintptr_t>(p.r.fp4) & 31u) == 0 &&
                          (reinterpret_cast<uintptr_t>(p.r.scales) & 3u) == 0;
 
+  for (uint64_t i = blockIdx.x * 256u + tid; i < p.zero_words; i += gridDim.x * 256u) p.zero[i] = make_uint4(0u, 0u, 0u, 0u);
+
   TileWalk next(tiles_x);
   uint32_t buf = 0;
   if (blockIdx.x < tile_count) issue_block(next.ty, next.tx);

@@ -129,3 +129,30 @@ def test_pair_any_scale(pkg, oracle, dev, tokens, out_dim, dtype, factor):
         assert np.array_equal(cpu(op["global_scales"]), ref[2]), name
     torch.cuda.synchronize()
     assert pkg.read_device_status() == 0
+
+
+@pytest.mark.parametrize("tokens,in_dim,out_dim,offset", [(4352, 64, 64, 0), (8192, 768, 200, 0), (4500, 128, 72, 0), (4352, 64, 64, 1),
+                                                          (256, 64, 64, 0)])
+def test_backward_clears_dweight_before_it_adds(pkg, dev, tokens, in_dim, out_dim, offset):
+    """A dW GEMM that splits K adds into dW, which the pair kernel clears on the way (a launch of its own does where dW is
+    not 16-byte aligned): whatever dW held before is gone, and nothing beside it is touched."""
+    q, gemm, bwd = pkg.Nvfp4QuantModule(), pkg.Nvfp4GemmModule(), pkg.LinearBackwardModule()
+    e = bf16_normal(731, (tokens, out_dim), 1e-3).to(dev)
+    xq = q.quantize_four_six(bf16_normal(732, (tokens, in_dim)).to(dev), rowwise=True, packed=True, decoded_amax=True)
+    wq = q.quantize_four_six(bf16_normal(733, (out_dim, in_dim), 0.02).to(dev), rowwise=False, packed=True)
+    sc = pkg.LinearBackwardScratch(tokens, in_dim, out_dim, dev)
+    memory = torch.full((out_dim * in_dim + 8,), float("nan"), device=dev)
+    dw = memory[offset: offset + out_dim * in_dim].view(out_dim, in_dim)
+    bwd.backward_ms_eden(e=e, weight=wq, input=xq, scratch=sc, sign_seed=SIGN, scale_seed=SCALE, dweight=dw)
+    k = -(-tokens // 64) * 64
+    a = pkg.Nvfp4Tensor(sc.e_t_h["bytes"], sc.e_t_h["scales_packed"], sc.e_t_h["global_scales"], out_dim, k, packed=True, rowwise=True)
+    b = pkg.Nvfp4Tensor(sc.input_t_h["bytes"], sc.input_t_h["scales_packed"], sc.input_t_h["global_scale"], in_dim, k, packed=True,
+                        rowwise=False)
+    want = torch.empty((out_dim, in_dim), device=dev)
+    assert (gemm.plan(a, b, out=want).k_splits > 1) == (tokens > 4096)
+    gemm.gemm(a, b, out=want)
+    # the same partial sums in another order: 32 additions at most
+    assert float((dw - want).norm() / want.norm()) <= 32 * 2.0 ** -24
+    assert bool(memory[:offset].isnan().all()) and bool(memory[offset + out_dim * in_dim:].isnan().all())
+    torch.cuda.synchronize()
+    assert pkg.read_device_status() == 0

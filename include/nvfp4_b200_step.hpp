@@ -396,6 +396,11 @@ class ProjectionStep {
 
   DriverError forward(cudaStream_t s, Linear& l) {
     const uint32_t T = opt_.tokens;
+    // The weight stream is ahead of the forward pass but for the first linear, whose quantizer need not wait for it.  Behind
+    // an event a kernel does not start early, so the wait stands before the quantizer and not between it and its GEMM.
+    const bool first = &l == &linears_.front();
+    if (!first)
+      if (auto e = cuda(cudaStreamWaitEvent(s, l.wq_ready, 0), "stream wait")) return e;
     if (opt_.fused_mlp && l.is_proj) {
       // the MLP activation relu(pre)^2 is computed on load from the fc projection's pre-activation; its row
       // amax came out of that GEMM's epilogue
@@ -404,7 +409,8 @@ class ProjectionStep {
       const DeviceBuffer<const uint16_t> x{x_.at(l.in), static_cast<size_t>(T) * l.in};
       if (auto e = quant_.quantize_row_amax<uint16_t>(s, x, l.xq)) return e;
     }
-    if (auto e = cuda(cudaStreamWaitEvent(s, l.wq_ready, 0), "stream wait")) return e;
+    if (first)
+      if (auto e = cuda(cudaStreamWaitEvent(s, l.wq_ready, 0), "stream wait")) return e;
     const DeviceBuffer<const float> bias{l.bias, l.bias ? l.out : 0};
     if (opt_.fused_mlp && l.is_fc)
       return gemm_.gemm<uint16_t>(s, l.xq, l.wq, pre_.as<uint16_t>(), Epilogue::Bias, bias, {}, pre_row_amax_.as<float>());
@@ -450,7 +456,8 @@ class ProjectionStep {
     bool reduced_any = false;
     for (size_t i = 0; i < n; ++i) {
       Linear& l = linears_[order[i]];
-      if (auto e = cuda(cudaStreamWaitEvent(s, l.wt_ready, 0), "stream wait")) return e;
+      // W^T is first read behind the join with the side stream: waiting there keeps the main stream's kernels in one chain
+      if (auto e = cuda(cudaStreamWaitEvent(side_stream_, l.wt_ready, 0), "stream wait")) return e;
       if (auto e = backward_.backward_ms_eden<uint16_t>(s, backward_args(l, i))) return e;
       // last linear of its bucket: the bucket is complete, its all-reduce goes to the communication stream
       const bool bucket_done = i + 1 == n || linears_[order[i + 1]].bucket != l.bucket;

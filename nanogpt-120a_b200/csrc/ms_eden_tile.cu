@@ -12,7 +12,8 @@
 //  * the E2M1 codes are widened with add.f32.f16 instead of cvt.f32.f16;
 //  * the reciprocal of a block scale, 1 / (s * gs + eps), depends on the scale byte only: a table per CTA;
 //  * every range check of a chunk (corrected scale inside the normal E4M3 range, finite quotients) is folded into one
-//    predicate at the end; a chunk that fails it is quantized again by the generic code, from the source.
+//    predicate at the end; a chunk that fails it has its scale bytes computed by the general code from what the straight line
+//    left (general_scales), and is quantized again from the source only for infinite sums and NaN.
 //    The common path is one straight line, so the chains of the 16-groups overlap; with a branch per check they did not;
 //  * output addresses are a pointer per tile plus an offset per thread; the row operand leaves in 32-byte stores;
 //  * warps share nothing but the table, so that they drift apart and the FP32 of one runs beside the conversions of another:
@@ -132,14 +133,17 @@ struct PairCode {
   uint4 lo, hi;      // nibble bytes of the low-lane and the high-lane chunk
   uint32_t scales;   // scale bytes: low-lane chunk in bits 0..15, high-lane chunk in bits 16..31 (group 0, group 1)
   float amax_lo, amax_hi;
-  bool ok;           // false: some value lies outside the straight-line path's range, the outputs are not valid
+  bool ok;           // false: some corrected scale lies outside the straight-line path's range, `scales` is not valid
+  float corrected[4];  // corrected scale of each group, in the order of the scale bytes, ...
+  uint32_t blocks;     // ... and the E4M3 code of its block scale: what general_scales needs
 };
 
 // One 16-group of both chunks; H: its 16 rotated values.  Returns the two scale bytes (low lane in bits 0..7, high lane
 // in bits 8..15).
 __device__ __forceinline__ uint32_t ms_eden_group(const f32x2_t* H, uint32_t inv_table, float so, float inv6,
                                                   uint32_t scale_seed, uint32_t opaque_zero, uint32_t group_lo, uint32_t group_hi, uint2& nib_lo,
-                                                  uint2& nib_hi, float& ga_lo, float& ga_hi, bool& ok) {
+                                                  uint2& nib_hi, float& ga_lo, float& ga_hi, bool& ok, uint32_t& block_codes,
+                                                  float& corrected_lo, float& corrected_hi) {
   ga_lo = ga_hi = 0.0f;
 #pragma unroll
   for (int i = 0; i < 16; i += 2) {
@@ -186,8 +190,10 @@ __device__ __forceinline__ uint32_t ms_eden_group(const f32x2_t* H, uint32_t inv
   // value is 0 up to |x| = 1/4 and at least 1/2 beyond, so den is 0 or at least 1/8, and where the sums stay finite den is
   // below 2^71, its reciprocal far inside the normal range.  den = 0 and infinite sums end as NaN, which the range check
   // of the product catches like every product outside [2^-6, 448).
-  const uint32_t s0 = __float_as_uint(__uint_as_float(t0.y) * div_in_range(num_a, den_a));
-  const uint32_t s1 = __float_as_uint(__uint_as_float(t1.y) * div_in_range(num_b, den_b));
+  corrected_lo = __uint_as_float(t0.y) * div_in_range(num_a, den_a);
+  corrected_hi = __uint_as_float(t1.y) * div_in_range(num_b, den_b);
+  block_codes = codes;
+  const uint32_t s0 = __float_as_uint(corrected_lo), s1 = __float_as_uint(corrected_hi);
   ok = ok && s0 - 0x3c800000u < 0x43e00000u - 0x3c800000u && s1 - 0x3c800000u < 0x43e00000u - 0x3c800000u;
   return stochastic_code(s0, scale_seed, group_lo) | (stochastic_code(s1, scale_seed, group_hi) << 8);
 }
@@ -215,8 +221,12 @@ __device__ __forceinline__ PairCode ms_eden_chunk_pair(f32x2_t (&P)[32], uint32_
   r.ok = true;
   uint2 lo0, lo1, hi0, hi1;
   float a0, a1, b0, b1;
-  const uint32_t g0 = ms_eden_group(&P[0], inv_table, so, inv6, scale_seed, opaque_zero, group_lo, group_hi, lo0, hi0, a0, b0, r.ok);
-  const uint32_t g1 = ms_eden_group(&P[16], inv_table, so, inv6, scale_seed, opaque_zero, group_lo + 1, group_hi + 1, lo1, hi1, a1, b1, r.ok);
+  uint32_t codes0, codes1;
+  const uint32_t g0 = ms_eden_group(&P[0], inv_table, so, inv6, scale_seed, opaque_zero, group_lo, group_hi, lo0, hi0, a0, b0, r.ok,
+                                    codes0, r.corrected[0], r.corrected[2]);
+  const uint32_t g1 = ms_eden_group(&P[16], inv_table, so, inv6, scale_seed, opaque_zero, group_lo + 1, group_hi + 1, lo1, hi1, a1,
+                                    b1, r.ok, codes1, r.corrected[1], r.corrected[3]);
+  r.blocks = __byte_perm(codes0, codes1, 0x5140);
   r.lo = make_uint4(lo0.x, lo0.y, lo1.x, lo1.y);
   r.hi = make_uint4(hi0.x, hi0.y, hi1.x, hi1.y);
   r.scales = __byte_perm(g0, g1, 0x5140);  // low lane: g0, g1; high lane: g0, g1
@@ -225,8 +235,38 @@ __device__ __forceinline__ PairCode ms_eden_chunk_pair(f32x2_t (&P)[32], uint32_
   return r;
 }
 
-// A chunk again by the generic code, any values (zero groups, scales outside the normal range, NaN), from the source:
-// `valid` values `step` elements apart, zeros behind them, K index k0 ...
+// The four scale bytes of a thread's two chunks whatever their corrected scales are: below 2^-6, saturating, negative, zero
+// groups.  The nibbles of the straight-line path hold for those too, so nothing else has to be done again.  A group has
+// den = 0 exactly where all its nibbles are zero (ms_eden_group); its correction is one.  `lost`: a sum was infinite or an
+// input NaN, the chunks need the generic code.  By value and not inlined, so that it costs the straight-line path no
+// registers.  dY of a cross-entropy over 32000 columns comes this way in 21 to 94 % of its chunks, masked tokens and dead units
+// in all of theirs: the linear backward of 8192 tokens x 32000 takes 676 us with normal dY, 752 to 788 with that gradient
+// (logits N(0, 0.02) to N(0, 6)), against 1725 to 2190 when each thread quantized such chunks again.
+struct GeneralScales {
+  uint32_t bytes;
+  bool lost;
+};
+__device__ __noinline__ GeneralScales general_scales(float4 corrected, uint32_t blocks, uint4 lo, uint4 hi, uint32_t scale_seed,
+                                                     uint32_t group_lo, uint32_t group_hi) {
+  const float c[4] = {corrected.x, corrected.y, corrected.z, corrected.w};
+  const uint32_t nibbles[4] = {lo.x | lo.y, lo.z | lo.w, hi.x | hi.y, hi.z | hi.w};
+  GeneralScales r = {0u, false};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float v = nz((nibbles[i] & 0x77777777u) ? c[i] : nz(e4m3_value((blocks >> (8 * i)) & 0xffu)));
+    r.bytes |= stochastic_e4m3_scale(v, scale_seed, (i < 2 ? group_lo : group_hi) + (i & 1)) << (8 * i);
+    r.lost = r.lost || v != v;
+  }
+  return r;
+}
+__device__ __forceinline__ bool finish_scales(PairCode& code, uint32_t scale_seed, uint32_t group_lo, uint32_t group_hi) {
+  const GeneralScales g = general_scales(make_float4(code.corrected[0], code.corrected[1], code.corrected[2], code.corrected[3]),
+                                         code.blocks, code.lo, code.hi, scale_seed, group_lo, group_hi);
+  code.scales = g.bytes;
+  return g.lost;
+}
+
+// A chunk again by the generic code, any values (infinite sums, NaN), from the source: `valid` values `step` elements apart, zeros behind them, K index k0 ...
 template <typename T>
 __device__ __noinline__ void requantize(const T* src, uint32_t step, uint32_t valid, uint32_t sign_seed, uint32_t k0,
                                         const MsEdenOut* o, float gs, float so, uint32_t row, uint32_t chunk_in_row) {
@@ -470,7 +510,7 @@ __global__ void __launch_bounds__(256, 2)
       // dbias partials: four sequential 32-row sums per column, added below in the order ((q0 + q1) + q2) + q3
       if (kColSum) *reinterpret_cast<float2*>(&quarter_sum[buf][warp][2 * lane]) = make_float2(sum_lo, sum_hi);
       const uint32_t group = at.group + c0 * p.t.group_row_stride + (r0 >> 4);
-      const PairCode code =
+      PairCode code =
           ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.t.scale_seed, p.opaque_zero, group, group + row_step.group);
       const uint32_t row = c0 + 2 * lane, chunk_in_row = (r0 >> 5) + warp;
       bool first = true, second = true;
@@ -483,8 +523,10 @@ __global__ void __launch_bounds__(256, 2)
         first = k_inside && row < p.t.rows;
         second = k_inside && row + 1 < p.t.rows;
       }
+      bool lost = false;
+      if (!code.ok && first) lost = finish_scales(code, p.t.scale_seed, group, group + row_step.group);
       store_column_pair(code, tile_nibbles(p.t, c0, r0 >> 5), tile_scales(p.t, c0, r0 >> 5), at, row_step, first, second);
-      if (!code.ok && first) {  // rare
+      if (lost) {
         const uint32_t k0 = r0 + warp * kBlockRows, valid = kEdge ? p.src_rows - min(p.src_rows, k0) : 32u;
 #pragma unroll 1
         for (uint32_t h = 0; h < (second ? 2u : 1u); ++h)
@@ -493,6 +535,7 @@ __global__ void __launch_bounds__(256, 2)
       }
       if (kColSum) {
         // two buffers: a warp that is here again has passed the barrier of the tile between, behind the sums of this one
+        __syncwarp();
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (warp < 2 && (!kEdge || c0 + tid < p.src_cols))
           p.col_sum_partials[static_cast<size_t>(ty) * p.src_cols + c0 + tid] =
@@ -525,7 +568,7 @@ __global__ void __launch_bounds__(256, 2)
       __syncwarp();
       if (more) issue_block(next.ty, next.tx);
       const uint32_t group = at.group + r0 * p.r.group_row_stride + (c0 >> 4);
-      const PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.r.scale_seed, p.opaque_zero, group, group + 2);
+      PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.r.scale_seed, p.opaque_zero, group, group + 2);
       uint8_t* const nibbles = tile_nibbles(p.r, r0, c0 >> 5) + at.nibbles;
       uint8_t* const scales = tile_scales(p.r, r0, c0 >> 5) + at.scales;
       const uint32_t row = r0 + row_in_tile + lane, chunk_in_row = c0 >> 5;
@@ -535,6 +578,8 @@ __global__ void __launch_bounds__(256, 2)
         if (second) store_pad_scales(p.r, row, chunk_in_row + 1, false);
       }
       if (inside) {
+        bool lost = false;
+        if (!code.ok) lost = finish_scales(code, p.r.scale_seed, group, group + 2);
         if (wide_rows) {  // 32 nibble bytes in one store, four scale bytes in one
           asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(nibbles), "r"(code.lo.x),
                        "r"(code.lo.y), "r"(code.lo.z), "r"(code.lo.w), "r"(code.hi.x), "r"(code.hi.y), "r"(code.hi.z), "r"(code.hi.w)
@@ -548,7 +593,7 @@ __global__ void __launch_bounds__(256, 2)
             *reinterpret_cast<uint16_t*>(scales + 2) = static_cast<uint16_t>(code.scales >> 16);
           }
         }
-        if (!code.ok) {  // rare
+        if (lost) {
 #pragma unroll 1
           for (uint32_t h = 0; h < (second ? 2u : 1u); ++h) {
             const uint32_t k0 = c0 + 32 * h, valid = kEdge ? p.src_cols - min(p.src_cols, k0) : 32u;
@@ -663,7 +708,7 @@ __global__ void __launch_bounds__(128, 4)
       P[k + 1] = sub2(ua, ub);
     }
     const uint32_t group = at.group + c0 * p.t.group_row_stride + (r0 >> 4);
-    const PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.t.scale_seed, p.opaque_zero, group, group + row_step.group);
+    PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.t.scale_seed, p.opaque_zero, group, group + row_step.group);
     const uint32_t row = c0 + 2 * lane, chunk_in_row = (r0 >> 5) + warp;
     bool first = true, second = true;
     if (kEdge) {
@@ -675,13 +720,15 @@ __global__ void __launch_bounds__(128, 4)
       first = k_inside && row < p.t.rows;
       second = k_inside && row + 1 < p.t.rows;
     }
+    bool lost = false;
+    if (!code.ok && first) lost = finish_scales(code, p.t.scale_seed, group, group + row_step.group);
     store_column_pair(code, tile_nibbles(p.t, c0, r0 >> 5), tile_scales(p.t, c0, r0 >> 5), at, row_step, first, second);
     if (p.t.chunk_amax) {
       const size_t chunk = static_cast<size_t>(row) * (p.t.dst_row_len >> 5) + chunk_in_row;
       if (first) p.t.chunk_amax[chunk] = code.amax_lo;
       if (second) p.t.chunk_amax[chunk + (p.t.dst_row_len >> 5)] = code.amax_hi;
     }
-    if (!code.ok && first) {
+    if (lost) {
       // the generic code, from the signed values still staged
       for (uint32_t h = 0; h < (second ? 2u : 1u); ++h)
         requantize_staged(src + h * 4, kNvPitch, &p.t, gs, p.scale_override, row + h, chunk_in_row);

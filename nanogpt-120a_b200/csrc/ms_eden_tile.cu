@@ -12,8 +12,9 @@
 //  * the E2M1 codes are widened with add.f32.f16 instead of cvt.f32.f16;
 //  * the reciprocal of a block scale, 1 / (s * gs + eps), depends on the scale byte only: a table per CTA;
 //  * every range check of a chunk (corrected scale inside the normal E4M3 range, finite quotients) is folded into one
-//    predicate at the end; a chunk that fails it has its scale bytes computed by the general code from what the straight line
-//    left (general_scales), and is quantized again from the source only for infinite sums and NaN.
+//    predicate at the end; of a chunk that fails it the pair kernel computes the scale bytes by the general code from what the
+//    straight line left (general_scales), and quantizes it again from the source only for infinite sums and NaN; the
+//    transposer quantizes it again from the staged values;
 //    The common path is one straight line, so the chains of the 16-groups overlap; with a branch per check they did not;
 //  * output addresses are a pointer per tile plus an offset per thread; the row operand leaves in 32-byte stores;
 //  * warps share nothing but the table, so that they drift apart and the FP32 of one runs beside the conversions of another:
@@ -259,14 +260,13 @@ __device__ __noinline__ GeneralScales general_scales(float4 corrected, uint32_t 
   }
   return r;
 }
-__device__ __forceinline__ bool finish_scales(PairCode& code, uint32_t scale_seed, uint32_t group_lo, uint32_t group_hi) {
-  const GeneralScales g = general_scales(make_float4(code.corrected[0], code.corrected[1], code.corrected[2], code.corrected[3]),
-                                         code.blocks, code.lo, code.hi, scale_seed, group_lo, group_hi);
-  code.scales = g.bytes;
-  return g.lost;
+__device__ __forceinline__ GeneralScales general_scales(const PairCode& code, uint32_t scale_seed, uint32_t group_lo, uint32_t group_hi) {
+  return general_scales(make_float4(code.corrected[0], code.corrected[1], code.corrected[2], code.corrected[3]), code.blocks, code.lo,
+                        code.hi, scale_seed, group_lo, group_hi);
 }
 
-// A chunk again by the generic code, any values (infinite sums, NaN), from the source: `valid` values `step` elements apart, zeros behind them, K index k0 ...
+// A chunk again by the generic code, any values (infinite sums, NaN), from the source: `valid` values `step` elements apart,
+// zeros behind them, K index k0 ...
 template <typename T>
 __device__ __noinline__ void requantize(const T* src, uint32_t step, uint32_t valid, uint32_t sign_seed, uint32_t k0,
                                         const MsEdenOut* o, float gs, float so, uint32_t row, uint32_t chunk_in_row) {
@@ -324,16 +324,16 @@ __device__ __forceinline__ void store_pad_scales(const MsEdenOut& o, uint32_t ro
       *reinterpret_cast<uint16_t*>(o.scales + packed_scale_offset(r, chunk_in_row * 2, o.dst_row_len >> 6)) = 0x3838;
 }
 // A transposed operand's column pair: two output rows, one chunk each.
-__device__ __forceinline__ void store_column_pair(const PairCode& c, uint8_t* nibbles, uint8_t* scales, const ChunkOffsets& at,
-                                                  const ChunkOffsets& row_step, bool first, bool second) {
-  if (first) {
-    *reinterpret_cast<uint4*>(nibbles + at.nibbles) = c.lo;
-    *reinterpret_cast<uint16_t*>(scales + at.scales) = static_cast<uint16_t>(c.scales);
-  }
-  if (second) {
-    *reinterpret_cast<uint4*>(nibbles + at.nibbles + row_step.nibbles) = c.hi;
-    *reinterpret_cast<uint16_t*>(scales + at.scales + row_step.scales) = static_cast<uint16_t>(c.scales >> 16);
-  }
+__device__ __forceinline__ void store_column_scales(uint32_t bytes, uint8_t* scales, const ChunkOffsets& row_step, bool second) {
+  *reinterpret_cast<uint16_t*>(scales) = static_cast<uint16_t>(bytes);
+  if (second) *reinterpret_cast<uint16_t*>(scales + row_step.scales) = static_cast<uint16_t>(bytes >> 16);
+}
+__device__ __forceinline__ void store_column_pair(const PairCode& c, uint8_t* nibbles, uint8_t* scales, const ChunkOffsets& row_step,
+                                                  bool first, bool second) {
+  if (!first) return;  // `second` implies `first`
+  *reinterpret_cast<uint4*>(nibbles) = c.lo;
+  if (second) *reinterpret_cast<uint4*>(nibbles + row_step.nibbles) = c.hi;
+  store_column_scales(c.scales, scales, row_step, second);
 }
 
 // The tiles of a persistent CTA: tile, tile + gridDim.x, ... as (row, column) of the tile grid without a division
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(256, 2)
       // dbias partials: four sequential 32-row sums per column, added below in the order ((q0 + q1) + q2) + q3
       if (kColSum) *reinterpret_cast<float2*>(&quarter_sum[buf][warp][2 * lane]) = make_float2(sum_lo, sum_hi);
       const uint32_t group = at.group + c0 * p.t.group_row_stride + (r0 >> 4);
-      PairCode code =
+      const PairCode code =
           ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.t.scale_seed, p.opaque_zero, group, group + row_step.group);
       const uint32_t row = c0 + 2 * lane, chunk_in_row = (r0 >> 5) + warp;
       bool first = true, second = true;
@@ -523,13 +523,14 @@ __global__ void __launch_bounds__(256, 2)
         first = k_inside && row < p.t.rows;
         second = k_inside && row + 1 < p.t.rows;
       }
-      bool lost = false;
-      if (!code.ok && first) lost = finish_scales(code, p.t.scale_seed, group, group + row_step.group);
-      store_column_pair(code, tile_nibbles(p.t, c0, r0 >> 5), tile_scales(p.t, c0, r0 >> 5), at, row_step, first, second);
-      if (lost) {
+      uint8_t* const scales = tile_scales(p.t, c0, r0 >> 5) + at.scales;
+      store_column_pair(code, tile_nibbles(p.t, c0, r0 >> 5) + at.nibbles, scales, row_step, first, second);
+      if (!code.ok && first) {
+        const GeneralScales g = general_scales(code, p.t.scale_seed, group, group + row_step.group);
+        store_column_scales(g.bytes, scales, row_step, second);
         const uint32_t k0 = r0 + warp * kBlockRows, valid = kEdge ? p.src_rows - min(p.src_rows, k0) : 32u;
 #pragma unroll 1
-        for (uint32_t h = 0; h < (second ? 2u : 1u); ++h)
+        for (uint32_t h = g.lost ? 0u : 2u; h < (second ? 2u : 1u); ++h)
           requantize<T>(x + static_cast<size_t>(k0) * p.src_cols + row + h, p.src_cols, valid, p.sign_seed, k0 + p.t.sign_offset, &p.t,
                         gs, p.scale_override, row + h, chunk_in_row);
       }
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(256, 2)
       __syncwarp();
       if (more) issue_block(next.ty, next.tx);
       const uint32_t group = at.group + r0 * p.r.group_row_stride + (c0 >> 4);
-      PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.r.scale_seed, p.opaque_zero, group, group + 2);
+      const PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.r.scale_seed, p.opaque_zero, group, group + 2);
       uint8_t* const nibbles = tile_nibbles(p.r, r0, c0 >> 5) + at.nibbles;
       uint8_t* const scales = tile_scales(p.r, r0, c0 >> 5) + at.scales;
       const uint32_t row = r0 + row_in_tile + lane, chunk_in_row = c0 >> 5;
@@ -578,8 +579,6 @@ __global__ void __launch_bounds__(256, 2)
         if (second) store_pad_scales(p.r, row, chunk_in_row + 1, false);
       }
       if (inside) {
-        bool lost = false;
-        if (!code.ok) lost = finish_scales(code, p.r.scale_seed, group, group + 2);
         if (wide_rows) {  // 32 nibble bytes in one store, four scale bytes in one
           asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(nibbles), "r"(code.lo.x),
                        "r"(code.lo.y), "r"(code.lo.z), "r"(code.lo.w), "r"(code.hi.x), "r"(code.hi.y), "r"(code.hi.z), "r"(code.hi.w)
@@ -593,9 +592,12 @@ __global__ void __launch_bounds__(256, 2)
             *reinterpret_cast<uint16_t*>(scales + 2) = static_cast<uint16_t>(code.scales >> 16);
           }
         }
-        if (lost) {
+        if (!code.ok) {
+          const GeneralScales g = general_scales(code, p.r.scale_seed, group, group + 2);
+          *reinterpret_cast<uint16_t*>(scales) = static_cast<uint16_t>(g.bytes);
+          if (second) *reinterpret_cast<uint16_t*>(scales + 2) = static_cast<uint16_t>(g.bytes >> 16);
 #pragma unroll 1
-          for (uint32_t h = 0; h < (second ? 2u : 1u); ++h) {
+          for (uint32_t h = g.lost ? 0u : 2u; h < (second ? 2u : 1u); ++h) {
             const uint32_t k0 = c0 + 32 * h, valid = kEdge ? p.src_cols - min(p.src_cols, k0) : 32u;
             requantize<T>(x + static_cast<size_t>(row) * p.src_cols + k0, 1, valid, p.sign_seed, k0 + p.r.sign_offset, &p.r, gs,
                           p.scale_override, row, chunk_in_row + h);
@@ -708,7 +710,7 @@ __global__ void __launch_bounds__(128, 4)
       P[k + 1] = sub2(ua, ub);
     }
     const uint32_t group = at.group + c0 * p.t.group_row_stride + (r0 >> 4);
-    PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.t.scale_seed, p.opaque_zero, group, group + row_step.group);
+    const PairCode code = ms_eden_chunk_pair(P, table, p.scale_override, inv6, p.t.scale_seed, p.opaque_zero, group, group + row_step.group);
     const uint32_t row = c0 + 2 * lane, chunk_in_row = (r0 >> 5) + warp;
     bool first = true, second = true;
     if (kEdge) {
@@ -720,16 +722,16 @@ __global__ void __launch_bounds__(128, 4)
       first = k_inside && row < p.t.rows;
       second = k_inside && row + 1 < p.t.rows;
     }
-    bool lost = false;
-    if (!code.ok && first) lost = finish_scales(code, p.t.scale_seed, group, group + row_step.group);
-    store_column_pair(code, tile_nibbles(p.t, c0, r0 >> 5), tile_scales(p.t, c0, r0 >> 5), at, row_step, first, second);
+    uint8_t* const scales = tile_scales(p.t, c0, r0 >> 5) + at.scales;
+    store_column_pair(code, tile_nibbles(p.t, c0, r0 >> 5) + at.nibbles, scales, row_step, first, second);
     if (p.t.chunk_amax) {
       const size_t chunk = static_cast<size_t>(row) * (p.t.dst_row_len >> 5) + chunk_in_row;
       if (first) p.t.chunk_amax[chunk] = code.amax_lo;
       if (second) p.t.chunk_amax[chunk + (p.t.dst_row_len >> 5)] = code.amax_hi;
     }
-    if (lost) {
-      // the generic code, from the signed values still staged
+    if (!code.ok && first) {
+      // the generic code, from the signed values still staged (general_scales takes the kernel from 120 to 121 registers a
+      // thread, and one GPT-2-small layer at 8192 tokens with it from 541 to 545 us)
       for (uint32_t h = 0; h < (second ? 2u : 1u); ++h)
         requantize_staged(src + h * 4, kNvPitch, &p.t, gs, p.scale_override, row + h, chunk_in_row);
     }

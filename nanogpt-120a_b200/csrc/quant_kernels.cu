@@ -275,7 +275,7 @@ struct FourSixScale {
   float d6, y6;    // 6 gs + eps and its reciprocal
   float d4, y4;
   float limit;     // groups with a larger amax (the caller's amax was not theirs) take the generic code
-  float tie;       // candidates whose cheap errors are this close are compared by the exact ones (four_six_group)
+  bool cheap;      // gs inside the range where the cheap errors can decide
   bool plain;      // gs inside the range of the straight-line code
   __device__ __forceinline__ explicit FourSixScale(float amax) {
     // amax / 1536 correctly rounded (the remainder form, exact for every amax the straight-line code accepts)
@@ -287,7 +287,7 @@ struct FourSixScale {
     y6 = rcp_in_range(d6);
     y4 = rcp_in_range(d4);
     limit = plain ? gs * 0x1p20f : -1.0f;
-    tie = plain && gs >= 0x1p-30f ? 0x1p-33f : INFINITY;
+    cheap = gs >= 0x1p-30f && gs <= 0x1p80f;
   }
 };
 
@@ -320,10 +320,14 @@ __device__ __forceinline__ float candidate16(const Group16& g, float inv, uint32
 }
 
 // Squared quantization error of the group for one candidate as the reference rounds it: sum of (v - q * dq)^2 in butterfly
-// order (utils/nvfp4/quant/kernels/convert.rs:27-35).  Not inlined: it is rare, and its registers would be the kernel's.
-__device__ __noinline__ float exact_error16(const Group16 g, const uint2 nib, float dq, uint32_t opaque_zero) {
-  const f32x2_t(&V)[8] = g.V;
-  const f32x2_t dq2 = pack2(dq, dq);
+// order (utils/nvfp4/quant/kernels/convert.rs:27-35).
+__device__ __forceinline__ float exact_error16(const f32x2_t (&V)[8], float inv, float dq, uint32_t opaque_zero, uint2& nib) {
+  const f32x2_t inv2 = pack2(inv, inv), dq2 = pack2(dq, dq);
+  float lo[8], hi[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) unpack2(mul2(V[i], inv2), lo[i], hi[i]);
+  nib = make_uint2(cvt_e2m1x8(lo[0], lo[1], lo[2], lo[3], lo[4], lo[5], lo[6], lo[7]),
+                   cvt_e2m1x8(hi[0], hi[1], hi[2], hi[3], hi[4], hi[5], hi[6], hi[7]));
   float qa[8], qb[8];
   e2m1x8_unpacked(nib.x, opaque_zero, qa);
   e2m1x8_unpacked(nib.y, opaque_zero, qb);
@@ -336,6 +340,17 @@ __device__ __noinline__ float exact_error16(const Group16 g, const uint2 nib, fl
     a8[i] = e0 + e1;  // scalar: never contracted with the product
   }
   return ((a8[0] + a8[4]) + (a8[2] + a8[6])) + ((a8[1] + a8[5]) + (a8[3] + a8[7]));
+}
+
+// The choice by the exact errors, with the winner's nibbles.  Not inlined: its registers would be the kernel's.
+struct FourSixChoice {
+  uint2 nib;
+  bool six;
+};
+__device__ __noinline__ FourSixChoice exact_choice(const Group16 g, float inv6, float inv4, float dq6, float dq4, uint32_t opaque_zero) {
+  uint2 nib6, nib4;
+  const bool six = exact_error16(g.V, inv6, dq6, opaque_zero, nib6) <= exact_error16(g.V, inv4, dq4, opaque_zero, nib4);
+  return {six ? nib6 : nib4, six};
 }
 
 __device__ __forceinline__ float2 e4m3x2_values(uint32_t codes) {
@@ -370,34 +385,45 @@ __device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float g
     codes = c;
   }
   float2 s = e4m3x2_values(codes);
-  inv6 = rcp_in_range((s.x == 0.0f ? sc.gs : s.x * sc.gs) + kDenomEps);
-  inv4 = rcp_in_range((s.y == 0.0f ? sc.gs : s.y * sc.gs) + kDenomEps);
+  float step6 = s.x == 0.0f ? sc.gs : s.x * sc.gs, step4 = s.y == 0.0f ? sc.gs : s.y * sc.gs;
+  inv6 = rcp_in_range(step6 + kDenomEps);
+  inv4 = rcp_in_range(step4 + kDenomEps);
   if (!(ga <= sc.limit)) {
     const FourSixCandidates any = four_six_scales_any(ga, sc.gs);
     codes = any.codes, inv6 = any.inv6, inv4 = any.inv4;
     s = e4m3x2_values(codes);
+    step6 = s.x == 0.0f ? sc.gs : s.x * sc.gs, step4 = s.y == 0.0f ? sc.gs : s.y * sc.gs;
   }
-  const float dq6 = s.x * sc.gs, dq4 = s.y * sc.gs;
   Group16 g;
 #pragma unroll
   for (int i = 0; i < 8; ++i) g.V[i] = pack2(v[i], v[i + 8]);
-  uint2 nib6, nib4;
-  const float e6 = candidate16(g, inv6, opaque_zero, nib6) * (dq6 * dq6);
-  const float e4 = candidate16(g, inv4, opaque_zero, nib4) * (dq4 * dq4);
   // How far the cheap errors can be off, with u = 2^-24, D the exact differences v - q dq and |q dq| <= |v| + |D| <= 2 |v|
   // (2-norms over the group; rounding to the grid never takes a value further than its own size):
   //   cheap: v * inv is v / dq within 3.1 u (1e-20 is below u / 10 of dq where gs >= 2^-30), then the difference, the
   //          products, the sums and two scalings:       | sqrt(e) - |D| |   <= 3.1 u |v| + 5 u |D|
   //   exact: q dq, the difference, square and sums:      | sqrt(err) - |D| | <= 2 u |v| + 3.5 u |D|
-  // With |D| <= |v| <= 4 ga both candidates together shift sqrt(e6) - sqrt(e4) by less than 120 u ga.  Multiplied by
-  // sqrt(e6) + sqrt(e4) <= sqrt(2 (e6 + e4)) and squared: the order is certain where (e6 - e4)^2 exceeds
-  // 2 (120 u)^2 < 2^-33 times ga^2 (e6 + e4).  Otherwise -- also a zero scale, NaN, overflow, 15 groups in 100000 of normal
-  // values -- the exact errors decide.
-  bool six = e6 <= e4;
-  const float gap = e6 - e4;
-  if (!(s.x > 0.0f && gap * gap > sc.tie * ga * ga * (e6 + e4)))
-    six = exact_error16(g, nib6, dq6, opaque_zero) <= exact_error16(g, nib4, dq4, opaque_zero);
-  packed = six ? nib6 : nib4;
+  // A scale byte of zero stands for the step gs in v * inv and for dq = 0: all q are 0 then, D = v, and with gs as the step
+  // the same bounds hold.  With |D| <= |v| <= 4 ga both candidates together shift sqrt(e6) - sqrt(e4) by less than 120 u ga.
+  // Multiplied by sqrt(e6) + sqrt(e4) <= sqrt(2 (e6 + e4)) and squared: the order is certain where (e6 - e4)^2 exceeds
+  // 2 (120 u)^2 < 2^-33 times ga^2 (e6 + e4).  Two candidates of one scale byte (zero groups, saturated ones) are the same
+  // candidate: "six", where the error is a number.  Otherwise -- NaN, overflow, gs outside the range of the bounds -- the
+  // exact errors decide.
+  bool six = false, certain = false;
+  if (sc.cheap) {
+    uint2 nib6, nib4;
+    const float e6 = candidate16(g, inv6, opaque_zero, nib6) * (step6 * step6);
+    const float e4 = candidate16(g, inv4, opaque_zero, nib4) * (step4 * step4);
+    const float gap = e6 - e4;
+    six = e6 <= e4;
+    packed = six ? nib6 : nib4;
+    certain = gap * gap > 0x1p-33f * ga * ga * (e6 + e4);
+    if (!certain) certain = (codes & 0xffu) == codes >> 8 && e6 == e4;
+  }
+  if (!certain) {
+    const FourSixChoice exact = exact_choice(g, inv6, inv4, s.x * sc.gs, s.y * sc.gs, opaque_zero);
+    six = exact.six;
+    packed = exact.nib;
+  }
   if (decoded_amax) {
     // Largest decoded magnitude of the group, (q * scale) * gs as the stand-alone NVFP4 amax kernel
     // evaluates it (utils/nvfp4/quant/kernels/ms_eden/amax.rs:23-64): rounding to E2M1 is monotonic

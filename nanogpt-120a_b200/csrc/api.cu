@@ -274,14 +274,14 @@ static int validate_ms_eden(const nvfp4_ms_eden_args* a) {
 // Row operand + transposed operand of one matrix in a single pass (same scale, same signs).
 static int ms_eden_pair(void* stream, nvfp4_ms_eden_args rows, nvfp4_ms_eden_args transposed,
                         float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr,
-                        void* zero = nullptr, uint64_t zero_words = 0) {
+                        void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false) {
   rows.src_kind = NVFP4_SRC_F32_ROWS;
   transposed.src_kind = NVFP4_SRC_F32_TRANSPOSED;
   int rc = validate_ms_eden(&rows);
   if (rc) return rc;
   rc = validate_ms_eden(&transposed);
   if (rc) return rc;
-  return launch_ms_eden_pair(S(stream), rows, transposed, col_sum_partials, amax_in, gs_out, zero, zero_words);
+  return launch_ms_eden_pair(S(stream), rows, transposed, col_sum_partials, amax_in, gs_out, zero, zero_words, beside_others);
 }
 
 static nvfp4_ms_eden_args rows_args(const float* x, uint8_t* out_fp4, uint8_t* out_scales, float* out_gss,
@@ -1034,7 +1034,8 @@ static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_
                     gemm_adds_into_output(dweight_gemm(a->dweight, a->dweight_dtype, T, I, O));
   zero_words = dweight_is_zero ? zero_words / 16 : 0;
   // one pass over dY for both orientations (+ column sums)
-  rc = ms_eden_pair(stream, q, qt, partials, amax_in, amax_in ? a->e_h.global_scale : nullptr, a->dweight, zero_words);
+  rc = ms_eden_pair(stream, q, qt, partials, amax_in, amax_in ? a->e_h.global_scale : nullptr, a->dweight, zero_words,
+                    ts != stream);
   if (rc) return rc;
   if (fuse_dbias) rc = launch_col_sum_reduce(s, partials, a->dbias, ms_eden_pair_row_tiles(T), O);
   return rc;

@@ -44,10 +44,11 @@ int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a, const float* ama
 // per-row-tile column sums [ms_eden_pair_row_tiles(rows)][cols] for launch_col_sum_reduce.
 // amax_in / gs_out (only when ms_eden_pair_takes_amax): the kernel derives the global scale from amax_in[0]
 // itself and writes it to gs_out[0]; rows.global_scale / transposed.global_scale are then not read.
+// beside_others: kernels of another stream are waiting for room on the SMs that this one would take by starting early.
 // zero (likewise only when ms_eden_pair_takes_amax): zero_words 16-byte words that the kernel clears beside its work.
 int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed,
                         float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr,
-                        void* zero = nullptr, uint64_t zero_words = 0);
+                        void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false);
 bool ms_eden_pair_takes_amax(const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed);
 bool ms_eden_pair_is_tiled(const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed);
 uint32_t ms_eden_pair_row_tiles(uint32_t rows);

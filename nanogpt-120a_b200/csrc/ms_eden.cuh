@@ -251,7 +251,7 @@ struct MsEdenTileParams {
 };
 
 bool ms_eden_pair_has_tile_form(const void* x, int dtype, uint32_t cols);
-int launch_ms_eden_pair_tiles(cudaStream_t s, const MsEdenTileParams& p, int dtype);
+int launch_ms_eden_pair_tiles(cudaStream_t s, const MsEdenTileParams& p, int dtype, bool beside_others);
 bool ms_eden_nvfp4_has_tile_form(const uint8_t* bytes, const uint8_t* scales, uint32_t cols);
 int launch_ms_eden_nvfp4_tiles(cudaStream_t s, const MsEdenTileParams& p, bool rowwise);
 

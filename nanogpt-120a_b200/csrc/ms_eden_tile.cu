@@ -759,21 +759,33 @@ int opt_in_shared(int bytes) {
 }
 
 template <typename T, bool kColSum, bool kEdge>
-int launch_pair(cudaStream_t s, const MsEdenTileParams& p) {
+int launch_pair(cudaStream_t s, const MsEdenTileParams& p, bool beside_others) {
   constexpr int kStage = 8 * PairBlock<T>::kBytes;
   const int rc = opt_in_shared<ms_eden_pair_kernel<T, kColSum, kEdge>>(kStage);
   if (rc) return rc;
   const uint32_t tiles_x = (p.src_cols + kTileCols - 1) / kTileCols;
   const uint32_t tiles = tiles_x * ((p.src_rows + kTileRows - 1) / kTileRows);
   const uint32_t resident = 148u * 2u;
+  // With a tile for every resident CTA this kernel takes every register of the chip.  Started early, its CTAs sit there waiting
+  // for the amax before it while the transposers of the other stream, enqueued earlier, may find no room until it ends.  A
+  // backward call behind another kernel, L2 cold, dY 8192 x 2304 bf16: 92 us started early, 105 with some side streams (which
+  // of them differs from process to process), 87 otherwise; 1000 x 3072 53 and 67 against 52.  Calls back to back gain 1 to 3
+  // us from the early start below 5000 tokens and lose 1 to 2 above.  With fewer CTAs (512 x 3072: 192) there is room for
+  // both streams.
+  if (beside_others && tiles >= resident) {
+    ms_eden_pair_kernel<T, kColSum, kEdge><<<resident, 256, kStage, s>>>(p, tiles_x, tiles);
+    count_launch();
+    return static_cast<int>(cudaGetLastError());
+  }
   return launch_chained(ms_eden_pair_kernel<T, kColSum, kEdge>, tiles < resident ? tiles : resident, 256, kStage, s, p, tiles_x,
                         tiles);
 }
 
 template <typename T>
-int launch_pair_of(cudaStream_t s, const MsEdenTileParams& p, bool edge) {
-  if (p.col_sum_partials) return edge ? launch_pair<T, true, true>(s, p) : launch_pair<T, true, false>(s, p);
-  return edge ? launch_pair<T, false, true>(s, p) : launch_pair<T, false, false>(s, p);
+int launch_pair_of(cudaStream_t s, const MsEdenTileParams& p, bool edge, bool beside_others) {
+  if (p.col_sum_partials)
+    return edge ? launch_pair<T, true, true>(s, p, beside_others) : launch_pair<T, true, false>(s, p, beside_others);
+  return edge ? launch_pair<T, false, true>(s, p, beside_others) : launch_pair<T, false, false>(s, p, beside_others);
 }
 
 }  // namespace
@@ -783,10 +795,11 @@ int launch_pair_of(cudaStream_t s, const MsEdenTileParams& p, bool edge) {
 bool ms_eden_pair_has_tile_form(const void* x, int dtype, uint32_t cols) {
   return (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && cols % (dtype == NVFP4_DTYPE_BF16 ? 8u : 4u) == 0;
 }
-int launch_ms_eden_pair_tiles(cudaStream_t s, const MsEdenTileParams& p, int dtype) {
+int launch_ms_eden_pair_tiles(cudaStream_t s, const MsEdenTileParams& p, int dtype, bool beside_others) {
   const bool edge = p.src_rows % 128 != 0 || p.src_cols % 128 != 0 || p.t.dst_row_len != p.src_rows ||
                     p.r.dst_row_len != p.src_cols;
-  return dtype == NVFP4_DTYPE_BF16 ? launch_pair_of<__nv_bfloat16>(s, p, edge) : launch_pair_of<float>(s, p, edge);
+  return dtype == NVFP4_DTYPE_BF16 ? launch_pair_of<__nv_bfloat16>(s, p, edge, beside_others)
+                                   : launch_pair_of<float>(s, p, edge, beside_others);
 }
 
 bool ms_eden_nvfp4_has_tile_form(const uint8_t* bytes, const uint8_t* scales, uint32_t cols) {

@@ -1659,7 +1659,8 @@ bool ms_eden_pair_takes_amax(const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_ar
 }
 
 int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_args& t,
-                        float* col_sum_partials, const float* amax_in, float* gs_out, void* zero, uint64_t zero_words) {
+                        float* col_sum_partials, const float* amax_in, float* gs_out, void* zero, uint64_t zero_words,
+                        bool beside_others) {
   const uint32_t rows = r.rows, cols = r.cols;
   if ((amax_in || zero_words) && !ms_eden_pair_takes_amax(r, t)) return static_cast<int>(cudaErrorInvalidValue);
   if (!ms_eden_pair_is_tiled(r, t)) {
@@ -1686,7 +1687,7 @@ int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& r, const nvfp4
   p.gs_out = gs_out;
   p.zero = static_cast<uint4*>(zero);
   p.zero_words = zero_words;
-  if (ms_eden_pair_has_tile_form(r.x, r.src_dtype, cols)) return launch_ms_eden_pair_tiles(s, p, r.src_dtype);
+  if (ms_eden_pair_has_tile_form(r.x, r.src_dtype, cols)) return launch_ms_eden_pair_tiles(s, p, r.src_dtype, beside_others);
   if (r.src_dtype == NVFP4_DTYPE_BF16) {
     launch_tile<0, __nv_bfloat16, true>(s, p);
   } else {

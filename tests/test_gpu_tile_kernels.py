@@ -224,3 +224,32 @@ def test_backward_clears_dweight_before_it_adds(pkg, dev, tokens, in_dim, out_di
     assert bool(memory[:offset].isnan().all()) and bool(memory[offset + out_dim * in_dim:].isnan().all())
     torch.cuda.synchronize()
     assert pkg.read_device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,out_dim", [(128, 64 * 295), (128, 64 * 296), (250, 64 * 148), (300, 64 * 100)])
+def test_pair_beside_a_side_stream(pkg, dev, tokens, out_dim, dtype):
+    """One CTA less than the chip holds, as many, more tiles than CTAs: beside the transposers of a side stream, where the pair
+    kernel starts early or not, the operands and gradients of a call that has one stream, call after call."""
+    q, bwd, in_dim = pkg.Nvfp4QuantModule(), pkg.LinearBackwardModule(), 64
+    xq = q.quantize_four_six(bf16_normal(781, (tokens, in_dim)).to(dev), rowwise=True, packed=True, decoded_amax=True)
+    wq = q.quantize_four_six(bf16_normal(782, (out_dim, in_dim), 0.02).to(dev), rowwise=False, packed=True)
+    es = [bf16_normal(783 + i, (tokens, out_dim), 1e-3).to(dev).to(dtype) for i in range(2)]
+    sc, side = pkg.LinearBackwardScratch(tokens, in_dim, out_dim, dev), pkg.SideStream(dev)
+
+    def call(e, stream):
+        # bf16 gradients: GEMMs into f32 of this K split it and add their partial sums in the order they arrive
+        grads = bwd.backward_ms_eden(e=e, weight=wq, input=xq, scratch=sc, sign_seed=SIGN, scale_seed=SCALE, side=stream,
+                                     grad_dtype=torch.bfloat16)
+        return [t.clone() for t in (*grads, sc.e_h["bytes"], sc.e_h["scales_packed"], sc.e_t_h["bytes"], sc.e_t_h["scales_packed"])]
+
+    want = []
+    for e in es:
+        torch.cuda.synchronize()
+        want.append(call(e, None))
+        torch.cuda.synchronize()
+    got = [call(es[i & 1], side) for i in range(8)]
+    torch.cuda.synchronize()
+    for i, tensors in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(tensors, want[i & 1])), i
+    assert pkg.read_device_status() == 0

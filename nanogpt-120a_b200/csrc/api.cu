@@ -1,6 +1,7 @@
 // extern "C" boundary of the NVFP4 projection path: argument checks, composition of the
 // kernels into the reference's host-level operations, and nothing else.  Each entry cites
 // the reference method it replaces in include/nvfp4_b200.h.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -831,7 +832,6 @@ int nvfp4_tc_matmul_ms_eden(void* stream, const float* a, const float* b_t, floa
   return nvfp4_gemm(stream, &g);
 }
 
-// The gradient GEMMs over quantized operands: dX = e_h . weight_t_h^T, dW = e_t_h . input_t_h^T.
 // Shapes, types and output of dW = dY^T . X.
 static nvfp4_gemm_args dweight_gemm(void* dweight, int dweight_dtype, uint32_t T, uint32_t I, uint32_t O) {
   nvfp4_gemm_args g;
@@ -848,6 +848,7 @@ static nvfp4_gemm_args dweight_gemm(void* dweight, int dweight_dtype, uint32_t T
   return g;
 }
 
+// The gradient GEMMs over quantized operands: dX = e_h . weight_t_h^T, dW = e_t_h . input_t_h^T.
 // dweight_is_zero: dweight holds zeros already
 static int backward_gemms(cudaStream_t s, const uint8_t* eh_b, const uint8_t* eh_s, const float* eh_g,
                           const uint8_t* wt_b, const uint8_t* wt_s, const float* wt_g, const uint8_t* et_b,
@@ -932,6 +933,33 @@ int nvfp4_linear_backward_prepare_weight_t(void* stream, const nvfp4_linear_back
       !op.global_scale || !op.chunk_amax)
     return invalid("linear_backward_prepare_weight_t: null pointer");
   return backward_weight_t(stream, a);
+}
+
+// Whether dweight lies apart from everything a backward call reads or writes ahead of its dW GEMM.  A caller may put dW into
+// memory that only the steps before it need (dY, the saved X, the operands of dX): then it must not be touched earlier.
+static bool dweight_lies_apart(const nvfp4_linear_backward_args* a, size_t dweight_bytes) {
+  const size_t T = a->token_count, I = a->input_dim, O = a->output_dim;
+  const uint32_t ok = padded_k(a->output_dim), tk = padded_k(a->token_count);
+  const uintptr_t begin = reinterpret_cast<uintptr_t>(a->dweight), end = begin + dweight_bytes;
+  auto apart = [&](const void* p, size_t bytes) {
+    const uintptr_t q = reinterpret_cast<uintptr_t>(p);
+    return q >= end || q + bytes <= begin;
+  };
+  auto element = [](int dtype) { return dtype == NVFP4_DTYPE_F32 ? size_t{4} : size_t{2}; };
+  auto scales = [](size_t rows, size_t cols, int layout) {
+    return layout == NVFP4_SCALES_PACKED ? nvfp4_scale_packed_len(static_cast<uint32_t>(rows), static_cast<uint32_t>(cols)) : rows * cols / 16;
+  };
+  auto operand_apart = [&](const nvfp4_ms_eden_operand& op, size_t rows, uint32_t k, size_t amax_words) {
+    return apart(op.bytes, rows * k / 2) && apart(op.scales_packed, scales(rows, k, NVFP4_SCALES_PACKED)) &&
+           apart(op.global_scales, rows * 4) && apart(op.global_scale, 4) && apart(op.chunk_amax, amax_words * 4);
+  };
+  const size_t e_chunks = std::max<size_t>(chunks1024(static_cast<uint64_t>(T) * O), a->precomputed_e_amax_chunks);
+  return apart(a->e, T * O * element(a->e_dtype)) && apart(a->w_bytes, O * I / 2) &&
+         apart(a->w_scales, scales(O, I, a->w_scale_layout)) && apart(a->w_global, 4) && apart(a->x_bytes, T * I / 2) &&
+         apart(a->x_scales, scales(T, I, a->x_scale_layout)) && apart(a->x_globals, T * 4) && apart(a->x_decoded_amax, 4) &&
+         apart(a->e_global_scale_override, 4) && apart(a->dinput, T * I * element(a->dinput_dtype)) && apart(a->dbias, O * 4) &&
+         operand_apart(a->e_h, T, ok, e_chunks) && operand_apart(a->weight_t_h, I, ok, 1) && operand_apart(a->e_t_h, O, tk, 1) &&
+         operand_apart(a->input_t_h, I, tk, 1);
 }
 
 // Everything of nvfp4_linear_backward_ms_eden that runs between the fork onto the caller's side stream and the
@@ -1031,7 +1059,8 @@ static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_
   // two GEMMs cost c_attn at 8192 tokens 3 us and kept the second GEMM from being set up early.
   uint64_t zero_words = static_cast<uint64_t>(O) * I * (a->dweight_dtype == NVFP4_DTYPE_F32 ? 4 : 2);
   dweight_is_zero = ms_eden_pair_takes_amax(q, qt) && ((reinterpret_cast<uintptr_t>(a->dweight) | zero_words) & 15u) == 0 &&
-                    gemm_adds_into_output(dweight_gemm(a->dweight, a->dweight_dtype, T, I, O));
+                    gemm_adds_into_output(dweight_gemm(a->dweight, a->dweight_dtype, T, I, O)) &&
+                    dweight_lies_apart(a, zero_words);
   zero_words = dweight_is_zero ? zero_words / 16 : 0;
   // one pass over dY for both orientations (+ column sums)
   rc = ms_eden_pair(stream, q, qt, partials, amax_in, amax_in ? a->e_h.global_scale : nullptr, a->dweight, zero_words,

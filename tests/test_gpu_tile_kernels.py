@@ -253,3 +253,41 @@ def test_pair_beside_a_side_stream(pkg, dev, tokens, out_dim, dtype):
     for i, tensors in enumerate(got):
         assert all(torch.equal(a, b) for a, b in zip(tensors, want[i & 1])), i
     assert pkg.read_device_status() == 0
+
+
+@pytest.mark.parametrize("with_side", [False, True])
+@pytest.mark.parametrize("inside", [None, "e", "input", "e_h", "weight_t_h"])
+def test_backward_dweight_inside_what_the_steps_before_it_read(pkg, dev, inside, with_side):
+    """dW may lie in memory that is free by the time its GEMM runs: dY, the saved X, the operands of dX.  Then it is not cleared
+    ahead of that.  Calls follow one another with changing inputs and nothing synchronised in between; dX and dbias are the
+    bits of calls that ran alone, dW the same partial sums in another order."""
+    q, bwd, tokens, in_dim, out_dim = pkg.Nvfp4QuantModule(), pkg.LinearBackwardModule(), 4352, 64, 64
+    wq = q.quantize_four_six(bf16_normal(761, (out_dim, in_dim), 0.02).to(dev), rowwise=False, packed=True)
+    side = pkg.SideStream(dev) if with_side else None
+    source = [(bf16_normal(762 + i, (tokens, out_dim), 1e-3).to(dev), bf16_normal(772 + i, (tokens, in_dim)).to(dev)) for i in range(3)]
+
+    def call(i, place):
+        e, x = source[i]
+        e, xq = e.clone(), q.quantize_four_six(x, rowwise=True, packed=True, decoded_amax=True)
+        memory = {None: None, "e": e, "input": xq.bytes, "e_h": sc.e_h["bytes"], "weight_t_h": sc.weight_t_h["bytes"]}[place]
+        dw = torch.full((out_dim, in_dim), float("nan"), device=dev) if memory is None else \
+            memory.view(-1).view(torch.float32)[: out_dim * in_dim].view(out_dim, in_dim)
+        dx, dw, db = bwd.backward_ms_eden(e=e, weight=wq, input=xq, scratch=sc, sign_seed=SIGN + i, scale_seed=SCALE, dweight=dw,
+                                          side=side)
+        return dx, dw.clone(), db
+
+    sc = pkg.LinearBackwardScratch(tokens, in_dim, out_dim, dev)
+    # room for dW inside the operands' buffers (they are larger than the call needs; the extents it passes stay the same)
+    sc.weight_t_h["bytes"] = torch.empty(out_dim * in_dim * 4, dtype=torch.uint8, device=dev)
+    want = []
+    for i in range(3):
+        torch.cuda.synchronize()
+        want.append(call(i, None))
+        torch.cuda.synchronize()
+    for repeat in range(4):
+        got = [call(i, inside) for i in range(3)]
+        torch.cuda.synchronize()
+        for (dx, dw, db), (dx0, dw0, db0) in zip(got, want):
+            assert torch.equal(dx, dx0) and torch.equal(db, db0)
+            assert float((dw - dw0).norm() / dw0.norm()) <= 32 * 2.0 ** -24
+    assert pkg.read_device_status() == 0

@@ -581,7 +581,8 @@ typedef struct nvfp4_linear_backward_args {
   nvfp4_ms_eden_operand e_h, e_t_h, weight_t_h, input_t_h;
   void* dinput;                      /* [token][in]                                           */
   int dinput_dtype;                  /* NVFP4_DTYPE_*                                         */
-  void* dweight;                     /* [out][in]                                             */
+  void* dweight;                     /* [out][in]; may be cleared ahead of the GEMMs, on `stream`, unless it
+                                        lies in memory of another argument that the steps before its GEMM use */
   int dweight_dtype;                 /* NVFP4_DTYPE_* (f32 lets long-K GEMMs split K)         */
   float* dbias;                      /* f32[out] or NULL                                      */
   uint32_t token_count, input_dim, output_dim;

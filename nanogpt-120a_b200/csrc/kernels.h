@@ -104,7 +104,9 @@ void count_launch();
 // Launches a kernel that may start while the kernel before it in the stream drains (programmatic stream serialization).
 // Only for kernels whose every thread waits for that one before its first access to memory
 // (wait_for_prior_then_allow_next): launch latency and the start of the thread blocks then cost nothing behind another
-// kernel.
+// kernel.  The main path's kernels are; those for shapes and alignments that it does not take (ms_eden_kernel,
+// ms_eden_tile_kernel, four_six_padded_kernel, decode_kernel, scale_pack_kernel, packed_scale_pad_kernel, bias_grad_kernel) and
+// relu2_backward_kernel are launched plainly: their loads are not pinned behind the wait.
 template <typename... Params, typename... Args>
 int launch_chained(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t shared_bytes, cudaStream_t s, const Args&... args) {
   cudaLaunchAttribute attr;

@@ -3,7 +3,7 @@
 //
 // Same bytes as the generic kernels of quant_kernels.cu (one thread per 32-chunk, utils/nvfp4/quant/kernels/
 // ms_eden/**), organised for the rate at which instructions issue: in the pair kernel the schedulers issue on 67 % of the
-// cycles, the FMA pipe is busy 61 % of them and the ALU 38 %, HBM 24 %.  Measured costs per warp instruction and scheduler are
+// cycles, the FMA pipe is busy 61 % of them and the ALU 37 %, HBM 25 %.  Measured costs per warp instruction and scheduler are
 // 1 cycle for scalar FP32 (mixed f32 += bf16 * bf16 included, either half of a word), 2 for the packed f32x2 forms, and 2 for
 // integer, logic and conversion instructions; the two pipes overlap as far as register reads allow (a butterfly stage beside
 // two conversions 5.3 cycles instead of 8, beside two three-input maxima 7.7).  So:

@@ -259,10 +259,10 @@ __global__ void ms_eden_scale_from_amax_kernel(const float* __restrict__ amax, f
 // candidate scales, two sets of nibbles and two error sums.  Only which error is the smaller leaves the group, so the sums
 // are taken the cheap way first (differences in scaled units, fused multiply-adds) and in the reference's order and
 // roundings only where the two lie closer together than both ways can differ (8192 x 768 bf16 rowwise 9.35 -> 8.65 us, 65536
-// x 768 57.4 -> 53.0; and out-of-line code that returns by value and keeps nothing in local memory 8.4 and 50.2).  The scalar side of a group -- two quotients by the global
-// scale, two reciprocals, two E4M3 conversions -- is straight-line code for global scales inside [2^-80, 2^80]
-// (four IEEE divisions with their range checks and branches cost a third of the group before); other global scales,
-// NaN included, take the generic code per group.
+// x 768 57.4 -> 53.0).  Code for rare cases stands out of line, returns by value and keeps nothing in local memory (8.4 and
+// 50.2).  The scalar side of a group -- two quotients by the global scale, two reciprocals, two E4M3 conversions -- is
+// straight-line code for global scales inside [2^-80, 2^80] (four IEEE divisions with their range checks and branches cost a
+// third of the group before); other global scales, NaN included, take the generic code per group.
 
 __device__ __forceinline__ float four_six_global_scale(float amax) {
   // utils/nvfp4/quant/kernels/four_six/helpers.rs:33-39 with scale_override = 1.0
@@ -503,7 +503,6 @@ __device__ __forceinline__ float cta_max_of(const float* partials, uint32_t coun
 // scales are packed (pad rows of the plane hold 1.0, the nibbles have none).  Rowwise: amax holds one value per row;
 // otherwise `amax_count` partial maxima whose maximum is the tensor's, published in out_amax when asked for.
 // decoded_amax (optional, zeroed by the launcher): max |decoded value| of the quantized tensor.
-// Measured, 8192 x 768 bf16 with a tensor scale: 8.5 -> 5.4 us (HBM allows 2.5).
 template <typename Source, bool kRowwise, bool kPacked, bool kQuads>
 __global__ void __launch_bounds__(256, 4)
     four_six_kernel(Source src, const float* __restrict__ amax, uint32_t amax_count, float* __restrict__ out_amax,

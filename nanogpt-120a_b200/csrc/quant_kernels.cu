@@ -591,7 +591,7 @@ struct RawGroup<__nv_bfloat16> {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         v[8 * i + 2 * j] = widen_bf16_lo(t[j]);
-        v[8 * i + 2 * j + 1] = __uint_as_float(t[j] & 0xffff0000u);
+        v[8 * i + 2 * j + 1] = widen_bf16_hi(t[j]);
       }
     }
   }

@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       smem_gen + (smem_bar - smem_base) + 8 * (2 * kMaxStages + 7 + 2 * C::kSfSets + 2 * C::kStoreBufs));
   volatile uint32_t* abort_flag = tmem_base_ptr + 1;
 
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 #ifdef NVFP4_GEMM_TRACE
   uint32_t trace_n = 0;
 #endif
@@ -627,24 +627,27 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == 0) {
     // ===================== TMA producer =====================
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, issued = 0, runs = 0, prev_n = 0xffffffffu;
-      bool ok = true;
-      for (uint32_t w = w_begin; w < w_end && ok; w += w_step) {
-        uint32_t m_blk, n_blk, split;
-        decode(w, m_blk, n_blk, split);
-        const uint32_t kt_begin = split * p.k_tiles_per_split;
-        const uint32_t kt_end = min(p.num_k_tiles, kt_begin + p.k_tiles_per_split);
-        const uint32_t first_blk128 = n_blk * kBlockN / 128u;
-        const uint32_t blks128 = min(static_cast<uint32_t>(C::kSfBlocks), p.sfb_blocks128 - first_blk128);
-        if (p.b_resident && n_blk != prev_n) {
-          // new column block: wait until the MMAs of the previous run have retired, then load the panel
-          if (runs > 0 && !mbar_wait(bar_b_empty, (runs - 1) & 1u, abort_flag, kStatusProducerTimeout, p.wait_timeout_ns)) {
-            ok = false;
-            break;
-          }
-          const uint32_t sf_total = p.k_atoms * kSfTileBytes * blks128;
-          mbar_expect_tx(bar_b_full, p.num_k_tiles * C::kBStageBytes + sf_total);
+    // Warp uniform like the MMA issuer: from inside a single-lane branch every copy took about 140 cycles to issue, and the six of
+    // a streamed k-tile 840 of the 1170 to 1300 the k-tile had (480 now).  8192 x 768 x K 3072 bf16 14.7 -> 13.2 us, 8192 x
+    // 32000 x K 768 142 -> 118, 16 x 2304 x K 768 5.7 -> 4.8, 65536 x 3072 x K 768 111 -> 101.
+    uint32_t stage = 0, phase = 0, issued = 0, runs = 0, prev_n = 0xffffffffu;
+    bool ok = true;
+    for (uint32_t w = w_begin; w < w_end && ok; w += w_step) {
+      uint32_t m_blk, n_blk, split;
+      decode(w, m_blk, n_blk, split);
+      const uint32_t kt_begin = split * p.k_tiles_per_split;
+      const uint32_t kt_end = min(p.num_k_tiles, kt_begin + p.k_tiles_per_split);
+      const uint32_t first_blk128 = n_blk * kBlockN / 128u;
+      const uint32_t blks128 = min(static_cast<uint32_t>(C::kSfBlocks), p.sfb_blocks128 - first_blk128);
+      if (p.b_resident && n_blk != prev_n) {
+        // new column block: wait until the MMAs of the previous run have retired, then load the panel
+        const bool free = runs == 0 || mbar_wait(bar_b_empty, (runs - 1) & 1u, abort_flag, kStatusProducerTimeout, p.wait_timeout_ns);
+        if (!__all_sync(0xffffffffu, free)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
+          mbar_expect_tx(bar_b_full, p.num_k_tiles * C::kBStageBytes + p.k_atoms * kSfTileBytes * blks128);
           for (uint32_t kt = 0; kt < p.num_k_tiles; ++kt) {
             const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
             tma_load_2d(smem_b + kt * C::kBStageBytes, &tmap_b, bar_b_full, static_cast<int32_t>(kt * kBlockKBytes),
@@ -654,62 +657,64 @@ __global__ void __launch_bounds__(kThreads, 1)
                         p.sfb + (static_cast<size_t>(first_blk128 + i) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
                         atoms * kSfTileBytes, bar_b_full);
           }
-          prev_n = n_blk;
-          ++runs;
         }
-        for (uint32_t kt = kt_begin; kt < kt_end; ++kt) {
-          if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, kStatusProducerTimeout, p.wait_timeout_ns)) {
-            ok = false;
-            break;
-          }
-          GEMM_TRACE(0, 1, true);
+        __syncwarp();
+        prev_n = n_blk;
+        ++runs;
+      }
+      // scale blocks of A inside the matrix (the second row half of a tall tile may lie below it)
+      const uint32_t a_blks = min(static_cast<uint32_t>(kMHalves), p.sfa_blocks128 - m_blk * kMHalves);
+      for (uint32_t kt = kt_begin; kt < kt_end; ++kt) {
+        const bool free = mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, kStatusProducerTimeout, p.wait_timeout_ns);
+        if (!__all_sync(0xffffffffu, free)) {
+          ok = false;
+          break;
+        }
+        GEMM_TRACE(0, 1, lane == 0);
+        // test hook: this stage is never armed nor loaded, so its consumers' waits run out
+        const bool skip = (p.debug_flags & 1u) && blockIdx.x == 0 && issued == 0;
+        if (!skip && elect_one()) {
           const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
           const uint32_t sf_bytes = atoms * kSfTileBytes;
           const uint32_t full = bar_full + 8 * stage;
-          if ((p.debug_flags & 1u) && blockIdx.x == 0 && issued == 0) {
-            // test hook: this stage is never armed nor loaded, so its consumers' waits run out
-            ++issued;
-            if (++stage == stages) {
-              stage = 0;
-              phase ^= 1u;
-            }
-            continue;
-          }
-          // scale blocks of A inside the matrix (the second row half of a tall tile may lie below it)
-          const uint32_t a_blks = min(static_cast<uint32_t>(kMHalves), p.sfa_blocks128 - m_blk * kMHalves);
           if (p.b_resident) {
             mbar_expect_tx(full, kAStageBytes + sf_bytes * a_blks);
           } else {
             mbar_expect_tx(full, kAStageBytes + C::kBStageBytes + sf_bytes * (a_blks + blks128));
             tma_load_2d(smem_b + stage * C::kBStageBytes, &tmap_b, full, static_cast<int32_t>(kt * kBlockKBytes),
                         static_cast<int32_t>(n_blk * kBlockN));
-            for (uint32_t i = 0; i < blks128; ++i)
-              bulk_load(smem_sfb + stage * C::kSfbStageBytes + i * kSfBlockStageBytes,
-                        p.sfb + (static_cast<size_t>(first_blk128 + i) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
-                        sf_bytes, full);
+#pragma unroll
+            for (uint32_t i = 0; i < static_cast<uint32_t>(C::kSfBlocks); ++i)
+              if (i < blks128)
+                bulk_load(smem_sfb + stage * C::kSfbStageBytes + i * kSfBlockStageBytes,
+                          p.sfb + (static_cast<size_t>(first_blk128 + i) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
+                          sf_bytes, full);
           }
           tma_load_2d(smem_a + stage * kAStageBytes, &tmap_a, full, static_cast<int32_t>(kt * kBlockKBytes),
                       static_cast<int32_t>(m_blk * kBlockM));
-          for (uint32_t h = 0; h < a_blks; ++h)
-            bulk_load(smem_sfa + stage * kSfaStageBytes + h * kSfBlockStageBytes,
-                      p.sfa + (static_cast<size_t>(m_blk * kMHalves + h) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
-                      sf_bytes, full);
-          GEMM_TRACE(0, 2, true);
-          ++issued;
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+#pragma unroll
+          for (uint32_t h = 0; h < static_cast<uint32_t>(kMHalves); ++h)
+            if (h < a_blks)
+              bulk_load(smem_sfa + stage * kSfaStageBytes + h * kSfBlockStageBytes,
+                        p.sfa + (static_cast<size_t>(m_blk * kMHalves + h) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
+                        sf_bytes, full);
+        }
+        __syncwarp();
+        GEMM_TRACE(0, 2, lane == 0);
+        ++issued;
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      if (!ok) {
-        // aborting: give copies already in flight a bounded chance to land before the CTA exits
-        const uint32_t pending = min(issued, stages);
-        for (uint32_t i = 0; i < pending; ++i) {
-          const uint32_t s = (stage + stages - 1 - i) % stages;
-          const uint32_t ph = (s < stage) ? phase : (phase ^ 1u);
-          for (int spin = 0; spin < 4096 && !mbar_try_wait(bar_full + 8 * s, ph); ++spin) {
-          }
+    }
+    if (!ok) {
+      // aborting: give copies already in flight a bounded chance to land before the CTA exits
+      const uint32_t pending = min(issued, stages);
+      for (uint32_t i = 0; i < pending; ++i) {
+        const uint32_t s = (stage + stages - 1 - i) % stages;
+        const uint32_t ph = (s < stage) ? phase : (phase ^ 1u);
+        for (int spin = 0; spin < 4096 && !mbar_try_wait(bar_full + 8 * s, ph); ++spin) {
         }
       }
     }
@@ -930,12 +935,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 2 || warp == 3) {
     // ===================== store warps (one per epilogue group) =====================
-    // Issuing a TMA store takes about 400 cycles and its read of the staging buffer as long again.  This thread waits for
-    // both, so that between two sub-tiles the epilogue warps have only the next sub-tile to do.  Measured against one
-    // epilogue thread issuing the stores between two barriers of its group: 65536 x 2304 and x 3072 bf16 at K = 768,
-    // 87.3 -> 83.0 us and 116.9 -> 111.3 us, 3.6 TB/s of output where a plain fill reaches 3.8.  A third or fourth buffer
-    // in place of an A stage gains nothing: at these sizes HBM takes the writes no faster.
-    if (kTmaStore && lane == 0) {
+    // Issuing a TMA store takes about 250 cycles and its read of the staging buffer up to 1000.  This warp waits for both, so
+    // that between two sub-tiles the epilogue warps have only the next sub-tile to do.  Measured against one epilogue thread
+    // issuing the stores between two barriers of its group: 65536 x 2304 and x 3072 bf16 at K = 768, 87.3 -> 83.0 us and
+    // 116.9 -> 111.3 us.
+    if (kTmaStore) {
       const uint32_t eg = warp - 2u;
       uint32_t buf = 0, phase = 0, tile_iter = 0, issued = 0;
       bool ok = true;
@@ -955,9 +959,12 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int item = load_item;
           load_item += 2;
           if (!item_valid(item, load_m, load_n)) continue;
-          mbar_expect_tx(bar_stored + 8 * slot, kStoreStageBytes);  // parts outside the matrix arrive as zeros
-          tma_load_2d(smem_store + slot * kStoreStageBytes, &tmap_out, bar_stored + 8 * slot, item_x(item, load_n),
-                      item_y(item, load_m));
+          if (elect_one()) {
+            mbar_expect_tx(bar_stored + 8 * slot, kStoreStageBytes);  // parts outside the matrix arrive as zeros
+            tma_load_2d(smem_store + slot * kStoreStageBytes, &tmap_out, bar_stored + 8 * slot, item_x(item, load_n),
+                        item_y(item, load_m));
+          }
+          __syncwarp();
           ++loads;
           return;
         }
@@ -977,9 +984,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!item_valid(item, m_blk, n_blk)) continue;
             due += pace;
             bool staged = false;
-            while (!staged && clock32() - t0 < due) staged = mbar_try_wait(bar_staged + 8 * (eg * kRing + buf), phase);
+            while (!staged && __any_sync(0xffffffffu, clock32() - t0 < due))
+              staged = __any_sync(0xffffffffu, mbar_try_wait(bar_staged + 8 * (eg * kRing + buf), phase));
             if (staged) break;
-            tma_prefetch_2d(&tmap_out, item_x(item, n_blk), item_y(item, m_blk));
+            if (elect_one()) tma_prefetch_2d(&tmap_out, item_x(item, n_blk), item_y(item, m_blk));
+            __syncwarp();
           }
         }
         for (int item = first_item_of(eg, tile_iter); item < kItems && ok; item += 2) {
@@ -987,28 +996,33 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int32_t x = item_x(item, n_blk), y = item_y(item, m_blk);
           for (int pass = 0; pass < item_passes; ++pass) {
             const uint32_t slot = eg * kRing + buf;
-            if (!mbar_wait(bar_staged + 8 * slot, phase, abort_flag, kStatusEpilogueTimeout, downstream_timeout_ns)) {
+            const bool staged = mbar_wait(bar_staged + 8 * slot, phase, abort_flag, kStatusEpilogueTimeout, downstream_timeout_ns);
+            if (!__all_sync(0xffffffffu, staged)) {
               ok = false;
               break;
             }
-            const CUtensorMap* map = item_passes == 2 && pass == 0 ? &tmap_aux : &tmap_out;
-            if (!kResidual && p.k_splits > 1)
-              tma_reduce_add_2d(map, smem_store + slot * kStoreStageBytes, x, y);
-            else
-              tma_store_2d(map, smem_store + slot * kStoreStageBytes, x, y);
-            bulk_commit_group();
-            // the buffer the epilogue needs next is handed back as soon as its store has read it: this one with a
-            // single buffer, the previous one with two; with a load to come into it, this one at once
-            if (kResidual) {
-              bulk_wait_group_read<0>();
-              load_next(slot);
-            } else {
-              bulk_wait_group_read<static_cast<int>(kRing) - 1>();
-              if (kRing == 1)
-                mbar_arrive(bar_stored + 8 * slot);
-              else if (issued > 0)
-                mbar_arrive(bar_stored + 8 * (eg * kRing + (buf ^ 1u)));
+            // the same lane is elected every time: it is the one whose bulk groups these are
+            if (elect_one()) {
+              const CUtensorMap* map = item_passes == 2 && pass == 0 ? &tmap_aux : &tmap_out;
+              if (!kResidual && p.k_splits > 1)
+                tma_reduce_add_2d(map, smem_store + slot * kStoreStageBytes, x, y);
+              else
+                tma_store_2d(map, smem_store + slot * kStoreStageBytes, x, y);
+              bulk_commit_group();
+              // the buffer the epilogue needs next is handed back as soon as its store has read it: this one with a
+              // single buffer, the previous one with two; with a load to come into it, this one at once
+              if (kResidual) {
+                bulk_wait_group_read<0>();
+              } else {
+                bulk_wait_group_read<static_cast<int>(kRing) - 1>();
+                if (kRing == 1)
+                  mbar_arrive(bar_stored + 8 * slot);
+                else if (issued > 0)
+                  mbar_arrive(bar_stored + 8 * (eg * kRing + (buf ^ 1u)));
+              }
             }
+            __syncwarp();
+            if (kResidual) load_next(slot);
             ++issued;
             if (++buf == kRing) {
               buf = 0;
@@ -1017,7 +1031,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      bulk_wait_group0();  // stores complete before the CTA exits
+      if (elect_one()) bulk_wait_group0();  // stores complete before the CTA exits
+      __syncwarp();
       if (kResidual && !ok) {
         // aborting: give loads already in flight a bounded chance to land; load j is phase j / kRing of its buffer
         for (uint32_t j = loads > kRing ? loads - kRing : 0; j < loads; ++j)

@@ -489,28 +489,31 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   const uint32_t stages = p.stages;
   const uint32_t b_slots = p.b_resident ? p.num_k_tiles : stages;
+  // No more column sets than stages: a scale-factor warp that has a free set for a k-tile, whose predecessor there has been
+  // issued, then knows that the `full` barrier it is going to arrive on is in that k-tile's phase.
+  const uint32_t sf_sets = min(static_cast<uint32_t>(C::kSfSets), stages);
   const uint32_t smem_a = smem_base;
   const uint32_t smem_b = smem_a + stages * kAStageBytes;
   const uint32_t smem_sfa = smem_b + b_slots * C::kBStageBytes;
   const uint32_t smem_sfb = smem_sfa + stages * kSfaStageBytes;
   const uint32_t smem_store = smem_sfb + b_slots * C::kSfbStageBytes;  // staging ring, 16 KB buffers, 1024-byte aligned
   const uint32_t smem_bar = smem_store + C::kStoreBufs * kStoreStageBytes;
-  // barrier block: full[8], empty[8], tmem_full[2], tmem_empty[2], b_full, b_empty, sf_full[4], sf_empty[4],
-  // mma_drain, staged[4], stored[4], tmem base, abort flag
+  // barrier block: full[8], empty[8], scales_full[8], tmem_full[2], tmem_empty[2], b_full, b_empty, sf_empty[4], mma_drain,
+  // staged[4], stored[4], tmem base, abort flag
   const uint32_t smem_bias = smem_bar + 512;  // kBlockN floats per epilogue group
   const uint32_t bar_full = smem_bar;
   const uint32_t bar_empty = bar_full + 8 * kMaxStages;
-  const uint32_t bar_tmem_full = bar_empty + 8 * kMaxStages;
+  const uint32_t bar_scales_full = bar_empty + 8 * kMaxStages;  // the scale tiles of a stage, ahead of its operands
+  const uint32_t bar_tmem_full = bar_scales_full + 8 * kMaxStages;
   const uint32_t bar_tmem_empty = bar_tmem_full + 16;
   const uint32_t bar_b_full = bar_tmem_empty + 16;
   const uint32_t bar_b_empty = bar_b_full + 8;
-  const uint32_t bar_sf_full = bar_b_empty + 8;
-  const uint32_t bar_sf_empty = bar_sf_full + 8 * C::kSfSets;
+  const uint32_t bar_sf_empty = bar_b_empty + 8;
   const uint32_t bar_mma_drain = bar_sf_empty + 8 * C::kSfSets;  // abort path only: issued MMAs have retired
   const uint32_t bar_staged = bar_mma_drain + 8;                 // one per staging buffer: a sub-tile is in it
   const uint32_t bar_stored = bar_staged + 8 * C::kStoreBufs;    // one per staging buffer: its TMA store has read it
   uint32_t* tmem_base_ptr = reinterpret_cast<uint32_t*>(
-      smem_gen + (smem_bar - smem_base) + 8 * (2 * kMaxStages + 7 + 2 * C::kSfSets + 2 * C::kStoreBufs));
+      smem_gen + (smem_bar - smem_base) + 8 * (3 * kMaxStages + 7 + C::kSfSets + 2 * C::kStoreBufs));
   volatile uint32_t* abort_flag = tmem_base_ptr + 1;
 
   const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -526,13 +529,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (p.aux) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_aux)) : "memory");
     }
     for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(bar_full + 8 * s, 1);
-      mbar_init(bar_empty + 8 * s, 1 + 4);  // the MMA commit and the four scale-factor warps
+      mbar_init(bar_full + 8 * s, 1 + 4);  // the operands, and the scale factors of the four warps
+      mbar_init(bar_empty + 8 * s, 1);
+      mbar_init(bar_scales_full + 8 * s, 1);
     }
-    for (int s = 0; s < C::kSfSets; ++s) {
-      mbar_init(bar_sf_full + 8 * s, 4);
-      mbar_init(bar_sf_empty + 8 * s, 1);
-    }
+    for (int s = 0; s < C::kSfSets; ++s) mbar_init(bar_sf_empty + 8 * s, 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(bar_tmem_full + 8 * a, 1);
       mbar_init(bar_tmem_empty + 8 * a, 8);
@@ -676,28 +677,28 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!skip && elect_one()) {
           const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
           const uint32_t sf_bytes = atoms * kSfTileBytes;
-          const uint32_t full = bar_full + 8 * stage;
-          if (p.b_resident) {
-            mbar_expect_tx(full, kAStageBytes + sf_bytes * a_blks);
-          } else {
-            mbar_expect_tx(full, kAStageBytes + C::kBStageBytes + sf_bytes * (a_blks + blks128));
-            tma_load_2d(smem_b + stage * C::kBStageBytes, &tmap_b, full, static_cast<int32_t>(kt * kBlockKBytes),
-                        static_cast<int32_t>(n_blk * kBlockN));
-#pragma unroll
-            for (uint32_t i = 0; i < static_cast<uint32_t>(C::kSfBlocks); ++i)
-              if (i < blks128)
-                bulk_load(smem_sfb + stage * C::kSfbStageBytes + i * kSfBlockStageBytes,
-                          p.sfb + (static_cast<size_t>(first_blk128 + i) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
-                          sf_bytes, full);
-          }
-          tma_load_2d(smem_a + stage * kAStageBytes, &tmap_a, full, static_cast<int32_t>(kt * kBlockKBytes),
-                      static_cast<int32_t>(m_blk * kBlockM));
+          // The scale tiles first and on a barrier of their own: they are in tensor memory when the operands land.  On one
+          // barrier with them a stage was occupied 460 cycles longer.
+          const uint32_t scales = bar_scales_full + 8 * stage, full = bar_full + 8 * stage;
+          mbar_expect_tx(scales, sf_bytes * (a_blks + (p.b_resident ? 0u : blks128)));
 #pragma unroll
           for (uint32_t h = 0; h < static_cast<uint32_t>(kMHalves); ++h)
             if (h < a_blks)
               bulk_load(smem_sfa + stage * kSfaStageBytes + h * kSfBlockStageBytes,
                         p.sfa + (static_cast<size_t>(m_blk * kMHalves + h) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
-                        sf_bytes, full);
+                        sf_bytes, scales);
+          if (!p.b_resident) {
+#pragma unroll
+            for (uint32_t i = 0; i < static_cast<uint32_t>(C::kSfBlocks); ++i)
+              if (i < blks128)
+                bulk_load(smem_sfb + stage * C::kSfbStageBytes + i * kSfBlockStageBytes,
+                          p.sfb + (static_cast<size_t>(first_blk128 + i) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
+                          sf_bytes, scales);
+          }
+          const int32_t x = static_cast<int32_t>(kt * kBlockKBytes);
+          mbar_expect_tx(full, kAStageBytes + (p.b_resident ? 0 : C::kBStageBytes));
+          tma_load_2d(smem_a + stage * kAStageBytes, &tmap_a, full, x, static_cast<int32_t>(m_blk * kBlockM));
+          if (!p.b_resident) tma_load_2d(smem_b + stage * C::kBStageBytes, &tmap_b, full, x, static_cast<int32_t>(n_blk * kBlockN));
         }
         __syncwarp();
         GEMM_TRACE(0, 2, lane == 0);
@@ -714,7 +715,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (uint32_t i = 0; i < pending; ++i) {
         const uint32_t s = (stage + stages - 1 - i) % stages;
         const uint32_t ph = (s < stage) ? phase : (phase ^ 1u);
-        for (int spin = 0; spin < 4096 && !mbar_try_wait(bar_full + 8 * s, ph); ++spin) {
+        for (int spin = 0; spin < 4096 && !(mbar_try_wait(bar_scales_full + 8 * s, ph) && mbar_try_wait(bar_full + 8 * s, ph)); ++spin) {
         }
       }
     }
@@ -725,7 +726,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // from inside a single-lane branch instead costs ~140 cycles per tcgen05.mma.
     {
       constexpr uint32_t idesc = make_idesc<kBlockN>();
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, runs = 0, prev_n = 0xffffffffu, sf_set = 0, sf_phase = 0;
+      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, runs = 0, prev_n = 0xffffffffu, sf_set = 0;
       bool ok = true;
       for (uint32_t w = w_begin; w < w_end && ok; w += w_step) {
         uint32_t m_blk, n_blk, split;
@@ -749,10 +750,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         tcgen05_fence_after();
         const uint32_t tmem_acc = tmem_base + acc * C::kAccCols;
         for (uint32_t kt = kt_begin; kt < kt_end; ++kt) {
-          // The scale-factor warps arrive on `sf_full` only after they have seen the stage's `full` barrier
-          // complete (operands and scale tiles share it), so this one wait covers both: operands in
-          // shared memory and column set `sf_set` filled.
-          const bool ready = mbar_wait(bar_sf_full + 8 * sf_set, sf_phase, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns);
+          // operands in shared memory, scale factors in column set `sf_set`
+          const bool ready = mbar_wait(bar_full + 8 * stage, phase, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns);
           if (!__all_sync(0xffffffffu, ready)) {
             ok = false;
             break;
@@ -784,10 +783,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           __syncwarp();
           GEMM_TRACE(1, 13, lane == 0);
-          if (++sf_set == C::kSfSets) {
-            sf_set = 0;
-            sf_phase ^= 1u;
-          }
+          if (++sf_set == sf_sets) sf_set = 0;
           if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
@@ -843,13 +839,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         ++runs;
       }
       for (uint32_t kt = kt_begin; kt < kt_end; ++kt) {
-        if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns) ||
-            !mbar_wait(bar_sf_empty + 8 * sf_set, sf_phase ^ 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) {
+        if (!mbar_wait(bar_scales_full + 8 * stage, phase, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) {
           ok = false;
           break;
         }
         GEMM_TRACE(2, 20, warp == 8 && lane == 0);
-        tcgen05_fence_after();
         const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
         const uint32_t b_slot = p.b_resident ? kt : stage;
         const uint32_t sfa_s = smem_sfa + stage * kSfaStageBytes + lane * 16;
@@ -874,6 +868,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                            : "r"(sfb_s + i * kSfBlockStageBytes + kb * kSfTileBytes));
           }
         }
+        if (!mbar_wait(bar_sf_empty + 8 * sf_set, sf_phase ^ 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) {
+          ok = false;
+          break;
+        }
+        tcgen05_fence_after();
+        __syncwarp();
         if constexpr (kBlockN == 192) {
           // Six scale words (192 rows of B) per k-atom out of the eight loaded: words 0..5 when the tile
           // starts on a 128-row block boundary (even column block), words 2..7 when it starts in the
@@ -918,12 +918,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(bar_sf_full + 8 * sf_set);  // scale factors visible to the MMA issuer
-          mbar_arrive(bar_empty + 8 * stage);     // this warp no longer reads the smem stage
-        }
+        // scale factors visible to the MMA issuer; that the slot has been read follows from the MMAs that need them
+        if (lane == 0) mbar_arrive(bar_full + 8 * stage);
         GEMM_TRACE(2, 21, warp == 8 && lane == 0);
-        if (++sf_set == C::kSfSets) {
+        if (++sf_set == sf_sets) {
           sf_set = 0;
           sf_phase ^= 1u;
         }

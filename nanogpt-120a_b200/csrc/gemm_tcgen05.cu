@@ -18,9 +18,8 @@
 //   warps 8..11 move the scale factors shared -> tensor memory (tcgen05.st).
 // Three tile widths.  BLOCK_N = 128 and 192 double buffer the accumulator (2 x 192 accumulator
 // columns + 3 x 40 scale-factor columns fill the 512 columns of tensor memory), so the epilogue of
-// one tile overlaps the main loop of the next; the 256-column tile has one accumulator buffer,
-// which every epilogue warp hands back as soon as its last tcgen05.ld of the tile has landed in
-// registers.  Every mbarrier wait is bounded: on expiry the kernel records a status word, drains,
+// one tile overlaps the main loop of the next; the 256-column accumulators of consecutive tiles share
+// 128 columns, which the epilogue takes first, so that all but a quarter of it overlaps as well.  Every mbarrier wait is bounded: on expiry the kernel records a status word, drains,
 // frees its tensor memory and returns.
 //
 // No thread-block clusters, no multicast: every load reads this GPU's own memory.
@@ -63,10 +62,12 @@ constexpr uint32_t kStatusProducerTimeout = 1u, kStatusMmaTimeout = 2u, kStatusE
 // streaming GEMMs are bound by the operand bytes an SM can pull from L2, and the tall tile moves 21 % fewer of
 // them per flop than 128 x 256.  Its two 192-column accumulators and two scale-factor column sets fill tensor
 // memory (2 x 192 + 2 x 56 = 496 of 512 columns), so the accumulator is single buffered.
-template <int kBlockM, int kBlockN>
+// kPanel: 0 streaming, else resident with a B panel of up to so many k-tiles
+template <int kBlockM, int kBlockN, int kPanel>
 struct Cfg {
+  static constexpr bool kResident = kPanel != 0;
   static constexpr int kMHalves = kBlockM / kRowBlock;
-  static_assert(kBlockM == 128 || (kBlockM == 256 && kBlockN == 192), "unsupported tile shape");
+  static_assert(kBlockM == 128 || (kBlockM == 256 && kBlockN == 192 && !kResident), "unsupported tile shape");
   static constexpr int kAStageBytes = kMHalves * kAHalfBytes;
   static constexpr int kSfaStageBytes = kMHalves * kSfBlockStageBytes;
   // 128-row scale-factor blocks of B a tile can touch: a 192-column tile starts either on a block
@@ -76,25 +77,33 @@ struct Cfg {
   static constexpr int kSfbStageBytes = kSfBlocks * kSfBlockStageBytes;
   static constexpr int kAccStages = (kBlockN == 256 || kMHalves == 2) ? 1 : 2;
   static constexpr int kAccCols = kMHalves * kBlockN;  // columns of one accumulator buffer (row halves side by side)
-  // Scale factors live in a ring of column sets behind the accumulators (one set per k-tile), so
-  // the copies for the next k-tile never overwrite columns an MMA in flight reads.
+  // The 256-column accumulator lies at columns 0 and 128 in turn: a tile's MMAs wait for the half of the tile before it that
+  // they overwrite, which the epilogue takes first, and run beside its other half.  With one fixed accumulator they waited
+  // 1900 cycles of a tile's 4700.  Together with the panel's scale factors kept in tensor memory, two staging buffers a group
+  // and A prefetched: 65536 x 2304 x K 768 bf16 76 -> 65 us, x 3072 99 -> 86, 8192 x 3072 17.5 -> 15.3; streaming, where only
+  // the accumulator changed: 4096 x 1024 x K 8192 f32 19.5 -> 18.2.
+  static constexpr bool kRotate = kBlockN == 256;
+  static constexpr int kAccRegion = kRotate ? 384 : kAccStages * kAccCols;
+  // Scale factors behind the accumulators.  Streaming: a ring of column sets (one per k-tile, A and B), so the copies for
+  // the next k-tile never overwrite columns an MMA in flight reads.  Resident: those of the whole B panel, and a ring for A.
   static constexpr int kSfaSetCols = kMHalves * 4 * kKAtomsPerStage;
   static constexpr int kSfbColsPerAtom = kBlockN / 32;
-  static constexpr int kSfSetCols = kSfaSetCols + kSfbColsPerAtom * kKAtomsPerStage;
-  static constexpr int kSfSets = kMHalves == 2 ? 2 : (kBlockN == 192 ? 3 : 4);
-  static constexpr int kTmemSfa = kAccStages * kAccCols;   // A scale factors of set 0
-  static constexpr int kTmemSfb = kTmemSfa + kSfaSetCols;  // B scale factors of set 0
-  static constexpr int kStreamStageBytes = kAStageBytes + kBStageBytes + kSfaStageBytes + kSfbStageBytes;
-  static constexpr int kResidentStageBytes = kAStageBytes + kSfaStageBytes;
-  static constexpr int kPanelSlotBytes = kBStageBytes + kSfbStageBytes;
-  // epilogue staging ring: deep for the narrow tile (short-K GEMMs are epilogue bound), shallow for
-  // the wide ones (long-K GEMMs need the shared memory for pipeline stages)
-  static constexpr int kStoreBufs = kBlockN == 128 ? 4 : 2;
+  static constexpr int kSfbTileCols = kSfbColsPerAtom * kKAtomsPerStage;
+  static constexpr int kTmemPanel = kAccRegion;           // resident: B scale factors of the panel
+  static constexpr int kTmemSfa = kAccRegion + kPanel * kSfbTileCols;  // set 0: A, streaming B behind it
+  static constexpr int kSfSetCols = kSfaSetCols + (kResident ? 0 : kSfbTileCols);
+  static constexpr int kSfSets = (kTmemCols - kTmemSfa) / kSfSetCols < 4 ? (kTmemCols - kTmemSfa) / kSfSetCols : 4;
+  static constexpr int kStageBytes = kAStageBytes + kSfaStageBytes;                    // of the ring, A side
+  static constexpr int kSlotBytes = kBStageBytes + (kResident ? 0 : kSfbStageBytes);  // of the panel or the ring, B side
+  // epilogue staging ring: deep for the narrow tile and for short K, which are epilogue bound, shallow where the shared memory
+  // goes to pipeline stages (streaming wide tiles) or the panel (four k-tiles of 192 columns: with two more buffers three A
+  // stages are left instead of five, 8192 x 32000 x K 1024 193 us against 154)
+  static constexpr int kStoreBufs = kBlockN == 128 || kPanel == 3 ? 4 : 2;
   static constexpr int kBiasSlots = (kBlockN + 127) / 128;  // bias values a thread of an epilogue group fetches
   static constexpr int kFixedBytes =
       1024 /*alignment slack*/ + kStoreBufs * kStoreStageBytes + 512 /*barriers*/ +
       2 * kBlockN * 4 /*bias of the tile, one copy per epilogue group*/;
-  static_assert(kTmemSfa + kSfSets * kSfSetCols <= kTmemCols, "tensor memory overflow");
+  static_assert(kSfSets >= 2, "tensor memory overflow");
 };
 
 // How a sub-tile leaves: registers to memory (outputs a tensor map cannot describe, a bf16 residual), staging buffer and
@@ -118,9 +127,8 @@ struct GemmParams {
   uint32_t num_m_blocks, num_n_blocks, k_atoms, sfa_blocks128, sfb_blocks128;
   uint32_t k_splits, k_tiles_per_split, num_k_tiles;
   uint32_t stages;  // depth of the A (and, when streaming, B) ring
-  int b_resident;   // the B panel of a column block stays in shared memory (short K)
   uint32_t resident_cpn;  // resident mode: CTAs per column block (0 = contiguous tile ranges instead)
-  int mode, epilogue, vec_store, tma_store;
+  int mode, epilogue, vec_store, tma_store, stream_out;
   float weight;
   uint64_t wait_timeout_ns;  // limit of every mbarrier wait
   uint32_t debug_flags;      // bit 0: CTA 0 never loads its first k-tile (exercises the bounded waits)
@@ -210,6 +218,9 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int32_t 
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y)
                : "memory");
 }
+__device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
@@ -220,6 +231,14 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t sr
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                    reinterpret_cast<uint64_t>(map)),
                "r"(src), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void tma_store_2d_streaming(const CUtensorMap* map, uint32_t src, int32_t x, int32_t y) {
+  uint64_t policy;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3}], [%1], %4;" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(src), "r"(x), "r"(y), "l"(policy)
                : "memory");
 }
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, uint32_t src, int32_t x, int32_t y) {
@@ -345,6 +364,12 @@ __device__ __forceinline__ float load_prior(const float* p) {
   float v;
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
   return v;
+}
+__device__ __forceinline__ void load_prior(const uint8_t* p, uint32_t* r) {  // 16 bytes
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void lds_128(uint32_t addr, uint32_t* r) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 __device__ __forceinline__ uint32_t load_prior(const uint8_t* p) {
   uint32_t v;
@@ -472,12 +497,13 @@ struct SubTile<__nv_bfloat16> {
 // Streaming mode: one B slot per pipeline stage.  Resident mode (short K): the whole
 // [kBlockN x K] B panel of the current column block stays in shared memory -- one slot per
 // k-tile -- while a CTA walks down the row blocks, so only A tiles stream through the ring.
-template <int kBlockM, int kBlockN, typename OutT, StorePath kStore>
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel>
 __global__ void __launch_bounds__(kThreads, 1)
     nvfp4_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                               const __grid_constant__ CUtensorMap tmap_out,
                               const __grid_constant__ CUtensorMap tmap_aux, const GemmParams p) {
-  using C = Cfg<kBlockM, kBlockN>;
+  using C = Cfg<kBlockM, kBlockN, kPanel>;
+  constexpr bool kResident = C::kResident;
   constexpr bool kTmaStore = kStore != StorePath::kDirect, kResidual = kStore == StorePath::kTmaResidual;
   static_assert(!kResidual || sizeof(OutT) == 4, "the residual stream of the TMA path is f32");
   constexpr int kMHalves = C::kMHalves;
@@ -488,7 +514,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
 
   const uint32_t stages = p.stages;
-  const uint32_t b_slots = p.b_resident ? p.num_k_tiles : stages;
+  const uint32_t b_slots = kResident ? p.num_k_tiles : stages;
   // No more column sets than stages: a scale-factor warp that has a free set for a k-tile, whose predecessor there has been
   // issued, then knows that the `full` barrier it is going to arrive on is in that k-tile's phase.
   const uint32_t sf_sets = min(static_cast<uint32_t>(C::kSfSets), stages);
@@ -496,7 +522,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t smem_b = smem_a + stages * kAStageBytes;
   const uint32_t smem_sfa = smem_b + b_slots * C::kBStageBytes;
   const uint32_t smem_sfb = smem_sfa + stages * kSfaStageBytes;
-  const uint32_t smem_store = smem_sfb + b_slots * C::kSfbStageBytes;  // staging ring, 16 KB buffers, 1024-byte aligned
+  const uint32_t smem_store = smem_sfb + (kResident ? 0 : stages * C::kSfbStageBytes);  // staging ring, 16 KB buffers, 1024-byte aligned
   const uint32_t smem_bar = smem_store + C::kStoreBufs * kStoreStageBytes;
   // barrier block: full[8], empty[8], scales_full[8], tmem_full[2], tmem_empty[2], b_full, b_empty, sf_empty[4], mma_drain,
   // staged[4], stored[4], tmem base, abort flag
@@ -561,7 +587,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   wait_for_prior_kernels();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_base_ptr;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_base_ptr, 0);  // warp uniform also to the compiler
 
   // Work list, identical in every role.  Streaming: work items (tile, k-split) strided over the
   // grid, column block fastest (neighbouring CTAs share A rows in L2).  Resident: each CTA owns a
@@ -569,7 +595,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // couple of times.
   const uint32_t tiles_mn = p.num_m_blocks * p.num_n_blocks;
   uint32_t w_begin, w_end, w_step, band_n = 0;
-  if (p.b_resident && p.resident_cpn) {
+  if (kResident && p.resident_cpn) {
     // Column block c / cpn, row blocks j, j + cpn, j + 2 cpn, ...: at any moment the CTAs of all
     // column blocks work on the same band of cpn row blocks, so whole output rows are written at
     // about the same time (full DRAM pages when L2 writes them back).
@@ -578,7 +604,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     w_begin = blockIdx.x - band_n * p.resident_cpn;
     w_end = has_work ? p.num_m_blocks : 0;
     w_step = p.resident_cpn;
-  } else if (p.b_resident) {
+  } else if (kResident) {
     w_begin = static_cast<uint32_t>(static_cast<uint64_t>(tiles_mn) * blockIdx.x / gridDim.x);
     w_end = static_cast<uint32_t>(static_cast<uint64_t>(tiles_mn) * (blockIdx.x + 1) / gridDim.x);
     w_step = 1;
@@ -588,11 +614,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     w_step = gridDim.x;
   }
   auto decode = [&](uint32_t w, uint32_t& m_blk, uint32_t& n_blk, uint32_t& split) {
-    if (p.b_resident && p.resident_cpn) {
+    if (kResident && p.resident_cpn) {
       n_blk = band_n;
       m_blk = w;
       split = 0;
-    } else if (p.b_resident) {
+    } else if (kResident) {
       n_blk = w / p.num_m_blocks;
       m_blk = w - n_blk * p.num_m_blocks;
       split = 0;
@@ -611,10 +637,16 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr int kNumSub = kBlockN / kSub;
   constexpr int kItems = kMHalves * kNumSub;
   constexpr uint32_t kRing = C::kStoreBufs / 2;  // staging buffers per group
-  auto first_item_of = [&](uint32_t group, uint32_t tile_iter) {
-    return static_cast<int>((kItems & 1) ? (group ^ (tile_iter & 1u)) : group);
+  // The rotating accumulator is taken from the half the next tile overwrites: columns 128.. of the tiles at column 0, 0.. of
+  // those at column 128.
+  constexpr int kTurns = (kItems + 1) / 2;               // items of a group and tile, at most
+  constexpr int kFirstTurns = C::kRotate ? kTurns / 2 : kTurns;  // of them, those the next tile's MMAs wait for
+  auto item_of = [&](uint32_t group, uint32_t tile_iter, int turn) {  // kItems: none
+    if (C::kRotate) return static_cast<int>(group) + 2 * ((tile_iter & 1u) ? turn : (turn + kFirstTurns) % kTurns);
+    return min(static_cast<int>((kItems & 1) ? (group ^ (tile_iter & 1u)) : group) + 2 * turn, kItems);
   };
-  auto item_valid = [&](int item, uint32_t m_blk, uint32_t n_blk) {  // not wholly outside the matrix
+  auto item_valid = [&](int item, uint32_t m_blk, uint32_t n_blk) {  // there is one, and not wholly outside the matrix
+    if (item >= kItems) return false;
     const uint32_t h = static_cast<uint32_t>(item / kNumSub), sub = static_cast<uint32_t>(item % kNumSub);
     return n_blk * kBlockN + sub * kSub < p.n && m_blk * kBlockM + h * kRowBlock < p.m;
   };
@@ -632,6 +664,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // a streamed k-tile 840 of the 1170 to 1300 the k-tile had (480 now).  8192 x 768 x K 3072 bf16 14.7 -> 13.2 us, 8192 x
     // 32000 x K 768 142 -> 118, 16 x 2304 x K 768 5.7 -> 4.8, 65536 x 3072 x K 768 111 -> 101.
     uint32_t stage = 0, phase = 0, issued = 0, runs = 0, prev_n = 0xffffffffu;
+    [[maybe_unused]] uint32_t tile_iter = 0;
     bool ok = true;
     for (uint32_t w = w_begin; w < w_end && ok; w += w_step) {
       uint32_t m_blk, n_blk, split;
@@ -640,7 +673,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t kt_end = min(p.num_k_tiles, kt_begin + p.k_tiles_per_split);
       const uint32_t first_blk128 = n_blk * kBlockN / 128u;
       const uint32_t blks128 = min(static_cast<uint32_t>(C::kSfBlocks), p.sfb_blocks128 - first_blk128);
-      if (p.b_resident && n_blk != prev_n) {
+      if (kResident && n_blk != prev_n) {
         // new column block: wait until the MMAs of the previous run have retired, then load the panel
         const bool free = runs == 0 || mbar_wait(bar_b_empty, (runs - 1) & 1u, abort_flag, kStatusProducerTimeout, p.wait_timeout_ns);
         if (!__all_sync(0xffffffffu, free)) {
@@ -648,16 +681,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         if (elect_one()) {
-          mbar_expect_tx(bar_b_full, p.num_k_tiles * C::kBStageBytes + p.k_atoms * kSfTileBytes * blks128);
-          for (uint32_t kt = 0; kt < p.num_k_tiles; ++kt) {
-            const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
+          mbar_expect_tx(bar_b_full, p.num_k_tiles * C::kBStageBytes);
+          for (uint32_t kt = 0; kt < p.num_k_tiles; ++kt)
             tma_load_2d(smem_b + kt * C::kBStageBytes, &tmap_b, bar_b_full, static_cast<int32_t>(kt * kBlockKBytes),
                         static_cast<int32_t>(n_blk * kBlockN));
-            for (uint32_t i = 0; i < blks128; ++i)
-              bulk_load(smem_sfb + kt * C::kSfbStageBytes + i * kSfBlockStageBytes,
-                        p.sfb + (static_cast<size_t>(first_blk128 + i) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
-                        atoms * kSfTileBytes, bar_b_full);
-          }
         }
         __syncwarp();
         prev_n = n_blk;
@@ -665,6 +692,21 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       // scale blocks of A inside the matrix (the second row half of a tall tile may lie below it)
       const uint32_t a_blks = min(static_cast<uint32_t>(kMHalves), p.sfa_blocks128 - m_blk * kMHalves);
+      if (kResident) {
+        // A goes to L2 two tiles ahead: from HBM, beside the output's writes, a k-tile takes 1900 cycles and more, longer than
+        // the ring covers (65536 x 2304 x K 768 80 us without).  In a banded schedule the column blocks' CTAs read the same A
+        // at about the same time and take turns.
+        const uint32_t ahead = w + 2 * w_step;
+        if (ahead < w_end && (p.resident_cpn == 0 || (tile_iter + band_n) % p.num_n_blocks == 0) && elect_one()) {
+          uint32_t m_ahead, n_ahead, none;
+          decode(ahead, m_ahead, n_ahead, none);
+          for (uint32_t kt = 0; kt < p.num_k_tiles; ++kt)
+            tma_prefetch_2d(&tmap_a, static_cast<int32_t>(kt * kBlockKBytes), static_cast<int32_t>(m_ahead * kBlockM));
+          bulk_prefetch(p.sfa + static_cast<size_t>(m_ahead) * p.k_atoms * kSfTileBytes, p.k_atoms * kSfTileBytes);
+        }
+        __syncwarp();
+        ++tile_iter;
+      }
       for (uint32_t kt = kt_begin; kt < kt_end; ++kt) {
         const bool free = mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, kStatusProducerTimeout, p.wait_timeout_ns);
         if (!__all_sync(0xffffffffu, free)) {
@@ -680,14 +722,14 @@ __global__ void __launch_bounds__(kThreads, 1)
           // The scale tiles first and on a barrier of their own: they are in tensor memory when the operands land.  On one
           // barrier with them a stage was occupied 460 cycles longer.
           const uint32_t scales = bar_scales_full + 8 * stage, full = bar_full + 8 * stage;
-          mbar_expect_tx(scales, sf_bytes * (a_blks + (p.b_resident ? 0u : blks128)));
+          mbar_expect_tx(scales, sf_bytes * (a_blks + (kResident ? 0u : blks128)));
 #pragma unroll
           for (uint32_t h = 0; h < static_cast<uint32_t>(kMHalves); ++h)
             if (h < a_blks)
               bulk_load(smem_sfa + stage * kSfaStageBytes + h * kSfBlockStageBytes,
                         p.sfa + (static_cast<size_t>(m_blk * kMHalves + h) * p.k_atoms + kt * kKAtomsPerStage) * kSfTileBytes,
                         sf_bytes, scales);
-          if (!p.b_resident) {
+          if (!kResident) {
 #pragma unroll
             for (uint32_t i = 0; i < static_cast<uint32_t>(C::kSfBlocks); ++i)
               if (i < blks128)
@@ -696,9 +738,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                           sf_bytes, scales);
           }
           const int32_t x = static_cast<int32_t>(kt * kBlockKBytes);
-          mbar_expect_tx(full, kAStageBytes + (p.b_resident ? 0 : C::kBStageBytes));
+          mbar_expect_tx(full, kAStageBytes + (kResident ? 0 : C::kBStageBytes));
           tma_load_2d(smem_a + stage * kAStageBytes, &tmap_a, full, x, static_cast<int32_t>(m_blk * kBlockM));
-          if (!p.b_resident) tma_load_2d(smem_b + stage * C::kBStageBytes, &tmap_b, full, x, static_cast<int32_t>(n_blk * kBlockN));
+          if (!kResident) tma_load_2d(smem_b + stage * C::kBStageBytes, &tmap_b, full, x, static_cast<int32_t>(n_blk * kBlockN));
         }
         __syncwarp();
         GEMM_TRACE(0, 2, lane == 0);
@@ -726,14 +768,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     // from inside a single-lane branch instead costs ~140 cycles per tcgen05.mma.
     {
       constexpr uint32_t idesc = make_idesc<kBlockN>();
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, runs = 0, prev_n = 0xffffffffu, sf_set = 0;
+      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, runs = 0, prev_n = 0xffffffffu, sf_set = 0, tile_iter = 0;
       bool ok = true;
-      for (uint32_t w = w_begin; w < w_end && ok; w += w_step) {
+      for (uint32_t w = w_begin; w < w_end && ok; w += w_step, ++tile_iter) {
         uint32_t m_blk, n_blk, split;
         decode(w, m_blk, n_blk, split);
         const uint32_t kt_begin = split * p.k_tiles_per_split;
         const uint32_t kt_end = min(p.num_k_tiles, kt_begin + p.k_tiles_per_split);
-        if (p.b_resident && n_blk != prev_n) {
+        if (kResident && n_blk != prev_n) {
           if (!__all_sync(0xffffffffu, mbar_wait(bar_b_full, runs & 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns))) {
             ok = false;
             break;
@@ -748,7 +790,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         GEMM_TRACE(1, 11, lane == 0);
         tcgen05_fence_after();
-        const uint32_t tmem_acc = tmem_base + acc * C::kAccCols;
+        const uint32_t tmem_acc = tmem_base + (C::kRotate ? (tile_iter & 1u) * 128u : acc * C::kAccCols);
         for (uint32_t kt = kt_begin; kt < kt_end; ++kt) {
           // operands in shared memory, scale factors in column set `sf_set`
           const bool ready = mbar_wait(bar_full + 8 * stage, phase, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns);
@@ -759,9 +801,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           GEMM_TRACE(1, 12, lane == 0);
           tcgen05_fence_after();
           const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
-          const uint32_t b_slot = p.b_resident ? kt : stage;
+          const uint32_t b_slot = kResident ? kt : stage;
           const uint32_t tsfa = tmem_base + C::kTmemSfa + sf_set * C::kSfSetCols;
-          const uint32_t tsfb = tmem_base + C::kTmemSfb + sf_set * C::kSfSetCols;
+          const uint32_t tsfb = kResident ? tmem_base + C::kTmemPanel + kt * C::kSfbTileCols : tsfa + C::kSfaSetCols;
           const uint64_t desc_a = make_ab_desc(smem_a + stage * kAStageBytes);
           const uint64_t desc_b = make_ab_desc(smem_b + b_slot * C::kBStageBytes);
           if (elect_one()) {
@@ -790,15 +832,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
         if (!ok) break;
-        // last tile of this column block (or of this CTA): the resident panel may be replaced once
-        // everything issued so far has retired
-        bool release_panel = false;
-        if (p.b_resident) {
-          uint32_t nm, nn = n_blk, ns;
-          const bool last = (w + w_step >= w_end);
-          if (!last) decode(w + w_step, nm, nn, ns);
-          release_panel = last || nn != n_blk;
-        }
+        // last tile of this column block: the resident panel may be replaced once everything issued so far has retired (a
+        // banded schedule keeps one column block)
+        const bool release_panel = kResident && p.resident_cpn == 0 && w + 1 == (n_blk + 1) * p.num_m_blocks;
         if (elect_one()) {
           tcgen05_commit(bar_tmem_full + 8 * acc);  // accumulator complete
           if (release_panel) tcgen05_commit(bar_b_empty);
@@ -833,8 +869,43 @@ __global__ void __launch_bounds__(kThreads, 1)
       decode(w, m_blk, n_blk, split);
       const uint32_t kt_begin = split * p.k_tiles_per_split;
       const uint32_t kt_end = min(p.num_k_tiles, kt_begin + p.k_tiles_per_split);
-      if (p.b_resident && n_blk != prev_n) {
-        if (!mbar_wait(bar_b_full, runs & 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) break;
+      if (kResident && n_blk != prev_n) {
+        // The panel's B scale factors, once per column block and from memory: its tiles then leave only those of A to move
+        // (500 to 600 cycles a k-tile with B, more than its MMAs take).  The MMAs of the column block before have retired.
+        if (runs > 0 && !mbar_wait(bar_b_empty, (runs - 1) & 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) break;
+        __syncwarp();
+        tcgen05_fence_after();
+        const uint32_t first_blk128 = n_blk * kBlockN / 128u;
+        const uint8_t* src = p.sfb + static_cast<size_t>(first_blk128) * p.k_atoms * kSfTileBytes + lane * 16;
+        const size_t block_bytes = static_cast<size_t>(p.k_atoms) * kSfTileBytes;
+#pragma unroll 1
+        for (uint32_t kt = 0; kt < p.num_k_tiles; ++kt) {
+          const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
+          const uint32_t dst = tmem_base + C::kTmemPanel + kt * C::kSfbTileCols + ((quad * 32u) << 16);
+          uint32_t r[kKAtomsPerStage][C::kSfBlocks * 4] = {};  // blocks outside the matrix: zeros
+#pragma unroll
+          for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb)
+#pragma unroll
+            for (uint32_t i = 0; i < static_cast<uint32_t>(C::kSfBlocks); ++i)
+              if (kb < atoms && first_blk128 + i < p.sfb_blocks128)
+                load_prior(src + i * block_bytes + (kt * kKAtomsPerStage + kb) * kSfTileBytes, &r[kb][4 * i]);
+#pragma unroll
+          for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb) {
+            if (kb < atoms) {
+              if constexpr (kBlockN == 192) {
+                const bool odd = (n_blk & 1u) != 0;  // the tile starts in the middle of its first block
+                uint32_t sel[6];
+#pragma unroll
+                for (int j = 0; j < 6; ++j) sel[j] = odd ? r[kb][j + 2] : r[kb][j];
+                tcgen05_st_x4(dst + kb * 6, sel);
+                tcgen05_st_x2(dst + kb * 6 + 4, sel + 4);
+              } else {
+#pragma unroll
+                for (int i = 0; i < C::kSfBlocks; ++i) tcgen05_st_x4(dst + kb * C::kSfbColsPerAtom + i * 4, &r[kb][4 * i]);
+              }
+            }
+          }
+        }
         prev_n = n_blk;
         ++runs;
       }
@@ -845,27 +916,26 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         GEMM_TRACE(2, 20, warp == 8 && lane == 0);
         const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
-        const uint32_t b_slot = p.b_resident ? kt : stage;
         const uint32_t sfa_s = smem_sfa + stage * kSfaStageBytes + lane * 16;
-        const uint32_t sfb_s = smem_sfb + b_slot * C::kSfbStageBytes + lane * 16;
         const uint32_t tsfa = tmem_base + C::kTmemSfa + sf_set * C::kSfSetCols + ((quad * 32u) << 16);
-        const uint32_t tsfb = tmem_base + C::kTmemSfb + sf_set * C::kSfSetCols + ((quad * 32u) << 16);
         // all shared-memory reads first (independent, pipelined), then the tensor-memory stores
         uint32_t ra[kMHalves][kKAtomsPerStage][4];
-        uint32_t rb[kKAtomsPerStage][C::kSfBlocks * 4];
 #pragma unroll
         for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb) {
           if (kb < atoms) {
 #pragma unroll
-            for (int h = 0; h < kMHalves; ++h)
-              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                           : "=r"(ra[h][kb][0]), "=r"(ra[h][kb][1]), "=r"(ra[h][kb][2]), "=r"(ra[h][kb][3])
-                           : "r"(sfa_s + h * kSfBlockStageBytes + kb * kSfTileBytes));
+            for (int h = 0; h < kMHalves; ++h) lds_128(sfa_s + h * kSfBlockStageBytes + kb * kSfTileBytes, ra[h][kb]);
+          }
+        }
+        [[maybe_unused]] uint32_t rb[kKAtomsPerStage][C::kSfBlocks * 4];
+        if constexpr (!kResident) {
+          const uint32_t sfb_s = smem_sfb + stage * C::kSfbStageBytes + lane * 16;
 #pragma unroll
-            for (int i = 0; i < C::kSfBlocks; ++i)
-              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                           : "=r"(rb[kb][4 * i]), "=r"(rb[kb][4 * i + 1]), "=r"(rb[kb][4 * i + 2]), "=r"(rb[kb][4 * i + 3])
-                           : "r"(sfb_s + i * kSfBlockStageBytes + kb * kSfTileBytes));
+          for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb) {
+            if (kb < atoms) {
+#pragma unroll
+              for (int i = 0; i < C::kSfBlocks; ++i) lds_128(sfb_s + i * kSfBlockStageBytes + kb * kSfTileBytes, &rb[kb][4 * i]);
+            }
           }
         }
         if (!mbar_wait(bar_sf_empty + 8 * sf_set, sf_phase ^ 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) {
@@ -874,44 +944,52 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         tcgen05_fence_after();
         __syncwarp();
-        if constexpr (kBlockN == 192) {
-          // Six scale words (192 rows of B) per k-atom out of the eight loaded: words 0..5 when the tile
-          // starts on a 128-row block boundary (even column block), words 2..7 when it starts in the
-          // middle of the first block (odd column block).
-          const bool odd = (n_blk & 1u) != 0;
-          uint32_t sel[kKAtomsPerStage][6];
+        if (atoms == kKAtomsPerStage) {
 #pragma unroll
-          for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb)
+          for (int h = 0; h < kMHalves; ++h) tcgen05_st_x16(tsfa + h * 4 * kKAtomsPerStage, &ra[h][0][0]);
+        } else {
 #pragma unroll
-            for (int j = 0; j < 6; ++j) sel[kb][j] = odd ? rb[kb][j + 2] : rb[kb][j];
-          if (atoms == kKAtomsPerStage) {
+          for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb) {
+            if (kb < atoms) {
 #pragma unroll
-            for (int h = 0; h < kMHalves; ++h) tcgen05_st_x16(tsfa + h * 4 * kKAtomsPerStage, &ra[h][0][0]);
-            tcgen05_st_x16(tsfb, &sel[0][0]);
-            tcgen05_st_x8(tsfb + 16, &sel[0][0] + 16);
+              for (int h = 0; h < kMHalves; ++h) tcgen05_st_x4(tsfa + h * 4 * kKAtomsPerStage + kb * 4, ra[h][kb]);
+            }
+          }
+        }
+        if constexpr (!kResident) {
+          const uint32_t tsfb = tsfa + C::kSfaSetCols;
+          if constexpr (kBlockN == 192) {
+            // Six scale words (192 rows of B) per k-atom out of the eight loaded: words 0..5 when the tile
+            // starts on a 128-row block boundary (even column block), words 2..7 when it starts in the
+            // middle of the first block (odd column block).
+            const bool odd = (n_blk & 1u) != 0;
+            uint32_t sel[kKAtomsPerStage][6];
+#pragma unroll
+            for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb)
+#pragma unroll
+              for (int j = 0; j < 6; ++j) sel[kb][j] = odd ? rb[kb][j + 2] : rb[kb][j];
+            if (atoms == kKAtomsPerStage) {
+              tcgen05_st_x16(tsfb, &sel[0][0]);
+              tcgen05_st_x8(tsfb + 16, &sel[0][0] + 16);
+            } else {
+#pragma unroll
+              for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb) {
+                if (kb < atoms) {
+                  tcgen05_st_x4(tsfb + kb * 6, sel[kb]);
+                  tcgen05_st_x2(tsfb + kb * 6 + 4, sel[kb] + 4);
+                }
+              }
+            }
+          } else if (atoms == kKAtomsPerStage) {
+            tcgen05_st_x16(tsfb, &rb[0][0]);
+            if constexpr (C::kSfBlocks == 2) tcgen05_st_x16(tsfb + 16, &rb[2][0]);
           } else {
 #pragma unroll
             for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb) {
               if (kb < atoms) {
 #pragma unroll
-                for (int h = 0; h < kMHalves; ++h) tcgen05_st_x4(tsfa + h * 4 * kKAtomsPerStage + kb * 4, ra[h][kb]);
-                tcgen05_st_x4(tsfb + kb * 6, sel[kb]);
-                tcgen05_st_x2(tsfb + kb * 6 + 4, sel[kb] + 4);
+                for (int i = 0; i < C::kSfBlocks; ++i) tcgen05_st_x4(tsfb + kb * C::kSfbColsPerAtom + i * 4, &rb[kb][4 * i]);
               }
-            }
-          }
-        } else if (atoms == kKAtomsPerStage) {
-          // one 16-column store for the A scales, one 16- or 32-column store for the B scales
-          tcgen05_st_x16(tsfa, &ra[0][0][0]);
-          tcgen05_st_x16(tsfb, &rb[0][0]);
-          if constexpr (C::kSfBlocks == 2) tcgen05_st_x16(tsfb + 16, &rb[2][0]);
-        } else {
-#pragma unroll
-          for (uint32_t kb = 0; kb < kKAtomsPerStage; ++kb) {
-            if (kb < atoms) {
-              tcgen05_st_x4(tsfa + kb * 4, ra[0][kb]);
-#pragma unroll
-              for (int i = 0; i < C::kSfBlocks; ++i) tcgen05_st_x4(tsfb + kb * C::kSfbColsPerAtom + i * 4, &rb[kb][4 * i]);
             }
           }
         }
@@ -945,17 +1023,17 @@ __global__ void __launch_bounds__(kThreads, 1)
       auto item_y = [&](int item, uint32_t m_blk) { return static_cast<int32_t>(m_blk * kBlockM + (item / kNumSub) * kRowBlock); };
       // residual stream: a second walk over the group's items, one ring ahead, loads what they will be added to
       uint32_t load_w = w_begin, load_tile = 0, load_m = 0, load_n = 0, load_split = 0, loads = 0;
-      int load_item = kItems;  // next item of the tile (load_m, load_n); kItems: on to the tile of load_w
+      int load_turn = kTurns;  // next turn in the tile (load_m, load_n); kTurns: on to the tile of load_w
       auto load_next = [&](uint32_t slot) {
         while (true) {
-          if (load_item >= kItems) {
+          if (load_turn >= kTurns) {
             if (load_w >= w_end) return;
             decode(load_w, load_m, load_n, load_split);
-            load_item = first_item_of(eg, load_tile++);
+            ++load_tile;
+            load_turn = 0;
             load_w += w_step;
           }
-          const int item = load_item;
-          load_item += 2;
+          const int item = item_of(eg, load_tile - 1, load_turn++);
           if (!item_valid(item, load_m, load_n)) continue;
           if (elect_one()) {
             mbar_expect_tx(bar_stored + 8 * slot, kStoreStageBytes);  // parts outside the matrix arrive as zeros
@@ -978,7 +1056,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           // 27.5 all at once, 23.4 spread; from L2 20.2.
           const uint32_t t0 = clock32(), pace = p.num_k_tiles * 700u / (kItems / 2);
           uint32_t due = 0;
-          for (int item = first_item_of(eg, tile_iter) + 2 * static_cast<int>(kRing); item < kItems; item += 2) {
+          for (int turn = kRing; turn < kTurns; ++turn) {
+            const int item = item_of(eg, tile_iter, turn);
             if (!item_valid(item, m_blk, n_blk)) continue;
             due += pace;
             bool staged = false;
@@ -989,7 +1068,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             __syncwarp();
           }
         }
-        for (int item = first_item_of(eg, tile_iter); item < kItems && ok; item += 2) {
+        for (int turn = 0; turn < kTurns && ok; ++turn) {
+          const int item = item_of(eg, tile_iter, turn);
           if (!item_valid(item, m_blk, n_blk)) continue;
           const int32_t x = item_x(item, n_blk), y = item_y(item, m_blk);
           for (int pass = 0; pass < item_passes; ++pass) {
@@ -1004,6 +1084,8 @@ __global__ void __launch_bounds__(kThreads, 1)
               const CUtensorMap* map = item_passes == 2 && pass == 0 ? &tmap_aux : &tmap_out;
               if (!kResidual && p.k_splits > 1)
                 tma_reduce_add_2d(map, smem_store + slot * kStoreStageBytes, x, y);
+              else if (kResident && p.stream_out)
+                tma_store_2d_streaming(map, smem_store + slot * kStoreStageBytes, x, y);
               else
                 tma_store_2d(map, smem_store + slot * kStoreStageBytes, x, y);
               bulk_commit_group();
@@ -1117,7 +1199,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int h = 0; h < kMHalves; ++h)
         scale_h[h] = __fmul_rn(__fmul_rn(p.weight, p.mode == NVFP4_GS_ROWWISE_A ? ga_row[h] : ga_scalar), gb);
-      const uint32_t taddr_row = tmem_base + acc * C::kAccCols + ((ew * 32u) << 16);
+      const uint32_t taddr_row = tmem_base + (C::kRotate ? (tile_iter & 1u) * 128u : acc * C::kAccCols) + ((ew * 32u) << 16);
       // The accumulator buffer goes back to the MMA warp as soon as this warp's last tcgen05.ld of the
       // tile has landed in registers: scaling, staging and the stores of that last sub-tile then run
       // beside the next tile's main loop.
@@ -1129,12 +1211,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (kTmaStore) {
         // the group's sub-tiles go through its shared-memory ring to the store warp; rows / columns outside the matrix
         // are clipped by the tensor map
-        const int first_item = first_item_of(eg, tile_iter);
-        int last_item = -1;
+        int last_turn = -1;  // behind which the accumulator, or the half of it that the next tile needs, is in registers
 #pragma unroll
-        for (int item = first_item; item < kItems; item += 2)
-          if (item_valid(item, m_blk, n_blk)) last_item = item;
-        if (last_item < 0) release_accumulator();  // nothing of this tile is for this group to read
+        for (int turn = 0; turn < kFirstTurns; ++turn)
+          if (item_valid(item_of(eg, tile_iter, turn), m_blk, n_blk)) last_turn = turn;
+        if (last_turn < 0) release_accumulator();  // nothing of it is for this group to read
         float row_max = -INFINITY;  // largest value this thread stores for its row in the current row half
         uint32_t max_h = 0;
         auto flush_row_max = [&]() {
@@ -1151,7 +1232,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           row_max = -INFINITY;
         };
 #pragma unroll 1
-        for (int item = first_item; item < kItems; item += 2) {
+        for (int turn = 0; turn < kTurns; ++turn) {
+          const int item = item_of(eg, tile_iter, turn);
           if (!item_valid(item, m_blk, n_blk)) continue;
           const uint32_t h = static_cast<uint32_t>(item / kNumSub);
           const int c = (item % kNumSub) * kSub;
@@ -1169,7 +1251,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int q = 0; q < kSub / 32; ++q) tcgen05_ld_32x32b_x32(taddr_row + h * kBlockN + c + 32 * q, r[q]);
             tcgen05_wait_ld();
             GEMM_TRACE(3 + eg, 32, elected);
-            if (item == last_item) release_accumulator();  // the group's last read of this tile
+            if (turn == last_turn) release_accumulator();
             if (kResidual) {
               // the roundings of the direct path: the product, the sum with the bias, then the one with the stream
 #pragma unroll
@@ -1252,11 +1334,13 @@ __global__ void __launch_bounds__(kThreads, 1)
           const bool row_ok = row < p.m;
           const float scale = kMHalves == 1 ? scale_h[0] : (h == 0 ? scale_h[0] : scale_h[kMHalves - 1]);
 #pragma unroll 1
-          for (int c = eg * 32; c < kBlockN; c += 64) {
+          for (int step = 0; step < kBlockN / 64; ++step) {
+            // 32 columns; a rotating accumulator's second half first where the tile lies at column 0
+            const int c = (C::kRotate && (tile_iter & 1u) == 0 ? (step + 2) % 4 : step) * 64 + eg * 32;
             uint32_t r[32];
             tcgen05_ld_32x32b_x32(taddr_row + h * kBlockN + c, r);
             tcgen05_wait_ld();
-            if (h + 1 == static_cast<uint32_t>(kMHalves) && c + 64 >= kBlockN) release_accumulator();
+            if (h + 1 == static_cast<uint32_t>(kMHalves) && step + 1 == (C::kRotate ? 2 : kBlockN / 64)) release_accumulator();
             const uint32_t col0 = n_blk * kBlockN + c;
             if (row_ok && col0 < p.n) {
               const uint32_t valid = min(32u, p.n - col0);
@@ -1459,26 +1543,30 @@ struct GemmTiming {
 // Everything the host decides about one launch.
 struct GemmPlan {
   uint32_t block_m = 128, block_n = 128, num_n_blocks = 0, k_splits = 1, k_tiles_per_split = 0;
-  uint32_t stages = 0, grid = 0, b_resident = 0, resident_cpn = 0, tma_store = 0, vec_store = 0;
+  uint32_t stages = 0, grid = 0, b_resident = 0, panel = 0, resident_cpn = 0, tma_store = 0, vec_store = 0;
   size_t smem_bytes = 0;
 };
 
 struct TileBytes {
-  int fixed, stream_stage, resident_stage, panel_slot, a_stage;
+  int fixed, stage, slot;  // see Cfg
 };
-template <int kBlockM, int kBlockN>
+template <int kBlockM, int kBlockN, int kPanel>
 constexpr TileBytes tile_bytes_of() {
-  using C = Cfg<kBlockM, kBlockN>;
-  return {C::kFixedBytes, C::kStreamStageBytes, C::kResidentStageBytes, C::kPanelSlotBytes,
-          C::kAStageBytes + C::kSfaStageBytes};
+  using C = Cfg<kBlockM, kBlockN, kPanel>;
+  return {C::kFixedBytes, C::kStageBytes, C::kSlotBytes};
 }
-TileBytes tile_bytes(uint32_t block_m, uint32_t block_n) {
-  if (block_m == 256) return tile_bytes_of<256, 192>();
-  return block_n == 256 ? tile_bytes_of<128, 256>() : block_n == 192 ? tile_bytes_of<128, 192>() : tile_bytes_of<128, 128>();
+// The resident form of a tile for so many k-tiles.
+constexpr uint32_t panel_of(uint32_t block_n, uint32_t num_k_tiles) { return block_n == 128 || num_k_tiles > 3 ? 4 : 3; }
+TileBytes tile_bytes(uint32_t block_m, uint32_t block_n, uint32_t panel) {
+  if (block_m == 256) return tile_bytes_of<256, 192, 0>();
+  if (block_n == 256) return panel ? tile_bytes_of<128, 256, 3>() : tile_bytes_of<128, 256, 0>();
+  if (block_n == 192)
+    return panel == 0 ? tile_bytes_of<128, 192, 0>() : panel == 3 ? tile_bytes_of<128, 192, 3>() : tile_bytes_of<128, 192, 4>();
+  return panel ? tile_bytes_of<128, 128, 4>() : tile_bytes_of<128, 128, 0>();
 }
 
-template <int kBlockM, int kBlockN, typename OutT, StorePath kStore>
-int launch_store_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo,
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel>
+int launch_schedule_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo,
                          const CUtensorMap& mx, const GemmParams& p, const GemmPlan& pl) {
   // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
   static std::atomic<int> attr_state[kMaxDevices];  // 0 = not set, 1 = set, -(error) = failed
@@ -1486,7 +1574,7 @@ int launch_store_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMa
   if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
   int st = attr_state[dev].load(std::memory_order_acquire);
   if (st == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore>,
+    const cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
     st = e == cudaSuccess ? 1 : -static_cast<int>(e);
     attr_state[dev].store(st, std::memory_order_release);
@@ -1515,11 +1603,25 @@ int launch_store_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMa
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int rc = static_cast<int>(
-      cudaLaunchKernelEx(&cfg, nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore>, ma, mb, mo, mx, p));
+      cudaLaunchKernelEx(&cfg, nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel>, ma, mb, mo, mx, p));
   count_launch();
   if (rc == 0) rc = static_cast<int>(cudaGetLastError());
   if (rec) cudaEventRecord(rec->stop, s);
   return rc;
+}
+
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore>
+int launch_store_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo,
+                         const CUtensorMap& mx, const GemmParams& p, const GemmPlan& pl) {
+  if constexpr (kBlockM == 128) {
+    if constexpr (kBlockN != 128) {
+      if (pl.panel == 3) return launch_schedule_variant<kBlockM, kBlockN, OutT, kStore, 3>(s, ma, mb, mo, mx, p, pl);
+    }
+    if constexpr (kBlockN != 256) {
+      if (pl.panel == 4) return launch_schedule_variant<kBlockM, kBlockN, OutT, kStore, 4>(s, ma, mb, mo, mx, p, pl);
+    }
+  }
+  return launch_schedule_variant<kBlockM, kBlockN, OutT, kStore, 0>(s, ma, mb, mo, mx, p, pl);
 }
 
 // The store path is a compile-time property of the kernel: each variant carries only its own epilogue code.  Deciding for
@@ -1709,27 +1811,32 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   // operand traffic per tile; these shapes are otherwise bound by L2 -> SM bandwidth).
   const bool want_resident =
       block_m == 128 && pl.k_splits == 1 && num_k_tiles <= (block_n == 256 ? 3u : 4u) && tiles >= 4 * pl.grid;
-  const TileBytes tb = tile_bytes(block_m, block_n);
-  const int budget = kSmemBudget - tb.fixed;
-  pl.b_resident = 0;
-  pl.resident_cpn = 0;
+  pl.b_resident = pl.panel = pl.resident_cpn = 0;
+  auto stages_beside = [&](const TileBytes& tb, uint32_t slots) {
+    return (kSmemBudget - tb.fixed - static_cast<int>(slots) * tb.slot) / tb.stage;
+  };
   if (want_resident) {
-    const int left = budget - static_cast<int>(num_k_tiles) * tb.panel_slot;
-    const int st = left / tb.resident_stage;
-    if (st >= 4) {
+    const uint32_t panel = panel_of(block_n, num_k_tiles);
+    const int st = stages_beside(tile_bytes(block_m, block_n, panel), num_k_tiles);
+    if (st >= 3) {
       pl.b_resident = 1;
+      pl.panel = panel;
       pl.stages = static_cast<uint32_t>(st > kMaxStages ? kMaxStages : st);
-      // banded schedule when the column blocks divide the grid almost evenly
-      const uint32_t cpn = pl.grid / pl.num_n_blocks;
-      if (cpn >= 1 && cpn * pl.num_n_blocks * 20 >= pl.grid * 19 && num_m_blocks >= 4 * cpn) pl.resident_cpn = cpn;
+      // banded schedule when the column blocks divide the grid almost evenly, or, for many row blocks, fill four fifths of it:
+      // one A tile for all CTAs at a time and whole output rows are worth that many idle SMs (65536 x 32000 x K 768 on
+      // 125 SMs 1003 us, contiguous on 148 1187; 8192 rows 112 and 114)
+      const uint32_t cpn = pl.grid / pl.num_n_blocks, used = cpn * pl.num_n_blocks;
+      if (cpn >= 1 && ((used * 20 >= pl.grid * 19 && num_m_blocks >= 4 * cpn) || (used * 5 >= pl.grid * 4 && num_m_blocks >= 16 * cpn)))
+        pl.resident_cpn = cpn;
     }
   }
+  const TileBytes tb = tile_bytes(block_m, block_n, pl.panel);
   if (!pl.b_resident) {
-    const int st = budget / tb.stream_stage;
+    const int st = (kSmemBudget - tb.fixed) / (tb.stage + tb.slot);
     pl.stages = static_cast<uint32_t>(st > kMaxStages ? kMaxStages : st);
   }
-  const uint32_t b_slots = pl.b_resident ? num_k_tiles : pl.stages;
-  pl.smem_bytes = tb.fixed + static_cast<size_t>(pl.stages) * tb.a_stage + static_cast<size_t>(b_slots) * tb.panel_slot;
+  const uint32_t slots = pl.b_resident ? num_k_tiles : pl.stages;
+  pl.smem_bytes = tb.fixed + static_cast<size_t>(pl.stages) * tb.stage + static_cast<size_t>(slots) * tb.slot;
 }
 
 }  // namespace
@@ -1884,10 +1991,14 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero) {
   p.k_splits = pl.k_splits;
   p.k_tiles_per_split = pl.k_tiles_per_split;
   p.stages = pl.stages;
-  p.b_resident = static_cast<int>(pl.b_resident);
   p.resident_cpn = pl.resident_cpn;
   p.vec_store = static_cast<int>(pl.vec_store);
   p.tma_store = static_cast<int>(pl.tma_store);
+  // An output that L2 (126 MB) does not hold leaves it first, so that the operands stay: the contiguous schedule, whose CTAs
+  // are all over the matrix, 1000 x 32000 x K 768 f32 36 -> 30 us, 8192 x 32000 x K 1024 bf16 150 -> 145.  Not the banded
+  // one: its rows are completed by several CTAs before they should leave (65536 x 2304 x K 768 65 -> 77 us).
+  p.stream_out = pl.b_resident && pl.resident_cpn == 0 &&
+                 static_cast<uint64_t>(a.m) * a.ldo * (a.out_dtype == NVFP4_DTYPE_F32 ? 4 : 2) > (96ull << 20);
   p.wait_timeout_ns = g_wait_timeout_ns.load(std::memory_order_relaxed);
   p.debug_flags = g_debug_flags.load(std::memory_order_relaxed);
 #ifdef NVFP4_GEMM_TRACE

@@ -556,25 +556,20 @@ __global__ void __launch_bounds__(kThreads, 1)
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_out)) : "memory");
       if (p.aux) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_aux)) : "memory");
     }
-    for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(bar_full + 8 * s, 1 + 4);  // the operands, and the scale factors of the four warps
-      mbar_init(bar_empty + 8 * s, 1);
-      mbar_init(bar_scales_full + 8 * s, 1);
-    }
-    for (int s = 0; s < C::kSfSets; ++s) mbar_init(bar_sf_empty + 8 * s, 1);
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(bar_tmem_full + 8 * a, 1);
-      mbar_init(bar_tmem_empty + 8 * a, 8);
-    }
-    mbar_init(bar_b_full, 1);
-    mbar_init(bar_b_empty, 1);
-    mbar_init(bar_mma_drain, 1);
-    for (uint32_t b = 0; b < kMaxFinal; ++b) mbar_init(bar_final + 8 * b, 4);
-    for (int b = 0; b < C::kStoreBufs; ++b) {
-      mbar_init(bar_staged + 8 * b, 4);  // the four warps of the epilogue group
-      mbar_init(bar_stored + 8 * b, 1);
-    }
     *abort_flag = 0;
+  }
+  if (warp == 1) {  // a barrier per lane and pass, in the order of the barrier block
+    constexpr uint32_t kTmemEmpty = 3 * kMaxStages + 2, kStaged = kTmemEmpty + 5 + C::kSfSets, kStored = kStaged + C::kStoreBufs,
+                       kFinal = kStored + C::kStoreBufs;
+    for (uint32_t b = lane; b < kFinal + kMaxFinal; b += 32) {
+      // full: the operands, and the scale factors of the four warps; a released accumulator: both groups' warps; a staged
+      // sub-tile: the group's warps
+      const uint32_t count = b < kMaxStages                                        ? 5
+                             : b == kTmemEmpty || b == kTmemEmpty + 1              ? 8
+                             : (b >= kStaged && b < kStored) || b >= kFinal ? 4
+                                                                                   : 1;
+      mbar_init(smem_bar + 8 * b, count);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -584,10 +579,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     tcgen05_fence_before();
   }
-  // Programmatic dependent launch: up to here the CTA has touched only its own SM.  Whatever runs before it in the stream
-  // is complete and visible beyond this point.  The GEMM itself does not allow the next kernel to start early: its CTAs end
-  // at different times, and the first SMs that come free would take all of a small grid's CTAs.
-  wait_for_prior_kernels();
+  // Programmatic dependent launch: the CTA touches only its own SM up to the roles' waits for what runs before it in the stream,
+  // each of which stands ahead of the role's first access to memory, behind the fetch of its code and of its first tile.  The
+  // GEMM itself does not allow the next kernel to start early: its CTAs end at different times, and the first SMs that come
+  // free would take all of a small grid's CTAs.
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_base_ptr, 0);  // warp uniform also to the compiler
@@ -692,6 +687,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = false;
           break;
         }
+        wait_for_prior_kernels();
         if (elect_one()) {
           mbar_expect_tx(bar_b_full, p.num_k_tiles * C::kBStageBytes);
           for (uint32_t kt = 0; kt < p.num_k_tiles; ++kt)
@@ -725,6 +721,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = false;
           break;
         }
+        if (issued == 0) wait_for_prior_kernels();
         GEMM_TRACE(0, 1, lane == 0);
         // test hook: this stage is never armed nor loaded, so its consumers' waits run out
         const bool skip = (p.debug_flags & 1u) && blockIdx.x == 0 && issued == 0;
@@ -887,6 +884,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (runs > 0 && !mbar_wait(bar_b_empty, (runs - 1) & 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) break;
         __syncwarp();
         tcgen05_fence_after();
+        wait_for_prior_kernels();
         const uint32_t first_blk128 = n_blk * kBlockN / 128u;
         const uint8_t* src = p.sfb + static_cast<size_t>(first_blk128) * p.k_atoms * kSfTileBytes + lane * 16;
         const size_t block_bytes = static_cast<size_t>(p.k_atoms) * kSfTileBytes;
@@ -1028,6 +1026,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // issuing the stores between two barriers of its group: 65536 x 2304 and x 3072 bf16 at K = 768, 87.3 -> 83.0 us and
     // 116.9 -> 111.3 us.
     if (kTmaStore) {
+      wait_for_prior_kernels();
       const uint32_t eg = warp - 2u;
       uint32_t buf = 0, phase = 0, tile_iter = 0, issued = 0;
       bool ok = true;
@@ -1160,6 +1159,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = true;  // warp uniform; false: some wait ran out, the rest of the list is walked without work
     const uint32_t my_bias = smem_bias + eg * kBlockN * 4;
     const float* my_bias_gen = reinterpret_cast<const float*>(smem_gen + (my_bias - smem_base));
+    wait_for_prior_kernels();
     const float gb = p.mode == NVFP4_GS_NONE ? 1.0f : load_prior(p.b_global);
     const float ga_scalar = p.mode == NVFP4_GS_TENSOR ? load_prior(p.a_global) : 1.0f;
     // the rows' global scales of a tile are fetched one tile ahead: their load latency would

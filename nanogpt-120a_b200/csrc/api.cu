@@ -275,14 +275,15 @@ static int validate_ms_eden(const nvfp4_ms_eden_args* a) {
 // Row operand + transposed operand of one matrix in a single pass (same scale, same signs).
 static int ms_eden_pair(void* stream, nvfp4_ms_eden_args rows, nvfp4_ms_eden_args transposed,
                         float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr,
-                        void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false) {
+                        uint32_t amax_count = 1, void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false) {
   rows.src_kind = NVFP4_SRC_F32_ROWS;
   transposed.src_kind = NVFP4_SRC_F32_TRANSPOSED;
   int rc = validate_ms_eden(&rows);
   if (rc) return rc;
   rc = validate_ms_eden(&transposed);
   if (rc) return rc;
-  return launch_ms_eden_pair(S(stream), rows, transposed, col_sum_partials, amax_in, gs_out, zero, zero_words, beside_others);
+  return launch_ms_eden_pair(S(stream), rows, transposed, col_sum_partials, amax_in, gs_out, amax_count, zero,
+                             zero_words, beside_others);
 }
 
 static nvfp4_ms_eden_args rows_args(const float* x, uint8_t* out_fp4, uint8_t* out_scales, float* out_gss,
@@ -436,17 +437,6 @@ static int nvfp4_source_transpose(void* stream, int kind, const uint8_t* in_byte
   if (source_cols % 16 != 0) return invalid("nvfp4 transpose: source_cols must be a multiple of 16");
   if (src_scale_layout == NVFP4_SCALES_PACKED && source_cols % 64 != 0)
     return invalid("nvfp4 transpose: a packed source scale layout needs source_cols % 64 == 0");
-  // The amax of the decoded source, unless the caller already holds it (the forward quantizer can emit it).
-  // When the chunk scratch is free (no chunk amax asked for) the amax accumulates in its word 0, away from
-  // out_gs, so that the transposer can derive the scale from it by itself.
-  int rc = 0;
-  const bool amax_in_scratch = !precomputed_amax && !chunk_amax_out && out_chunk_amax != nullptr;
-  if (!precomputed_amax)
-    rc = launch_nvfp4_amax(S(stream), in_bytes, in_scales, in_global, source_rows, source_cols,
-                           kind == NVFP4_SRC_ROWWISE_NVFP4_TRANSPOSED, src_scale_layout == NVFP4_SCALES_PACKED,
-                           amax_in_scratch ? nullptr : out_chunk_amax, amax_in_scratch ? out_chunk_amax : out_gs);
-  if (rc) return rc;
-  (void)n;
   nvfp4_ms_eden_args a;
   std::memset(&a, 0, sizeof(a));
   a.src_kind = kind;
@@ -469,6 +459,18 @@ static int nvfp4_source_transpose(void* stream, int kind, const uint8_t* in_byte
   a.scale_layout = scale_layout;
   a.out_global_scales = out_gss;
   a.out_chunk_amax = chunk_amax_out ? out_chunk_amax : nullptr;
+  // The amax of the decoded source, unless the caller already holds it (the forward quantizer can emit it).  When the chunk
+  // scratch is free (no chunk amax asked for) it goes there, away from out_gs, so that the transposer can derive the scale
+  // from it by itself: as partial maxima where that is a tiled one, else in word 0.
+  int rc = 0;
+  const bool amax_in_scratch = !precomputed_amax && !chunk_amax_out && out_chunk_amax != nullptr;
+  const bool partials = amax_in_scratch && ms_eden_takes_amax(a);
+  if (!precomputed_amax)
+    rc = launch_nvfp4_amax(S(stream), in_bytes, in_scales, in_global, source_rows, source_cols,
+                           kind == NVFP4_SRC_ROWWISE_NVFP4_TRANSPOSED, src_scale_layout == NVFP4_SCALES_PACKED,
+                           amax_in_scratch ? nullptr : out_chunk_amax, amax_in_scratch ? out_chunk_amax : out_gs,
+                           partials ? out_chunk_amax : nullptr);
+  if (rc) return rc;
   rc = validate_ms_eden(&a);
   if (rc) return rc;
   // amax -> global scale inside the transposer where it can (whole tiles), by a one-thread kernel otherwise;
@@ -479,7 +481,7 @@ static int nvfp4_source_transpose(void* stream, int kind, const uint8_t* in_byte
     rc = launch_ms_eden_scale_from_amax(S(stream), out_gs, out_gs);
     return rc ? rc : launch_ms_eden(S(stream), a);
   }
-  return launch_ms_eden(S(stream), a, amax_ptr, out_gs);
+  return launch_ms_eden(S(stream), a, amax_ptr, out_gs, partials ? tensor_amax_partials(n, kAmaxScratchPartials) : 1u);
 }
 
 int nvfp4_nvfp4_transpose_to_quartet_backward_ms_eden_derived_device_scale(
@@ -958,8 +960,8 @@ static bool dweight_lies_apart(const nvfp4_linear_backward_args* a, size_t dweig
          apart(a->w_scales, scales(O, I, a->w_scale_layout)) && apart(a->w_global, 4) && apart(a->x_bytes, T * I / 2) &&
          apart(a->x_scales, scales(T, I, a->x_scale_layout)) && apart(a->x_globals, T * 4) && apart(a->x_decoded_amax, 4) &&
          apart(a->e_global_scale_override, 4) && apart(a->dinput, T * I * element(a->dinput_dtype)) && apart(a->dbias, O * 4) &&
-         operand_apart(a->e_h, T, ok, e_chunks) && operand_apart(a->weight_t_h, I, ok, 1) && operand_apart(a->e_t_h, O, tk, 1) &&
-         operand_apart(a->input_t_h, I, tk, 1);
+         operand_apart(a->e_h, T, ok, e_chunks) && operand_apart(a->weight_t_h, I, ok, chunks1024(static_cast<uint64_t>(O) * I)) &&
+         operand_apart(a->e_t_h, O, tk, 1) && operand_apart(a->input_t_h, I, tk, chunks1024(static_cast<uint64_t>(T) * I));
 }
 
 // Everything of nvfp4_linear_backward_ms_eden that runs between the fork onto the caller's side stream and the
@@ -1039,14 +1041,21 @@ static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_
     if (rc) return rc;
   }
   const float* amax_in = nullptr;
+  uint32_t amax_count = 1;
   if (!a->e_global_scale_override) {
-    if (a->precomputed_e_amax_chunks != 0) {
-      rc = launch_amax_from_chunks(s, a->e_h.chunk_amax, a->e_h.global_scale, a->precomputed_e_amax_chunks, 1);
-    } else if (ms_eden_pair_takes_amax(q, qt)) {
-      // the amax accumulates in word 0 of the (otherwise unused) chunk scratch; the pair kernel derives the
-      // scale from it and publishes it in e_h.global_scale
-      rc = launch_tensor_amax(s, a->e, a->e_dtype, nullptr, a->e_h.chunk_amax, ne);
+    // Partial maxima in the chunk scratch, by the caller or by a pass over dY: the pair kernel derives the scale from them and
+    // publishes it in e_h.global_scale.  With a word cleared ahead of that pass, and of the side stream's over W, a
+    // backward of 1000 x 3072 f32 took 41.0 us instead of 37.6.  Every CTA reads all of them, so a caller's many thousands are reduced by a kernel first.
+    const bool takes_amax = ms_eden_pair_takes_amax(q, qt);
+    if (takes_amax && a->precomputed_e_amax_chunks <= kAmaxScratchPartials) {
       amax_in = a->e_h.chunk_amax;
+      amax_count = a->precomputed_e_amax_chunks;
+      if (amax_count == 0) {
+        rc = launch_tensor_amax(s, a->e, a->e_dtype, nullptr, nullptr, ne, a->e_h.chunk_amax, kAmaxScratchPartials);
+        amax_count = tensor_amax_partials(ne, kAmaxScratchPartials);
+      }
+    } else if (a->precomputed_e_amax_chunks != 0) {
+      rc = launch_amax_from_chunks(s, a->e_h.chunk_amax, a->e_h.global_scale, a->precomputed_e_amax_chunks, 1);
     } else {
       rc = launch_tensor_amax(s, a->e, a->e_dtype, a->e_h.chunk_amax, a->e_h.global_scale, ne);
       if (rc) return rc;
@@ -1063,8 +1072,8 @@ static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_
                     dweight_lies_apart(a, zero_words);
   zero_words = dweight_is_zero ? zero_words / 16 : 0;
   // one pass over dY for both orientations (+ column sums)
-  rc = ms_eden_pair(stream, q, qt, partials, amax_in, amax_in ? a->e_h.global_scale : nullptr, a->dweight, zero_words,
-                    ts != stream);
+  rc = ms_eden_pair(stream, q, qt, partials, amax_in, amax_in ? a->e_h.global_scale : nullptr, amax_count, a->dweight,
+                    zero_words, ts != stream);
   if (rc) return rc;
   if (fuse_dbias) rc = launch_col_sum_reduce(s, partials, a->dbias, ms_eden_pair_row_tiles(T), O);
   return rc;

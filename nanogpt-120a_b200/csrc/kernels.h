@@ -13,11 +13,14 @@ int launch_row_amax(cudaStream_t s, const void* x, int dtype, float* out, uint32
 // partials (optional, kAmaxPartials floats): every CTA leaves its maximum there -- tensor_amax_partials(n) of them -- for
 // a consumer that reduces them, and `out` is not touched (no zeroing launch, no atomics).
 constexpr uint32_t kAmaxPartials = 148u * 4u;
-uint32_t tensor_amax_partials(uint64_t n);
+// max_partials: more of them where the buffer holds a float per 1024 values (chunk scratch): twice the loads in flight, 524 MB of
+// bf16 80 us instead of 91.
+constexpr uint32_t kAmaxScratchPartials = 148u * 8u;
+uint32_t tensor_amax_partials(uint64_t n, uint32_t max_partials = kAmaxPartials);
 int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_amax, float* out, uint64_t n,
-                       float* partials = nullptr);
+                       float* partials = nullptr, uint32_t max_partials = kAmaxPartials);
 int launch_nvfp4_amax(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, const float* gscales, uint32_t rows,
-                      uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out);
+                      uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out, float* partials = nullptr);  // kAmaxScratchPartials
 // transform 0: out[0] = max(chunks); 1: out[0] = MS-EDEN global scale of that max
 int launch_amax_from_chunks(cudaStream_t s, const float* chunk_amax, float* out, uint32_t chunk_count, int transform);
 int launch_ms_eden_scale_from_amax(cudaStream_t s, const float* amax, float* out);
@@ -36,19 +39,21 @@ int launch_packed_scale_pad(cudaStream_t s, uint8_t* packed, uint32_t rows, uint
 int launch_schedule_free_materialize(cudaStream_t s, const float* z, const float* x, float beta, float* chunk_amax,
                                      float* amax, uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs,
                                      uint32_t rows, uint32_t cols, float* partials = nullptr);
-// amax_in / gs_out (optional): the global scale is the MS-EDEN scale of amax_in[0] (derived inside the kernel
-// where the kernel supports it, by a one-thread kernel otherwise) and is written to gs_out[0]; a.global_scale
-// and a.host_global_scale are then not read.
-int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a, const float* amax_in = nullptr, float* gs_out = nullptr);
+// amax_in / gs_out (optional): the global scale is the MS-EDEN scale of max(amax_in[0 .. amax_count - 1]) (derived inside the
+// kernel where the kernel supports it, by a one-thread kernel otherwise) and is written to gs_out[0]; a.global_scale
+// and a.host_global_scale are then not read.  amax_count > 1 only where ms_eden_takes_amax.
+int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a, const float* amax_in = nullptr, float* gs_out = nullptr,
+                   uint32_t amax_count = 1);
+bool ms_eden_takes_amax(const nvfp4_ms_eden_args& a);
 // Pair quantization; when col_sum_partials != nullptr (and ms_eden_pair_is_tiled) it also writes the
 // per-row-tile column sums [ms_eden_pair_row_tiles(rows)][cols] for launch_col_sum_reduce.
-// amax_in / gs_out (only when ms_eden_pair_takes_amax): the kernel derives the global scale from amax_in[0]
+// amax_in / gs_out (only when ms_eden_pair_takes_amax): the kernel derives the global scale from max(amax_in[0 .. amax_count - 1])
 // itself and writes it to gs_out[0]; rows.global_scale / transposed.global_scale are then not read.
 // beside_others: kernels of another stream are waiting for room on the SMs that this one would take by starting early.
 // zero (likewise only when ms_eden_pair_takes_amax): zero_words 16-byte words that the kernel clears beside its work.
 int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed,
                         float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr,
-                        void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false);
+                        uint32_t amax_count = 1, void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false);
 bool ms_eden_pair_takes_amax(const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed);
 bool ms_eden_pair_is_tiled(const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed);
 uint32_t ms_eden_pair_row_tiles(uint32_t rows);

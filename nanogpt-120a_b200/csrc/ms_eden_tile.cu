@@ -362,7 +362,22 @@ __device__ __forceinline__ void fill_inv_table(float2* table, float safe_gs) {
 
 __device__ __forceinline__ float tile_global_scale(const MsEdenTileParams& p) {
   if (!p.amax_in) return p.use_host_scale ? p.global_scale_host : after_prior(p.global_scale_dev)[0];
-  const float gs = ms_eden_scale_of_amax(after_prior(p.amax_in)[0]);
+  const float* const in = after_prior(p.amax_in);
+  float amax;
+  if (p.amax_count == 1) {
+    amax = in[0];
+  } else {  // partial maxima, non-negative: the pass before neither waited for a cleared word nor added to it
+    __shared__ uint32_t amax_bits;
+    if (threadIdx.x == 0) amax_bits = 0u;
+    __syncthreads();
+    float m = 0.0f;
+    for (uint32_t i = threadIdx.x; i < p.amax_count; i += blockDim.x) m = max_f32(m, in[i]);
+    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31u) == 0) atomicMax(&amax_bits, w);
+    __syncthreads();
+    amax = __uint_as_float(amax_bits);
+  }
+  const float gs = ms_eden_scale_of_amax(amax);
   if (blockIdx.x == 0 && threadIdx.x == 0) p.gs_out[0] = gs;
   return gs;
 }
@@ -406,9 +421,6 @@ __global__ void __launch_bounds__(256, 2)
   __shared__ float2 inv_table[kScaleCodes];
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const T* x = after_prior(static_cast<const T*>(p.x));
-  const float gs = tile_global_scale(p), safe_gs = nz(gs);
-  fill_inv_table(inv_table, safe_gs);
-  const float inv6 = inv_scale(6.0f, safe_gs);
   const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(pair_stage)) + warp * PB::kBytes;
   const uint32_t signs = static_cast<uint32_t>(__cvta_generic_to_shared(sign_words[warp]));
   const uint32_t table = static_cast<uint32_t>(__cvta_generic_to_shared(inv_table));
@@ -435,6 +447,13 @@ __global__ void __launch_bounds__(256, 2)
     }
   };
 
+  TileWalk next(tiles_x);
+  uint32_t buf = 0;
+  if (blockIdx.x < tile_count) issue_block(next.ty, next.tx);  // in flight while the scale is derived
+  const float gs = tile_global_scale(p), safe_gs = nz(gs);
+  fill_inv_table(inv_table, safe_gs);
+  const float inv6 = inv_scale(6.0f, safe_gs);
+
   const uint32_t src = stage + (warp < 4 ? lane * 2 * kSize : lane * PB::kPitch);
   const ChunkOffsets at = warp < 4 ? chunk_offsets(p.t, 2 * lane, warp) : chunk_offsets(p.r, row_in_tile + lane, 0);
   const ChunkOffsets row_step = {(p.t.dst_row_len >> 5) * 16, p.t.packed ? 16u : (p.t.dst_row_len >> 5) * 2, p.t.group_row_stride};
@@ -443,9 +462,6 @@ __global__ void __launch_bounds__(256, 2)
 
   for (uint64_t i = blockIdx.x * 256u + tid; i < p.zero_words; i += gridDim.x * 256u) p.zero[i] = make_uint4(0u, 0u, 0u, 0u);
 
-  TileWalk next(tiles_x);
-  uint32_t buf = 0;
-  if (blockIdx.x < tile_count) issue_block(next.ty, next.tx);
   __syncthreads();  // the table
 #pragma unroll 1
   for (uint32_t tile = blockIdx.x; tile < tile_count; tile += gridDim.x, buf ^= 1) {

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256) nvfp4_amax_kernel(const uint8_t* __restri
                                                           const uint8_t* __restrict__ scales,
                                                           const float* __restrict__ gscales, uint64_t n, uint32_t cols,
                                                           int rowwise, int packed, float* __restrict__ chunk_amax,
-                                                          float* __restrict__ out) {
+                                                          float* __restrict__ out, float* __restrict__ partials) {
   wait_for_prior_then_allow_next();
   bytes = after_prior(bytes);
   scales = after_prior(scales);
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256) nvfp4_amax_kernel(const uint8_t* __restri
     if (lane == 0 && chunk_amax) chunk_amax[chunk] = m;
     running = max_f32(running, m);
   }
-  cta_atomic_max(running, out);
+  cta_publish_max(running, out, partials);
 }
 
 // max over chunk values -> out[0] (transform 0) or the MS-EDEN global scale (transform 1).
@@ -1330,15 +1330,16 @@ int launch_row_amax(cudaStream_t s, const void* x, int dtype, float* out, uint32
                         rows, row_len);
 }
 
-uint32_t tensor_amax_partials(uint64_t n) { return blocks_for((n + 1023) / 1024, 8, kAmaxPartials); }
+uint32_t tensor_amax_partials(uint64_t n, uint32_t max_partials) { return blocks_for((n + 1023) / 1024, 8, max_partials); }
 
-int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_amax, float* out, uint64_t n, float* partials) {
+int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_amax, float* out, uint64_t n, float* partials,
+                       uint32_t max_partials) {
   if (!partials) {
     const cudaError_t err = cudaMemsetAsync(out, 0, sizeof(float), s);
     if (err != cudaSuccess) return static_cast<int>(err);
     if (n == 0) return 0;
   }
-  const uint32_t grid = partials ? tensor_amax_partials(n) : blocks_for((n + 1023) / 1024, 8, 148 * 8);
+  const uint32_t grid = partials ? tensor_amax_partials(n, max_partials) : blocks_for((n + 1023) / 1024, 8, 148 * 8);
   if (dtype == 0)
     return launch_chained(tensor_amax_kernel<float>, grid, 256, 0, s, static_cast<const float*>(x), chunk_amax, out, partials, n);
   return launch_chained(tensor_amax_kernel<__nv_bfloat16>, grid, 256, 0, s, static_cast<const __nv_bfloat16*>(x), chunk_amax, out,
@@ -1346,13 +1347,15 @@ int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_am
 }
 
 int launch_nvfp4_amax(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, const float* gscales, uint32_t rows,
-                      uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out) {
+                      uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out, float* partials) {
   const uint64_t n = static_cast<uint64_t>(rows) * cols;
-  cudaError_t err = cudaMemsetAsync(out, 0, sizeof(float), s);
-  if (err != cudaSuccess) return static_cast<int>(err);
-  if (n == 0) return 0;
-  return launch_chained(nvfp4_amax_kernel, blocks_for((n + 1023) / 1024, 8, 148 * 8), 256, 0, s, bytes, scales, gscales, n, cols,
-                        rowwise, packed, chunk_amax, out);
+  if (!partials) {
+    const cudaError_t err = cudaMemsetAsync(out, 0, sizeof(float), s);
+    if (err != cudaSuccess) return static_cast<int>(err);
+    if (n == 0) return 0;
+  }
+  return launch_chained(nvfp4_amax_kernel, tensor_amax_partials(n, kAmaxScratchPartials), 256, 0, s, bytes, scales, gscales, n, cols, rowwise, packed, chunk_amax, out,
+                        partials);
 }
 
 int launch_amax_from_chunks(cudaStream_t s, const float* chunk_amax, float* out, uint32_t chunk_count, int transform) {
@@ -1540,11 +1543,16 @@ static bool tile_covers(uint32_t src_rows, uint32_t dst_row_len) {
   return dst_row_len <= (src_rows + kTileRows - 1) / kTileRows * kTileRows;
 }
 
-int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a_in, const float* amax_in, float* gs_out) {
-  nvfp4_ms_eden_args a = a_in;
+bool ms_eden_takes_amax(const nvfp4_ms_eden_args& a) {
   const bool nv_kind = a.src_kind == NVFP4_SRC_NVFP4_TRANSPOSED || a.src_kind == NVFP4_SRC_ROWWISE_NVFP4_TRANSPOSED;
-  const bool nv_tiles = nv_kind && a.rows != 0 && a.cols != 0 && tile_covers(a.rows, a.dst_row_len) &&
-                        ms_eden_nvfp4_has_tile_form(a.src_bytes, a.src_scales, a.cols);
+  return nv_kind && a.rows != 0 && a.cols != 0 && a.dst_row_len >= 32 && tile_covers(a.rows, a.dst_row_len) &&
+         ms_eden_nvfp4_has_tile_form(a.src_bytes, a.src_scales, a.cols);
+}
+
+int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a_in, const float* amax_in, float* gs_out, uint32_t amax_count) {
+  nvfp4_ms_eden_args a = a_in;
+  const bool nv_tiles = ms_eden_takes_amax(a);
+  if (amax_count > 1 && !nv_tiles) return static_cast<int>(cudaErrorInvalidValue);
   if (amax_in) {
     // the tiled NVFP4 transposer derives the scale from the amax itself; every other kernel gets it from a
     // one-thread kernel first
@@ -1581,6 +1589,7 @@ int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a_in, const float* 
     p.col_sum_partials = nullptr;
     p.amax_in = amax_in;
     p.gs_out = gs_out;
+    p.amax_count = amax_count;
     if (nv_tiles) return launch_ms_eden_nvfp4_tiles(s, p, a.src_kind == NVFP4_SRC_ROWWISE_NVFP4_TRANSPOSED);
     switch (a.src_kind) {
       case NVFP4_SRC_F32_TRANSPOSED:
@@ -1658,8 +1667,8 @@ bool ms_eden_pair_takes_amax(const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_ar
 }
 
 int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& r, const nvfp4_ms_eden_args& t,
-                        float* col_sum_partials, const float* amax_in, float* gs_out, void* zero, uint64_t zero_words,
-                        bool beside_others) {
+                        float* col_sum_partials, const float* amax_in, float* gs_out, uint32_t amax_count, void* zero,
+                        uint64_t zero_words, bool beside_others) {
   const uint32_t rows = r.rows, cols = r.cols;
   if ((amax_in || zero_words) && !ms_eden_pair_takes_amax(r, t)) return static_cast<int>(cudaErrorInvalidValue);
   if (!ms_eden_pair_is_tiled(r, t)) {
@@ -1684,6 +1693,7 @@ int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& r, const nvfp4
   p.col_sum_partials = col_sum_partials;
   p.amax_in = amax_in;
   p.gs_out = gs_out;
+  p.amax_count = amax_count;
   p.zero = static_cast<uint4*>(zero);
   p.zero_words = zero_words;
   if (ms_eden_pair_has_tile_form(r.x, r.src_dtype, cols)) return launch_ms_eden_pair_tiles(s, p, r.src_dtype, beside_others);

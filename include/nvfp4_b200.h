@@ -171,6 +171,16 @@ int nvfp4_quantize_relu2_four_six_rowwise(void* stream, const void* pre_activati
                                           uint8_t* out_scales, int scale_layout, float* out_global_scale,
                                           float* out_row_amax, float* out_decoded_amax);
 
+/* The two quantizers above and nvfp4_gemm for a caller that has cleared out_decoded_amax / relu2_row_amax itself (one
+ * memset for all of a step's): the call does not clear it, and takes the maximum with what it holds. */
+int nvfp4_quantize_four_six_rowwise_fused_cleared(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols,
+                                                  uint8_t* out_fp4, uint8_t* out_scales, int scale_layout,
+                                                  float* out_global_scale, float* out_row_amax, float* out_decoded_amax);
+int nvfp4_quantize_relu2_four_six_rowwise_cleared(void* stream, const void* pre_activation, int dtype, uint32_t rows,
+                                                  uint32_t cols, const float* row_amax_in, uint8_t* out_fp4,
+                                                  uint8_t* out_scales, int scale_layout, float* out_global_scale,
+                                                  float* out_row_amax, float* out_decoded_amax);
+
 /* gpt/mlp/launcher.rs:66-76  MlpModule::relu2_backward / relu2_backward_f16 (kernels gpt/mlp/kernels.rs:72-104):
  * d_pre = (d_out * 2) * max(pre, 0) between the two MLP linears of the backward pass. */
 int nvfp4_relu2_backward(void* stream, const float* pre_activation, const float* d_out, float* d_pre_activation,
@@ -393,6 +403,7 @@ typedef struct nvfp4_gemm_args {
  * memory by tcgen05.mma kind::mxf4nvf4.  Replaces pack + prepare_tma + gemm_tma + post-op
  * (utils/nvfp4_tma_matmul/launcher.rs:106-328, gpt/projection_postop.rs:50-162).           */
 int nvfp4_gemm(void* stream, const nvfp4_gemm_args* args /* host */);
+int nvfp4_gemm_cleared(void* stream, const nvfp4_gemm_args* args /* host */);  /* see ..._fused_cleared */
 
 /* What nvfp4_gemm would choose for `args` on the current device, without launching (no reference
  * counterpart: the reference has one tile shape, utils/nvfp4_tma_matmul/kernels.rs:1314).  Lets a caller

@@ -141,33 +141,32 @@ class Nvfp4QuantModule {
   }
   // `RowwiseNvfp4Scratch::quantize_row_amax` (crates/gpt2-nvfp4/src/types/nvfp4_scratch/scratch.rs:35-52):
   // row amax and rowwise four-six in one pass.  `row_amax` may be empty for rows of up to 4096 values;
-  // `out.decoded_amax`, when set, receives max |decoded value| for the backward pass.
+  // `out.decoded_amax`, when set, receives max |decoded value| for the backward pass; `amax_cleared`: it is zero already.
   template <typename T>
   DriverError quantize_row_amax(Stream s, DeviceBuffer<const T> x, const Nvfp4TensorView& out,
-                                DeviceBuffer<float> row_amax = {}) const {
+                                DeviceBuffer<float> row_amax = {}, bool amax_cleared = false) const {
     if (auto e = out.check()) return e;
     if (!out.rowwise) return detail::invalid("quantize_row_amax: output must be rowwise");
     if (x.len < static_cast<size_t>(out.rows) * out.cols) return detail::invalid("quantize_row_amax: input too short");
     if (row_amax.ptr && row_amax.len < out.rows) return detail::invalid("quantize_row_amax: row_amax too short");
-    return detail::from_rc(nvfp4_quantize_four_six_rowwise_fused(s, x.ptr, dtype_of<T>::value, out.rows, out.cols,
-                                                                 out.bytes.ptr, out.scales.ptr, out.scale_layout,
-                                                                 out.global_scales.ptr, row_amax.ptr,
-                                                                 out.decoded_amax.ptr));
+    const auto entry = amax_cleared ? nvfp4_quantize_four_six_rowwise_fused_cleared : nvfp4_quantize_four_six_rowwise_fused;
+    return detail::from_rc(entry(s, x.ptr, dtype_of<T>::value, out.rows, out.cols, out.bytes.ptr, out.scales.ptr,
+                                 out.scale_layout, out.global_scales.ptr, row_amax.ptr, out.decoded_amax.ptr));
   }
   // The same quantizer applied to relu(pre)^2 computed on load: the MLP activation is never stored
   // (`RowwiseNvfp4Scratch::quantize_precomputed_amax` fed by the ReLU^2 post-op's row amax in the reference,
   // crates/gpt2-nvfp4/src/types/l3_mlp/forward.rs:60-76).  `row_amax_in` may be empty.
   template <typename T>
   DriverError quantize_relu2(Stream s, DeviceBuffer<const T> pre_activation, DeviceBuffer<const float> row_amax_in,
-                             const Nvfp4TensorView& out) const {
+                             const Nvfp4TensorView& out, bool amax_cleared = false) const {
     if (auto e = out.check()) return e;
     if (!out.rowwise) return detail::invalid("quantize_relu2: output must be rowwise");
     if (pre_activation.len < static_cast<size_t>(out.rows) * out.cols) return detail::invalid("quantize_relu2: input too short");
     if (row_amax_in.ptr && row_amax_in.len < out.rows) return detail::invalid("quantize_relu2: row_amax_in too short");
-    return detail::from_rc(nvfp4_quantize_relu2_four_six_rowwise(s, pre_activation.ptr, dtype_of<T>::value, out.rows,
-                                                                 out.cols, row_amax_in.ptr, out.bytes.ptr, out.scales.ptr,
-                                                                 out.scale_layout, out.global_scales.ptr, nullptr,
-                                                                 out.decoded_amax.ptr));
+    const auto entry = amax_cleared ? nvfp4_quantize_relu2_four_six_rowwise_cleared : nvfp4_quantize_relu2_four_six_rowwise;
+    return detail::from_rc(entry(s, pre_activation.ptr, dtype_of<T>::value, out.rows, out.cols, row_amax_in.ptr,
+                                 out.bytes.ptr, out.scales.ptr, out.scale_layout, out.global_scales.ptr, nullptr,
+                                 out.decoded_amax.ptr));
   }
   // Tensor amax of an f32 / bf16 tensor (quant/amax.rs:19-23)
   template <typename T>
@@ -206,7 +205,7 @@ class Nvfp4GemmModule {
   template <typename T>
   DriverError gemm(Stream s, const Nvfp4TensorView& a, const Nvfp4TensorView& b, DeviceBuffer<T> out,
                    Epilogue epilogue = Epilogue::None, DeviceBuffer<const float> bias = {},
-                   DeviceBuffer<T> aux = {}, DeviceBuffer<float> relu2_row_amax = {}) const {
+                   DeviceBuffer<T> aux = {}, DeviceBuffer<float> relu2_row_amax = {}, bool row_amax_cleared = false) const {
     if (auto e = a.check()) return e;
     if (auto e = b.check()) return e;
     if (a.cols != b.cols) return detail::invalid("gemm: A and B must share K");
@@ -227,7 +226,7 @@ class Nvfp4GemmModule {
     g.out_dtype = dtype_of<T>::value;
     if (relu2_row_amax.ptr && relu2_row_amax.len < a.rows) return detail::invalid("gemm: relu2_row_amax too short");
     g.relu2_row_amax = relu2_row_amax.ptr;
-    return detail::from_rc(nvfp4_gemm(s, &g));
+    return detail::from_rc(row_amax_cleared ? nvfp4_gemm_cleared(s, &g) : nvfp4_gemm(s, &g));
   }
   // launcher.rs:39-166: validates the operands and puts their tensor maps into the calling thread's cache
   DriverError prepare_tma_nvfp4_device_scales(Stream s, const Nvfp4TensorView& a, const Nvfp4TensorView& b) const {

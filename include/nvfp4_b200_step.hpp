@@ -163,7 +163,7 @@ class ProjectionStep {
     const uint16_t* weight = nullptr;
     const float* bias = nullptr;
     Nvfp4TensorView wq, xq;
-    DeviceBuffer<float> w_amax, w_chunk, dweight, dbias;
+    DeviceBuffer<float> w_partials, dweight, dbias;
     MsEdenOperandBuffers weight_t_h;      // W^T of this step, quantized early on the weight stream
     cudaEvent_t wq_ready = nullptr, wt_ready = nullptr;
     uint32_t sign_seed = 0, scale_seed = 0;  // this step's MS-EDEN seeds
@@ -233,6 +233,9 @@ class ProjectionStep {
     }
     if (auto e = weight_side(s, weights_changed || !weights_quantized_)) return e;
     weights_quantized_ = true;
+    // every amax that the forward pass's kernels add to, in one go: a memset of their own ahead of each quantizer and fc GEMM
+    // cost them their early start, 3 us each
+    if (auto e = cuda(cudaMemsetAsync(forward_amax_.as<float>().ptr, 0, forward_amax_.bytes(), s), "memset")) return e;
     for (auto& l : linears_)
       if (auto e = forward(s, l)) return e;
     return backward(s);
@@ -286,6 +289,9 @@ class ProjectionStep {
     };
     const Kind kinds[4] = {{d, 3 * d, NVFP4_EPI_BIAS}, {d, d, NVFP4_EPI_BIAS}, {d, h, NVFP4_EPI_RELU2}, {h, d, NVFP4_EPI_BIAS}};
     linears_.resize(n_lin);
+    // decoded amax of every X, and the pre-activation row amax of every layer
+    forward_amax_ = DeviceBlock((n_lin + static_cast<size_t>(shape_.n_layer) * T) * sizeof(float));
+    if (!forward_amax_.ok()) error_ = "cudaMalloc failed";
     for (size_t i = 0; i < n_lin; ++i) {
       Linear& l = linears_[i];
       const bool head = i + 1 == n_lin;
@@ -295,9 +301,9 @@ class ProjectionStep {
       l.weight = in.weight[i], l.bias = in.bias[i];
       l.bucket = head ? shape_.n_layer : static_cast<uint32_t>(i / 4);
       l.wq = alloc_tensor(l.out, l.in, false, false);
-      l.xq = alloc_tensor(T, l.in, true, true);
-      l.w_amax = alloc(sizeof(float)).as<float>();
-      l.w_chunk = alloc(sizeof(float) * ((static_cast<size_t>(l.out) * l.in + 1023) / 1024)).as<float>();
+      l.xq = alloc_tensor(T, l.in, true, false);
+      l.xq.decoded_amax = {forward_amax_.as<float>().ptr + i, 1};
+      l.w_partials = alloc(sizeof(float) * nvfp4_tensor_amax_partials()).as<float>();
       l.weight_t_h = alloc_operand(LinearBackwardMsEdenScratchSizes(T, l.in, l.out).weight_t_h);
       if (cudaEventCreateWithFlags(&l.wq_ready, cudaEventDisableTiming) != cudaSuccess ||
           cudaEventCreateWithFlags(&l.wt_ready, cudaEventDisableTiming) != cudaSuccess)
@@ -336,7 +342,6 @@ class ProjectionStep {
       if (!dx_.count(l.in)) dx_.emplace(l.in, DeviceBlock(static_cast<size_t>(T) * l.in * 2));
     }
     pre_ = DeviceBlock(static_cast<size_t>(T) * h * 2);
-    pre_row_amax_ = DeviceBlock(static_cast<size_t>(T) * sizeof(float));
     amax_vec_ = DeviceBlock(2 * n_lin * sizeof(float));
     e_scales_ = DeviceBlock(n_lin * sizeof(float));
     bool streams = cudaStreamCreateWithFlags(&weight_stream_, cudaStreamNonBlocking) == cudaSuccess &&
@@ -345,7 +350,7 @@ class ProjectionStep {
     for (cudaEvent_t* e : {&fork_, &join_, &weights_free_, &layer_done_, &comm_done_})
       streams = streams && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
     if (!streams && error_.empty()) error_ = "could not create the step's streams / events";
-    if (!pre_.ok() || !pre_row_amax_.ok() || !amax_vec_.ok() || !e_scales_.ok()) error_ = "cudaMalloc failed";
+    if (!pre_.ok() || !amax_vec_.ok() || !e_scales_.ok()) error_ = "cudaMalloc failed";
   }
 
   // The weight side of a step, on its own stream beside the forward pass: (when the masters changed) four-six of
@@ -357,9 +362,9 @@ class ProjectionStep {
     if (auto e = cuda(cudaStreamWaitEvent(weight_stream_, weights_free_, 0), "stream wait")) return e;
     if (requantize) {
       for (auto& l : linears_) {
-        const DeviceBuffer<const uint16_t> w{l.weight, static_cast<size_t>(l.out) * l.in};
-        if (auto e = quant_.tensor_amax<uint16_t>(weight_stream_, w, l.w_chunk, l.w_amax)) return e;
-        if (auto e = quant_.quantize_four_six<uint16_t>(weight_stream_, w, l.w_amax, l.wq)) return e;
+        if (int rc = nvfp4_quantize_four_six_tensor(weight_stream_, l.weight, NVFP4_DTYPE_BF16, l.out, l.in, l.w_partials.ptr,
+                                                    l.wq.bytes.ptr, l.wq.scales.ptr, l.wq.scale_layout, l.wq.global_scales.ptr))
+          return detail::from_rc(rc);
         if (auto e = cuda(cudaEventRecord(l.wq_ready, weight_stream_), "event record")) return e;
       }
     }
@@ -396,6 +401,10 @@ class ProjectionStep {
 
   DriverError forward(cudaStream_t s, Linear& l) {
     const uint32_t T = opt_.tokens;
+    const bool in_layer = l.bucket < shape_.n_layer;
+    const DeviceBuffer<float> pre_row_amax{
+        in_layer ? forward_amax_.as<float>().ptr + linears_.size() + static_cast<size_t>(l.bucket) * T : nullptr, in_layer ? T : 0};
+    const DeviceBuffer<const float> row_amax{pre_row_amax.ptr, pre_row_amax.len};
     // Behind an event a kernel does not start early, so the wait stands before the quantizer and not between it and its GEMM.
     // The first linear's quantizer does not wait; the others' need not either, but the weight stream is taken to be ahead of
     // them: 2 to 7 % less per step for 4 layers of d_model 768 and 1024 at 128 to 2048 tokens, the same time for 3 of d_model
@@ -406,16 +415,17 @@ class ProjectionStep {
     if (opt_.fused_mlp && l.is_proj) {
       // the MLP activation relu(pre)^2 is computed on load from the fc projection's pre-activation; its row
       // amax came out of that GEMM's epilogue
-      if (auto e = quant_.quantize_relu2<uint16_t>(s, pre_.as<const uint16_t>(), pre_row_amax_.as<const float>(), l.xq)) return e;
+      if (auto e = quant_.quantize_relu2<uint16_t>(s, pre_.as<const uint16_t>(), row_amax, l.xq, true)) return e;
     } else {
       const DeviceBuffer<const uint16_t> x{x_.at(l.in), static_cast<size_t>(T) * l.in};
-      if (auto e = quant_.quantize_row_amax<uint16_t>(s, x, l.xq)) return e;
+      if (auto e = quant_.quantize_row_amax<uint16_t>(s, x, l.xq, {}, true)) return e;
     }
     if (first)
       if (auto e = cuda(cudaStreamWaitEvent(s, l.wq_ready, 0), "stream wait")) return e;
     const DeviceBuffer<const float> bias{l.bias, l.bias ? l.out : 0};
     if (opt_.fused_mlp && l.is_fc)
-      return gemm_.gemm<uint16_t>(s, l.xq, l.wq, pre_.as<uint16_t>(), Epilogue::Bias, bias, {}, pre_row_amax_.as<float>());
+      return gemm_.gemm<uint16_t>(s, l.xq, l.wq, pre_.as<uint16_t>(), Epilogue::Bias, bias, {},
+                                  pre_row_amax, true);
     const DeviceBuffer<uint16_t> aux = l.is_fc ? pre_.as<uint16_t>() : DeviceBuffer<uint16_t>{};
     return gemm_.gemm<uint16_t>(s, l.xq, l.wq, y_.at(l.out).as<uint16_t>(), static_cast<Epilogue>(l.epilogue), bias, aux);
   }
@@ -488,7 +498,7 @@ class ProjectionStep {
   std::map<std::pair<uint32_t, uint32_t>, LinearBackwardMsEdenScratchBuffers> scratch_;
   std::map<uint32_t, DeviceBlock> y_, dx_;
   std::map<uint32_t, const uint16_t*> x_, dy_;
-  DeviceBlock pre_, pre_row_amax_, amax_vec_, e_scales_;
+  DeviceBlock pre_, forward_amax_, amax_vec_, e_scales_;
   cudaStream_t weight_stream_ = nullptr, side_stream_ = nullptr, comm_stream_ = nullptr;
   cudaEvent_t fork_ = nullptr, join_ = nullptr, weights_free_ = nullptr, layer_done_ = nullptr, comm_done_ = nullptr;
   bool weights_quantized_ = false;

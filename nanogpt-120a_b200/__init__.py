@@ -139,7 +139,9 @@ _SIGNATURES = {
     "nvfp4_quantize_four_six": [_P, _P, c_int, _P, c_int, _U, _U, _P, _P, c_int, _P],
     "nvfp4_quantize_four_six_tensor": [_P, _P, c_int, _U, _U, _P, _P, _P, c_int, _P],
     "nvfp4_quantize_four_six_rowwise_fused": [_P, _P, c_int, _U, _U, _P, _P, c_int, _P, _P, _P],
+    "nvfp4_quantize_four_six_rowwise_fused_cleared": [_P, _P, c_int, _U, _U, _P, _P, c_int, _P, _P, _P],
     "nvfp4_quantize_relu2_four_six_rowwise": [_P, _P, c_int, _U, _U, _P, _P, _P, c_int, _P, _P, _P],
+    "nvfp4_quantize_relu2_four_six_rowwise_cleared": [_P, _P, c_int, _U, _U, _P, _P, _P, c_int, _P, _P, _P],
     "nvfp4_tc_matmul_ms_eden": [_P, _P, _P, _P, POINTER(MsEdenOperand), _F, POINTER(MsEdenOperand), _F, _U, _U, _U, _U, _U],
     "nvfp4_relu2_backward": [_P, _P, _P, _P, _U],
     "nvfp4_relu2_backward_f16": [_P, _P, _P, _P, _U],
@@ -173,6 +175,7 @@ _SIGNATURES = {
     "nvfp4_transpose_pad_f32": [_P, _P, _P, _U, _U, _U, _U],
     "nvfp4_crop_f32": [_P, _P, _P, _U, _U, _U],
     "nvfp4_gemm": [_P, POINTER(GemmArgs)],
+    "nvfp4_gemm_cleared": [_P, POINTER(GemmArgs)],
     "nvfp4_gemm_plan_query": [POINTER(GemmArgs), POINTER(GemmPlan)],
     "nvfp4_prepare_tma_nvfp4_device_scales": [_P, _P, _P, _P, _P, _U, _U, _U],
     "nvfp4_prepare_tma_nvfp4_device_scales_into": [_P, _P, _P, _P, _P, _U, _U, _U, _P],

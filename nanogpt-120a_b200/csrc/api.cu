@@ -129,10 +129,9 @@ int nvfp4_quantize_four_six_tensor(void* stream, const void* x, int dtype, uint3
                          scale_layout == NVFP4_SCALES_PACKED, out_gs, 0, nullptr, tensor_amax_partials(n));
 }
 
-int nvfp4_quantize_four_six_rowwise_fused(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols,
-                                          uint8_t* out_fp4, uint8_t* out_scales, int scale_layout,
-                                          float* out_global_scale, float* out_row_amax,
-                                          float* out_decoded_amax) {
+static int quantize_rowwise_fused(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols, uint8_t* out_fp4,
+                                  uint8_t* out_scales, int scale_layout, float* out_global_scale, float* out_row_amax,
+                                  float* out_decoded_amax, bool cleared) {
   if (cols % 16 != 0) return invalid("quantize_four_six_rowwise_fused: cols must be a multiple of 16");
   if (scale_layout == NVFP4_SCALES_PACKED && cols % 64 != 0)
     return invalid("quantize_four_six_rowwise_fused: the packed scale layout needs cols % 64 == 0");
@@ -140,7 +139,7 @@ int nvfp4_quantize_four_six_rowwise_fused(void* stream, const void* x, int dtype
   if (reinterpret_cast<uintptr_t>(x) & 15u) return invalid("quantize_four_six_rowwise_fused: input must be 16-byte aligned");
   const int packed = scale_layout == NVFP4_SCALES_PACKED;
   int rc = launch_four_six_rowwise_fused(S(stream), x, dtype, rows, cols, out_fp4, out_scales, packed,
-                                         out_global_scale, out_row_amax, out_decoded_amax);
+                                         out_global_scale, out_row_amax, out_decoded_amax, 0, cleared);
   if (rc != -1) return rc;
   // rows too long for one thread block: a row amax pass, then the rowwise quantizer
   if (!out_row_amax) return invalid("quantize_four_six_rowwise_fused: rows longer than 4096 need out_row_amax");
@@ -152,11 +151,22 @@ int nvfp4_quantize_four_six_rowwise_fused(void* stream, const void* x, int dtype
   return launch_nvfp4_amax(S(stream), out_fp4, out_scales, out_global_scale, rows, cols, 1, packed, nullptr,
                            out_decoded_amax);
 }
+int nvfp4_quantize_four_six_rowwise_fused(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols,
+                                          uint8_t* out_fp4, uint8_t* out_scales, int scale_layout,
+                                          float* out_global_scale, float* out_row_amax, float* out_decoded_amax) {
+  return quantize_rowwise_fused(stream, x, dtype, rows, cols, out_fp4, out_scales, scale_layout, out_global_scale,
+                                out_row_amax, out_decoded_amax, false);
+}
+int nvfp4_quantize_four_six_rowwise_fused_cleared(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols,
+                                                  uint8_t* out_fp4, uint8_t* out_scales, int scale_layout,
+                                                  float* out_global_scale, float* out_row_amax, float* out_decoded_amax) {
+  return quantize_rowwise_fused(stream, x, dtype, rows, cols, out_fp4, out_scales, scale_layout, out_global_scale,
+                                out_row_amax, out_decoded_amax, true);
+}
 
-int nvfp4_quantize_relu2_four_six_rowwise(void* stream, const void* pre_activation, int dtype, uint32_t rows,
-                                          uint32_t cols, const float* row_amax_in, uint8_t* out_fp4,
-                                          uint8_t* out_scales, int scale_layout, float* out_global_scale,
-                                          float* out_row_amax, float* out_decoded_amax) {
+static int quantize_relu2_rowwise(void* stream, const void* pre_activation, int dtype, uint32_t rows, uint32_t cols,
+                                  const float* row_amax_in, uint8_t* out_fp4, uint8_t* out_scales, int scale_layout,
+                                  float* out_global_scale, float* out_row_amax, float* out_decoded_amax, bool cleared) {
   if (cols % 16 != 0) return invalid("quantize_relu2_four_six_rowwise: cols must be a multiple of 16");
   if (scale_layout == NVFP4_SCALES_PACKED && cols % 64 != 0)
     return invalid("quantize_relu2_four_six_rowwise: the packed scale layout needs cols % 64 == 0");
@@ -172,12 +182,26 @@ int nvfp4_quantize_relu2_four_six_rowwise(void* stream, const void* pre_activati
       if (e != cudaSuccess) return static_cast<int>(e);
     }
     return launch_four_six(S(stream), pre_activation, dtype, row_amax_in, 1, rows, cols, out_fp4, out_scales, packed,
-                           out_global_scale, 1, out_decoded_amax);
+                           out_global_scale, 1, out_decoded_amax, 1, cleared);
   }
   int rc = launch_four_six_rowwise_fused(S(stream), pre_activation, dtype, rows, cols, out_fp4, out_scales, packed,
-                                         out_global_scale, out_row_amax, out_decoded_amax, 1);
+                                         out_global_scale, out_row_amax, out_decoded_amax, 1, cleared);
   if (rc != -1) return rc;
   return invalid("quantize_relu2_four_six_rowwise: rows longer than 4096 need row_amax_in");
+}
+int nvfp4_quantize_relu2_four_six_rowwise(void* stream, const void* pre_activation, int dtype, uint32_t rows,
+                                          uint32_t cols, const float* row_amax_in, uint8_t* out_fp4,
+                                          uint8_t* out_scales, int scale_layout, float* out_global_scale,
+                                          float* out_row_amax, float* out_decoded_amax) {
+  return quantize_relu2_rowwise(stream, pre_activation, dtype, rows, cols, row_amax_in, out_fp4, out_scales, scale_layout,
+                                out_global_scale, out_row_amax, out_decoded_amax, false);
+}
+int nvfp4_quantize_relu2_four_six_rowwise_cleared(void* stream, const void* pre_activation, int dtype, uint32_t rows,
+                                                  uint32_t cols, const float* row_amax_in, uint8_t* out_fp4,
+                                                  uint8_t* out_scales, int scale_layout, float* out_global_scale,
+                                                  float* out_row_amax, float* out_decoded_amax) {
+  return quantize_relu2_rowwise(stream, pre_activation, dtype, rows, cols, row_amax_in, out_fp4, out_scales, scale_layout,
+                                out_global_scale, out_row_amax, out_decoded_amax, true);
 }
 
 // ---- ReLU^2 backward -------------------------------------------------------------------------
@@ -558,6 +582,10 @@ int nvfp4_crop_f32(void* stream, const float* src, float* dst, uint32_t rows, ui
 int nvfp4_gemm(void* stream, const nvfp4_gemm_args* args) {
   if (!args) return invalid("nvfp4_gemm: null args");
   return launch_gemm(S(stream), *args);
+}
+int nvfp4_gemm_cleared(void* stream, const nvfp4_gemm_args* args) {
+  if (!args) return invalid("nvfp4_gemm: null args");
+  return launch_gemm(S(stream), *args, false, true);
 }
 
 int nvfp4_gemm_plan_query(const nvfp4_gemm_args* args, nvfp4_gemm_plan* out) {

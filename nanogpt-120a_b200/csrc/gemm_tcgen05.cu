@@ -1991,7 +1991,7 @@ bool gemm_adds_into_output(const nvfp4_gemm_args& a) {
   return pl.k_splits > 1;
 }
 
-int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero) {
+int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool row_amax_cleared) {
   if (a.m == 0 || a.n == 0) return 0;
   int rc = validate_gemm(a);
   if (rc) return rc;
@@ -2065,7 +2065,7 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero) {
     cudaError_t e = cudaMemset2DAsync(a.out, static_cast<size_t>(a.ldo) * esz, 0, static_cast<size_t>(a.n) * esz, a.m, s);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  if (a.relu2_row_amax) {
+  if (a.relu2_row_amax && !row_amax_cleared) {
     cudaError_t e = cudaMemsetAsync(a.relu2_row_amax, 0, static_cast<size_t>(a.m) * sizeof(float), s);
     if (e != cudaSuccess) return static_cast<int>(e);
   }

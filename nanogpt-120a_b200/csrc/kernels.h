@@ -24,13 +24,14 @@ int launch_nvfp4_amax(cudaStream_t s, const uint8_t* bytes, const uint8_t* scale
 // transform 0: out[0] = max(chunks); 1: out[0] = MS-EDEN global scale of that max
 int launch_amax_from_chunks(cudaStream_t s, const float* chunk_amax, float* out, uint32_t chunk_count, int transform);
 int launch_ms_eden_scale_from_amax(cudaStream_t s, const float* amax, float* out);
-// relu2: quantize relu(x)^2 computed on load; decoded_amax (optional f32[1]): max |decoded value| of the result
+// relu2: quantize relu(x)^2 computed on load; decoded_amax (optional f32[1]): max |decoded value| of the result, cleared first
+// unless decoded_cleared
 int launch_four_six(cudaStream_t s, const void* x, int dtype, const float* amax, int rowwise, uint32_t rows,
                     uint32_t cols, uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, int relu2 = 0,
-                    float* decoded_amax = nullptr, uint32_t amax_count = 1);
+                    float* decoded_amax = nullptr, uint32_t amax_count = 1, bool decoded_cleared = false);
 int launch_four_six_rowwise_fused(cudaStream_t s, const void* x, int dtype, uint32_t rows, uint32_t cols,
                                   uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, float* out_amax,
-                                  float* decoded_amax, int relu2 = 0);
+                                  float* decoded_amax, int relu2 = 0, bool decoded_cleared = false);
 int launch_four_six_padded(cudaStream_t s, const float* x, const float* amax, uint8_t* out_fp4, uint8_t* out_scales,
                            float* out_gs, uint32_t rows, uint32_t cols, uint32_t padded_rows, uint32_t padded_cols,
                            int transposed);
@@ -80,7 +81,8 @@ uint32_t relu2_backward_grid(uint64_t n);
 
 // gemm_tcgen05.cu ---------------------------------------------------------------------------
 // out_is_zero: the output holds zeros already (it is cleared first where gemm_adds_into_output otherwise)
-int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero = false);
+// row_amax_cleared: so does a.relu2_row_amax
+int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero = false, bool row_amax_cleared = false);
 // Whether launch_gemm splits K and sums the partial tiles in the output.
 bool gemm_adds_into_output(const nvfp4_gemm_args& a);
 // What launch_gemm would choose for these arguments on the current device (no launch).

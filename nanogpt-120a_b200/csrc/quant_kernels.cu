@@ -1423,8 +1423,8 @@ static int launch_four_six_source(cudaStream_t s, const Source& src, const float
 
 int launch_four_six(cudaStream_t s, const void* x, int dtype, const float* amax, int rowwise, uint32_t rows,
                     uint32_t cols, uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, int relu2,
-                    float* decoded_amax, uint32_t amax_count) {
-  if (decoded_amax) {
+                    float* decoded_amax, uint32_t amax_count, bool decoded_cleared) {
+  if (decoded_amax && !decoded_cleared) {
     const cudaError_t err = cudaMemsetAsync(decoded_amax, 0, sizeof(float), s);
     if (err != cudaSuccess) return static_cast<int>(err);
   }
@@ -1441,10 +1441,10 @@ int launch_four_six(cudaStream_t s, const void* x, int dtype, const float* amax,
 // caller then runs the two-kernel path).
 int launch_four_six_rowwise_fused(cudaStream_t s, const void* x, int dtype, uint32_t rows, uint32_t cols,
                                   uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, float* out_amax,
-                                  float* decoded_amax, int relu2) {
+                                  float* decoded_amax, int relu2, bool decoded_cleared) {
   const uint32_t gpr = cols / 16;
   if (gpr == 0 || gpr > 256) return -1;
-  if (decoded_amax) {
+  if (decoded_amax && !decoded_cleared) {
     const cudaError_t err = cudaMemsetAsync(decoded_amax, 0, sizeof(float), s);
     if (err != cudaSuccess) return static_cast<int>(err);
   }

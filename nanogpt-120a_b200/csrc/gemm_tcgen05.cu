@@ -22,7 +22,7 @@
 // 128 columns, which the epilogue takes first, so that all but a quarter of it overlaps as well.  Every mbarrier wait is bounded: on expiry the kernel records a status word, drains,
 // frees its tensor memory and returns.
 //
-// No thread-block clusters, no multicast: every load reads this GPU's own memory.
+// Clusters only as CTA pairs for long main loops (cta_group::2), no multicast loads: every load reads this GPU's own memory.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -63,10 +63,12 @@ constexpr uint32_t kStatusProducerTimeout = 1u, kStatusMmaTimeout = 2u, kStatusE
 // streaming GEMMs are bound by the operand bytes an SM can pull from L2, and the tall tile moves 21 % fewer of
 // them per flop than 128 x 256.  Its two 192-column accumulators and two scale-factor column sets fill tensor
 // memory (2 x 192 + 2 x 56 = 496 of 512 columns), so the accumulator is single buffered.
-// kPanel: 0 streaming, else resident with a B panel of up to so many k-tiles
-template <int kBlockM, int kBlockN, int kPanel>
+// kPanel: 0 streaming, else resident with a B panel of up to so many k-tiles.  kPair: two CTAs of a cluster on neighbouring SMs
+// (cta_group::2) work on 256 x 256; each loads its 128 rows of A and half of B, a third fewer operand bytes per flop.
+template <int kBlockM, int kBlockN, int kPanel, bool kPair>
 struct Cfg {
   static constexpr bool kResident = kPanel != 0;
+  static_assert(!kPair || (kPanel == 0 && kBlockM == 128 && kBlockN == 256), "a pair streams 128 x 256 tiles");
   static constexpr int kMHalves = kBlockM / kRowBlock;
   static_assert(kBlockM == 128 || (kBlockM == 256 && kBlockN == 192 && !kResident), "unsupported tile shape");
   static constexpr int kAStageBytes = kMHalves * kAHalfBytes;
@@ -74,7 +76,8 @@ struct Cfg {
   // 128-row scale-factor blocks of B a tile can touch: a 192-column tile starts either on a block
   // boundary or in the middle of a block, and spans two blocks either way
   static constexpr int kSfBlocks = (kBlockN + 127) / 128;
-  static constexpr int kBStageBytes = kBlockN * kBlockKBytes;
+  static constexpr int kBRows = kPair ? kBlockN / 2 : kBlockN;  // rows of B a CTA loads
+  static constexpr int kBStageBytes = kBRows * kBlockKBytes;
   static constexpr int kSfbStageBytes = kSfBlocks * kSfBlockStageBytes;
   static constexpr int kAccStages = (kBlockN == 256 || kMHalves == 2) ? 1 : 2;
   static constexpr int kAccCols = kMHalves * kBlockN;  // columns of one accumulator buffer (row halves side by side)
@@ -275,6 +278,48 @@ __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fe
 __device__ __forceinline__ void tcgen05_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// The forms of a CTA pair (two CTAs of a cluster on neighbouring SMs, cta_group::2).  `kBothCtas`: the signal goes to the
+// barrier at this offset in both.
+constexpr uint16_t kBothCtas = 3;
+template <bool kPair>
+__device__ __forceinline__ void commit(uint32_t bar) {
+  if constexpr (kPair)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"(kBothCtas)
+                 : "memory");
+  else
+    tcgen05_commit(bar);
+}
+__device__ __forceinline__ uint32_t leader_address(uint32_t addr) {  // of the same variable in the pair's first CTA
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+// At CTA scope: what the other CTA's MMAs read has been ordered by the tcgen05 fences, and a release at cluster scope in this
+// place waited 1200 cycles for the thread's other memory operations.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// An operand load of either CTA of a pair, counted by the barrier `bar` of one of them.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int32_t x, int32_t y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+          dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tcgen05_mma_nvf4_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                      uint32_t accumulate, uint32_t tmem_sfa, uint32_t tmem_sfb) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n\t}" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
+      : "memory");
+}
 __device__ __forceinline__ void tcgen05_mma_nvf4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                                  uint32_t accumulate, uint32_t tmem_sfa, uint32_t tmem_sfb) {
   asm volatile(
@@ -352,11 +397,11 @@ __device__ __forceinline__ uint64_t make_ab_desc(uint32_t smem_addr) {
   return d;
 }
 // Instruction descriptor of kind::mxf4nvf4: E2M1 x E2M1, UE4M3 scales, K-major A and B,
-// M = 128, N = kBlockN, K = 64.
-template <int kBlockN>
+// M = 128 (256 of a pair), N = kBlockN, K = 64.
+template <int kBlockN, bool kPair>
 __device__ __forceinline__ constexpr uint32_t make_idesc() {
   return (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kBlockN >> 3) << 17) | (0u << 23) |
-         (static_cast<uint32_t>(kRowBlock >> 4) << 24);
+         (static_cast<uint32_t>(((kPair ? 2 : 1) * kRowBlock) >> 4) << 24);
 }
 
 // Loads of values that the kernel before this one may have written.  Volatile and through the coherent path: a read-only
@@ -498,12 +543,12 @@ struct SubTile<__nv_bfloat16> {
 // Streaming mode: one B slot per pipeline stage.  Resident mode (short K): the whole
 // [kBlockN x K] B panel of the current column block stays in shared memory -- one slot per
 // k-tile -- while a CTA walks down the row blocks, so only A tiles stream through the ring.
-template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel>
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel, bool kPair>
 __global__ void __launch_bounds__(kThreads, 1)
     nvfp4_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                               const __grid_constant__ CUtensorMap tmap_out,
                               const __grid_constant__ CUtensorMap tmap_aux, const GemmParams p) {
-  using C = Cfg<kBlockM, kBlockN, kPanel>;
+  using C = Cfg<kBlockM, kBlockN, kPanel, kPair>;
   constexpr bool kResident = C::kResident;
   constexpr bool kTmaStore = kStore != StorePath::kDirect, kResidual = kStore == StorePath::kTmaResidual;
   static_assert(!kResidual || sizeof(OutT) == 4, "the residual stream of the TMA path is f32");
@@ -558,14 +603,19 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     *abort_flag = 0;
   }
+  // In a pair, a tile is two CTAs' blocks of rows beside one block of columns, of which each loads a half; the first issues the
+  // MMAs of both.  Its `full` and `tmem_empty` barriers count both CTAs.
+  uint32_t rank = 0;
+  if (kPair) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  rank = __shfl_sync(0xffffffffu, rank, 0);
   if (warp == 1) {  // a barrier per lane and pass, in the order of the barrier block
     constexpr uint32_t kTmemEmpty = 3 * kMaxStages + 2, kStaged = kTmemEmpty + 5 + C::kSfSets, kStored = kStaged + C::kStoreBufs,
                        kFinal = kStored + C::kStoreBufs;
     for (uint32_t b = lane; b < kFinal + kMaxFinal; b += 32) {
       // full: the operands, and the scale factors of the four warps; a released accumulator: both groups' warps; a staged
       // sub-tile: the group's warps
-      const uint32_t count = b < kMaxStages                                        ? 5
-                             : b == kTmemEmpty || b == kTmemEmpty + 1              ? 8
+      const uint32_t count = b < kMaxStages                                        ? (kPair ? 9 : 5)
+                             : b == kTmemEmpty || b == kTmemEmpty + 1              ? (kPair ? 16 : 8)
                              : (b >= kStaged && b < kStored) || b >= kFinal ? 4
                                                                                    : 1;
       mbar_init(smem_bar + 8 * b, count);
@@ -573,17 +623,27 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_ptr)),
-                 "r"(static_cast<uint32_t>(kTmemCols))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (kPair) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_ptr)),
+                   "r"(static_cast<uint32_t>(kTmemCols))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_ptr)),
+                   "r"(static_cast<uint32_t>(kTmemCols))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
     tcgen05_fence_before();
   }
   // Programmatic dependent launch: the CTA touches only its own SM up to the roles' waits for what runs before it in the stream,
   // each of which stands ahead of the role's first access to memory, behind the fetch of its code and of its first tile.  The
   // GEMM itself does not allow the next kernel to start early: its CTAs end at different times, and the first SMs that come
   // free would take all of a small grid's CTAs.
-  __syncthreads();
+  if (kPair)
+    cluster_sync();
+  else
+    __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_base_ptr, 0);  // warp uniform also to the compiler
 
@@ -607,9 +667,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     w_end = static_cast<uint32_t>(static_cast<uint64_t>(tiles_mn) * (blockIdx.x + 1) / gridDim.x);
     w_step = 1;
   } else {
-    w_begin = blockIdx.x;
+    w_begin = kPair ? blockIdx.x / 2 : blockIdx.x;
     w_end = tiles_mn * p.k_splits;
-    w_step = gridDim.x;
+    w_step = kPair ? gridDim.x / 2 : gridDim.x;
   }
   auto decode = [&](uint32_t w, uint32_t& m_blk, uint32_t& n_blk, uint32_t& split) {
     if (kResident && p.resident_cpn) {
@@ -625,6 +685,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       split = w / tiles_mn;
       m_blk = tile / p.num_n_blocks;
       n_blk = tile - m_blk * p.num_n_blocks;
+      if (kPair) m_blk = 2 * m_blk + rank;  // may lie below the matrix
     }
   };
 
@@ -646,11 +707,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   // The last tile of a CTA has the shared memory of the operands to itself: what the ring does not hold of it is staged there,
   // every sub-tile in a buffer of its own, and no sub-tile waits for a store: 2304 x 768 x K 8192 f32 17.4 -> 16.0 us, 1024 x
   // 1024 x K 8192 13.4 -> 12.0, 8192 x 768 x K 2304 bf16 11.2 -> 10.8.  (Not for 192 columns and four k-tiles: it spills.)
+  constexpr int kOperandBytes = 3 * (kAStageBytes + (kResident ? 0 : C::kBStageBytes)) + kPanel * C::kBStageBytes / 2;  // at least
+  constexpr int kBeyondRing = kTurns - static_cast<int>(kRing), kSpare = kOperandBytes / (2 * kStoreStageBytes);
   constexpr int kFinalTurns =
-      kResidual || (kPanel == 4 && kBlockN == 192) || kTurns <= static_cast<int>(kRing) ? 0 : kTurns - static_cast<int>(kRing);
+      kResidual || (kPanel == 4 && kBlockN == 192) || kBeyondRing < 0 ? 0 : kBeyondRing < kSpare ? kBeyondRing : kSpare;
   static_assert(2 * kFinalTurns <= static_cast<int>(kMaxFinal), "buffers of the last tile");
-  static_assert(2 * kFinalTurns * kStoreStageBytes <= 3 * (kAStageBytes + (kResident ? 0 : C::kBStageBytes)) + kPanel * C::kBStageBytes / 2,
-                "the last tile's buffers lie in the operands' stages");
+  auto in_final = [&](int turn) { return turn >= static_cast<int>(kRing) && turn < static_cast<int>(kRing) + kFinalTurns; };
   auto final_index = [&](uint32_t group, int turn) { return static_cast<uint32_t>(turn - static_cast<int>(kRing)) * 2u + group; };
   auto item_valid = [&](int item, uint32_t m_blk, uint32_t n_blk) {  // there is one, and not wholly outside the matrix
     if (item >= kItems) return false;
@@ -699,7 +761,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ++runs;
       }
       // scale blocks of A inside the matrix (the second row half of a tall tile may lie below it)
-      const uint32_t a_blks = min(static_cast<uint32_t>(kMHalves), p.sfa_blocks128 - m_blk * kMHalves);
+      const uint32_t a_blks = min(static_cast<uint32_t>(kMHalves), p.sfa_blocks128 - min(m_blk * kMHalves, p.sfa_blocks128));
       if (kResident) {
         // A goes to L2 two tiles ahead: from HBM, beside the output's writes, a k-tile takes 1900 cycles and more, longer than
         // the ring covers (65536 x 2304 x K 768 80 us without).  In a banded schedule the column blocks' CTAs read the same A
@@ -747,13 +809,31 @@ __global__ void __launch_bounds__(kThreads, 1)
                           sf_bytes, scales);
           }
           const int32_t x = static_cast<int32_t>(kt * kBlockKBytes);
-          mbar_expect_tx(full, kAStageBytes + (kResident ? 0 : C::kBStageBytes));
-          tma_load_2d(smem_a + stage * kAStageBytes, &tmap_a, full, x, static_cast<int32_t>(m_blk * kBlockM));
-          if (!kResident) tma_load_2d(smem_b + stage * C::kBStageBytes, &tmap_b, full, x, static_cast<int32_t>(n_blk * kBlockN));
+          if constexpr (kPair) {
+            const uint32_t both = leader_address(full);
+            if (rank == 0) mbar_expect_tx(full, 2 * (kAStageBytes + C::kBStageBytes));
+            tma_load_2d_pair(smem_a + stage * kAStageBytes, &tmap_a, both, x, static_cast<int32_t>(m_blk * kBlockM));
+            tma_load_2d_pair(smem_b + stage * C::kBStageBytes, &tmap_b, both, x,
+                             static_cast<int32_t>(n_blk * kBlockN + rank * C::kBRows));
+          } else {
+            mbar_expect_tx(full, kAStageBytes + (kResident ? 0 : C::kBStageBytes));
+            tma_load_2d(smem_a + stage * kAStageBytes, &tmap_a, full, x, static_cast<int32_t>(m_blk * kBlockM));
+            if (!kResident) tma_load_2d(smem_b + stage * C::kBStageBytes, &tmap_b, full, x, static_cast<int32_t>(n_blk * kBlockN));
+          }
         }
         __syncwarp();
         GEMM_TRACE(0, 2, lane == 0);
         ++issued;
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    if (kPair) {
+      // the commits that hand the last stages back come from the other CTA: they arrive before this one ends
+      for (uint32_t i = 0; i < stages && ok; ++i) {  // (a stage never used is free at once)
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, kStatusProducerTimeout, p.wait_timeout_ns));
         if (++stage == stages) {
           stage = 0;
           phase ^= 1u;
@@ -776,10 +856,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     // uniform (uniform registers); one elected lane issues the tensor-core instructions.  Issuing
     // from inside a single-lane branch instead costs ~140 cycles per tcgen05.mma.
     {
-      constexpr uint32_t idesc = make_idesc<kBlockN>();
+      constexpr uint32_t idesc = make_idesc<kBlockN, kPair>();
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, runs = 0, prev_n = 0xffffffffu, sf_set = 0, tile_iter = 0;
       bool ok = true;
-      for (uint32_t w = w_begin; w < w_end && ok; w += w_step, ++tile_iter) {
+      for (uint32_t w = rank == 0 ? w_begin : w_end; w < w_end && ok; w += w_step, ++tile_iter) {
         uint32_t m_blk, n_blk, split;
         decode(w, m_blk, n_blk, split);
         const uint32_t kt_begin = split * p.k_tiles_per_split;
@@ -824,13 +904,13 @@ __global__ void __launch_bounds__(kThreads, 1)
               if (kb < atoms) {
 #pragma unroll
                 for (uint32_t h = 0; h < static_cast<uint32_t>(kMHalves); ++h)
-                  tcgen05_mma_nvf4(tmem_acc + h * kBlockN, desc_a + h * (kAHalfBytes >> 4) + kb * 2, desc_b + kb * 2, idesc,
+                  (kPair ? tcgen05_mma_nvf4_pair : tcgen05_mma_nvf4)(tmem_acc + h * kBlockN, desc_a + h * (kAHalfBytes >> 4) + kb * 2, desc_b + kb * 2, idesc,
                                    (kt > kt_begin || kb > 0) ? 1u : 0u, tsfa + h * 4 * kKAtomsPerStage + kb * 4,
                                    tsfb + kb * C::kSfbColsPerAtom);
               }
             }
-            tcgen05_commit(bar_empty + 8 * stage);       // frees the smem stage once these MMAs retire
-            tcgen05_commit(bar_sf_empty + 8 * sf_set);   // ... and the scale-factor column set
+            commit<kPair>(bar_empty + 8 * stage);      // frees the smem stage once these MMAs retire
+            commit<kPair>(bar_sf_empty + 8 * sf_set);  // ... and the scale-factor column set
           }
           __syncwarp();
           GEMM_TRACE(1, 13, lane == 0);
@@ -845,7 +925,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // banded schedule keeps one column block)
         const bool release_panel = kResident && p.resident_cpn == 0 && w + 1 == (n_blk + 1) * p.num_m_blocks;
         if (elect_one()) {
-          tcgen05_commit(bar_tmem_full + 8 * acc);  // accumulator complete
+          commit<kPair>(bar_tmem_full + 8 * acc);  // accumulator complete
           if (release_panel) tcgen05_commit(bar_b_empty);
         }
         __syncwarp();
@@ -857,7 +937,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (!ok) {
         // aborting: give the MMAs already issued a bounded chance to retire before tensor memory is freed
-        if (elect_one()) tcgen05_commit(bar_mma_drain);
+        if (elect_one()) commit<kPair>(bar_mma_drain);
         __syncwarp();
         for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(bar_mma_drain, 0); ++spin) {
         }
@@ -1007,7 +1087,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         tcgen05_fence_before();
         __syncwarp();
         // scale factors visible to the MMA issuer; that the slot has been read follows from the MMAs that need them
-        if (lane == 0) mbar_arrive(bar_full + 8 * stage);
+        if (lane == 0) {
+          if (kPair)
+            mbar_arrive_cluster(leader_address(bar_full + 8 * stage));
+          else
+            mbar_arrive(bar_full + 8 * stage);
+        }
         GEMM_TRACE(2, 21, warp == 8 && lane == 0);
         if (++sf_set == sf_sets) {
           sf_set = 0;
@@ -1018,6 +1103,17 @@ __global__ void __launch_bounds__(kThreads, 1)
           phase ^= 1u;
         }
       }
+    }
+    if (kPair) {
+      // as the producer does for its stages: the sets' last commits come from the other CTA (a set never used is free at once)
+      for (uint32_t i = 0; i < sf_sets && ok; ++i) {
+        ok = mbar_wait(bar_sf_empty + 8 * sf_set, sf_phase ^ 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns);
+        if (++sf_set == sf_sets) {
+          sf_set = 0;
+          sf_phase ^= 1u;
+        }
+      }
+      __syncwarp();
     }
   } else if (warp == 2 || warp == 3) {
     // ===================== store warps (one per epilogue group) =====================
@@ -1084,7 +1180,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int item = item_of(eg, tile_iter, turn);
           if (!item_valid(item, m_blk, n_blk)) continue;
           const int32_t x = item_x(item, n_blk), y = item_y(item, m_blk);
-          if (final_tile && turn >= static_cast<int>(kRing)) {
+          if (final_tile && in_final(turn)) {
             const uint32_t f = final_index(eg, turn);
             ok = __all_sync(0xffffffffu, mbar_wait(bar_final + 8 * f, 0, abort_flag, kStatusEpilogueTimeout, downstream_timeout_ns));
             if (ok && elect_one()) {
@@ -1234,7 +1330,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       auto release_accumulator = [&]() {
         tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_tmem_empty + 8 * acc);
+        if (lane == 0) {
+          if (kPair)
+            mbar_arrive_cluster(leader_address(bar_tmem_empty + 8 * acc));
+          else
+            mbar_arrive(bar_tmem_empty + 8 * acc);
+        }
       };
       if (kTmaStore) {
         // the group's sub-tiles go through its shared-memory ring to the store warp; rows / columns outside the matrix
@@ -1337,7 +1438,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 square_f32x2(v[i], v[i + 1]);
               }
             }
-            if (final_tile && turn >= static_cast<int>(kRing)) {
+            if (final_tile && in_final(turn)) {
               const uint32_t f = final_index(eg, turn);
               if (ok) {
                 SubTile<OutT>::stage(smem_base + f * kStoreStageBytes + gtid * 128, gtid, v);
@@ -1429,12 +1530,20 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   // ===================== teardown =====================
   tcgen05_fence_before();
-  __syncthreads();
+  if (kPair) {
+    __syncwarp();
+    cluster_sync();  // neither CTA ends while the other may still signal it
+  } else {
+    __syncthreads();
+  }
   if (warp == 2) {
     tcgen05_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(static_cast<uint32_t>(kTmemCols))
-                 : "memory");
+    if constexpr (kPair)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(static_cast<uint32_t>(kTmemCols))
+                   : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(static_cast<uint32_t>(kTmemCols))
+                   : "memory");
   }
 }
 
@@ -1582,21 +1691,22 @@ struct GemmTiming {
 // Everything the host decides about one launch.
 struct GemmPlan {
   uint32_t block_m = 128, block_n = 128, num_n_blocks = 0, k_splits = 1, k_tiles_per_split = 0;
-  uint32_t stages = 0, grid = 0, b_resident = 0, panel = 0, resident_cpn = 0, tma_store = 0, vec_store = 0;
+  uint32_t stages = 0, grid = 0, b_resident = 0, panel = 0, resident_cpn = 0, tma_store = 0, vec_store = 0, pair = 0;
   size_t smem_bytes = 0;
 };
 
 struct TileBytes {
   int fixed, stage, slot;  // see Cfg
 };
-template <int kBlockM, int kBlockN, int kPanel>
+template <int kBlockM, int kBlockN, int kPanel, bool kPair = false>
 constexpr TileBytes tile_bytes_of() {
-  using C = Cfg<kBlockM, kBlockN, kPanel>;
+  using C = Cfg<kBlockM, kBlockN, kPanel, kPair>;
   return {C::kFixedBytes, C::kStageBytes, C::kSlotBytes};
 }
 // The resident form of a tile for so many k-tiles.
 constexpr uint32_t panel_of(uint32_t block_n, uint32_t num_k_tiles) { return block_n == 128 || num_k_tiles > 3 ? 4 : 3; }
-TileBytes tile_bytes(uint32_t block_m, uint32_t block_n, uint32_t panel) {
+TileBytes tile_bytes(uint32_t block_m, uint32_t block_n, uint32_t panel, bool pair) {
+  if (pair) return tile_bytes_of<128, 256, 0, true>();
   if (block_m == 256) return tile_bytes_of<256, 192, 0>();
   if (block_n == 256) return panel ? tile_bytes_of<128, 256, 3>() : tile_bytes_of<128, 256, 0>();
   if (block_n == 192)
@@ -1604,7 +1714,7 @@ TileBytes tile_bytes(uint32_t block_m, uint32_t block_n, uint32_t panel) {
   return panel ? tile_bytes_of<128, 128, 4>() : tile_bytes_of<128, 128, 0>();
 }
 
-template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel>
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel, bool kPair = false>
 int launch_schedule_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo,
                          const CUtensorMap& mx, const GemmParams& p, const GemmPlan& pl) {
   // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
@@ -1613,7 +1723,7 @@ int launch_schedule_variant(cudaStream_t s, const CUtensorMap& ma, const CUtenso
   if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
   int st = attr_state[dev].load(std::memory_order_acquire);
   if (st == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel>,
+    const cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel, kPair>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
     st = e == cudaSuccess ? 1 : -static_cast<int>(e);
     attr_state[dev].store(st, std::memory_order_release);
@@ -1631,18 +1741,21 @@ int launch_schedule_variant(cudaStream_t s, const CUtensorMap& ma, const CUtenso
   // The kernel may be set up while the one before it in the stream drains (the quantizers allow it from their start).
   // Every allocation, barrier and tensor-map fetch of the prologue and the launch itself then cost nothing behind a
   // quantizer: 16 tokens x 768 -> 2304 with its quantizer 12.3 -> 10.5 us, 8192 tokens 30.8 -> 28.5 us.
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = 2;
+  attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(pl.grid);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = pl.smem_bytes;
   cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = kPair ? 2 : 1;
   int rc = static_cast<int>(
-      cudaLaunchKernelEx(&cfg, nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel>, ma, mb, mo, mx, p));
+      cudaLaunchKernelEx(&cfg, nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel, kPair>, ma, mb, mo, mx, p));
   count_launch();
   if (rc == 0) rc = static_cast<int>(cudaGetLastError());
   if (rec) cudaEventRecord(rec->stop, s);
@@ -1659,6 +1772,9 @@ int launch_store_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMa
     if constexpr (kBlockN != 256) {
       if (pl.panel == 4) return launch_schedule_variant<kBlockM, kBlockN, OutT, kStore, 4>(s, ma, mb, mo, mx, p, pl);
     }
+  }
+  if constexpr (kStore != StorePath::kDirect && kBlockN == 256) {
+    if (pl.pair) return launch_schedule_variant<kBlockM, kBlockN, OutT, kStore, 0, true>(s, ma, mb, mo, mx, p, pl);
   }
   return launch_schedule_variant<kBlockM, kBlockN, OutT, kStore, 0>(s, ma, mb, mo, mx, p, pl);
 }
@@ -1856,7 +1972,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   };
   if (want_resident) {
     const uint32_t panel = panel_of(block_n, num_k_tiles);
-    const int st = stages_beside(tile_bytes(block_m, block_n, panel), num_k_tiles);
+    const int st = stages_beside(tile_bytes(block_m, block_n, panel, false), num_k_tiles);
     if (st >= 3) {
       pl.b_resident = 1;
       pl.panel = panel;
@@ -1869,7 +1985,20 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
         pl.resident_cpn = cpn;
     }
   }
-  const TileBytes tb = tile_bytes(block_m, block_n, pl.panel);
+  // CTA pairs for the main loops that are long enough, at 64 operand bytes per cycle and SM, to earn back what setting up and
+  // tearing down a pair and the signals between its CTAs cost (about 1.5 us): 8192 x 1024 x K 32000 bf16 127 -> 102 us, 32000 x
+  // 1024 x K 8192 f32 125 -> 110, 4096 x 2048 x K 8192 f32 residual 41 -> 38; 8192 x 1024 x K 4096 bf16 18.2 either way, 1024 x
+  // 1024 x K 2048 (a split of 8192) f32 12.9 -> 14.2.  Not the tall tile: its two column sets for scale factors leave no slack
+  // for those signals (8192 x 768 x K 32000 81 -> 85).  A pair per two SMs must need no more waves.
+  pl.pair = 0;
+  if (!pl.b_resident && pl.tma_store && block_m == 128 && block_n == 256 && pl.k_tiles_per_split >= 32 && usms % 2 == 0) {
+    const uint32_t pair_work = (a.m + 255u) / 256u * pl.num_n_blocks * pl.k_splits, pairs = usms / 2;
+    if ((pair_work + pairs - 1) / pairs <= (work + usms - 1) / usms) {
+      pl.pair = 1;
+      pl.grid = 2 * (pair_work < pairs ? pair_work : pairs);
+    }
+  }
+  const TileBytes tb = tile_bytes(block_m, block_n, pl.panel, pl.pair != 0);
   if (!pl.b_resident) {
     const int st = (kSmemBudget - tb.fixed) / (tb.stage + tb.slot);
     pl.stages = static_cast<uint32_t>(st > kMaxStages ? kMaxStages : st);
@@ -2023,7 +2152,8 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool
   p.weight = a.weight_global_scale;
   p.k_atoms = a.k / 64;
   p.num_k_tiles = (p.k_atoms + kKAtomsPerStage - 1) / kKAtomsPerStage;
-  p.num_m_blocks = (a.m + pl.block_m - 1) / pl.block_m;
+  const uint32_t tile_rows = pl.pair ? 2 * pl.block_m : pl.block_m;
+  p.num_m_blocks = (a.m + tile_rows - 1) / tile_rows;
   p.num_n_blocks = pl.num_n_blocks;
   p.sfa_blocks128 = (a.m + 127) / 128;
   p.sfb_blocks128 = (a.n + 127) / 128;
@@ -2047,7 +2177,7 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool
   CUtensorMap ma, mb, mo, mx;
   rc = encode_operand_map(&ma, a.a_bytes, a.m, a.k, pl.block_m);
   if (rc) return rc;
-  rc = encode_operand_map(&mb, a.b_bytes, a.n, a.k, pl.block_n);
+  rc = encode_operand_map(&mb, a.b_bytes, a.n, a.k, pl.pair ? pl.block_n / 2 : pl.block_n);
   if (rc) return rc;
   mo = ma;
   mx = ma;

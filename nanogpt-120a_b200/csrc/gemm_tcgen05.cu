@@ -1850,39 +1850,65 @@ int validate_gemm(const nvfp4_gemm_args& a) {
 void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   const uint32_t k_atoms = a.k / 64;
   const uint32_t num_k_tiles = (k_atoms + kKAtomsPerStage - 1) / kKAtomsPerStage;
-  const uint32_t m_blocks128 = (a.m + kRowBlock - 1) / kRowBlock;
   const uint32_t usms = static_cast<uint32_t>(sms);
-  // Tile shape.  A block-scaled FP4 tcgen05.mma occupies the tensor pipe for about as long at N = 128 as
-  // at N = 256 (the 128-column form is bound by shared-memory operand reads), so wide tiles do more work
-  // per instruction and are preferred whenever the shape can still fill the SMs:
-  //  * long K: enough wide tiles, or (f32 output, linear epilogue) enough tiles x K splits;
-  //  * short K with many row blocks: wide tile with its whole B panel resident in shared memory.
-  // 128 x 192 keeps a double-buffered accumulator (the drain of one tile hides behind the next main loop);
-  // 128 x 256 has one buffer; the tall 256 x 192 tile moves the fewest operand bytes per flop and is for
-  // streamed long-K GEMMs; 128 x 128 remains for everything else.
+  const size_t esz = a.out_dtype == NVFP4_DTYPE_F32 ? 4 : 2;
+  const uint32_t vec_elems = 16 / static_cast<uint32_t>(esz);
+  pl.vec_store = ((reinterpret_cast<uintptr_t>(a.out) & 15u) == 0 && a.ldo % vec_elems == 0 &&
+                  (!a.aux || (reinterpret_cast<uintptr_t>(a.aux) & 15u) == 0))
+                     ? 1
+                     : 0;
+  // TMA-store epilogue whenever the output satisfies the tensor-map rules (16-byte aligned base
+  // and row pitch); odd layouts use direct stores.  The f32 residual stream goes through the staging buffers as well, where
+  // its lanes would read and write a row each: 4096 x 2048 x K 8192 100 us with direct stores, 54 us.  A TMA reduction into
+  // the stream took 48 us, but every f32 reduction in global memory takes subnormals for zero.  A bf16 residual stays on
+  // the direct path, which adds in f32 and rounds once.
+  pl.tma_store = (pl.vec_store && (a.epilogue != NVFP4_EPI_RESIDUAL || a.out_dtype == NVFP4_DTYPE_F32)) ? 1 : 0;
   const bool can_split = a.out_dtype == NVFP4_DTYPE_F32 &&
                          (a.epilogue == NVFP4_EPI_NONE || a.epilogue == NVFP4_EPI_BIAS) && num_k_tiles >= 16;
-  //
   // The f32 residual stream is loaded into the staging buffers its sums leave from.  Two buffers per group (128 x 128)
   // keep a load in flight beside a store; one (the wider tiles) has them take turns, which a main loop of up to eight
   // k-tiles does not hide: 65536 x 768 x K 768 82 us at 128 x 128, 98 to 100 at the others, K 1536 96 against 106 to 110;
   // 8192 x 768 x K 3072 25 against 24.  Beyond, the estimate carries what the turns add to a tile.
   const bool f32_residual = a.epilogue == NVFP4_EPI_RESIDUAL && a.out_dtype == NVFP4_DTYPE_F32;
-  // Work items, waves and an estimated duration (SM cycles) of a candidate shape.  The constants are fits to
-  // B200 measurements of the training step's shapes: a streamed k-tile costs what its operand bytes take
-  // through the SM's L2 port (about 47 bytes per cycle: 128 x 128 700, 128 x 192 980, 128 x 256 1150,
-  // 256 x 192 1360 cycles), a tile adds the part of its epilogue that the next main loop does not hide (one
-  // accumulator buffer: all of the drain).
+  // CTA pairs for the main loops that are long enough, at 64 operand bytes per cycle and SM, to earn back what setting up and
+  // tearing down a pair and the signals between its CTAs cost (about 1.5 us): 8192 x 1024 x K 32000 bf16 127 -> 102 us, 32000 x
+  // 1024 x K 8192 f32 125 -> 110, 4096 x 2048 x K 8192 f32 residual 41 -> 38; 8192 x 1024 x K 4096 bf16 18.2 either way, 1024 x
+  // 1024 x K 2048 (a split of 8192) f32 12.9 -> 14.2.  Not the tall tile: its two column sets for scale factors leave no slack
+  // for those signals (8192 x 768 x K 32000 81 -> 85).  A pair per two SMs must need no more waves.
+  auto pairs_of = [&](uint32_t splits) { return (a.m + 255u) / 256u * ((a.n + 255u) / 256u) * splits; };
+  auto tiles_of = [&](uint32_t bm, uint32_t bn) { return ((a.m + bm - 1) / bm) * ((a.n + bn - 1) / bn); };
+  auto pair_fits = [&](uint32_t bm, uint32_t bn, uint32_t splits, uint32_t k_tiles_per_split) {
+    if (!pl.tma_store || bm != 128 || bn != 256 || k_tiles_per_split < 32 || usms % 2 != 0) return false;
+    return (pairs_of(splits) + usms / 2 - 1) / (usms / 2) <= (tiles_of(bm, bn) * splits + usms - 1) / usms;
+  };
+  // Short K and many row blocks: keep the B panel resident and stream only A (halves the
+  // operand traffic per tile; these shapes are otherwise bound by L2 -> SM bandwidth).
+  auto resident_shape = [&](uint32_t bm, uint32_t bn, uint32_t splits) {
+    const uint32_t tiles = tiles_of(bm, bn);
+    return bm == 128 && splits == 1 && num_k_tiles <= (bn == 256 ? 3u : 4u) && tiles >= 4 * (tiles < usms ? tiles : usms);
+  };
+  // Waves and an estimated duration (SM cycles) of a candidate shape: per wave the k-tiles, at what their operand bytes or
+  // MMAs take, and the part of the epilogue that no main loop hides; a split adds the clearing of the output and the
+  // reduction.  The constants are a fit, in round figures, to the four tiles measured on 58 shapes (16 to 65536 rows, 512 to
+  // 32000 columns, K 320 to 65536).  On 47 of them the tile taken was 8 % slower than the fastest one on average with the
+  // constants from before tiles overlapped their epilogues (k-tiles 700, 980, 1150, 1360; epilogues 1500, 2000, 3500, 5000),
+  // and is 2 % slower with these: 3072 x 768 x K 8192 f32 17.2 -> 14.2 us (128 x 128 in one wave, not three splits of 256 x
+  // 192), 3072 x 1024 x K 8192 f32 26.3 -> 17.7, 4096 x 8192 x K 2048 f32 ReLU^2 with its second output 80 -> 61, 4096 x 4096 x
+  // K 2048 bf16 24.5 -> 20.9, 2048 x 2304 x K 768 bf16 7.4 -> 6.0.
   struct Candidate {
     uint32_t splits;
     uint64_t cost;
   };
-  auto tiles_of = [&](uint32_t bm, uint32_t bn) { return ((a.m + bm - 1) / bm) * ((a.n + bn - 1) / bn); };
   auto evaluate = [&](uint32_t bm, uint32_t bn) {
     const uint32_t tiles = tiles_of(bm, bn);
-    const uint64_t ck = bm == 256 ? 1360 : bn == 256 ? 1150 : bn == 192 ? 980 : 700;
-    const uint64_t ce = (bm == 256 ? 5000 : bn == 256 ? 3500 : bn == 192 ? 2000 : 1500) +
-                        (!f32_residual ? 0 : bm == 256 ? 11000 : bn == 256 ? 6000 : bn == 192 ? 1000 : 0);
+    const int shape = bm == 256 ? 3 : bn == 256 ? 2 : bn == 192 ? 1 : 0;
+    constexpr uint64_t kTileCycles[4] = {550, 700, 850, 1050}, kResidentTileCycles = 300, kPairTileCycles = 800;
+    constexpr uint64_t kEpilogue[4] = {2000, 3000, 2500, 4000}, kF32Epilogue[4] = {4000, 3000, 6000, 6000};
+    constexpr uint64_t kSecondOutput[4] = {7500, 500, 3500, 12500}, kResidualTurns[4] = {0, 1000, 6000, 11000};
+    constexpr uint64_t kSplitCycles = 4000;
+    const uint64_t ce = kEpilogue[shape] + (a.out_dtype == NVFP4_DTYPE_F32 ? kF32Epilogue[shape] : 0) +
+                        (a.epilogue == NVFP4_EPI_RELU2 && a.aux ? kSecondOutput[shape] : 0) +
+                        (f32_residual ? kResidualTurns[shape] : 0);
     Candidate best{1, ~0ull};
     uint32_t max_splits = 1;
     if (can_split && tiles < 2 * usms) {
@@ -1894,8 +1920,11 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
     for (uint32_t sp = 1; sp <= max_splits; ++sp) {
       const uint32_t per = (num_k_tiles + sp - 1) / sp;
       const uint32_t real = (num_k_tiles + per - 1) / per;
-      const uint64_t waves = (static_cast<uint64_t>(tiles) * real + usms - 1) / usms;
-      const uint64_t cost = waves * (per * ck + ce);
+      const bool pair = pair_fits(bm, bn, real, per);
+      const uint64_t waves = pair ? (pairs_of(real) + usms / 2 - 1) / (usms / 2)
+                                  : (static_cast<uint64_t>(tiles) * real + usms - 1) / usms;
+      const uint64_t ck = resident_shape(bm, bn, real) ? kResidentTileCycles : pair ? kPairTileCycles : kTileCycles[shape];
+      const uint64_t cost = waves * (per * ck + ce) + (real > 1 ? kSplitCycles : 0);
       if (cost < best.cost) best = Candidate{real, cost};  // ties go to fewer splits
     }
     return best;
@@ -1914,31 +1943,32 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
     const bool wide_shape = a.n % 256 == 0 || a.n > 1024;
     const bool ok256 = wide_shape && ((num_k_tiles >= 4 && (tiles256 >= usms || can_split)) ||
                                       (a.n % 256 == 0 && num_k_tiles <= 3 && tiles256 >= 4u * usms));
+    uint64_t best = ~0ull;
+    auto consider = [&](uint32_t bm, uint32_t bn) {
+      const uint64_t cost = evaluate(bm, bn).cost;
+      if (cost >= best) return;
+      best = cost;
+      block_m = bm;
+      block_n = bn;
+    };
+    // Short K with a resident B panel is bound by writing the output, which the estimate does not see: the widest tile.
+    const bool wide_resident = num_k_tiles <= 3 && ok192 && (ok256 || resident_shape(128, 192, 1));
+    if (wide_resident) {
+      consider(128, ok256 ? 256 : 192);
+    } else {
+      if (ok192) consider(128, 192);
+      if (ok256) consider(128, 256);
+      // The narrow tile where its finer waves pay: six k-tiles and more that cannot be split go to the wide ones.
+      if (can_split || num_k_tiles < 6 || (!ok192 && !ok256)) consider(128, 128);
+    }
     // the tall tile: streamed long-K GEMMs only (its A stages leave no room for a resident panel, and short-K
-    // GEMMs are bound by writing their output); the wave count in the estimate decides against it when its
-    // tiles are too few
-    const bool ok_tall = fits192 && num_k_tiles >= 6;
-    if (ok192 && ok256) {
-      // short K (resident B panel, bound by writing the output): the wider tile; otherwise the cheaper estimate
-      if (num_k_tiles <= 3)
-        block_n = a.n % 256 == 0 ? 256 : 192;
-      else
-        block_n = evaluate(128, 192).cost < evaluate(128, 256).cost ? 192 : 256;
-    } else if (ok256) {
-      block_n = 256;
-    } else if (ok192) {
-      block_n = 192;
-    }
-    if (ok_tall && g_allow_tall.load(std::memory_order_relaxed) && evaluate(256, 192).cost < evaluate(128, block_n).cost) {
-      block_m = 256;
-      block_n = 192;
-    }
+    // GEMMs are bound by writing their output)
+    if (fits192 && num_k_tiles >= 6 && g_allow_tall.load(std::memory_order_relaxed)) consider(256, 192);
   }
   pl.block_m = block_m;
   pl.block_n = block_n;
   pl.num_n_blocks = (a.n + block_n - 1) / block_n;
   const uint32_t num_m_blocks = (a.m + block_m - 1) / block_m;
-  (void)m_blocks128;
   const uint32_t tiles = num_m_blocks * pl.num_n_blocks;
 
   // split-K for long GEMMs with few tiles (dW = dY^T.X): f32 output, linear epilogue only; the split count is
@@ -1947,30 +1977,13 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   pl.k_tiles_per_split = (num_k_tiles + pl.k_splits - 1) / pl.k_splits;
   pl.k_splits = (num_k_tiles + pl.k_tiles_per_split - 1) / pl.k_tiles_per_split;
 
-  const size_t esz = a.out_dtype == NVFP4_DTYPE_F32 ? 4 : 2;
-  const uint32_t vec_elems = 16 / static_cast<uint32_t>(esz);
-  pl.vec_store = ((reinterpret_cast<uintptr_t>(a.out) & 15u) == 0 && a.ldo % vec_elems == 0 &&
-                  (!a.aux || (reinterpret_cast<uintptr_t>(a.aux) & 15u) == 0))
-                     ? 1
-                     : 0;
-  // TMA-store epilogue whenever the output satisfies the tensor-map rules (16-byte aligned base
-  // and row pitch); odd layouts use direct stores.  The f32 residual stream goes through the staging buffers as well, where
-  // its lanes would read and write a row each: 4096 x 2048 x K 8192 100 us with direct stores, 54 us.  A TMA reduction into
-  // the stream took 48 us, but every f32 reduction in global memory takes subnormals for zero.  A bf16 residual stays on
-  // the direct path, which adds in f32 and rounds once.
-  pl.tma_store = (pl.vec_store && (a.epilogue != NVFP4_EPI_RESIDUAL || a.out_dtype == NVFP4_DTYPE_F32)) ? 1 : 0;
-
   const uint32_t work = tiles * pl.k_splits;
   pl.grid = work < usms ? work : usms;
-  // Short K and many row blocks: keep the B panel resident and stream only A (halves the
-  // operand traffic per tile; these shapes are otherwise bound by L2 -> SM bandwidth).
-  const bool want_resident =
-      block_m == 128 && pl.k_splits == 1 && num_k_tiles <= (block_n == 256 ? 3u : 4u) && tiles >= 4 * pl.grid;
   pl.b_resident = pl.panel = pl.resident_cpn = 0;
   auto stages_beside = [&](const TileBytes& tb, uint32_t slots) {
     return (kSmemBudget - tb.fixed - static_cast<int>(slots) * tb.slot) / tb.stage;
   };
-  if (want_resident) {
+  if (resident_shape(block_m, block_n, pl.k_splits)) {
     const uint32_t panel = panel_of(block_n, num_k_tiles);
     const int st = stages_beside(tile_bytes(block_m, block_n, panel, false), num_k_tiles);
     if (st >= 3) {
@@ -1985,19 +1998,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
         pl.resident_cpn = cpn;
     }
   }
-  // CTA pairs for the main loops that are long enough, at 64 operand bytes per cycle and SM, to earn back what setting up and
-  // tearing down a pair and the signals between its CTAs cost (about 1.5 us): 8192 x 1024 x K 32000 bf16 127 -> 102 us, 32000 x
-  // 1024 x K 8192 f32 125 -> 110, 4096 x 2048 x K 8192 f32 residual 41 -> 38; 8192 x 1024 x K 4096 bf16 18.2 either way, 1024 x
-  // 1024 x K 2048 (a split of 8192) f32 12.9 -> 14.2.  Not the tall tile: its two column sets for scale factors leave no slack
-  // for those signals (8192 x 768 x K 32000 81 -> 85).  A pair per two SMs must need no more waves.
-  pl.pair = 0;
-  if (!pl.b_resident && pl.tma_store && block_m == 128 && block_n == 256 && pl.k_tiles_per_split >= 32 && usms % 2 == 0) {
-    const uint32_t pair_work = (a.m + 255u) / 256u * pl.num_n_blocks * pl.k_splits, pairs = usms / 2;
-    if ((pair_work + pairs - 1) / pairs <= (work + usms - 1) / usms) {
-      pl.pair = 1;
-      pl.grid = 2 * (pair_work < pairs ? pair_work : pairs);
-    }
-  }
+  pl.pair = !pl.b_resident && pair_fits(block_m, block_n, pl.k_splits, pl.k_tiles_per_split) ? 1 : 0;
+  if (pl.pair) pl.grid = 2 * (pairs_of(pl.k_splits) < usms / 2 ? pairs_of(pl.k_splits) : usms / 2);
   const TileBytes tb = tile_bytes(block_m, block_n, pl.panel, pl.pair != 0);
   if (!pl.b_resident) {
     const int st = (kSmemBudget - tb.fixed) / (tb.stage + tb.slot);

@@ -1894,7 +1894,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   // constants from before tiles overlapped their epilogues (k-tiles 700, 980, 1150, 1360; epilogues 1500, 2000, 3500, 5000),
   // and is 2 % slower with these: 3072 x 768 x K 8192 f32 17.2 -> 14.2 us (128 x 128 in one wave, not three splits of 256 x
   // 192), 3072 x 1024 x K 8192 f32 26.3 -> 17.7, 4096 x 8192 x K 2048 f32 ReLU^2 with its second output 80 -> 61, 4096 x 4096 x
-  // K 2048 bf16 24.5 -> 20.9, 2048 x 2304 x K 768 bf16 7.4 -> 6.0.
+  // K 2048 bf16 24.5 -> 20.9, 2048 x 2304 x K 768 bf16 7.4 -> 6.0.  A pair's setting up and tearing down count once, not per
+  // wave: 32000 x 768 x K 8192 f32 99 -> 93, where a split of 768 x 768 x K 65536 over pairs stays with the tall tile.
   struct Candidate {
     uint32_t splits;
     uint64_t cost;
@@ -1902,13 +1903,14 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   auto evaluate = [&](uint32_t bm, uint32_t bn) {
     const uint32_t tiles = tiles_of(bm, bn);
     const int shape = bm == 256 ? 3 : bn == 256 ? 2 : bn == 192 ? 1 : 0;
-    constexpr uint64_t kTileCycles[4] = {550, 700, 850, 1050}, kResidentTileCycles = 300, kPairTileCycles = 800;
+    constexpr uint64_t kTileCycles[4] = {550, 700, 850, 1050}, kResidentTileCycles = 300;
+    constexpr uint64_t kPairTileCycles = 710, kPairF32Epilogue = 2000, kPairSetup = 6000;
     constexpr uint64_t kEpilogue[4] = {2000, 3000, 2500, 4000}, kF32Epilogue[4] = {4000, 3000, 6000, 6000};
     constexpr uint64_t kSecondOutput[4] = {7500, 500, 3500, 12500}, kResidualTurns[4] = {0, 1000, 6000, 11000};
     constexpr uint64_t kSplitCycles = 4000;
-    const uint64_t ce = kEpilogue[shape] + (a.out_dtype == NVFP4_DTYPE_F32 ? kF32Epilogue[shape] : 0) +
-                        (a.epilogue == NVFP4_EPI_RELU2 && a.aux ? kSecondOutput[shape] : 0) +
+    const uint64_t ce = kEpilogue[shape] + (a.epilogue == NVFP4_EPI_RELU2 && a.aux ? kSecondOutput[shape] : 0) +
                         (f32_residual ? kResidualTurns[shape] : 0);
+    const bool f32_out = a.out_dtype == NVFP4_DTYPE_F32;
     Candidate best{1, ~0ull};
     uint32_t max_splits = 1;
     if (can_split && tiles < 2 * usms) {
@@ -1924,7 +1926,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
       const uint64_t waves = pair ? (pairs_of(real) + usms / 2 - 1) / (usms / 2)
                                   : (static_cast<uint64_t>(tiles) * real + usms - 1) / usms;
       const uint64_t ck = resident_shape(bm, bn, real) ? kResidentTileCycles : pair ? kPairTileCycles : kTileCycles[shape];
-      const uint64_t cost = waves * (per * ck + ce) + (real > 1 ? kSplitCycles : 0);
+      const uint64_t cf = !f32_out ? 0 : pair ? kPairF32Epilogue : kF32Epilogue[shape];
+      const uint64_t cost = waves * (per * ck + ce + cf) + (real > 1 ? kSplitCycles : 0) + (pair ? kPairSetup : 0);
       if (cost < best.cost) best = Candidate{real, cost};  // ties go to fewer splits
     }
     return best;

@@ -113,7 +113,7 @@ def test_backward_scale_from_partial_maxima(pkg, dev, chunks):
 @pytest.mark.parametrize("m,n,k,dtype,epi,want", [
     (3072, 768, 8192, f32, 0, (128, 128, 1)), (2304, 768, 8192, f32, 0, (128, 192, 2)), (768, 768, 65536, f32, 0, (256, 192, 12)),
     (4096, 4096, 2048, bf16, 1, (128, 256, 1)), (4096, 8192, 2048, f32, 2, (128, 192, 1)), (2048, 2304, 768, bf16, 1, (128, 128, 1)),
-    (16, 768, 768, bf16, 1, (128, 128, 1)), (200, 768, 4352, f32, 0, (128, 128, 2))])
+    (32000, 768, 8192, f32, 0, (128, 256, 1)), (16, 768, 768, bf16, 1, (128, 128, 1)), (200, 768, 4352, f32, 0, (128, 128, 2))])
 def test_the_estimate_takes_the_measured_tile(pkg, dev, m, n, k, dtype, epi, want):
     """The fastest tile, or one within a few per cent of it, where a wave more or less, the f32 or the second output decides."""
     stub, one = torch.zeros(16, dtype=torch.uint8, device=dev), torch.ones(1, device=dev)

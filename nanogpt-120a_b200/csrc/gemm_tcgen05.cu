@@ -19,8 +19,8 @@
 // Three tile widths.  BLOCK_N = 128 and 192 double buffer the accumulator (2 x 192 accumulator
 // columns + 3 x 40 scale-factor columns fill the 512 columns of tensor memory), so the epilogue of
 // one tile overlaps the main loop of the next; the 256-column accumulators of consecutive tiles share
-// 128 columns, which the epilogue takes first, so that all but a quarter of it overlaps as well.  Every mbarrier wait is bounded: on expiry the kernel records a status word, drains,
-// frees its tensor memory and returns.
+// 128 columns, which the epilogue takes first, so that half of it overlaps as well.  Every mbarrier
+// wait is bounded: on expiry the kernel records a status word, drains, frees its tensor memory and returns.
 //
 // Clusters only as CTA pairs for long main loops (cta_group::2), no multicast loads: every load reads this GPU's own memory.
 #include <cuda.h>
@@ -1883,9 +1883,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   };
   // Short K and many row blocks: keep the B panel resident and stream only A (halves the
   // operand traffic per tile; these shapes are otherwise bound by L2 -> SM bandwidth).
-  auto resident_shape = [&](uint32_t bm, uint32_t bn, uint32_t splits) {
-    const uint32_t tiles = tiles_of(bm, bn);
-    return bm == 128 && splits == 1 && num_k_tiles <= (bn == 256 ? 3u : 4u) && tiles >= 4 * (tiles < usms ? tiles : usms);
+  auto resident_shape = [&](uint32_t bm, uint32_t bn, uint32_t splits, uint32_t tiles) {
+    return bm == 128 && splits == 1 && num_k_tiles <= (bn == 256 ? 3u : 4u) && tiles >= 4 * usms;
   };
   // Waves and an estimated duration (SM cycles) of a candidate shape: per wave the k-tiles, at what their operand bytes or
   // MMAs take, and the part of the epilogue that no main loop hides; a split adds the clearing of the output and the
@@ -1923,9 +1922,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
       const uint32_t per = (num_k_tiles + sp - 1) / sp;
       const uint32_t real = (num_k_tiles + per - 1) / per;
       const bool pair = pair_fits(bm, bn, real, per);
-      const uint64_t waves = pair ? (pairs_of(real) + usms / 2 - 1) / (usms / 2)
-                                  : (static_cast<uint64_t>(tiles) * real + usms - 1) / usms;
-      const uint64_t ck = resident_shape(bm, bn, real) ? kResidentTileCycles : pair ? kPairTileCycles : kTileCycles[shape];
+      const uint32_t waves = pair ? (pairs_of(real) + usms / 2 - 1) / (usms / 2) : (tiles * real + usms - 1) / usms;
+      const uint64_t ck = resident_shape(bm, bn, real, tiles) ? kResidentTileCycles : pair ? kPairTileCycles : kTileCycles[shape];
       const uint64_t cf = !f32_out ? 0 : pair ? kPairF32Epilogue : kF32Epilogue[shape];
       const uint64_t cost = waves * (per * ck + ce + cf) + (real > 1 ? kSplitCycles : 0) + (pair ? kPairSetup : 0);
       if (cost < best.cost) best = Candidate{real, cost};  // ties go to fewer splits
@@ -1933,6 +1931,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
     return best;
   };
   uint32_t block_m = 128, block_n = 128;
+  Candidate best{1, ~0ull};
   const int forced = tile_override();
   if (forced) {
     block_m = static_cast<uint32_t>(forced) >> 16;
@@ -1946,16 +1945,15 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
     const bool wide_shape = a.n % 256 == 0 || a.n > 1024;
     const bool ok256 = wide_shape && ((num_k_tiles >= 4 && (tiles256 >= usms || can_split)) ||
                                       (a.n % 256 == 0 && num_k_tiles <= 3 && tiles256 >= 4u * usms));
-    uint64_t best = ~0ull;
     auto consider = [&](uint32_t bm, uint32_t bn) {
-      const uint64_t cost = evaluate(bm, bn).cost;
-      if (cost >= best) return;
-      best = cost;
+      const Candidate c = evaluate(bm, bn);
+      if (c.cost >= best.cost) return;
+      best = c;
       block_m = bm;
       block_n = bn;
     };
     // Short K with a resident B panel is bound by writing the output, which the estimate does not see: the widest tile.
-    const bool wide_resident = num_k_tiles <= 3 && ok192 && (ok256 || resident_shape(128, 192, 1));
+    const bool wide_resident = num_k_tiles <= 3 && ok192 && (ok256 || resident_shape(128, 192, 1, tiles192));
     if (wide_resident) {
       consider(128, ok256 ? 256 : 192);
     } else {
@@ -1976,7 +1974,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
 
   // split-K for long GEMMs with few tiles (dW = dY^T.X): f32 output, linear epilogue only; the split count is
   // the one that minimises waves x (main loop + exposed epilogue) of one work item
-  pl.k_splits = evaluate(block_m, block_n).splits;
+  if (best.cost == ~0ull) best = evaluate(block_m, block_n);  // a tile that was not chosen by its cost
+  pl.k_splits = best.splits;
   pl.k_tiles_per_split = (num_k_tiles + pl.k_splits - 1) / pl.k_splits;
   pl.k_splits = (num_k_tiles + pl.k_tiles_per_split - 1) / pl.k_tiles_per_split;
 
@@ -1986,7 +1985,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   auto stages_beside = [&](const TileBytes& tb, uint32_t slots) {
     return (kSmemBudget - tb.fixed - static_cast<int>(slots) * tb.slot) / tb.stage;
   };
-  if (resident_shape(block_m, block_n, pl.k_splits)) {
+  if (resident_shape(block_m, block_n, pl.k_splits, tiles)) {
     const uint32_t panel = panel_of(block_n, num_k_tiles);
     const int st = stages_beside(tile_bytes(block_m, block_n, panel, false), num_k_tiles);
     if (st >= 3) {

@@ -141,7 +141,7 @@ class Nvfp4QuantModule {
   }
   // `RowwiseNvfp4Scratch::quantize_row_amax` (crates/gpt2-nvfp4/src/types/nvfp4_scratch/scratch.rs:35-52):
   // row amax and rowwise four-six in one pass.  `row_amax` may be empty for rows of up to 4096 values;
-  // `out.decoded_amax`, when set, receives max |decoded value| for the backward pass; `amax_cleared`: it is zero already.
+  // `out.decoded_amax`, when set, receives max |decoded value| for the backward pass; `amax_cleared`: what it holds takes part.
   template <typename T>
   DriverError quantize_row_amax(Stream s, DeviceBuffer<const T> x, const Nvfp4TensorView& out,
                                 DeviceBuffer<float> row_amax = {}, bool amax_cleared = false) const {

@@ -149,7 +149,7 @@ static int quantize_rowwise_fused(void* stream, const void* x, int dtype, uint32
                        out_global_scale);
   if (rc || !out_decoded_amax) return rc;
   return launch_nvfp4_amax(S(stream), out_fp4, out_scales, out_global_scale, rows, cols, 1, packed, nullptr,
-                           out_decoded_amax);
+                           out_decoded_amax, nullptr, cleared);
 }
 int nvfp4_quantize_four_six_rowwise_fused(void* stream, const void* x, int dtype, uint32_t rows, uint32_t cols,
                                           uint8_t* out_fp4, uint8_t* out_scales, int scale_layout,

@@ -19,8 +19,10 @@ constexpr uint32_t kAmaxScratchPartials = 148u * 8u;
 uint32_t tensor_amax_partials(uint64_t n, uint32_t max_partials = kAmaxPartials);
 int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_amax, float* out, uint64_t n,
                        float* partials = nullptr, uint32_t max_partials = kAmaxPartials);
+// partials (optional): kAmaxScratchPartials floats, as above.  out_cleared: out[0] is not cleared first, its value takes part
 int launch_nvfp4_amax(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, const float* gscales, uint32_t rows,
-                      uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out, float* partials = nullptr);  // kAmaxScratchPartials
+                      uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out, float* partials = nullptr,
+                      bool out_cleared = false);
 // transform 0: out[0] = max(chunks); 1: out[0] = MS-EDEN global scale of that max
 int launch_amax_from_chunks(cudaStream_t s, const float* chunk_amax, float* out, uint32_t chunk_count, int transform);
 int launch_ms_eden_scale_from_amax(cudaStream_t s, const float* amax, float* out);

@@ -1347,15 +1347,18 @@ int launch_tensor_amax(cudaStream_t s, const void* x, int dtype, float* chunk_am
 }
 
 int launch_nvfp4_amax(cudaStream_t s, const uint8_t* bytes, const uint8_t* scales, const float* gscales, uint32_t rows,
-                      uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out, float* partials) {
+                      uint32_t cols, int rowwise, int packed, float* chunk_amax, float* out, float* partials,
+                      bool out_cleared) {
   const uint64_t n = static_cast<uint64_t>(rows) * cols;
   if (!partials) {
-    const cudaError_t err = cudaMemsetAsync(out, 0, sizeof(float), s);
-    if (err != cudaSuccess) return static_cast<int>(err);
+    if (!out_cleared) {
+      const cudaError_t err = cudaMemsetAsync(out, 0, sizeof(float), s);
+      if (err != cudaSuccess) return static_cast<int>(err);
+    }
     if (n == 0) return 0;
   }
-  return launch_chained(nvfp4_amax_kernel, tensor_amax_partials(n, kAmaxScratchPartials), 256, 0, s, bytes, scales, gscales, n, cols, rowwise, packed, chunk_amax, out,
-                        partials);
+  return launch_chained(nvfp4_amax_kernel, tensor_amax_partials(n, kAmaxScratchPartials), 256, 0, s, bytes, scales, gscales, n, cols,
+                        rowwise, packed, chunk_amax, out, partials);
 }
 
 int launch_amax_from_chunks(cudaStream_t s, const float* chunk_amax, float* out, uint32_t chunk_count, int transform) {

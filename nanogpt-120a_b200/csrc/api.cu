@@ -299,7 +299,7 @@ static int validate_ms_eden(const nvfp4_ms_eden_args* a) {
 // Row operand + transposed operand of one matrix in a single pass (same scale, same signs).
 static int ms_eden_pair(void* stream, nvfp4_ms_eden_args rows, nvfp4_ms_eden_args transposed,
                         float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr,
-                        uint32_t amax_count = 1, void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false) {
+                        uint32_t amax_count = 0, void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false) {
   rows.src_kind = NVFP4_SRC_F32_ROWS;
   transposed.src_kind = NVFP4_SRC_F32_TRANSPOSED;
   int rc = validate_ms_eden(&rows);
@@ -505,7 +505,7 @@ static int nvfp4_source_transpose(void* stream, int kind, const uint8_t* in_byte
     rc = launch_ms_eden_scale_from_amax(S(stream), out_gs, out_gs);
     return rc ? rc : launch_ms_eden(S(stream), a);
   }
-  return launch_ms_eden(S(stream), a, amax_ptr, out_gs, partials ? tensor_amax_partials(n, kAmaxScratchPartials) : 1u);
+  return launch_ms_eden(S(stream), a, amax_ptr, out_gs, partials ? tensor_amax_partials(n, kAmaxScratchPartials) : 0u);
 }
 
 int nvfp4_nvfp4_transpose_to_quartet_backward_ms_eden_derived_device_scale(
@@ -1069,7 +1069,7 @@ static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_
     if (rc) return rc;
   }
   const float* amax_in = nullptr;
-  uint32_t amax_count = 1;
+  uint32_t amax_count = 0;
   if (!a->e_global_scale_override) {
     // Partial maxima in the chunk scratch, by the caller or by a pass over dY: the pair kernel derives the scale from them and
     // publishes it in e_h.global_scale.  With a word cleared ahead of that pass, and of the side stream's over W, a

@@ -42,21 +42,22 @@ int launch_packed_scale_pad(cudaStream_t s, uint8_t* packed, uint32_t rows, uint
 int launch_schedule_free_materialize(cudaStream_t s, const float* z, const float* x, float beta, float* chunk_amax,
                                      float* amax, uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs,
                                      uint32_t rows, uint32_t cols, float* partials = nullptr);
-// amax_in / gs_out (optional): the global scale is the MS-EDEN scale of max(amax_in[0 .. amax_count - 1]) (derived inside the
-// kernel where the kernel supports it, by a one-thread kernel otherwise) and is written to gs_out[0]; a.global_scale
-// and a.host_global_scale are then not read.  amax_count > 1 only where ms_eden_takes_amax.
+// amax_in / gs_out (optional): the global scale is the MS-EDEN scale of max(0, amax_in[0 .. amax_count - 1]), or of amax_in[0]
+// as it stands for a count of 0 (derived inside the kernel where the kernel supports it, by a one-thread kernel otherwise),
+// and is written to gs_out[0]; a.global_scale and a.host_global_scale are then not read.  amax_count > 0 only where
+// ms_eden_takes_amax.
 int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a, const float* amax_in = nullptr, float* gs_out = nullptr,
-                   uint32_t amax_count = 1);
+                   uint32_t amax_count = 0);
 bool ms_eden_takes_amax(const nvfp4_ms_eden_args& a);
 // Pair quantization; when col_sum_partials != nullptr (and ms_eden_pair_is_tiled) it also writes the
 // per-row-tile column sums [ms_eden_pair_row_tiles(rows)][cols] for launch_col_sum_reduce.
-// amax_in / gs_out (only when ms_eden_pair_takes_amax): the kernel derives the global scale from max(amax_in[0 .. amax_count - 1])
+// amax_in / gs_out (only when ms_eden_pair_takes_amax): the kernel derives the global scale from the same maximum
 // itself and writes it to gs_out[0]; rows.global_scale / transposed.global_scale are then not read.
 // beside_others: kernels of another stream are waiting for room on the SMs that this one would take by starting early.
 // zero (likewise only when ms_eden_pair_takes_amax): zero_words 16-byte words that the kernel clears beside its work.
 int launch_ms_eden_pair(cudaStream_t s, const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed,
                         float* col_sum_partials = nullptr, const float* amax_in = nullptr, float* gs_out = nullptr,
-                        uint32_t amax_count = 1, void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false);
+                        uint32_t amax_count = 0, void* zero = nullptr, uint64_t zero_words = 0, bool beside_others = false);
 bool ms_eden_pair_takes_amax(const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed);
 bool ms_eden_pair_is_tiled(const nvfp4_ms_eden_args& rows, const nvfp4_ms_eden_args& transposed);
 uint32_t ms_eden_pair_row_tiles(uint32_t rows);

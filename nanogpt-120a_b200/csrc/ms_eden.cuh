@@ -243,10 +243,10 @@ struct MsEdenTileParams {
   float* col_sum_partials;  // pair mode, optional: [row tiles][src_cols] column sums of each tile
   // whole-tile pair kernel, optional: take the global scale from the source amax (every thread
   // evaluates the same two operations) and publish it, instead of a one-thread kernel in between
-  // (amax_count > 1: the maximum of so many partial maxima)
+  // (amax_count: so many partial maxima, of which NaN drop out and none counts as less than zero; 0: one word as it stands)
   const float* amax_in;
   float* gs_out;
-  uint32_t amax_count = 1;
+  uint32_t amax_count = 0;
   uint4* zero = nullptr;  // pair kernel, optional: words to clear
   uint64_t zero_words = 0;
   uint32_t opaque_zero = 0;  // always 0; keeps the assembler from seeing through a pack / unpack pair (ms_eden_tile.cu)

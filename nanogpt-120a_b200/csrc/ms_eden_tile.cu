@@ -364,8 +364,8 @@ __device__ __forceinline__ float tile_global_scale(const MsEdenTileParams& p) {
   if (!p.amax_in) return p.use_host_scale ? p.global_scale_host : after_prior(p.global_scale_dev)[0];
   const float* const in = after_prior(p.amax_in);
   float amax;
-  if (p.amax_count == 1) {
-    amax = in[0];
+  if (p.amax_count <= 1) {
+    amax = p.amax_count == 0 ? in[0] : max_f32(in[0], 0.0f);  // a single partial maximum by the rule of several
   } else {  // partial maxima, non-negative: the pass before neither waited for a cleared word nor added to it
     __shared__ uint32_t amax_bits;
     if (threadIdx.x == 0) amax_bits = 0u;

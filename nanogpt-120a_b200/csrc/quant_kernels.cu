@@ -1555,7 +1555,7 @@ bool ms_eden_takes_amax(const nvfp4_ms_eden_args& a) {
 int launch_ms_eden(cudaStream_t s, const nvfp4_ms_eden_args& a_in, const float* amax_in, float* gs_out, uint32_t amax_count) {
   nvfp4_ms_eden_args a = a_in;
   const bool nv_tiles = ms_eden_takes_amax(a);
-  if (amax_count > 1 && !nv_tiles) return static_cast<int>(cudaErrorInvalidValue);
+  if (amax_count > 0 && !nv_tiles) return static_cast<int>(cudaErrorInvalidValue);
   if (amax_in) {
     // the tiled NVFP4 transposer derives the scale from the amax itself; every other kernel gets it from a
     // one-thread kernel first

@@ -110,6 +110,24 @@ def test_backward_scale_from_partial_maxima(pkg, dev, chunks):
         assert torch.equal(own, theirs)
 
 
+@pytest.mark.parametrize("maxima", [[float("nan")], [-2.0], [-0.0], [float("inf")], [3e-3], [float("nan"), 2e-3], [-2.0, float("nan")]])
+def test_backward_scale_from_unusual_partial_maxima(pkg, dev, maxima):
+    """A NaN among a caller's maxima drops out and a negative one counts as zero, however many there are: the scale that
+    nvfp4_quartet_backward_ms_eden_global_scale_from_chunks derives from them."""
+    t, i, o = 128, 64, 64
+    q = pkg.Nvfp4QuantModule()
+    e = (torch.randn(t, o, device=dev) * 1e-3).to(bf16)
+    w = q.quantize_four_six(torch.randn(o, i, device=dev).to(bf16), rowwise=False, packed=True)
+    x = q.quantize_four_six(torch.randn(t, i, device=dev).to(bf16), rowwise=True, packed=True, decoded_amax=True)
+    s = pkg.LinearBackwardScratch(t, i, o, dev)
+    given = torch.tensor(maxima, device=dev)
+    s.e_h["chunk_amax"][:len(maxima)] = given
+    want = q.quartet_backward_ms_eden_global_scale_from_chunks(given, len(maxima))
+    pkg.LinearBackwardModule().backward_ms_eden(e=e, weight=w, input=x, scratch=s, sign_seed=5, scale_seed=6, want_dbias=False,
+                                                precomputed_e_amax_chunks=len(maxima))
+    assert torch.equal(s.e_h["global_scale"].reshape(-1)[:1], want.reshape(-1)[:1])
+
+
 @pytest.mark.parametrize("m,n,k,dtype,epi,want", [
     (3072, 768, 8192, f32, 0, (128, 128, 1)), (2304, 768, 8192, f32, 0, (128, 192, 2)), (768, 768, 65536, f32, 0, (256, 192, 12)),
     (4096, 4096, 2048, bf16, 1, (128, 256, 1)), (4096, 8192, 2048, f32, 2, (128, 192, 1)), (2048, 2304, 768, bf16, 1, (128, 128, 1)),

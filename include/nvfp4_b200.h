@@ -481,7 +481,8 @@ int nvfp4_gemm_set_tile_override(int block_m, int block_n);
 int nvfp4_gemm_set_wait_timeout_ns(uint64_t ns);
 /* Test aid: bit 0 makes CTA 0 of every following GEMM skip the loads of its first k-tile, so that the
  * waits on that stage run out (the safe way to exercise the time-out path: nothing faults, the kernel
- * returns).  0 (default) = normal operation. */
+ * returns).  Bit 1 treats every output's tensor maps as refused by the driver: such a GEMM is planned again with direct
+ * stores.  0 (default) = normal operation. */
 int nvfp4_gemm_set_debug_flags(uint32_t flags);
 
 /* Measurement aid (no reference counterpart; off by default).  Between begin and end every GEMM

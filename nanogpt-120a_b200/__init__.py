@@ -353,7 +353,8 @@ def set_gemm_wait_timeout_ns(ns: int) -> None:
 
 
 def set_gemm_debug_flags(flags: int) -> None:
-    """Test aid: bit 0 makes CTA 0 of every following GEMM skip the loads of its first k-tile."""
+    """Test aid: bit 0 makes CTA 0 of every following GEMM skip the loads of its first k-tile, bit 1 has the output's
+    tensor maps refused (direct stores)."""
     _call("nvfp4_gemm_set_debug_flags", flags)
 
 

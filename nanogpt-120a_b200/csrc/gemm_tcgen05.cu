@@ -57,6 +57,7 @@ constexpr uint32_t kMaxFinal = 10;  // staging buffers of a CTA's last tile besi
 constexpr uint64_t kDefaultWaitTimeoutNs = 2000000000ull;  // 2 s
 
 constexpr uint32_t kStatusProducerTimeout = 1u, kStatusMmaTimeout = 2u, kStatusEpilogueTimeout = 4u;
+constexpr uint32_t kDebugSkipFirstLoad = 1u, kDebugRefuseOutputMaps = 2u;
 
 // Tile shapes: 128 x {128, 192, 256} and the tall 256 x 192.  The tall tile issues two MMAs per k-atom (rows
 // 0..127 and 128..255 of the A stage against the same B stage), so a stage's B bytes feed twice the flops:
@@ -786,7 +787,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (issued == 0) wait_for_prior_kernels();
         GEMM_TRACE(0, 1, lane == 0);
         // test hook: this stage is never armed nor loaded, so its consumers' waits run out
-        const bool skip = (p.debug_flags & 1u) && blockIdx.x == 0 && issued == 0;
+        const bool skip = (p.debug_flags & kDebugSkipFirstLoad) && blockIdx.x == 0 && issued == 0;
         if (!skip && elect_one()) {
           const uint32_t atoms = min(static_cast<uint32_t>(kKAtomsPerStage), p.k_atoms - kt * kKAtomsPerStage);
           const uint32_t sf_bytes = atoms * kSfTileBytes;
@@ -1847,7 +1848,8 @@ int validate_gemm(const nvfp4_gemm_args& a) {
 }
 
 // Tile width, split-K count, shared-memory plan and grid of one GEMM on `sms` SMs.
-void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
+// maps_refused: the output's tensor maps could not be encoded, direct stores it is.
+void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refused = false) {
   const uint32_t k_atoms = a.k / 64;
   const uint32_t num_k_tiles = (k_atoms + kKAtomsPerStage - 1) / kKAtomsPerStage;
   const uint32_t usms = static_cast<uint32_t>(sms);
@@ -1862,7 +1864,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl) {
   // its lanes would read and write a row each: 4096 x 2048 x K 8192 100 us with direct stores, 54 us.  A TMA reduction into
   // the stream took 48 us, but every f32 reduction in global memory takes subnormals for zero.  A bf16 residual stays on
   // the direct path, which adds in f32 and rounds once.
-  pl.tma_store = (pl.vec_store && (a.epilogue != NVFP4_EPI_RESIDUAL || a.out_dtype == NVFP4_DTYPE_F32)) ? 1 : 0;
+  pl.tma_store = (pl.vec_store && !maps_refused && (a.epilogue != NVFP4_EPI_RESIDUAL || a.out_dtype == NVFP4_DTYPE_F32)) ? 1 : 0;
   const bool can_split = a.out_dtype == NVFP4_DTYPE_F32 &&
                          (a.epilogue == NVFP4_EPI_NONE || a.epilogue == NVFP4_EPI_BIAS) && num_k_tiles >= 16;
   // The f32 residual stream is loaded into the staging buffers its sums leave from.  Two buffers per group (128 x 128)
@@ -2077,8 +2079,8 @@ int gemm_plan_query(const nvfp4_gemm_args& a, nvfp4_gemm_plan* out) {
   if (rc) return rc;
   GemmPlan pl;
   plan_gemm(a, sm_count(), pl);
-  // the kernel falls back to direct stores when the output map cannot be encoded; that cannot happen for
-  // outputs that pass the alignment test above, so the plan reports the test's verdict
+  // launch_gemm plans again when an output map cannot be encoded; that has not been seen for outputs that pass the plan's
+  // alignment test, so the query reports the test's verdict
   out->block_m = pl.block_m;
   out->block_n = pl.block_n;
   out->acc_stages = (pl.block_n == 256 || pl.block_m == 256) ? 1 : 2;
@@ -2128,8 +2130,16 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool
   if (a.m == 0 || a.n == 0) return 0;
   int rc = validate_gemm(a);
   if (rc) return rc;
+  const uint32_t debug_flags = g_debug_flags.load(std::memory_order_relaxed);
   GemmPlan pl;
   plan_gemm(a, sm_count(), pl);
+  CUtensorMap ma, mb, mo, mx;
+  // An output that passes the plan's test of its alignment has not been seen refused.  Should it be, the whole plan is made again:
+  // pairs, for one, have no direct stores.
+  if (pl.tma_store &&
+      ((debug_flags & kDebugRefuseOutputMaps) || encode_output_map(&mo, a.out, a.out_dtype, a.m, a.n, a.ldo) != 0 ||
+       (a.aux && encode_output_map(&mx, a.aux, a.out_dtype, a.m, a.n, a.ldo) != 0)))
+    plan_gemm(a, sm_count(), pl, true);
   if (a.relu2_row_amax && (!pl.tma_store || a.epilogue == NVFP4_EPI_RESIDUAL)) {
     set_last_error("nvfp4_gemm: relu2_row_amax needs a 16-byte aligned output and row pitch and no residual epilogue");
     return static_cast<int>(cudaErrorInvalidValue);
@@ -2173,26 +2183,17 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool
   p.stream_out = pl.b_resident && pl.resident_cpn == 0 &&
                  static_cast<uint64_t>(a.m) * a.ldo * (a.out_dtype == NVFP4_DTYPE_F32 ? 4 : 2) > (96ull << 20);
   p.wait_timeout_ns = g_wait_timeout_ns.load(std::memory_order_relaxed);
-  p.debug_flags = g_debug_flags.load(std::memory_order_relaxed);
+  p.debug_flags = debug_flags;
 #ifdef NVFP4_GEMM_TRACE
   p.trace = g_trace_buffer.load(std::memory_order_relaxed);
 #endif
 
-  CUtensorMap ma, mb, mo, mx;
   rc = encode_operand_map(&ma, a.a_bytes, a.m, a.k, pl.block_m);
   if (rc) return rc;
   rc = encode_operand_map(&mb, a.b_bytes, a.n, a.k, pl.pair ? pl.block_n / 2 : pl.block_n);
   if (rc) return rc;
-  mo = ma;
-  mx = ma;
-  if (p.tma_store) {
-    if (encode_output_map(&mo, a.out, a.out_dtype, a.m, a.n, a.ldo) != 0) p.tma_store = 0;
-    if (p.tma_store && a.aux && encode_output_map(&mx, a.aux, a.out_dtype, a.m, a.n, a.ldo) != 0) p.tma_store = 0;
-    if (!p.tma_store && a.relu2_row_amax) {
-      set_last_error("nvfp4_gemm: relu2_row_amax needs an output the TMA store path accepts");
-      return static_cast<int>(cudaErrorInvalidValue);
-    }
-  }
+  if (!pl.tma_store) mo = ma;
+  if (!pl.tma_store || !a.aux) mx = ma;
 
   const size_t esz = a.out_dtype == NVFP4_DTYPE_F32 ? 4 : 2;
   if (p.k_splits > 1 && !out_is_zero) {

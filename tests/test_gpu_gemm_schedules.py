@@ -85,6 +85,18 @@ def test_pair_wait_runs_out(pkg, dev, tile):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("m,n,k,epi,dtype", [(300, 520, 8256, 1, bf16), (300, 520, 8256, 2, bf16), (512, 512, 8192, 0, f32),
+                                             (700, 840, 16384, 1, f32)])
+def test_refused_output_maps_plan_again(pkg, oracle, dev, tile, m, n, k, epi, dtype):
+    """Without its TMA stores a GEMM that would run on pairs, split or not, is planned for direct stores, one CTA a tile."""
+    tile(256)
+    pkg.set_gemm_debug_flags(2)
+    try:
+        run_case(pkg, oracle, dev, m, n, k, out_dtype=dtype, epi=epi)
+    finally:
+        pkg.set_gemm_debug_flags(0)
+
+
 @pytest.mark.parametrize("chunks", [1, 2, 257, 1184, 1185])
 def test_backward_scale_from_partial_maxima(pkg, dev, chunks):
     """A caller's chunk maxima, the largest in the last place, up to what the pair kernel reduces itself (1184) and one more:

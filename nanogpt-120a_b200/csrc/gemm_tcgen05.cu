@@ -1996,10 +1996,11 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
       pl.stages = static_cast<uint32_t>(st > kMaxStages ? kMaxStages : st);
       // banded schedule when the column blocks divide the grid almost evenly, or, for many row blocks, fill four fifths of it:
       // one A tile for all CTAs at a time and whole output rows are worth that many idle SMs (65536 x 32000 x K 768 on
-      // 125 SMs 1003 us, contiguous on 148 1187; 8192 rows 112 and 114)
+      // 125 SMs 1003 us, contiguous on 148 1187; 8192 rows 112 and 114).  Direct stores take an SM's time and not the memory's:
+      // 28928 x 5695 x K 448 bf16 1774 us on all, 2193 on 132; 27392 x 6272 x K 960 bf16 residual 1177 and 1337
       const uint32_t cpn = pl.grid / pl.num_n_blocks, used = cpn * pl.num_n_blocks;
-      if (cpn >= 1 && ((used * 20 >= pl.grid * 19 && num_m_blocks >= 4 * cpn) || (used * 5 >= pl.grid * 4 && num_m_blocks >= 16 * cpn)))
-        pl.resident_cpn = cpn;
+      const bool most = pl.tma_store && used * 5 >= pl.grid * 4 && num_m_blocks >= 16 * cpn;
+      if (cpn >= 1 && ((used * 20 >= pl.grid * 19 && num_m_blocks >= 4 * cpn) || most)) pl.resident_cpn = cpn;
     }
   }
   pl.pair = !pl.b_resident && pair_fits(block_m, block_n, pl.k_splits, pl.k_tiles_per_split) ? 1 : 0;

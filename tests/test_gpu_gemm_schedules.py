@@ -31,6 +31,13 @@ def test_vocabulary_walks(pkg, oracle, dev, m, n, k, cpn, dtype):
              blocks=row_blocks(m)[::2])
 
 
+@pytest.mark.parametrize("n,cpn,tma", [(5696, 4, 1), (5695, 0, 0)])
+def test_direct_stores_walk_on_every_sm(pkg, oracle, dev, n, cpn, tma):
+    """30 column blocks: four CTAs for each leave 28 SMs idle, which outputs with TMA stores are worth and direct ones are not."""
+    run_case(pkg, oracle, dev, 8192, n, 448, out_dtype=bf16, epi=1,
+             want_plan=dict(block_n=192, b_resident=1, resident_cpn=cpn, tma_store=tma))
+
+
 @pytest.mark.parametrize("m,n,k,epi,dtype", [(128, 256, 8192, 0, bf16), (300, 520, 8256, 1, bf16), (384, 512, 8128, 2, bf16),
                                              (10000, 768, 8192, 0, bf16), (1000, 512, 8256, 2, f32), (4096, 1024, 8192, 0, f32)])
 def test_pairs(pkg, oracle, dev, tile, m, n, k, epi, dtype):

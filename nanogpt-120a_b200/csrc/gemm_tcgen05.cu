@@ -1896,7 +1896,11 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
   // and is 2 % slower with these: 3072 x 768 x K 8192 f32 17.2 -> 14.2 us (128 x 128 in one wave, not three splits of 256 x
   // 192), 3072 x 1024 x K 8192 f32 26.3 -> 17.7, 4096 x 8192 x K 2048 f32 ReLU^2 with its second output 80 -> 61, 4096 x 4096 x
   // K 2048 bf16 24.5 -> 20.9, 2048 x 2304 x K 768 bf16 7.4 -> 6.0.  A pair's setting up and tearing down count once, not per
-  // wave: 32000 x 768 x K 8192 f32 99 -> 93, where a split of 768 x 768 x K 65536 over pairs stays with the tall tile.
+  // wave: 32000 x 768 x K 8192 f32 99 -> 93, where a split of 768 x 768 x K 65536 over pairs stays with the tall tile.  Direct
+  // stores (odd pitches) take an SM 24 us for every 128 x 128 elements of bf16, 15 of f32, and half of that again for a second
+  // output or the stream they add to, more in the tall tile, where no main loop runs beside them.  Weighed like the TMA stores' epilogue they put 696 x 3101 x K 8320 bf16 on the
+  // tall tile (87 us, 49 at 128 x 128), 1024 x 2979 x K 1536 too (71 us, 52) and split 768 x 1685 x K 12736 f32 five ways (47
+  // us, 31 unsplit).
   struct Candidate {
     uint32_t splits;
     uint64_t cost;
@@ -1908,10 +1912,15 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
     constexpr uint64_t kPairTileCycles = 710, kPairF32Epilogue = 2000, kPairSetup = 6000;
     constexpr uint64_t kEpilogue[4] = {2000, 3000, 2500, 4000}, kF32Epilogue[4] = {4000, 3000, 6000, 6000};
     constexpr uint64_t kSecondOutput[4] = {7500, 500, 3500, 12500}, kResidualTurns[4] = {0, 1000, 6000, 11000};
+    constexpr uint64_t kDirectBf16[4] = {46000, 68000, 90000, 125000}, kDirectSecondBf16[4] = {26000, 42000, 57000, 92000};
+    constexpr uint64_t kDirectF32[4] = {29000, 42000, 56000, 76000}, kDirectSecondF32[4] = {14000, 22000, 28000, 75000};
+    constexpr uint64_t kDirectResidual[4] = {42000, 63000, 84000, 145000};
     constexpr uint64_t kSplitCycles = 4000;
-    const uint64_t ce = kEpilogue[shape] + (a.epilogue == NVFP4_EPI_RELU2 && a.aux ? kSecondOutput[shape] : 0) +
-                        (f32_residual ? kResidualTurns[shape] : 0);
-    const bool f32_out = a.out_dtype == NVFP4_DTYPE_F32;
+    const bool f32_out = a.out_dtype == NVFP4_DTYPE_F32, second = a.epilogue == NVFP4_EPI_RELU2 && a.aux;
+    const uint64_t direct = (f32_residual ? kDirectResidual : f32_out ? kDirectF32 : kDirectBf16)[shape] +
+                            (second ? (f32_out ? kDirectSecondF32 : kDirectSecondBf16)[shape] : 0);
+    const uint64_t staged = kEpilogue[shape] + (second ? kSecondOutput[shape] : 0) + (f32_residual ? kResidualTurns[shape] : 0);
+    const uint64_t ce = pl.tma_store ? staged : direct;
     Candidate best{1, ~0ull};
     uint32_t max_splits = 1;
     if (can_split && tiles < 2 * usms) {
@@ -1926,7 +1935,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
       const bool pair = pair_fits(bm, bn, real, per);
       const uint32_t waves = pair ? (pairs_of(real) + usms / 2 - 1) / (usms / 2) : (tiles * real + usms - 1) / usms;
       const uint64_t ck = resident_shape(bm, bn, real, tiles) ? kResidentTileCycles : pair ? kPairTileCycles : kTileCycles[shape];
-      const uint64_t cf = !f32_out ? 0 : pair ? kPairF32Epilogue : kF32Epilogue[shape];
+      const uint64_t cf = !f32_out || !pl.tma_store ? 0 : pair ? kPairF32Epilogue : kF32Epilogue[shape];
       const uint64_t cost = waves * (per * ck + ce + cf) + (real > 1 ? kSplitCycles : 0) + (pair ? kPairSetup : 0);
       if (cost < best.cost) best = Candidate{real, cost};  // ties go to fewer splits
     }
@@ -1996,10 +2005,11 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
       pl.stages = static_cast<uint32_t>(st > kMaxStages ? kMaxStages : st);
       // banded schedule when the column blocks divide the grid almost evenly, or, for many row blocks, fill four fifths of it:
       // one A tile for all CTAs at a time and whole output rows are worth that many idle SMs (65536 x 32000 x K 768 on
-      // 125 SMs 1003 us, contiguous on 148 1187; 8192 rows 112 and 114).  Direct stores take an SM's time and not the memory's:
-      // 28928 x 5695 x K 448 bf16 1774 us on all, 2193 on 132; 27392 x 6272 x K 960 bf16 residual 1177 and 1337
+      // 125 SMs 1003 us, contiguous on 148 1187; 8192 rows 112 and 114).  Direct stores of bf16 take an SM's time and not the
+      // memory's: 28928 x 5695 x K 448 1774 us on all, 2193 on 132; 27392 x 6272 x K 960 residual 1177 and 1337; those of f32 gain
+      // like TMA stores (31744 x 3759 x K 448 918 and 817)
       const uint32_t cpn = pl.grid / pl.num_n_blocks, used = cpn * pl.num_n_blocks;
-      const bool most = pl.tma_store && used * 5 >= pl.grid * 4 && num_m_blocks >= 16 * cpn;
+      const bool most = (pl.tma_store || a.out_dtype == NVFP4_DTYPE_F32) && used * 5 >= pl.grid * 4 && num_m_blocks >= 16 * cpn;
       if (cpn >= 1 && ((used * 20 >= pl.grid * 19 && num_m_blocks >= 4 * cpn) || most)) pl.resident_cpn = cpn;
     }
   }

@@ -31,10 +31,12 @@ def test_vocabulary_walks(pkg, oracle, dev, m, n, k, cpn, dtype):
              blocks=row_blocks(m)[::2])
 
 
-@pytest.mark.parametrize("n,cpn,tma", [(5696, 4, 1), (5695, 0, 0)])
-def test_direct_stores_walk_on_every_sm(pkg, oracle, dev, n, cpn, tma):
-    """30 column blocks: four CTAs for each leave 28 SMs idle, which outputs with TMA stores are worth and direct ones are not."""
-    run_case(pkg, oracle, dev, 8192, n, 448, out_dtype=bf16, epi=1,
+@pytest.mark.parametrize("n,dtype,cpn,tma", [(5696, bf16, 4, 1), (5695, bf16, 0, 0), (5695, f32, 4, 0)])
+def test_bf16_direct_stores_walk_on_every_sm(pkg, oracle, dev, tile, n, dtype, cpn, tma):
+    """30 column blocks: four CTAs for each leave 28 SMs idle, which TMA stores are worth, and direct ones of f32; those of bf16
+    are not."""
+    tile(192)
+    run_case(pkg, oracle, dev, 8192, n, 448, out_dtype=dtype, epi=1,
              want_plan=dict(block_n=192, b_resident=1, resident_cpn=cpn, tma_store=tma))
 
 
@@ -150,9 +152,12 @@ def test_backward_scale_from_unusual_partial_maxima(pkg, dev, maxima):
 @pytest.mark.parametrize("m,n,k,dtype,epi,want", [
     (3072, 768, 8192, f32, 0, (128, 128, 1)), (2304, 768, 8192, f32, 0, (128, 192, 2)), (768, 768, 65536, f32, 0, (256, 192, 12)),
     (4096, 4096, 2048, bf16, 1, (128, 256, 1)), (4096, 8192, 2048, f32, 2, (128, 192, 1)), (2048, 2304, 768, bf16, 1, (128, 128, 1)),
-    (32000, 768, 8192, f32, 0, (128, 256, 1)), (16, 768, 768, bf16, 1, (128, 128, 1)), (200, 768, 4352, f32, 0, (128, 128, 2))])
+    (32000, 768, 8192, f32, 0, (128, 256, 1)), (16, 768, 768, bf16, 1, (128, 128, 1)), (200, 768, 4352, f32, 0, (128, 128, 2)),
+    (1024, 2979, 1536, bf16, 1, (128, 128, 1)), (13568, 571, 2432, bf16, 0, (128, 192, 1)), (31360, 3039, 5312, f32, 0, (256, 192, 1)),
+    (768, 1685, 12736, f32, 1, (128, 128, 1))])
 def test_the_estimate_takes_the_measured_tile(pkg, dev, m, n, k, dtype, epi, want):
-    """The fastest tile, or one within a few per cent of it, where a wave more or less, the f32 or the second output decides."""
+    """The fastest tile, or one within a few per cent of it, where a wave more or less, the f32 or the second output, or the time
+    of direct stores (odd columns) decides."""
     stub, one = torch.zeros(16, dtype=torch.uint8, device=dev), torch.ones(1, device=dev)
     A = pkg.Nvfp4Tensor(stub, stub, one, m, k, packed=True, rowwise=True)
     B = pkg.Nvfp4Tensor(stub, stub, one, n, k, packed=True, rowwise=False)

@@ -421,6 +421,9 @@ typedef struct nvfp4_gemm_plan {
   uint32_t smem_bytes;    /* dynamic shared memory of the launch                                           */
 } nvfp4_gemm_plan;
 int nvfp4_gemm_plan_query(const nvfp4_gemm_args* args /* host */, nvfp4_gemm_plan* out /* host */);
+/* *pair = 1: the 128 x 256 tiles of that plan run on CTA pairs, two SMs for 256 x 256 (an entry of its own: nvfp4_gemm_plan keeps
+ * its size). */
+int nvfp4_gemm_plan_is_pair(const nvfp4_gemm_args* args /* host */, uint32_t* pair /* host */);
 
 /* utils/nvfp4_tma_matmul/launcher.rs:39-166  Nvfp4GemmModule::prepare_tma_nvfp4_device_scales{,_into}.
  * The reference encodes four tensor maps per GEMM on the host and copies them into caller-owned device

@@ -73,6 +73,7 @@ class GemmPlan(Structure):
     _fields_ = [("block_m", c_uint32), ("block_n", c_uint32), ("acc_stages", c_uint32), ("k_splits", c_uint32), ("b_resident", c_uint32),
                 ("resident_cpn", c_uint32), ("stages", c_uint32), ("grid", c_uint32), ("tma_store", c_uint32),
                 ("smem_bytes", c_uint32)]
+    pair = 0  # 1: the 128 x 256 tiles run on CTA pairs (nvfp4_gemm_plan_is_pair)
 
 
 class ProjectionArgs(Structure):
@@ -177,6 +178,7 @@ _SIGNATURES = {
     "nvfp4_gemm": [_P, POINTER(GemmArgs)],
     "nvfp4_gemm_cleared": [_P, POINTER(GemmArgs)],
     "nvfp4_gemm_plan_query": [POINTER(GemmArgs), POINTER(GemmPlan)],
+    "nvfp4_gemm_plan_is_pair": [POINTER(GemmArgs), POINTER(c_uint32)],
     "nvfp4_prepare_tma_nvfp4_device_scales": [_P, _P, _P, _P, _P, _U, _U, _U],
     "nvfp4_prepare_tma_nvfp4_device_scales_into": [_P, _P, _P, _P, _P, _U, _U, _U, _P],
     "nvfp4_tensor_map_cache_stats": [POINTER(ctypes.c_uint64), POINTER(ctypes.c_uint64)],
@@ -857,8 +859,10 @@ class Nvfp4GemmModule:
             out = torch.empty((m, ldo), dtype=out_dtype, device=a.bytes.device)
         if plan_only:
             g, keep = self._args(a, b, out, aux, bias, mode, epilogue, weight_global_scale, n, ldo, relu2_row_amax)
-            plan = GemmPlan()
+            plan, pair = GemmPlan(), c_uint32()
             _call("nvfp4_gemm_plan_query", ctypes.byref(g), ctypes.byref(plan))
+            _call("nvfp4_gemm_plan_is_pair", ctypes.byref(g), ctypes.byref(pair))
+            plan.pair = pair.value
             return plan
         # (possibly temporary) packed planes: referenced until the launch is enqueued
         a_scales, b_scales = _packed_scales(a), _packed_scales(b)

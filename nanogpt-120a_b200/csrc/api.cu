@@ -590,7 +590,13 @@ int nvfp4_gemm_cleared(void* stream, const nvfp4_gemm_args* args) {
 
 int nvfp4_gemm_plan_query(const nvfp4_gemm_args* args, nvfp4_gemm_plan* out) {
   if (!args || !out) return invalid("nvfp4_gemm_plan_query: null pointer");
-  return gemm_plan_query(*args, out);
+  uint32_t pair;
+  return gemm_plan_query(*args, out, &pair);
+}
+int nvfp4_gemm_plan_is_pair(const nvfp4_gemm_args* args, uint32_t* pair) {
+  if (!args || !pair) return invalid("nvfp4_gemm_plan_is_pair: null pointer");
+  nvfp4_gemm_plan plan;
+  return gemm_plan_query(*args, &plan, pair);
 }
 int nvfp4_prepare_tma_nvfp4_device_scales_into(void* stream, const uint8_t* input_bytes,
                                                const uint8_t* input_scale_data, const uint8_t* weight_bytes,

@@ -2082,9 +2082,9 @@ uint32_t* device_status_word() {
   return ptr;
 }
 
-int gemm_plan_query(const nvfp4_gemm_args& a, nvfp4_gemm_plan* out) {
-  if (!out) return static_cast<int>(cudaErrorInvalidValue);
+int gemm_plan_query(const nvfp4_gemm_args& a, nvfp4_gemm_plan* out, uint32_t* pair) {
   std::memset(out, 0, sizeof(*out));
+  *pair = 0;
   if (a.m == 0 || a.n == 0) return 0;
   const int rc = validate_gemm(a);
   if (rc) return rc;
@@ -2102,6 +2102,7 @@ int gemm_plan_query(const nvfp4_gemm_args& a, nvfp4_gemm_plan* out) {
   out->grid = pl.grid;
   out->tma_store = pl.tma_store;
   out->smem_bytes = static_cast<uint32_t>(pl.smem_bytes);
+  *pair = pl.pair;
   return 0;
 }
 

@@ -89,7 +89,7 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero = fal
 // Whether launch_gemm splits K and sums the partial tiles in the output.
 bool gemm_adds_into_output(const nvfp4_gemm_args& a);
 // What launch_gemm would choose for these arguments on the current device (no launch).
-int gemm_plan_query(const nvfp4_gemm_args& a, nvfp4_gemm_plan* out);
+int gemm_plan_query(const nvfp4_gemm_args& a, nvfp4_gemm_plan* out, uint32_t* pair);
 // Encodes (and keeps in the calling thread's cache) the operand tensor maps of a GEMM ahead of its launch.
 int gemm_prepare_operand_maps(const uint8_t* a_bytes, const uint8_t* b_bytes, uint32_t m, uint32_t k, uint32_t n);
 // Measurement / test aids: forced tile shape (block_n 0 = automatic), limit of the kernel's bounded waits,

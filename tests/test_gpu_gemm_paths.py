@@ -227,13 +227,15 @@ def test_tall_tile_streaming_auto(pkg, oracle, dev, n, k, out_dtype):
 
 # ------------------------------------------------------------------------------------------ split-K (dW)
 
-@pytest.mark.parametrize("m,n,k", [(3072, 768, 65536), (768, 768, 65536), (2304, 768, 65536), (768, 3072, 65536),
-                                   (4096, 1024, 32768)])
-def test_split_k_dw_shapes(pkg, oracle, dev, m, n, k):
+@pytest.mark.parametrize("m,n,k,want", [(3072, 768, 65536, (256, 192, 3)), (768, 768, 65536, (256, 192, 12)),
+                                        (2304, 768, 65536, (256, 192, 4)), (768, 3072, 65536, (256, 192, 3)),
+                                        (2304, 768, 8192, (128, 192, 2)), (4096, 1024, 32768, (128, 256, 1))])
+def test_split_k_dw_shapes(pkg, oracle, dev, m, n, k, want):
     """dW = dY^T . X at the training step's shapes (K = tokens): f32 output, K split over CTAs, partial tiles
-    summed by TMA reduce-add.  Checked on sampled output rows."""
+    summed by TMA reduce-add; the last one fills the SMs with CTA pairs unsplit.  Checked on sampled output rows."""
     plan, _ = run_case(pkg, oracle, dev, m, n, k, out_dtype=torch.float32, epi=0,
                        want_plan=dict(b_resident=0), blocks=row_blocks(m)[:2])
+    assert (plan.block_m, plan.block_n, plan.k_splits) == want
     assert plan.k_splits >= 2 or plan.grid >= 96, (plan.k_splits, plan.grid)
 
 

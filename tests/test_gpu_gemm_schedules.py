@@ -11,7 +11,6 @@ from test_gpu_gemm_paths import GEMM_TOL, assert_plan, check_rows, cpu, no_timeo
 
 pytestmark = pytest.mark.gpu
 bf16, f32 = torch.bfloat16, torch.float32
-PAIR_STAGES = 5  # a stage of a pair's CTA holds half of B: five fit, of a single CTA's three
 
 
 @pytest.mark.parametrize("m,n,k,epi", [(19072, 1024, 768, 1), (19000, 1000, 768, 2), (19072, 2304, 1024, 1), (19072, 768, 832, 0)])
@@ -20,6 +19,18 @@ def test_resident_forms(pkg, oracle, dev, m, n, k, epi, dtype):
     """Resident panels of three and four k-tiles (the last one short), many tiles per CTA, ragged rows and columns: 1000
     columns end in the first half of a 256-column tile, so that the half taken first may be empty."""
     run_case(pkg, oracle, dev, m, n, k, out_dtype=dtype, epi=epi, want_plan=dict(b_resident=1, tma_store=1))
+
+
+@pytest.mark.parametrize("width", [128, 192, 256])
+@pytest.mark.parametrize("k", [64, 256, 320, 512])
+@pytest.mark.parametrize("dtype", [bf16, f32])
+def test_resident_forms_of_one_and_two_k_tiles(pkg, oracle, dev, tile, width, k, dtype):
+    """Shorter panels leave room for more A stages, over which a CTA's last tile is staged; the second k-tile whole and of one atom.
+    Many tiles per CTA, ragged rows and columns; banded (19000 rows), and contiguous with the panel replaced (1000)."""
+    tile(width)
+    for m, n, epi in ((19000, 1000, 1), (1000, 20400, 0)):
+        run_case(pkg, oracle, dev, m, n, k, out_dtype=dtype, epi=epi, blocks=row_blocks(m)[-2:],
+                 want_plan=dict(block_n=width, b_resident=1, resident_cpn=(lambda c: c > 0) if m == 19000 else (lambda c: c <= 1)))
 
 
 @pytest.mark.parametrize("m,n,k,cpn,dtype", [(840, 32000, 768, 0, f32), (2176, 32000, 768, 1, bf16), (2000, 32000, 768, 1, bf16),
@@ -46,12 +57,34 @@ def test_pairs(pkg, oracle, dev, tile, m, n, k, epi, dtype):
     """CTA pairs from 32 k-tiles: one tile and several a pair, a second CTA without rows, with some, ragged columns and K."""
     tile(256)
     run_case(pkg, oracle, dev, m, n, k, out_dtype=dtype, epi=epi, blocks=row_blocks(m)[-2:],
-             want_plan=dict(block_m=128, block_n=256, stages=PAIR_STAGES, k_splits=1, grid=lambda g: g % 2 == 0))
+             want_plan=dict(block_m=128, block_n=256, pair=1, k_splits=1, grid=lambda g: g % 2 == 0))
+
+
+@pytest.mark.parametrize("m,n,k,splits", [(1024, 1024, 32768, 4), (3072, 1024, 32768, 3), (768, 2048, 24576, 3)])
+@pytest.mark.parametrize("epi", [0, 1])
+def test_split_k_over_pairs(pkg, oracle, dev, m, n, k, splits, epi):
+    """dW of d_model 1024 and a like shape: even splits and uneven ones (43 + 43 + 42 k-tiles), whose partial tiles both CTAs of a
+    pair add into the output; a bias joins with the first split."""
+    run_case(pkg, oracle, dev, m, n, k, out_dtype=f32, epi=epi, blocks=row_blocks(m)[:2],
+             want_plan=dict(block_m=128, block_n=256, pair=1, k_splits=splits, tma_store=1))
+
+
+@pytest.mark.parametrize("m,n,k,epi,deterministic", [(1000, 1020, 32768, 0, False), (1000, 1020, 32832, 1, False),
+                                                     (900, 776, 32832, 1, False), (300, 520, 24832, 1, True), (100, 260, 16640, 0, True)])
+def test_split_k_over_pairs_with_tails(pkg, oracle, dev, tile, m, n, k, epi, deterministic):
+    """Ragged rows, columns and K; a second CTA with few rows and with none; capped at two splits."""
+    tile(256)
+    pkg.set_deterministic_reductions(deterministic)
+    try:
+        run_case(pkg, oracle, dev, m, n, k, out_dtype=f32, epi=epi, blocks=row_blocks(m)[-2:],
+                 want_plan=dict(block_n=256, pair=1, k_splits=(lambda s: s == 2) if deterministic else (lambda s: s > 1)))
+    finally:
+        pkg.set_deterministic_reductions(False)
 
 
 def test_pairs_begin_at_32_k_tiles(pkg, oracle, dev, tile):
     tile(256)
-    run_case(pkg, oracle, dev, 300, 512, 7936, out_dtype=bf16, epi=0, want_plan=dict(block_n=256, stages=3))
+    run_case(pkg, oracle, dev, 300, 512, 7936, out_dtype=bf16, epi=0, want_plan=dict(block_n=256, pair=0))
 
 
 @pytest.mark.parametrize("m", [256, 700])
@@ -65,7 +98,7 @@ def test_pairs_on_the_residual_stream(pkg, oracle, dev, tile, m):
     out = torch.from_numpy(res).to(dev)
     kw = dict(bias=torch.from_numpy(bias).to(dev), epilogue=pkg.EPI_RESIDUAL, out=out)
     gemm = pkg.Nvfp4GemmModule()
-    assert_plan(gemm.plan(A, B, **kw), block_n=256, stages=PAIR_STAGES, tma_store=1)
+    assert_plan(gemm.plan(A, B, **kw), block_n=256, pair=1, tma_store=1)
     gemm.gemm(A, B, **kw)
     no_timeouts(pkg)
     assert rel_fro(cpu(out), oracle.gemm(a, b, m, k, n, 2, bias=bias, epi=3, residual=res)) <= GEMM_TOL
@@ -95,13 +128,13 @@ def test_pair_wait_runs_out(pkg, dev, tile):
 
 
 @pytest.mark.parametrize("m,n,k,epi,dtype", [(300, 520, 8256, 1, bf16), (300, 520, 8256, 2, bf16), (512, 512, 8192, 0, f32),
-                                             (700, 840, 16384, 1, f32)])
+                                             (900, 776, 32832, 1, f32)])
 def test_refused_output_maps_plan_again(pkg, oracle, dev, tile, m, n, k, epi, dtype):
     """Without its TMA stores a GEMM that would run on pairs, split or not, is planned for direct stores, one CTA a tile."""
     tile(256)
     pkg.set_gemm_debug_flags(2)
     try:
-        run_case(pkg, oracle, dev, m, n, k, out_dtype=dtype, epi=epi)
+        run_case(pkg, oracle, dev, m, n, k, out_dtype=dtype, epi=epi, blocks=row_blocks(m)[-2:], want_plan=dict(pair=1))
     finally:
         pkg.set_gemm_debug_flags(0)
 

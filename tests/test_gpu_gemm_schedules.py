@@ -127,7 +127,7 @@ def test_pair_wait_runs_out(pkg, dev, tile):
     assert torch.equal(got, want)
 
 
-@pytest.mark.parametrize("m,n,k,epi,dtype", [(300, 520, 8256, 1, bf16), (300, 520, 8256, 2, bf16), (512, 512, 8192, 0, f32),
+@pytest.mark.parametrize("m,n,k,epi,dtype", [(300, 520, 8256, 1, bf16), (300, 520, 8256, 2, bf16), (512, 512, 8192, 2, f32),
                                              (900, 776, 32832, 1, f32)])
 def test_refused_output_maps_plan_again(pkg, oracle, dev, tile, m, n, k, epi, dtype):
     """Without its TMA stores a GEMM that would run on pairs, split or not, is planned for direct stores, one CTA a tile."""

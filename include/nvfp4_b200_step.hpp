@@ -251,13 +251,12 @@ class ProjectionStep {
     if (!blocks_.back().ok() && error_.empty()) error_ = "cudaMalloc failed";
     return blocks_.back();
   }
-  Nvfp4TensorView alloc_tensor(uint32_t rows, uint32_t cols, bool rowwise, bool decoded) {
+  Nvfp4TensorView alloc_tensor(uint32_t rows, uint32_t cols, bool rowwise) {
     Nvfp4TensorView t;
     t.rows = rows, t.cols = cols, t.rowwise = rowwise, t.scale_layout = NVFP4_SCALES_PACKED;
     t.bytes = alloc(Nvfp4TensorView::bytes_len(rows, cols)).as<uint8_t>();
     t.scales = alloc(scale_packed_len(rows, cols)).as<uint8_t>();
     t.global_scales = alloc(sizeof(float) * (rowwise ? rows : 1)).as<float>();
-    if (decoded) t.decoded_amax = alloc(sizeof(float)).as<float>();
     return t;
   }
   MsEdenOperandBuffers alloc_operand(const MsEdenOperandSizes& n) {
@@ -300,8 +299,8 @@ class ProjectionStep {
       l.is_fc = !head && i % 4 == 2, l.is_proj = !head && i % 4 == 3;
       l.weight = in.weight[i], l.bias = in.bias[i];
       l.bucket = head ? shape_.n_layer : static_cast<uint32_t>(i / 4);
-      l.wq = alloc_tensor(l.out, l.in, false, false);
-      l.xq = alloc_tensor(T, l.in, true, false);
+      l.wq = alloc_tensor(l.out, l.in, false);
+      l.xq = alloc_tensor(T, l.in, true);
       l.xq.decoded_amax = {forward_amax_.as<float>().ptr + i, 1};
       l.w_partials = alloc(sizeof(float) * nvfp4_tensor_amax_partials()).as<float>();
       l.weight_t_h = alloc_operand(LinearBackwardMsEdenScratchSizes(T, l.in, l.out).weight_t_h);

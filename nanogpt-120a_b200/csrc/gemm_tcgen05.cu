@@ -540,10 +540,11 @@ struct SubTile<__nv_bfloat16> {
 // ---- the kernel -----------------------------------------------------------------------------
 
 // Shared-memory plan of one launch, chosen on the host (all offsets from the 1024-byte aligned
-// base): A stages, B slots, SFA stages, SFB slots, two epilogue staging buffers, barriers.
-// Streaming mode: one B slot per pipeline stage.  Resident mode (short K): the whole
+// base): A stages, B slots, SFA stages, SFB stages, kStoreBufs epilogue staging buffers, barriers.
+// Streaming mode: one B slot and one SFB stage per pipeline stage.  Resident mode (short K): the whole
 // [kBlockN x K] B panel of the current column block stays in shared memory -- one slot per
-// k-tile -- while a CTA walks down the row blocks, so only A tiles stream through the ring.
+// k-tile, its scale factors in tensor memory only -- while a CTA walks down the row blocks, so only A
+// tiles stream through the ring.  A CTA's last tile is staged over the A stages and B slots.
 template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel, bool kPair>
 __global__ void __launch_bounds__(kThreads, 1)
     nvfp4_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -1861,20 +1862,21 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
                      : 0;
   // TMA-store epilogue whenever the output satisfies the tensor-map rules (16-byte aligned base
   // and row pitch); odd layouts use direct stores.  The f32 residual stream goes through the staging buffers as well, where
-  // its lanes would read and write a row each: 4096 x 2048 x K 8192 100 us with direct stores, 54 us.  A TMA reduction into
-  // the stream took 48 us, but every f32 reduction in global memory takes subnormals for zero.  A bf16 residual stays on
-  // the direct path, which adds in f32 and rounds once.
+  // its lanes would read and write a row each: 4096 x 2048 x K 8192 100 us with direct stores, 54 us (36 on CTA pairs).  A TMA
+  // reduction into the stream took 48 us where this took 54, but every f32 reduction in global memory takes subnormals for
+  // zero.  A bf16 residual stays on the direct path, which adds in f32 and rounds once.
   pl.tma_store = (pl.vec_store && !maps_refused && (a.epilogue != NVFP4_EPI_RESIDUAL || a.out_dtype == NVFP4_DTYPE_F32)) ? 1 : 0;
   const bool can_split = a.out_dtype == NVFP4_DTYPE_F32 &&
                          (a.epilogue == NVFP4_EPI_NONE || a.epilogue == NVFP4_EPI_BIAS) && num_k_tiles >= 16;
   // The f32 residual stream is loaded into the staging buffers its sums leave from.  Two buffers per group (128 x 128)
-  // keep a load in flight beside a store; one (the wider tiles) has them take turns, which a main loop of up to eight
-  // k-tiles does not hide: 65536 x 768 x K 768 82 us at 128 x 128, 98 to 100 at the others, K 1536 96 against 106 to 110;
-  // 8192 x 768 x K 3072 25 against 24.  Beyond, the estimate carries what the turns add to a tile.
+  // keep a load in flight beside a store; one (the wider streaming tiles) has them take turns, which a main loop of up to eight
+  // k-tiles does not hide: 65536 x 768 x K 1536 81 us at 128 x 128, 113 to 120 at the others; K 768, where the panels of up to
+  // three k-tiles have two buffers as well, 79 against 77 to 80 (tall 111).  Beyond, the estimate carries what the turns add to
+  // a tile (8192 x 768 x K 3072 20 us at 128 x 128, 21 at 128 x 192).
   const bool f32_residual = a.epilogue == NVFP4_EPI_RESIDUAL && a.out_dtype == NVFP4_DTYPE_F32;
   // CTA pairs for the main loops that are long enough, at 64 operand bytes per cycle and SM, to earn back what setting up and
   // tearing down a pair and the signals between its CTAs cost (about 1.5 us): 8192 x 1024 x K 32000 bf16 127 -> 102 us, 32000 x
-  // 1024 x K 8192 f32 125 -> 110, 4096 x 2048 x K 8192 f32 residual 41 -> 38; 8192 x 1024 x K 4096 bf16 18.2 either way, 1024 x
+  // 1024 x K 8192 f32 125 -> 110, 4096 x 2048 x K 8192 f32 residual 41 -> 36.4; 8192 x 1024 x K 4096 bf16 18.2 either way, 1024 x
   // 1024 x K 2048 (a split of 8192) f32 12.9 -> 14.2.  Not the tall tile: its two column sets for scale factors leave no slack
   // for those signals (8192 x 768 x K 32000 81 -> 85).  A pair per two SMs must need no more waves.
   auto pairs_of = [&](uint32_t splits) { return (a.m + 255u) / 256u * ((a.n + 255u) / 256u) * splits; };

@@ -258,61 +258,82 @@ __global__ void ms_eden_scale_from_amax_kernel(const float* __restrict__ amax, f
 // Bound by instruction dispatch like the MS-EDEN kernels (ms_eden_tile.cu has the measured costs): per 16-group two
 // candidate scales, two sets of nibbles and two error sums.  Only which error is the smaller leaves the group, so the sums
 // are taken the cheap way first (differences in scaled units, fused multiply-adds) and in the reference's order and
-// roundings only where the two lie closer together than both ways can differ (8192 x 768 bf16 rowwise 9.35 -> 8.65 us, 65536
-// x 768 57.4 -> 53.0).  Code for rare cases stands out of line, returns by value and keeps nothing in local memory (8.4 and
-// 50.2).  The scalar side of a group -- two quotients by the global scale, two reciprocals, two E4M3 conversions -- is
-// straight-line code for global scales inside [2^-80, 2^80] (four IEEE divisions with their range checks and branches cost a
-// third of the group before); other global scales, NaN included, take the generic code per group.
+// roundings only where the two lie closer together than both ways can differ.  Code for rare cases stands out of line, returns
+// by value and keeps nothing in local memory.  The scalar side of a group -- two quotients by the global scale, two reciprocals,
+// two E4M3 conversions -- is straight-line code, both candidates in the lanes of packed operations, for global scales inside
+// [2^-80, 2^80]; other global scales, NaN included, take the generic code per group.  One branch decides between cheap and exact
+// errors, one more takes the latter (24.5 -> 23.0 instructions an element, 65536 x 768 bf16 rowwise 46.4 -> 43.2 us in
+// four_six_rowwise_kernel, of zeros 73 -> 44).
 
 __device__ __forceinline__ float four_six_global_scale(float amax) {
   // utils/nvfp4/quant/kernels/four_six/helpers.rs:33-39 with scale_override = 1.0
   return nz(amax == 0.0f ? 1.0f : amax * 1.0f / (256.0f * 6.0f));
 }
 
+// Quotient a / b and reciprocal of two operands at once, correctly rounded in each lane (div_by_rcp, rcp_in_range).
+__device__ __forceinline__ f32x2_t neg2(f32x2_t v) { return v ^ 0x8000000080000000ull; }
+__device__ __forceinline__ f32x2_t rcp_in_range2(f32x2_t b) {
+  float lo, hi;
+  unpack2(b, lo, hi);
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(lo));
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(hi));
+  const f32x2_t y = pack2(lo, hi);
+  return fma2(y, fma2(neg2(b), y, pack2(1.0f, 1.0f)), y);
+}
+__device__ __forceinline__ f32x2_t div_by_rcp2(f32x2_t a, f32x2_t b, f32x2_t y) {
+  const f32x2_t q = mul2(a, y);
+  return fma2(fma2(neg2(b), q, a), y, q);
+}
+
 // What the groups of one global scale share.
+__device__ __noinline__ float four_six_global_scale_any(float amax) { return four_six_global_scale(amax); }
 struct FourSixScale {
-  float gs;        // global scale
-  float d6, y6;    // 6 gs + eps and its reciprocal
-  float d4, y4;
-  float limit;     // groups with a larger amax (the caller's amax was not theirs) take the generic code
-  bool cheap;      // gs inside the range where the cheap errors can decide
-  bool plain;      // gs inside the range of the straight-line code
+  float gs;       // global scale
+  f32x2_t d, y;   // 6 gs + eps and 4 gs + eps, and their reciprocals
+  float limit;    // groups with a larger amax (the caller's was not theirs, or gs is outside the straight-line code's range) take
+                  // the generic code; up to 2^60, where the reference's squares do not overflow
+  FourSixScale() = default;
   __device__ __forceinline__ explicit FourSixScale(float amax) {
-    // amax / 1536 correctly rounded (the remainder form, exact for every amax the straight-line code accepts)
-    const float quick = div_by_rcp(amax, 1536.0f, 1.0f / 1536.0f);
-    plain = quick >= 0x1p-80f && quick <= 0x1p80f;
-    gs = plain ? quick : four_six_global_scale(amax);
-    d6 = 6.0f * gs + kDenomEps;
-    d4 = 4.0f * gs + kDenomEps;
-    y6 = rcp_in_range(d6);
-    y4 = rcp_in_range(d4);
-    limit = plain ? gs * 0x1p20f : -1.0f;
-    cheap = gs >= 0x1p-30f && gs <= 0x1p80f;
+    // amax / 1536 correctly rounded (the remainder form, exact for every amax the straight-line code accepts); one for zero
+    gs = amax == 0.0f ? 1.0f : div_by_rcp(amax, 1536.0f, 1.0f / 1536.0f);
+    const bool plain = gs >= 0x1p-80f && gs <= 0x1p80f;
+    if (!plain) gs = four_six_global_scale_any(amax);
+    d = add2(mul2_rounded(pack2(gs, gs), pack2(6.0f, 4.0f)), pack2(kDenomEps, kDenomEps));
+    y = rcp_in_range2(d);
+    limit = plain ? fminf(gs * 0x1p20f, 0x1p60f) : -1.0f;
   }
 };
 
-// V[i] = (v[i], v[i + 8]) of a group
+// V[i] = (v[2 i], v[2 i + 1]) of a group
 struct Group16 {
   f32x2_t V[8];
 };
 
+// V * inv and its nibble bytes
+__device__ __forceinline__ uint2 trial16(const f32x2_t (&V)[8], float inv, float (&x)[16]) {
+  const f32x2_t inv2 = pack2(inv, inv);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) unpack2(mul2(V[i], inv2), x[2 * i], x[2 * i + 1]);
+  return make_uint2(cvt_e2m1x8(x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]),
+                    cvt_e2m1x8(x[8], x[9], x[10], x[11], x[12], x[13], x[14], x[15]));
+}
+
 // One candidate scale: the nibble bytes q(v * inv) (the winner's are the output) and the squared error in units of the
 // candidate's step, sum of (q - v * inv)^2, in four partial sums.
 __device__ __forceinline__ float candidate16(const Group16& g, float inv, uint32_t opaque_zero, uint2& nib) {
-  const f32x2_t inv2 = pack2(inv, inv);
-  float lo[8], hi[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) unpack2(mul2(g.V[i], inv2), lo[i], hi[i]);
-  nib = make_uint2(cvt_e2m1x8(lo[0], lo[1], lo[2], lo[3], lo[4], lo[5], lo[6], lo[7]),
-                   cvt_e2m1x8(hi[0], hi[1], hi[2], hi[3], hi[4], hi[5], hi[6], hi[7]));
-  float da[8], db[8];
-  e2m1x8_minus(nib.x, opaque_zero, lo, da);
-  e2m1x8_minus(nib.y, opaque_zero, hi, db);
+  float x[16];
+  nib = trial16(g.V, inv, x);
   f32x2_t sum[2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const f32x2_t d = pack2(da[i], db[i]);
-    sum[i & 1] = i < 2 ? mul2(d, d) : fma2(d, d, sum[i & 1]);
+  for (int h = 0; h < 2; ++h) {
+    const float t[8] = {x[8 * h], x[8 * h + 1], x[8 * h + 2], x[8 * h + 3], x[8 * h + 4], x[8 * h + 5], x[8 * h + 6], x[8 * h + 7]};
+    float d[8];
+    e2m1x8_minus(h ? nib.y : nib.x, opaque_zero, t, d);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const f32x2_t e = pack2(d[2 * i], d[2 * i + 1]);
+      sum[h] = i == 0 ? mul2(e, e) : fma2(e, e, sum[h]);
+    }
   }
   float a, b;
   unpack2(add2(sum[0], sum[1]), a, b);
@@ -322,35 +343,21 @@ __device__ __forceinline__ float candidate16(const Group16& g, float inv, uint32
 // Squared quantization error of the group for one candidate as the reference rounds it: sum of (v - q * dq)^2 in butterfly
 // order (utils/nvfp4/quant/kernels/convert.rs:27-35).
 __device__ __forceinline__ float exact_error16(const f32x2_t (&V)[8], float inv, float dq, uint32_t opaque_zero, uint2& nib) {
-  const f32x2_t inv2 = pack2(inv, inv), dq2 = pack2(dq, dq);
-  float lo[8], hi[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) unpack2(mul2(V[i], inv2), lo[i], hi[i]);
-  nib = make_uint2(cvt_e2m1x8(lo[0], lo[1], lo[2], lo[3], lo[4], lo[5], lo[6], lo[7]),
-                   cvt_e2m1x8(hi[0], hi[1], hi[2], hi[3], hi[4], hi[5], hi[6], hi[7]));
-  float qa[8], qb[8];
+  const f32x2_t dq2 = pack2(dq, dq);
+  float x[16], qa[8], qb[8];
+  nib = trial16(V, inv, x);
   e2m1x8_unpacked(nib.x, opaque_zero, qa);
   e2m1x8_unpacked(nib.y, opaque_zero, qb);
-  float a8[8];  // first butterfly level: e[i] + e[i + 8]
+  f32x2_t e[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const f32x2_t d = sub2(V[i], mul2_rounded(pack2(qa[i], qb[i]), dq2));
-    float e0, e1;
-    unpack2(mul2(d, d), e0, e1);
-    a8[i] = e0 + e1;  // scalar: never contracted with the product
+    const f32x2_t q = i < 4 ? pack2(qa[2 * i], qa[2 * i + 1]) : pack2(qb[2 * i - 8], qb[2 * i - 7]);
+    const f32x2_t d = sub2(V[i], mul2_rounded(q, dq2));
+    e[i] = mul2_rounded(d, d);
   }
-  return ((a8[0] + a8[4]) + (a8[2] + a8[6])) + ((a8[1] + a8[5]) + (a8[3] + a8[7]));
-}
-
-// The choice by the exact errors, with the winner's nibbles.  Not inlined: its registers would be the kernel's.
-struct FourSixChoice {
-  uint2 nib;
-  bool six;
-};
-__device__ __noinline__ FourSixChoice exact_choice(const Group16 g, float inv6, float inv4, float dq6, float dq4, uint32_t opaque_zero) {
-  uint2 nib6, nib4;
-  const bool six = exact_error16(g.V, inv6, dq6, opaque_zero, nib6) <= exact_error16(g.V, inv4, dq4, opaque_zero, nib4);
-  return {six ? nib6 : nib4, six};
+  float a, b;  // e[i] + e[i + 8], then + 4, + 2, + 1: even places in one lane, odd ones in the other
+  unpack2(add2(add2(add2(e[0], e[4]), add2(e[2], e[6])), add2(add2(e[1], e[5]), add2(e[3], e[7]))), a, b);
+  return a + b;
 }
 
 __device__ __forceinline__ float2 e4m3x2_values(uint32_t codes) {
@@ -359,15 +366,32 @@ __device__ __forceinline__ float2 e4m3x2_values(uint32_t codes) {
   return __half22float2(*reinterpret_cast<__half2*>(&h2));
 }
 
-// The scale byte of one candidate pair and everything that follows from it, any values.
-struct FourSixCandidates {
-  uint32_t codes;  // scale bytes: six in bits 0..7, four in bits 8..15
-  float inv6, inv4;
+// Largest decoded magnitude of a group, (q * scale) * gs as the stand-alone NVFP4 amax kernel evaluates it
+// (utils/nvfp4/quant/kernels/ms_eden/amax.rs:23-64): rounding to E2M1 is monotonic in |x|, so the largest nibble is the one of
+// the element with the largest magnitude, ga.
+__device__ __forceinline__ float decoded_max(float ga, float inv, float scale, float gs) {
+  const float q = e2m1x2_values(cvt_e2m1x2(0.0f, ga * inv)).x;
+  return fabsf(q * scale * gs);
+}
+
+// A group by the exact errors.  Not inlined: its registers would be the kernel's.
+struct FourSixChoice {
+  uint2 nib;
+  uint32_t code;
+  float inv, scale;
 };
-__device__ __noinline__ FourSixCandidates four_six_scales_any(float ga, float gs) {
+// codes: the two scale bytes (six in bits 0..7, four in bits 8..15) with their reciprocals
+__device__ __noinline__ FourSixChoice exact_choice(const Group16 g, float gs, uint32_t codes, float inv6, float inv4, uint32_t opaque_zero) {
+  const float2 s = e4m3x2_values(codes);
+  uint2 nib6, nib4;
+  const bool six = exact_error16(g.V, inv6, s.x * gs, opaque_zero, nib6) <= exact_error16(g.V, inv4, s.y * gs, opaque_zero, nib4);
+  return {six ? nib6 : nib4, six ? codes & 0xffu : codes >> 8, six ? inv6 : inv4, six ? s.x : s.y};
+}
+// The same with the scale bytes, any values.
+__device__ __noinline__ FourSixChoice exact_choice_any(const Group16 g, float ga, float gs, uint32_t opaque_zero) {
   const uint32_t b6 = cvt_e4m3(ga * 1.0f / (6.0f * gs + kDenomEps));
   const uint32_t b4 = cvt_e4m3(ga * 1.0f / (4.0f * gs + kDenomEps));
-  return {b6 | (b4 << 8), inv_scale(e4m3_value(b6), gs), inv_scale(e4m3_value(b4), gs)};
+  return exact_choice(g, gs, b6 | (b4 << 8), inv_scale(e4m3_value(b6), gs), inv_scale(e4m3_value(b4), gs), opaque_zero);
 }
 
 // v: one 16-group, ga its amax.  Returns the scale byte and writes the 8 nibble bytes into `packed`.
@@ -376,62 +400,64 @@ __device__ __noinline__ FourSixCandidates four_six_scales_any(float ga, float gs
 __device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float ga, const FourSixScale& sc, uint32_t opaque_zero,
                                                    uint2& packed, float* decoded_amax = nullptr) {
   uint32_t codes;
-  float inv6, inv4;
   {
+    float q6, q4;
+    unpack2(div_by_rcp2(pack2(ga, ga), sc.d, sc.y), q6, q4);
     uint16_t c;
-    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;"
-        : "=h"(c)
-        : "f"(div_by_rcp(ga, sc.d4, sc.y4)), "f"(div_by_rcp(ga, sc.d6, sc.y6)));
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(c) : "f"(q4), "f"(q6));
     codes = c;
   }
-  float2 s = e4m3x2_values(codes);
-  float step6 = s.x == 0.0f ? sc.gs : s.x * sc.gs, step4 = s.y == 0.0f ? sc.gs : s.y * sc.gs;
-  inv6 = rcp_in_range(step6 + kDenomEps);
-  inv4 = rcp_in_range(step4 + kDenomEps);
-  if (!(ga <= sc.limit)) {
-    const FourSixCandidates any = four_six_scales_any(ga, sc.gs);
-    codes = any.codes, inv6 = any.inv6, inv4 = any.inv4;
-    s = e4m3x2_values(codes);
-    step6 = s.x == 0.0f ? sc.gs : s.x * sc.gs, step4 = s.y == 0.0f ? sc.gs : s.y * sc.gs;
-  }
+  // a zero scale byte counts as one
+  uint32_t h2;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"(static_cast<uint16_t>(codes)));
+  const __half2 raw = *reinterpret_cast<const __half2*>(&h2);
+  const float2 s = __half22float2(__hadd2(raw, __heq2(raw, __floats2half2_rn(0.0f, 0.0f))));
+  const f32x2_t step = mul2_rounded(pack2(s.x, s.y), pack2(sc.gs, sc.gs));
+  float step6, step4, inv6, inv4;
+  unpack2(step, step6, step4);
+  unpack2(rcp_in_range2(add2(step, pack2(kDenomEps, kDenomEps))), inv6, inv4);
   Group16 g;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) g.V[i] = pack2(v[i], v[i + 8]);
+  for (int i = 0; i < 8; ++i) g.V[i] = pack2(v[2 * i], v[2 * i + 1]);
   // How far the cheap errors can be off, with u = 2^-24, D the exact differences v - q dq and |q dq| <= |v| + |D| <= 2 |v|
-  // (2-norms over the group; rounding to the grid never takes a value further than its own size):
-  //   cheap: v * inv is v / dq within 3.1 u (1e-20 is below u / 10 of dq where gs >= 2^-30), then the difference, the
-  //          products, the sums and two scalings:       | sqrt(e) - |D| |   <= 3.1 u |v| + 5 u |D|
+  // (2-norms over the group; rounding to the grid never takes a value further than its own size), all in steps of "six":
+  //   cheap: v * inv is v / dq within 4.6 u (1e-20 is below 1.5 u of a step of 2^-43 and more), then the difference, the
+  //          products, the sums, and for "four" the ratio of the steps, its square and a product:
+  //                                                      | sqrt(e) - |D| |   <= 4.6 u |v| + 7 u |D|
   //   exact: q dq, the difference, square and sums:      | sqrt(err) - |D| | <= 2 u |v| + 3.5 u |D|
   // A scale byte of zero stands for the step gs in v * inv and for dq = 0: all q are 0 then, D = v, and with gs as the step
-  // the same bounds hold.  With |D| <= |v| <= 4 ga both candidates together shift sqrt(e6) - sqrt(e4) by less than 120 u ga.
-  // Multiplied by sqrt(e6) + sqrt(e4) <= sqrt(2 (e6 + e4)) and squared: the order is certain where (e6 - e4)^2 exceeds
-  // 2 (120 u)^2 < 2^-33 times ga^2 (e6 + e4).  Two candidates of one scale byte (zero groups, saturated ones) are the same
-  // candidate: "six", where the error is a number.  Otherwise -- NaN, overflow, gs outside the range of the bounds -- the
-  // exact errors decide.
-  bool six = false, certain = false;
-  if (sc.cheap) {
+  // the same bounds hold.  With |D| <= |v| <= 4 ga both candidates together shift sqrt(e6) - sqrt(e4) by less than 128 u ga,
+  // and ga is at most 9 steps of "six" (the largest quotient that rounds to the smallest scale byte is 1.5 times it) unless both
+  // scale bytes saturate.  Multiplied by sqrt(e6) + sqrt(e4) <= sqrt(2 (e6 + e4)) and squared: the order is certain where
+  // (e6 - e4)^2 exceeds 2 (1152 u)^2 < 2^-26 times e6 + e4.  Two candidates of one scale byte (zero groups, saturated ones) are
+  // the same candidate: "six", where the error is a number, and the same bytes either way.  Otherwise -- NaN, scales and values
+  // outside the range of the bounds -- the exact errors decide.
+  bool certain = false;
+  uint32_t code;
+  float inv, scale;
+  if (ga <= sc.limit && step6 >= 0x1p-43f) {
     uint2 nib6, nib4;
-    const float e6 = candidate16(g, inv6, opaque_zero, nib6) * (step6 * step6);
-    const float e4 = candidate16(g, inv4, opaque_zero, nib4) * (step4 * step4);
-    const float gap = e6 - e4;
-    six = e6 <= e4;
+    const float e6 = candidate16(g, inv6, opaque_zero, nib6), e4 = candidate16(g, inv4, opaque_zero, nib4);
+    const float ratio = step4 * inv6, e4_in_six = e4 * (ratio * ratio);
+    const float gap = e6 - e4_in_six;
+    const bool six = e6 <= e4_in_six;
     packed = six ? nib6 : nib4;
-    certain = gap * gap > 0x1p-33f * ga * ga * (e6 + e4);
+    code = six ? codes & 0xffu : codes >> 8;
+    inv = six ? inv6 : inv4;
+    scale = six ? s.x : s.y;
+    certain = gap * gap > 0x1p-26f * (e6 + e4_in_six);
     if (!certain) certain = (codes & 0xffu) == codes >> 8 && e6 == e4;
   }
   if (!certain) {
-    const FourSixChoice exact = exact_choice(g, inv6, inv4, s.x * sc.gs, s.y * sc.gs, opaque_zero);
-    six = exact.six;
+    const FourSixChoice exact = ga <= sc.limit ? exact_choice(g, sc.gs, codes, inv6, inv4, opaque_zero)
+                                               : exact_choice_any(g, ga, sc.gs, opaque_zero);
     packed = exact.nib;
+    code = exact.code;
+    inv = exact.inv;
+    scale = exact.scale;
   }
-  if (decoded_amax) {
-    // Largest decoded magnitude of the group, (q * scale) * gs as the stand-alone NVFP4 amax kernel
-    // evaluates it (utils/nvfp4/quant/kernels/ms_eden/amax.rs:23-64): rounding to E2M1 is monotonic
-    // in |x|, so the largest nibble is the one of the element with the largest magnitude, ga.
-    const float q = e2m1x2_values(cvt_e2m1x2(0.0f, ga * (six ? inv6 : inv4))).x;
-    *decoded_amax = fabsf(q * (six ? s.x : s.y) * sc.gs);
-  }
-  return six ? codes & 0xffu : codes >> 8;
+  if (decoded_amax) *decoded_amax = decoded_max(ga, inv, scale, sc.gs);
+  return code;
 }
 
 __device__ __forceinline__ float group_amax16(const float (&v)[16]) {
@@ -441,6 +467,88 @@ __device__ __forceinline__ float group_amax16(const float (&v)[16]) {
   return ga;
 }
 
+// The stored words of a 16-group, widened as they are or as relu(x)^2 (max(x, 0) drops NaN like the reference's max_f32, the
+// square is one rounded multiply); bf16 pairs meet the zero before they are widened.
+template <typename T>
+struct RawGroup;
+template <>
+struct RawGroup<float> {
+  uint4 w[4];
+  __device__ __forceinline__ void load(const float* p) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
+  }
+  template <bool kRelu2>
+  __device__ __forceinline__ void widen(float (&v)[16]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[4 * i] = __uint_as_float(w[i].x);
+      v[4 * i + 1] = __uint_as_float(w[i].y);
+      v[4 * i + 2] = __uint_as_float(w[i].z);
+      v[4 * i + 3] = __uint_as_float(w[i].w);
+    }
+    if (kRelu2) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = max_f32(v[i], 0.0f);
+      square_all(v);
+    }
+  }
+  __device__ __forceinline__ static void square_all(float (&v)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+      const f32x2_t t = pack2(v[i], v[i + 1]);
+      unpack2(mul2(t, t), v[i], v[i + 1]);
+    }
+  }
+  template <bool kRelu2>
+  __device__ __forceinline__ float amax() const {  // of the widened values
+    float v[16];
+    widen<kRelu2>(v);
+    return group_amax16(v);
+  }
+};
+template <>
+struct RawGroup<__nv_bfloat16> {
+  uint4 w[2];
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) w[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
+  }
+  template <bool kRelu2>
+  __device__ __forceinline__ void widen(float (&v)[16]) const {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint32_t t[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (kRelu2) {
+          const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&t[j]), __floats2bfloat162_rn(0.0f, 0.0f));
+          t[j] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+        v[8 * i + 2 * j] = widen_bf16_lo(t[j]);
+        v[8 * i + 2 * j + 1] = widen_bf16_hi(t[j]);
+      }
+    }
+    if (kRelu2) RawGroup<float>::square_all(v);
+  }
+  // Of the widened values, on packed pairs (a maximum rounds nothing and drops NaN; the largest square is that of the largest).
+  template <bool kRelu2>
+  __device__ __forceinline__ float amax() const {
+    __nv_bfloat162 m = __floats2bfloat162_rn(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t t[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(&t[j]);
+        m = __hmax2(m, kRelu2 ? b : __habs2(b));
+      }
+    }
+    const float a = max_f32(__low2float(m), __high2float(m));
+    return kRelu2 ? a * a : a;
+  }
+};
+
 // What a quantizer reads: a group of 16 values of a stored tensor, relu(x)^2 of it (the MLP activation computed on load
 // from the stored pre-activation: max(x, 0) drops NaN like the reference's max_f32, the square is one rounded multiply),
 // or the schedule-free weight y = z + beta (x - z) of two f32 masters, which is never written out in f32
@@ -449,15 +557,16 @@ template <typename T, bool kRelu2>
 struct TensorSource {
   const T* x;
   __device__ __forceinline__ void pin_loads() { x = after_prior(x); }
+  struct Words {
+    RawGroup<T> raw;
+    __device__ __forceinline__ float amax() const { return raw.template amax<kRelu2>(); }
+    __device__ __forceinline__ void widen(float (&v)[16]) const { raw.template widen<kRelu2>(v); }
+  };
+  __device__ __forceinline__ void load(size_t group, Words& w) const { w.raw.load(x + group * 16); }
   __device__ __forceinline__ void load16(size_t group, float (&v)[16]) const {
-    Load16<T>::run(x + group * 16, v);
-    if (kRelu2) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float r = max_f32(v[i], 0.0f);
-        v[i] = r * r;
-      }
-    }
+    Words w;
+    load(group, w);
+    w.widen(v);
   }
 };
 __device__ __forceinline__ float schedule_free_value(float z, float x, float beta) { return z + beta * (x - z); }
@@ -476,6 +585,15 @@ struct ScheduleFreeSource {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = schedule_free_value(zv[i], xv[i], beta);
   }
+  struct Words {
+    float value[16];
+    __device__ __forceinline__ float amax() const { return group_amax16(value); }
+    __device__ __forceinline__ void widen(float (&v)[16]) const {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = value[i];
+    }
+  };
+  __device__ __forceinline__ void load(size_t group, Words& w) const { load16(group, w.value); }
 };
 
 // Scale bytes of four neighbouring lanes (one k-atom of a row) as one 32-bit store; every lane of the warp calls it.
@@ -497,6 +615,92 @@ __device__ __forceinline__ float cta_max_of(const float* partials, uint32_t coun
   if ((threadIdx.x & 31u) == 0) atomicMax(&bits, w);
   __syncthreads();
   return __uint_as_float(bits);
+}
+
+// Rowwise four-six of rows that whole warps cover.  A warp takes 32 kGroups groups at a time, a lane kGroups of them: kRows = 2
+// whole rows, a row, or, where the rows' maxima are given (kOwn = false), a part of one.  All of them are loaded before the first
+// is quantized, the row maximum is a reduction of the warp, so that nothing ties the warps of a CTA together, and what depends
+// on the row alone -- its maximum, its scale, the place of its scale bytes -- is computed once.  Bound by issue slots like its
+// neighbours (20 instructions an element in place of 24, and four groups of a lane give the schedulers independent chains): bf16
+// with own maxima 65536 x 768 46.4 -> 35.8 us, 8192 x 768 7.6 -> 5.9, 16384 x 2048 29.5 -> 20.7 (against a CTA per row block
+// with a barrier, four_six_rowwise_kernel, which takes the other widths and few rows); relu^2 with given maxima
+// 65536 x 3072 166 -> 146, 8192 x 4096 29.3 -> 25.3.  With 80 registers and three CTAs an SM 8192 x 768 took 8.1 us.
+template <typename Source, bool kOwn, int kGroups, int kRows>
+__global__ void __launch_bounds__(256, 2)
+    four_six_rows_kernel(Source src, const float* __restrict__ amax, uint8_t* __restrict__ out_fp4, uint8_t* __restrict__ out_scales,
+                         float* __restrict__ out_gs, float* __restrict__ out_amax, float* __restrict__ decoded_amax, uint32_t rows,
+                         uint32_t plane_rows, uint32_t units, uint32_t groups_per_row, const FastDiv units_per_row,
+                         int packed_scales, uint32_t opaque_zero) {
+  static_assert(kOwn || kRows == 1, "parts of a row only where its maximum is given");
+  wait_for_prior_then_allow_next();
+  src.pin_loads();
+  amax = after_prior(amax);
+  constexpr uint32_t kRowGroups = 32 / kRows * kGroups;  // of a row in a unit
+  const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * 8u;
+  // this lane's groups inside a unit: row, scale byte
+  bool in_second[kGroups];
+  uint32_t scale_at[kGroups];
+#pragma unroll
+  for (int i = 0; i < kGroups; ++i) {
+    const uint32_t g = lane + 32u * i;
+    in_second[i] = kRows == 2 && g >= kRowGroups;
+    const uint32_t kg = in_second[i] ? g - kRowGroups : g;
+    scale_at[i] = packed_scales ? (kg >> 2) * 512u + (kg & 3u) + (in_second[i] ? 16u : 0u) : g;
+  }
+  float dec = 0.0f;
+  for (uint32_t u = blockIdx.x * 8u + (threadIdx.x >> 5); u < units; u += warps) {
+    const uint32_t row = kOwn ? u * kRows : units_per_row.div(u), kg0 = kOwn ? 0u : (u - row * units_per_row.d) * kRowGroups;
+    const bool first = row < rows, second = kRows == 2 && row + 1 < rows;
+    const size_t group = static_cast<size_t>(u) * (32u * kGroups) + lane;
+    typename Source::Words words[kGroups] = {};
+    float ga[kGroups], row_amax[kRows] = {};
+    if (!kOwn && first) row_amax[0] = amax[row];
+#pragma unroll
+    for (int i = 0; i < kGroups; ++i)
+      if (in_second[i] ? second : first) src.load(group + 32u * i, words[i]);
+#pragma unroll
+    for (int i = 0; i < kGroups; ++i) {
+      ga[i] = words[i].amax();
+      if (!kOwn) {
+        continue;
+      } else if (kRows == 1 || 32u * (i + 1) <= kRowGroups) {
+        row_amax[0] = max_f32(row_amax[0], ga[i]);
+      } else if (32u * i >= kRowGroups) {
+        row_amax[kRows - 1] = max_f32(row_amax[kRows - 1], ga[i]);
+      } else {
+        row_amax[0] = max_f32(row_amax[0], in_second[i] ? 0.0f : ga[i]);
+        row_amax[kRows - 1] = max_f32(row_amax[kRows - 1], in_second[i] ? ga[i] : 0.0f);
+      }
+    }
+    FourSixScale sc[kRows];
+#pragma unroll
+    for (int h = 0; h < kRows; ++h) {  // non-negative floats order like their bit patterns
+      if (kOwn) row_amax[h] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(row_amax[h])));
+      sc[h] = FourSixScale(row_amax[h]);
+    }
+    if (kg0 == 0 && lane < kRows && row + lane < rows) {
+      out_gs[row + lane] = lane ? sc[kRows - 1].gs : sc[0].gs;
+      if (kOwn && out_amax) out_amax[row + lane] = lane ? row_amax[kRows - 1] : row_amax[0];
+    }
+    uint8_t* const scales = out_scales + (packed_scales ? packed_scale_offset(row, kg0, groups_per_row >> 2)
+                                                             : static_cast<size_t>(row) * groups_per_row + kg0);
+#pragma unroll
+    for (int i = 0; i < kGroups; ++i) {
+      float v[16], d;
+      words[i].widen(v);
+      FourSixScale mine = sc[0];
+      if (in_second[i]) mine = sc[kRows - 1];
+      uint2 nibbles;
+      uint32_t b = four_six_group(v, ga[i], mine, opaque_zero, nibbles, decoded_amax ? &d : nullptr);
+      const bool inside = in_second[i] ? second : first;
+      if (inside) *reinterpret_cast<uint2*>(out_fp4 + (group + 32u * i) * 8) = nibbles;
+      if (inside && decoded_amax) dec = max_f32(dec, d);
+      if (!inside) b = 0x38u;  // pad rows of a packed plane hold 1.0
+      if (row + (in_second[i] ? 1u : 0u) < plane_rows) scales[scale_at[i]] = static_cast<uint8_t>(b);
+    }
+    if (u + warps < u) break;  // the index space ends below 2^32
+  }
+  if (decoded_amax) cta_atomic_max(warp_max(dec), decoded_amax);  // uniform across the CTA
 }
 
 // One thread per 16-group and step over a [rows][cols] tensor; `groups` counts those of the pad rows too where the
@@ -558,45 +762,6 @@ __global__ void __launch_bounds__(256, 4)
 // decoded_amax (optional, zeroed by the launcher): max |decoded value| of the whole quantized tensor, i.e. what
 // utils/nvfp4/quant/kernels/ms_eden/amax.rs:23-64 computes from the stored tensor before the backward transposer --
 // handed over so that pass can be skipped.
-template <typename T>
-struct RawGroup;
-template <>
-struct RawGroup<float> {
-  uint4 w[4];
-  __device__ __forceinline__ void load(const float* p) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
-  }
-  __device__ __forceinline__ void widen(float (&v)[16]) const {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      v[4 * i] = __uint_as_float(w[i].x);
-      v[4 * i + 1] = __uint_as_float(w[i].y);
-      v[4 * i + 2] = __uint_as_float(w[i].z);
-      v[4 * i + 3] = __uint_as_float(w[i].w);
-    }
-  }
-};
-template <>
-struct RawGroup<__nv_bfloat16> {
-  uint4 w[2];
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) w[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
-  }
-  __device__ __forceinline__ void widen(float (&v)[16]) const {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint32_t t[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        v[8 * i + 2 * j] = widen_bf16_lo(t[j]);
-        v[8 * i + 2 * j + 1] = widen_bf16_hi(t[j]);
-      }
-    }
-  }
-};
-
 constexpr int kStreamMaxRowsPerCta = 256;
 template <typename T, bool kPacked, bool kRelu2>
 __global__ void __launch_bounds__(256, 3)
@@ -608,70 +773,57 @@ __global__ void __launch_bounds__(256, 3)
   x = after_prior(x);
   __shared__ unsigned int row_amax_bits[3][kStreamMaxRowsPerCta];
   const uint32_t t = threadIdx.x, lane_id = t & 31u;
-  for (uint32_t i = t; i < 3 * rows_per_cta; i += blockDim.x) row_amax_bits[i / rows_per_cta][i % rows_per_cta] = 0u;
+  for (uint32_t i = t; i < kStreamMaxRowsPerCta; i += blockDim.x) row_amax_bits[0][i] = row_amax_bits[1][i] = row_amax_bits[2][i] = 0u;
   __syncthreads();
   const uint32_t local_row = t / groups_per_row;
   const uint32_t kg = t - local_row * groups_per_row;
   const bool in_use = local_row < rows_per_cta;
   // four neighbouring lanes hold four neighbouring scale bytes of one aligned word
   const bool quads = (groups_per_row & 3u) == 0 && (reinterpret_cast<uintptr_t>(out_scales) & 3u) == 0;
-  RawGroup<T> raw;
-  uint32_t blk = blockIdx.x;
-  {
-    const uint32_t row = blk * rows_per_cta + local_row;
-    if (blk < row_blocks && in_use && row < rows) raw.load(x + (static_cast<size_t>(row) * groups_per_row + kg) * 16);
-  }
+  const bool first_of_quad = (kg & 3u) == 0;
+  // Row max: non-negative floats order like their bit patterns.  With at least 32 groups per row a warp touches at most two
+  // rows: two warp-wide integer maxima, of the lanes in its first row and of the others, and an atomic max of one lane each.
+  const bool two_rows = groups_per_row >= 32;
+  const bool in_first = !two_rows || local_row == __shfl_sync(0xffffffffu, local_row, 0);
+  const uint32_t other_lanes = __ballot_sync(0xffffffffu, !in_first && in_use);
+  const bool leads_row = two_rows ? in_use && (lane_id == 0 || (other_lanes != 0u && lane_id + 1u == __ffs(other_lanes))) : in_use;
+
+  uint32_t row = blockIdx.x * rows_per_cta + local_row;
+  const uint32_t row_step = gridDim.x * rows_per_cta;
+  size_t group = static_cast<size_t>(row) * groups_per_row + kg;
+  const size_t group_step = static_cast<size_t>(row_step) * groups_per_row;
+  RawGroup<T> raw = {};
+  if (in_use && row < rows) raw.load(x + group * 16);
   float dec_running = 0.0f;
-  uint32_t buf = 0;
-  for (; blk < row_blocks; blk += gridDim.x) {
-    const uint32_t row = blk * rows_per_cta + local_row;
+  unsigned int *here = row_amax_bits[0], *next = row_amax_bits[1], *stale = row_amax_bits[2];
+  for (uint32_t blk = blockIdx.x; blk < row_blocks; blk += gridDim.x, row += row_step, group += group_step) {
     const bool active = in_use && row < rows;
     float v[16];
-    float ga = 0.0f;
-    if (active) {
-      raw.widen(v);
-      if (kRelu2) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float r = max_f32(v[i], 0.0f);
-          v[i] = r * r;
-        }
-      }
-      ga = group_amax16(v);
-    }
-    {
-      // the next row block's words: in flight across the barrier and the whole quantization below
-      const uint32_t nblk = blk + gridDim.x;
-      const uint32_t nrow = nblk * rows_per_cta + local_row;
-      if (nblk < row_blocks && in_use && nrow < rows) raw.load(x + (static_cast<size_t>(nrow) * groups_per_row + kg) * 16);
-    }
-    // Row max: non-negative floats order like their bit patterns.  With at least 32 groups per row a warp
-    // touches at most two rows: two warp-wide integer maxima and two shared-memory atomics.
+    raw.template widen<kRelu2>(v);
+    const float ga = group_amax16(v);
+    // the next row block's words: in flight across the barrier and the whole quantization below (row numbers end below 2^32)
+    if (in_use && row < rows - min(rows, row_step)) raw.load(x + (group + group_step) * 16);
     const uint32_t ga_bits = active ? __float_as_uint(ga) : 0u;
-    if (groups_per_row >= 32) {
-      const uint32_t first_row = __shfl_sync(0xffffffffu, local_row, 0);
-      const bool in_first = local_row == first_row;
-      const uint32_t m_first = __reduce_max_sync(0xffffffffu, in_first ? ga_bits : 0u);
-      const uint32_t m_other = __reduce_max_sync(0xffffffffu, in_first ? 0u : ga_bits);
-      const uint32_t other_lanes = __ballot_sync(0xffffffffu, !in_first && active);
-      if (lane_id == 0 && active) atomicMax(&row_amax_bits[buf][local_row], m_first);
-      if (other_lanes != 0u && lane_id == static_cast<uint32_t>(__ffs(other_lanes) - 1))
-        atomicMax(&row_amax_bits[buf][local_row], m_other);
-    } else if (active) {
-      atomicMax(&row_amax_bits[buf][local_row], ga_bits);
+    uint32_t row_bits = ga_bits;
+    if (two_rows) {
+      row_bits = __reduce_max_sync(0xffffffffu, in_first ? ga_bits : 0u);
+      if (other_lanes != 0u) {
+        const uint32_t m_other = __reduce_max_sync(0xffffffffu, in_first ? 0u : ga_bits);
+        if (!in_first) row_bits = m_other;
+      }
     }
+    if (leads_row) atomicMax(&here[local_row], row_bits);
     __syncthreads();
     // every thread is past its reads of the buffer of the previous row block: clear it for the block after next
-    const uint32_t stale = buf == 0 ? 2u : buf - 1u;
-    if (t < rows_per_cta) row_amax_bits[stale][t] = 0u;
+    if (t < rows_per_cta) stale[t] = 0u;
     uint32_t b = 0x38u;
     if (active) {
-      const float amax = __uint_as_float(row_amax_bits[buf][local_row]);
+      const float amax = __uint_as_float(here[local_row]);
       const FourSixScale sc(amax);
       uint2 packed;
       float dec;
       b = four_six_group(v, ga, sc, opaque_zero, packed, decoded_amax ? &dec : nullptr);
-      *reinterpret_cast<uint2*>(out_fp4 + (static_cast<size_t>(row) * groups_per_row + kg) * 8) = packed;
+      *reinterpret_cast<uint2*>(out_fp4 + group * 8) = packed;
       if (kg == 0) {
         out_gs[row] = sc.gs;
         if (out_amax) out_amax[row] = amax;
@@ -679,13 +831,15 @@ __global__ void __launch_bounds__(256, 3)
       if (decoded_amax) dec_running = max_f32(dec_running, dec);
     }
     const bool in_plane = in_use && row < (kPacked ? padded_rows : rows);
-    uint8_t* const dst = out_scales + (kPacked ? packed_scale_offset(row, kg, groups_per_row >> 2)
-                                               : static_cast<size_t>(row) * groups_per_row + kg);
+    uint8_t* const dst = out_scales + (kPacked ? packed_scale_offset(row, kg, groups_per_row >> 2) : group);
     if (quads)
-      store_scale_quad(dst, b, in_plane && (kg & 3u) == 0);
+      store_scale_quad(dst, b, in_plane && first_of_quad);
     else if (in_plane)
       *dst = static_cast<uint8_t>(b);
-    buf = buf == 2 ? 0u : buf + 1u;
+    unsigned int* const done = here;
+    here = next;
+    next = stale;
+    stale = done;
   }
   if (decoded_amax) {  // uniform across the CTA; the CTA may have fewer than eight warps
     __shared__ unsigned int dec_bits;
@@ -1383,6 +1537,48 @@ TensorSource<__nv_bfloat16, true> advance(const TensorSource<__nv_bfloat16, true
 template <>
 ScheduleFreeSource advance(const ScheduleFreeSource& s, size_t n) { return {s.z + n, s.x + n, s.beta}; }
 
+template <typename Source, bool kOwn, int kGroups, int kRows>
+static int launch_four_six_rows(cudaStream_t s, const Source& src, const float* amax, uint32_t rows, uint32_t plane_rows, uint32_t gpr,
+                                uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, float* out_amax, float* decoded_amax) {
+  const uint32_t per_row = kRows == 2 ? 1u : gpr / (32 * kGroups);
+  const uint32_t units = kRows == 2 ? (plane_rows + 1) / 2 : plane_rows * per_row;
+  // CTAs of eight warps, as many of the latter as are resident where that gives each the same number of units, fewer otherwise
+  const uint32_t resident = 148u * 8u * 2u, per_warp = (units + resident - 1) / resident;
+  const uint32_t grid = ((units + per_warp - 1) / per_warp + 7) / 8;
+  return launch_chained(four_six_rows_kernel<Source, kOwn, kGroups, kRows>, grid, 256, 0, s, src, amax, out_fp4, out_scales, out_gs,
+                        out_amax, decoded_amax, rows, plane_rows, units, gpr, FastDiv(per_row), packed, 0u);
+}
+// -1: no form of the kernel takes such rows
+template <typename Source>
+static int launch_four_six_own_rows(cudaStream_t s, const Source& src, uint32_t rows, uint32_t plane_rows, uint32_t gpr, uint8_t* out_fp4,
+                                    uint8_t* out_scales, int packed, float* out_gs, float* out_amax, float* decoded_amax) {
+  // Fewer than four warps an SM leave most of it idle while a lane quantizes its groups one after the other: 1000 x 768 2.75 us by
+  // four_six_rowwise_kernel, 2.87 here; 1500 x 768 3.17 and 2.87.
+  if (plane_rows / (gpr == 16 || gpr == 48 ? 2u : 1u) < 148u * 4u) return -1;
+#define NVFP4_ROWS(G, R)                                                                                                    \
+  return launch_four_six_rows<Source, true, G, R>(s, src, nullptr, rows, plane_rows, gpr, out_fp4, out_scales, packed, out_gs, \
+                                                  out_amax, decoded_amax)
+  switch (gpr) {
+    case 16: NVFP4_ROWS(1, 2);
+    case 32: NVFP4_ROWS(1, 1);
+    case 48: NVFP4_ROWS(3, 2);
+    case 64: NVFP4_ROWS(2, 1);
+    case 96: NVFP4_ROWS(3, 1);
+    case 128: NVFP4_ROWS(4, 1);
+    default: return -1;
+  }
+#undef NVFP4_ROWS
+}
+// Sources whose rows with given maxima go to four_six_rows_kernel.
+template <typename Source>
+struct TakesGivenRows {
+  static constexpr bool value = false;
+};
+template <bool kRelu2>
+struct TakesGivenRows<TensorSource<__nv_bfloat16, kRelu2>> {
+  static constexpr bool value = true;
+};
+
 template <typename Source>
 static int launch_four_six_source(cudaStream_t s, const Source& src, const float* amax, uint32_t amax_count, float* out_amax,
                                   int rowwise, uint32_t rows, uint32_t cols, uint8_t* out_fp4, uint8_t* out_scales, int packed,
@@ -1405,6 +1601,19 @@ static int launch_four_six_source(cudaStream_t s, const Source& src, const float
   const uint64_t plane_rows = packed ? (rows + 127u) / 128u * 128u : rows;
   const bool pad_apart = plane_rows * gpr > limit;
   const uint32_t groups = static_cast<uint32_t>((pad_apart ? rows : plane_rows) * gpr);
+  if constexpr (TakesGivenRows<Source>::value) {
+    // bf16 sources; f32 ones are bound by HBM and L2 as they are (4096 x 8192 26.5 us one group at a time, 26.8 and more by
+    // rows).  With fewer than twelve warps an SM a lane's groups one after the other take longer: 500 x 4096 3.4 us in place of 3.8,
+    // 1000 x 4096 5.4 and 5.3.
+    if (rowwise && (gpr % 64 == 0 || gpr % 96 == 0) && plane_rows * (gpr / (gpr % 128 == 0 ? 128u : gpr % 96 == 0 ? 96u : 64u)) >= 148u * 12u) {
+      const uint32_t launched_rows = static_cast<uint32_t>(pad_apart ? rows : plane_rows);
+      const auto launch = gpr % 128 == 0 ? launch_four_six_rows<Source, false, 4, 1>
+                          : gpr % 96 == 0 ? launch_four_six_rows<Source, false, 3, 1>
+                                          : launch_four_six_rows<Source, false, 2, 1>;
+      const int rc = launch(s, src, amax, rows, launched_rows, gpr, out_fp4, out_scales, packed, out_gs, nullptr, decoded_amax);
+      return rc == 0 && pad_apart ? launch_packed_scale_pad(s, out_scales, rows, cols) : rc;
+    }
+  }
   // one wave of resident CTAs where the prologue reduces partial maxima or the tensor is large; each thread then walks
   const uint32_t grid = blocks_for(groups, 256, 148u * 4u);
   const bool quads = gpr % 4 == 0 && (reinterpret_cast<uintptr_t>(out_scales) & 3u) == 0;
@@ -1452,6 +1661,17 @@ int launch_four_six_rowwise_fused(cudaStream_t s, const void* x, int dtype, uint
     if (err != cudaSuccess) return static_cast<int>(err);
   }
   if (rows == 0) return 0;
+  const uint64_t plane_rows = packed ? (static_cast<uint64_t>(rows) + 127u) / 128u * 128u : rows;
+  if (plane_rows * gpr <= 0xfff00000ull) {
+    const uint32_t plane = static_cast<uint32_t>(plane_rows);
+#define NVFP4_OWN_ROWS(T, R)                                                                                          \
+  launch_four_six_own_rows(s, TensorSource<T, R>{static_cast<const T*>(x)}, rows, plane, gpr, out_fp4, out_scales, packed, \
+                           out_gs, out_amax, decoded_amax)
+    const int rc = dtype == NVFP4_DTYPE_F32 ? (relu2 ? NVFP4_OWN_ROWS(float, true) : NVFP4_OWN_ROWS(float, false))
+                                            : (relu2 ? NVFP4_OWN_ROWS(__nv_bfloat16, true) : NVFP4_OWN_ROWS(__nv_bfloat16, false));
+#undef NVFP4_OWN_ROWS
+    if (rc >= 0) return rc;
+  }
   const uint32_t rpc = 256 / gpr;
   const uint32_t threads = (rpc * gpr + 31) / 32 * 32;
   const uint32_t padded_rows = packed ? (rows + 127u) / 128u * 128u : rows;

@@ -885,12 +885,12 @@ static nvfp4_gemm_args dweight_gemm(void* dweight, int dweight_dtype, uint32_t T
 }
 
 // The gradient GEMMs over quantized operands: dX = e_h . weight_t_h^T, dW = e_t_h . input_t_h^T.
-// dweight_is_zero: dweight holds zeros already
+// dweight_is_zero: dweight holds zeros already.  side_by_side: dweight lies apart from what the dX GEMM reads and writes.
 static int backward_gemms(cudaStream_t s, const uint8_t* eh_b, const uint8_t* eh_s, const float* eh_g,
                           const uint8_t* wt_b, const uint8_t* wt_s, const float* wt_g, const uint8_t* et_b,
                           const uint8_t* et_s, const float* et_g, const uint8_t* xt_b, const uint8_t* xt_s,
                           const float* xt_g, void* dinput, int dinput_dtype, void* dweight, int dweight_dtype,
-                          uint32_t T, uint32_t I, uint32_t O, bool dweight_is_zero = false) {
+                          uint32_t T, uint32_t I, uint32_t O, bool dweight_is_zero = false, bool side_by_side = false) {
   nvfp4_gemm_args g;
   std::memset(&g, 0, sizeof(g));
   g.global_scale_mode = NVFP4_GS_ROWWISE_A;
@@ -908,7 +908,8 @@ static int backward_gemms(cudaStream_t s, const uint8_t* eh_b, const uint8_t* eh
   g.n = I;
   g.k = padded_k(O);
   g.ldo = I;
-  int rc = launch_gemm(s, g);
+  side_by_side = side_by_side && T != 0 && I != 0 && O != 0;
+  int rc = launch_gemm(s, g, false, false, side_by_side ? GemmNeighbour::kLetsNextBeside : GemmNeighbour::kNone);
   if (rc) return rc;
   g = dweight_gemm(dweight, dweight_dtype, T, I, O);
   g.a_bytes = et_b;
@@ -917,7 +918,7 @@ static int backward_gemms(cudaStream_t s, const uint8_t* eh_b, const uint8_t* eh
   g.b_bytes = xt_b;
   g.b_scales = xt_s;
   g.b_global = xt_g;
-  return launch_gemm(s, g, dweight_is_zero);
+  return launch_gemm(s, g, dweight_is_zero, false, side_by_side ? GemmNeighbour::kBesidePrior : GemmNeighbour::kNone);
 }
 
 static int backward_device_scale(void* stream, const nvfp4_linear_backward_device_scale_args* a) {
@@ -1001,7 +1002,8 @@ static bool dweight_lies_apart(const nvfp4_linear_backward_args* a, size_t dweig
 // Everything of nvfp4_linear_backward_ms_eden that runs between the fork onto the caller's side stream and the
 // join; `ts` is the stream the two transposers go to (the side stream, or the main one when there is none).
 // dweight_is_zero: set where dweight was cleared along the way for a dW GEMM that adds into it.
-static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_backward_args* a, bool& dweight_is_zero) {
+static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_backward_args* a, bool dweight_apart,
+                                     bool& dweight_is_zero) {
   const uint32_t T = a->token_count, I = a->input_dim, O = a->output_dim;
   const uint32_t ok = padded_k(O), tk = padded_k(T);
   cudaStream_t s = S(stream);
@@ -1103,8 +1105,7 @@ static int backward_ms_eden_quantize(void* stream, void* ts, const nvfp4_linear_
   // two GEMMs cost c_attn at 8192 tokens 3 us and kept the second GEMM from being set up early.
   uint64_t zero_words = static_cast<uint64_t>(O) * I * (a->dweight_dtype == NVFP4_DTYPE_F32 ? 4 : 2);
   dweight_is_zero = ms_eden_pair_takes_amax(q, qt) && ((reinterpret_cast<uintptr_t>(a->dweight) | zero_words) & 15u) == 0 &&
-                    gemm_adds_into_output(dweight_gemm(a->dweight, a->dweight_dtype, T, I, O)) &&
-                    dweight_lies_apart(a, zero_words);
+                    dweight_apart && gemm_adds_into_output(dweight_gemm(a->dweight, a->dweight_dtype, T, I, O));
   zero_words = dweight_is_zero ? zero_words / 16 : 0;
   // one pass over dY for both orientations (+ column sums)
   rc = ms_eden_pair(stream, q, qt, partials, amax_in, amax_in ? a->e_h.global_scale : nullptr, amax_count, a->dweight,
@@ -1145,8 +1146,9 @@ int nvfp4_linear_backward_ms_eden(void* stream, const nvfp4_linear_backward_args
     ts = a->side_stream;
     forked = true;
   }
+  const bool dweight_apart = dweight_lies_apart(a, static_cast<size_t>(O) * I * (a->dweight_dtype == NVFP4_DTYPE_F32 ? 4 : 2));
   bool dweight_is_zero = false;
-  int rc = backward_ms_eden_quantize(stream, ts, a, dweight_is_zero);
+  int rc = backward_ms_eden_quantize(stream, ts, a, dweight_apart, dweight_is_zero);
   if (forked) {
     // join: the GEMMs need W^T and X^T; on an error path this leaves neither stream (nor a capture in
     // progress) dangling
@@ -1161,7 +1163,7 @@ int nvfp4_linear_backward_ms_eden(void* stream, const nvfp4_linear_backward_args
                         a->weight_t_h.scales_packed, a->weight_t_h.global_scale, a->e_t_h.bytes, a->e_t_h.scales_packed,
                         a->e_t_h.global_scales, a->input_t_h.bytes, a->input_t_h.scales_packed,
                         a->input_t_h.global_scale, a->dinput, a->dinput_dtype, a->dweight, a->dweight_dtype, T, I, O,
-                        dweight_is_zero);
+                        dweight_is_zero, dweight_apart);
 }
 
 }  // extern "C"

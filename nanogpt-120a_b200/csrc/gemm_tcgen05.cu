@@ -137,6 +137,7 @@ struct GemmParams {
   float weight;
   uint64_t wait_timeout_ns;  // limit of every mbarrier wait
   uint32_t debug_flags;      // bit 0: CTA 0 never loads its first k-tile (exercises the bounded waits)
+  uint32_t neighbour;        // GemmNeighbour
 #ifdef NVFP4_GEMM_TRACE
   unsigned long long* trace;  // measurement builds only: [5 roles][1024] (clock << 8 | tag) records of CTA 0
 #endif
@@ -265,6 +266,12 @@ __device__ __forceinline__ void epilogue_barrier(uint32_t group) {
 }
 
 __device__ __forceinline__ void wait_for_prior_kernels() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A GEMM beside its predecessor does not wait for it: that one let it start only behind its own wait, so that everything before
+// it is complete.
+__device__ __forceinline__ void wait_for_inputs(const GemmParams& p) {
+  if (p.neighbour != static_cast<uint32_t>(GemmNeighbour::kBesidePrior)) wait_for_prior_kernels();
+}
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -641,7 +648,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // Programmatic dependent launch: the CTA touches only its own SM up to the roles' waits for what runs before it in the stream,
   // each of which stands ahead of the role's first access to memory, behind the fetch of its code and of its first tile.  The
   // GEMM itself does not allow the next kernel to start early: its CTAs end at different times, and the first SMs that come
-  // free would take all of a small grid's CTAs.
+  // free would take all of a small grid's CTAs.  Another GEMM that needs nothing of it is the exception (GemmNeighbour).
   if (kPair)
     cluster_sync();
   else
@@ -751,7 +758,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = false;
           break;
         }
-        wait_for_prior_kernels();
+        wait_for_inputs(p);
         if (elect_one()) {
           mbar_expect_tx(bar_b_full, p.num_k_tiles * C::kBStageBytes);
           for (uint32_t kt = 0; kt < p.num_k_tiles; ++kt)
@@ -785,7 +792,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = false;
           break;
         }
-        if (issued == 0) wait_for_prior_kernels();
+        if (issued == 0) wait_for_inputs(p);
         GEMM_TRACE(0, 1, lane == 0);
         // test hook: this stage is never armed nor loaded, so its consumers' waits run out
         const bool skip = (p.debug_flags & kDebugSkipFirstLoad) && blockIdx.x == 0 && issued == 0;
@@ -966,7 +973,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (runs > 0 && !mbar_wait(bar_b_empty, (runs - 1) & 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) break;
         __syncwarp();
         tcgen05_fence_after();
-        wait_for_prior_kernels();
+        wait_for_inputs(p);
         const uint32_t first_blk128 = n_blk * kBlockN / 128u;
         const uint8_t* src = p.sfb + static_cast<size_t>(first_blk128) * p.k_atoms * kSfTileBytes + lane * 16;
         const size_t block_bytes = static_cast<size_t>(p.k_atoms) * kSfTileBytes;
@@ -1124,7 +1131,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // issuing the stores between two barriers of its group: 65536 x 2304 and x 3072 bf16 at K = 768, 87.3 -> 83.0 us and
     // 116.9 -> 111.3 us.
     if (kTmaStore) {
-      wait_for_prior_kernels();
+      wait_for_inputs(p);
       const uint32_t eg = warp - 2u;
       uint32_t buf = 0, phase = 0, tile_iter = 0, issued = 0;
       bool ok = true;
@@ -1257,7 +1264,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = true;  // warp uniform; false: some wait ran out, the rest of the list is walked without work
     const uint32_t my_bias = smem_bias + eg * kBlockN * 4;
     const float* my_bias_gen = reinterpret_cast<const float*>(smem_gen + (my_bias - smem_base));
-    wait_for_prior_kernels();
+    wait_for_inputs(p);
+    if (gtid == 0 && eg == 0 && p.neighbour == static_cast<uint32_t>(GemmNeighbour::kLetsNextBeside)) allow_next_kernel();
     const float gb = p.mode == NVFP4_GS_NONE ? 1.0f : load_prior(p.b_global);
     const float ga_scalar = p.mode == NVFP4_GS_TENSOR ? load_prior(p.a_global) : 1.0f;
     // the rows' global scales of a tile are fetched one tile ahead: their load latency would
@@ -1547,6 +1555,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(static_cast<uint32_t>(kTmemCols))
                    : "memory");
   }
+  // this grid is not complete before the one beside it
+  if (p.neighbour == static_cast<uint32_t>(GemmNeighbour::kBesidePrior) && blockIdx.x == 0) wait_for_prior_kernels();
 }
 
 // ---- host side ------------------------------------------------------------------------------
@@ -2140,7 +2150,7 @@ bool gemm_adds_into_output(const nvfp4_gemm_args& a) {
   return pl.k_splits > 1;
 }
 
-int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool row_amax_cleared) {
+int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool row_amax_cleared, GemmNeighbour neighbour) {
   if (a.m == 0 || a.n == 0) return 0;
   int rc = validate_gemm(a);
   if (rc) return rc;
@@ -2213,7 +2223,10 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool
   if (p.k_splits > 1 && !out_is_zero) {
     cudaError_t e = cudaMemset2DAsync(a.out, static_cast<size_t>(a.ldo) * esz, 0, static_cast<size_t>(a.n) * esz, a.m, s);
     if (e != cudaSuccess) return static_cast<int>(e);
+    neighbour = GemmNeighbour::kNone;  // not directly behind the other GEMM
   }
+  if (g_timing.enabled) neighbour = GemmNeighbour::kNone;  // events between the launches
+  p.neighbour = static_cast<uint32_t>(neighbour);
   if (a.relu2_row_amax && !row_amax_cleared) {
     cudaError_t e = cudaMemsetAsync(a.relu2_row_amax, 0, static_cast<size_t>(a.m) * sizeof(float), s);
     if (e != cudaSuccess) return static_cast<int>(e);

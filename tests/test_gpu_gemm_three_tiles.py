@@ -1,0 +1,41 @@
+"""Which GEMMs of three to four tiles a CTA keep their B panel: those whose banded schedule keeps every CTA busy; and that they compute
+what the narrow streaming tile computes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# (rows, columns, K): tile width, resident, CTAs per column block on 148 SMs
+@pytest.mark.parametrize("m,n,k,width,resident,cpn", [
+    (8192, 2304, 768, 256, 1, 16),    # 64 row blocks on 16 CTAs
+    (8100, 2304, 704, 256, 1, 16),    # ragged rows, K of three k-tiles less an atom
+    (4096, 2304, 768, 128, 1, 8),
+    (7424, 2304, 768, None, 0, 0),    # 58 row blocks: 3.6 turns of 16
+    (16384, 768, 768, None, None, None),
+])
+def test_three_tiles_a_cta(pkg, dev, m, n, k, width, resident, cpn):
+    if torch.cuda.get_device_properties(dev).multi_processor_count != 148:
+        pytest.skip("the expectations are for a 148-SM part")
+    q, gemm = pkg.Nvfp4QuantModule(), pkg.Nvfp4GemmModule()
+    g = torch.Generator(device=dev)
+    g.manual_seed(m + n)
+    x = q.quantize_four_six(torch.randn(m, k, generator=g, device=dev).to(torch.bfloat16), rowwise=True, packed=True)
+    w = q.quantize_four_six((torch.randn(n, k, generator=g, device=dev) * 0.02).to(torch.bfloat16), rowwise=False, packed=True)
+    bias = torch.randn(n, generator=g, device=dev)
+    plan = gemm.plan(x, w, bias=bias, epilogue=pkg.EPI_BIAS, out=torch.empty(m, n, device=dev, dtype=torch.bfloat16))
+    if width is not None:
+        assert (plan.block_n, plan.b_resident, plan.resident_cpn) == (width, resident, cpn)
+    elif resident is not None:
+        assert plan.block_n != 256 or plan.b_resident == resident
+    for dtype in (torch.bfloat16, torch.float32):
+        y = gemm.gemm(x, w, bias=bias, epilogue=pkg.EPI_BIAS, out_dtype=dtype)
+        pkg.set_gemm_tile_override(128)
+        try:
+            want = gemm.gemm(x, w, bias=bias, epilogue=pkg.EPI_BIAS, out_dtype=torch.float32)
+        finally:
+            pkg.set_gemm_tile_override(0)
+        # sums over K of 704 to 768 in f32, each of order sqrt(K) 0.02 beside a bias of order 1: a bf16 rounding, or some f32 ones
+        limit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -18
+        assert float((y.float() - want).norm() / want.norm()) < limit
+    assert pkg.read_device_status() == 0

@@ -1919,6 +1919,8 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
   // output or the stream they add to, more in the tall tile, where no main loop runs beside them.  Weighed like the TMA stores' epilogue they put 696 x 3101 x K 8320 bf16 on the
   // tall tile (87 us, 49 at 128 x 128), 1024 x 2979 x K 1536 too (71 us, 52) and split 768 x 1685 x K 12736 f32 five ways (47
   // us, 31 unsplit).
+  // Two outputs at 128 x 128 cost less than their first fit, at 4096 x 8192 x K 2048 alone, said (its buffers come in pairs): 8192 x
+  // 4096 x K 1024 f32 62 -> 51 us, bf16 38.7 -> 31.7, 1000 x 4096 14.2 -> 9.6, 4096 x 3072 x K 768 bf16 16.9 -> 13.3.
   struct Candidate {
     uint32_t splits;
     uint64_t cost;
@@ -1929,7 +1931,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
     constexpr uint64_t kTileCycles[4] = {550, 700, 850, 1050}, kResidentTileCycles = 300;
     constexpr uint64_t kPairTileCycles = 710, kPairF32Epilogue = 2000, kPairSetup = 6000;
     constexpr uint64_t kEpilogue[4] = {2000, 3000, 2500, 4000}, kF32Epilogue[4] = {4000, 3000, 6000, 6000};
-    constexpr uint64_t kSecondOutput[4] = {7500, 500, 3500, 12500}, kResidualTurns[4] = {0, 1000, 6000, 11000};
+    constexpr uint64_t kSecondOutput[4] = {0, 500, 3500, 7000}, kResidualTurns[4] = {0, 1000, 6000, 11000};
     constexpr uint64_t kDirectBf16[4] = {46000, 68000, 90000, 125000}, kDirectSecondBf16[4] = {26000, 42000, 57000, 92000};
     constexpr uint64_t kDirectF32[4] = {29000, 42000, 56000, 76000}, kDirectSecondF32[4] = {14000, 22000, 28000, 75000};
     constexpr uint64_t kDirectResidual[4] = {42000, 63000, 84000, 145000};
@@ -1939,6 +1941,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
                             (second ? (f32_out ? kDirectSecondF32 : kDirectSecondBf16)[shape] : 0);
     const uint64_t staged = kEpilogue[shape] + (second ? kSecondOutput[shape] : 0) + (f32_residual ? kResidualTurns[shape] : 0);
     const uint64_t ce = pl.tma_store ? staged : direct;
+    const bool two_outputs = second && pl.tma_store;
     Candidate best{1, ~0ull};
     uint32_t max_splits = 1;
     if (can_split && tiles < 2 * usms) {
@@ -1953,8 +1956,12 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
       const bool pair = pair_fits(bm, bn, real, per);
       const uint32_t waves = pair ? (pairs_of(real) + usms / 2 - 1) / (usms / 2) : (tiles * real + usms - 1) / usms;
       const uint64_t ck = resident_shape(bm, bn, real, tiles) ? kResidentTileCycles : pair ? kPairTileCycles : kTileCycles[shape];
-      const uint64_t cf = !f32_out || !pl.tma_store ? 0 : pair ? kPairF32Epilogue : kF32Epilogue[shape];
-      const uint64_t cost = waves * (per * ck + ce + cf) + (real > 1 ? kSplitCycles : 0) + (pair ? kPairSetup : 0);
+      const uint64_t cf = !f32_out || !pl.tma_store ? 0 : pair ? kPairF32Epilogue : two_outputs && shape == 0 ? 3000 : kF32Epilogue[shape];
+      // however short the main loop is: two outputs of a 128 x 192 tile take turns with its stores (one staging buffer a group), those
+      // of a 128 x 128 tile take their time to memory
+      const uint64_t least = !two_outputs || shape > 1 ? 0 : shape == 1 ? (f32_out ? 11500 : 7300) : (f32_out ? 6500 : 4000);
+      const uint64_t wave = per * ck + ce + cf;
+      const uint64_t cost = waves * (wave > least ? wave : least) + (real > 1 ? kSplitCycles : 0) + (pair ? kPairSetup : 0);
       if (cost < best.cost) best = Candidate{real, cost};  // ties go to fewer splits
     }
     return best;

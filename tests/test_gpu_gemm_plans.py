@@ -1,5 +1,5 @@
-"""Which GEMMs of three to four tiles a CTA keep their B panel: those whose banded schedule keeps every CTA busy; and that they compute
-what the narrow streaming tile computes."""
+"""Which GEMMs of three to four tiles a CTA keep their B panel (those whose banded schedule keeps every CTA busy), which tile two
+outputs take, and that they compute what another tile computes."""
 import pytest
 import torch
 
@@ -38,4 +38,36 @@ def test_three_tiles_a_cta(pkg, dev, m, n, k, width, resident, cpn):
         # sums over K of 704 to 768 in f32, each of order sqrt(K) 0.02 beside a bias of order 1: a bf16 rounding, or some f32 ones
         limit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -18
         assert float((y.float() - want).norm() / want.norm()) < limit
+    assert pkg.read_device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,dtype,width", [
+    (1000, 4096, 1024, torch.float32, 128), (1000, 4096, 1024, torch.bfloat16, 128), (2048, 4096, 1024, torch.float32, 128),
+    (4096, 3072, 768, torch.bfloat16, 128),
+    (4096, 8192, 2048, torch.float32, 192),   # a main loop that hides the turns of 192 columns
+    (8192, 3072, 768, torch.bfloat16, 256),   # resident, two staging buffers a group
+])
+def test_two_outputs(pkg, dev, m, n, k, dtype, width):
+    if torch.cuda.get_device_properties(dev).multi_processor_count != 148:
+        pytest.skip("the expectations are for a 148-SM part")
+    q, gemm = pkg.Nvfp4QuantModule(), pkg.Nvfp4GemmModule()
+    g = torch.Generator(device=dev)
+    g.manual_seed(m + n)
+    x = q.quantize_four_six(torch.randn(m, k, generator=g, device=dev).to(torch.bfloat16), rowwise=True, packed=True)
+    w = q.quantize_four_six((torch.randn(n, k, generator=g, device=dev) * 0.02).to(torch.bfloat16), rowwise=False, packed=True)
+    bias = torch.randn(n, generator=g, device=dev) * 0.02
+    out, pre = torch.empty(m, n, device=dev, dtype=dtype), torch.empty(m, n, device=dev, dtype=dtype)
+    kw = dict(bias=bias, epilogue=pkg.EPI_RELU2)
+    assert gemm.plan(x, w, out=out, aux=pre, **kw).block_n == width
+    gemm.gemm(x, w, out=out, aux=pre, **kw)
+    pkg.set_gemm_tile_override(192, 256)
+    try:
+        want_pre = torch.empty(m, n, device=dev)
+        want = gemm.gemm(x, w, out=torch.empty(m, n, device=dev), aux=want_pre, **kw)
+    finally:
+        pkg.set_gemm_tile_override(0)
+    # f32 sums over K up to 2048 in another order, or one bf16 rounding (doubled by the square)
+    limit = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -17
+    assert float((pre.float() - want_pre).norm() / want_pre.norm()) < limit
+    assert float((out.float() - want).norm() / want.norm()) < limit
     assert pkg.read_device_status() == 0

@@ -5,8 +5,10 @@
 // ms_eden/**), organised for the rate at which instructions issue: in the pair kernel the schedulers issue on 67 % of the
 // cycles, the FMA pipe is busy 61 % of them and the ALU 37 %, HBM 25 %.  Measured costs per warp instruction and scheduler are
 // 1 cycle for scalar FP32 (mixed f32 += bf16 * bf16 included, either half of a word), 2 for the packed f32x2 forms, and 2 for
-// integer, logic and conversion instructions; the two pipes overlap as far as register reads allow (a butterfly stage beside
-// two conversions 5.3 cycles instead of 8, beside two three-input maxima 7.7).  So:
+// integer, logic and conversion instructions, one for the rest.  Alone, a butterfly stage beside two conversions takes 5.3
+// cycles instead of 8 (beside two three-input maxima 7.7), but these kernels take the sum: of the 47.5 cycles of a scheduler for
+// an element of each lane the pair kernel's FP32 accounts for 26.8, integer, logic and conversions for 17.4 and the rest for 3;
+// the transposer's 31 are 14.5, 12.4 and 4.  So fewer and cheaper operations are what helps:
 //  * a bf16 source is widened, sign-flipped and taken through the first butterfly stage by mixed-precision FMAs,
 //    x * (+-1) + u (exact product, one rounding), which read either half of a word;
 //  * the E2M1 codes are widened with add.f32.f16 instead of cvt.f32.f16;

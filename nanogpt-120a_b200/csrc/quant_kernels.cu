@@ -1556,8 +1556,8 @@ static int launch_four_six_rows(cudaStream_t s, const Source& src, const float* 
 template <typename Source>
 static int launch_four_six_own_rows(cudaStream_t s, const Source& src, uint32_t rows, uint32_t plane_rows, uint32_t gpr, uint8_t* out_fp4,
                                     uint8_t* out_scales, int packed, float* out_gs, float* out_amax, float* decoded_amax) {
-  // Fewer than four warps an SM leave most of it idle while a lane quantizes its groups one after the other: 1000 x 768 2.75 us by
-  // four_six_rowwise_kernel, 2.87 here; 1500 x 768 3.17 and 2.87.
+  // Fewer than four warps an SM leave most of it idle while a lane quantizes its groups one after the other: 1000 x 768 2.48 us by
+  // four_six_rowwise_kernel, 2.87 here; 1500 x 768 3.17 (ahead of that kernel's early set-up) and 2.87.
   if (plane_rows / (gpr == 16 || gpr == 48 ? 2u : 1u) < 148u * 4u) return -1;
 #define NVFP4_ROWS(G, R)                                                                                                    \
   return launch_four_six_rows<Source, true, G, R>(s, src, nullptr, rows, plane_rows, gpr, out_fp4, out_scales, packed, out_gs, \

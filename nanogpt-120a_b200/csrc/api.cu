@@ -909,7 +909,8 @@ static int backward_gemms(cudaStream_t s, const uint8_t* eh_b, const uint8_t* eh
   g.k = padded_k(O);
   g.ldo = I;
   side_by_side = side_by_side && T != 0 && I != 0 && O != 0;
-  int rc = launch_gemm(s, g, false, false, side_by_side ? GemmNeighbour::kLetsNextBeside : GemmNeighbour::kNone);
+  GemmNeighbour dx = side_by_side ? GemmNeighbour::kLetsNextBeside : GemmNeighbour::kNone;
+  int rc = launch_gemm(s, g, false, false, dx, &dx);
   if (rc) return rc;
   g = dweight_gemm(dweight, dweight_dtype, T, I, O);
   g.a_bytes = et_b;
@@ -918,7 +919,8 @@ static int backward_gemms(cudaStream_t s, const uint8_t* eh_b, const uint8_t* eh
   g.b_bytes = xt_b;
   g.b_scales = xt_s;
   g.b_global = xt_g;
-  return launch_gemm(s, g, dweight_is_zero, false, side_by_side ? GemmNeighbour::kBesidePrior : GemmNeighbour::kNone);
+  return launch_gemm(s, g, dweight_is_zero, false,
+                     dx == GemmNeighbour::kLetsNextBeside ? GemmNeighbour::kBesidePrior : GemmNeighbour::kNone);
 }
 
 static int backward_device_scale(void* stream, const nvfp4_linear_backward_device_scale_args* a) {

@@ -2160,7 +2160,8 @@ bool gemm_adds_into_output(const nvfp4_gemm_args& a) {
   return pl.k_splits > 1;
 }
 
-int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool row_amax_cleared, GemmNeighbour neighbour) {
+int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool row_amax_cleared, GemmNeighbour neighbour,
+                GemmNeighbour* launched_as) {
   if (a.m == 0 || a.n == 0) return 0;
   int rc = validate_gemm(a);
   if (rc) return rc;
@@ -2233,10 +2234,12 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool
   if (p.k_splits > 1 && !out_is_zero) {
     cudaError_t e = cudaMemset2DAsync(a.out, static_cast<size_t>(a.ldo) * esz, 0, static_cast<size_t>(a.n) * esz, a.m, s);
     if (e != cudaSuccess) return static_cast<int>(e);
-    neighbour = GemmNeighbour::kNone;  // not directly behind the other GEMM
+    // not directly behind the other GEMM; one that lets its follower start has waited for the clearing by then
+    if (neighbour == GemmNeighbour::kBesidePrior) neighbour = GemmNeighbour::kNone;
   }
   if (g_timing.enabled) neighbour = GemmNeighbour::kNone;  // events between the launches
   p.neighbour = static_cast<uint32_t>(neighbour);
+  if (launched_as) *launched_as = neighbour;
   if (a.relu2_row_amax && !row_amax_cleared) {
     cudaError_t e = cudaMemsetAsync(a.relu2_row_amax, 0, static_cast<size_t>(a.m) * sizeof(float), s);
     if (e != cudaSuccess) return static_cast<int>(e);

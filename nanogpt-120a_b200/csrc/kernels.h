@@ -92,8 +92,10 @@ uint32_t relu2_backward_grid(uint64_t n);
 enum class GemmNeighbour { kNone, kLetsNextBeside, kBesidePrior };
 // out_is_zero: the output holds zeros already (it is cleared first where gemm_adds_into_output otherwise)
 // row_amax_cleared: so does a.relu2_row_amax
+// neighbour: the role asked for; launched_as: the one taken.  A GEMM that is timed, or would run beside its predecessor but clears
+// its output itself, takes none.
 int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero = false, bool row_amax_cleared = false,
-                GemmNeighbour neighbour = GemmNeighbour::kNone);
+                GemmNeighbour neighbour = GemmNeighbour::kNone, GemmNeighbour* launched_as = nullptr);
 // Whether launch_gemm splits K and sums the partial tiles in the output.
 bool gemm_adds_into_output(const nvfp4_gemm_args& a);
 // What launch_gemm would choose for these arguments on the current device (no launch).

@@ -2,6 +2,7 @@
 small and large grids, split K, with and without a side stream, captured."""
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 pytestmark = pytest.mark.gpu
 
@@ -34,12 +35,13 @@ class Call:
         return dx, dw
 
 
-# grids: a few tiles each; dX below and dW at the SMs' number; split K with the output cleared along the way; pairs; ragged; many
-# waves
+# grids: a few tiles each; dX below and dW at the SMs' number; split K with the output cleared along the way; pairs; ragged; dX split
+# and clearing its own output; many waves
 @pytest.mark.parametrize("tokens,i,o,dtype,grad", [
     (128, 256, 256, torch.bfloat16, torch.bfloat16), (1000, 768, 3072, torch.float32, torch.float32),
     (4096, 768, 768, torch.bfloat16, torch.bfloat16), (8192, 768, 2304, torch.bfloat16, torch.bfloat16),
     (1024, 1024, 8192, torch.bfloat16, torch.bfloat16), (515, 320, 264, torch.bfloat16, torch.float32),
+    (512, 768, 8192, torch.bfloat16, torch.float32),
     (16384, 1024, 4096, torch.bfloat16, torch.bfloat16)])
 @pytest.mark.parametrize("side", [False, True])
 def test_side_by_side_is_one_after_the_other(pkg, dev, tokens, i, o, dtype, grad, side):
@@ -67,3 +69,29 @@ def test_side_by_side_is_one_after_the_other(pkg, dev, tokens, i, o, dtype, grad
         assert pkg.read_device_status() == 0
     finally:
         pkg.set_deterministic_reductions(False)
+
+
+@pytest.mark.parametrize("tokens,dx_splits", [(1000, False), (512, True)])
+def test_dw_starts_before_dx_has_ended(pkg, dev, tokens, dx_splits):
+    """Also behind a dX whose output is cleared in front of it: its wait for what runs before it covers the clearing."""
+    i, o = 768, 8192 if dx_splits else 3072
+    c = Call(pkg, dev, tokens, i, o, torch.bfloat16, torch.float32, True)
+    c.run(0)
+    torch.cuda.synchronize()
+    e_h, weight_t_h = c.scratch.as_tensor("e_h"), c.scratch.as_tensor("weight_t_h")
+    assert (pkg.Nvfp4GemmModule().plan(e_h, weight_t_h, out=c.dx).k_splits > 1) == dx_splits
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+        c.run(0)
+    graph.replay()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
+        graph.replay()
+        torch.cuda.synchronize()
+    spans = sorted((e.time_range.start, e.time_range.end) for e in prof.events() if "nvfp4_gemm_tcgen05_kernel" in e.name)
+    if not spans:
+        pytest.skip("no kernel activity records on this machine")
+    (dx_start, dx_end), (dw_start, _) = spans
+    assert dw_start < dx_start + 0.75 * (dx_end - dx_start), spans
+    assert pkg.read_device_status() == 0

@@ -858,6 +858,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     }
+    // This grid is not complete before the one beside it.  One CTA waits, so that the SMs of the others go to the CTAs still to start
+    // (all of them: backward of 1000 x 3072 f32 39.4 -> 41.6 us), and its producer does: behind all roles, the test cost the
+    // streaming 128 x 256 bf16 form 36 bytes of spilled registers.
+    if (p.neighbour == static_cast<uint32_t>(GemmNeighbour::kBesidePrior) && blockIdx.x == 0) wait_for_prior_kernels();
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
     // The whole warp walks the loops so that tile / stage bookkeeping and the descriptors stay warp
@@ -1552,8 +1556,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(static_cast<uint32_t>(kTmemCols))
                    : "memory");
   }
-  // this grid is not complete before the one beside it
-  if (p.neighbour == static_cast<uint32_t>(GemmNeighbour::kBesidePrior) && blockIdx.x == 0) wait_for_prior_kernels();
 }
 
 // ---- host side ------------------------------------------------------------------------------

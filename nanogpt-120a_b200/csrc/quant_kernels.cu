@@ -260,10 +260,15 @@ __global__ void ms_eden_scale_from_amax_kernel(const float* __restrict__ amax, f
 // are taken the cheap way first (differences in scaled units, fused multiply-adds) and in the reference's order and
 // roundings only where the two lie closer together than both ways can differ.  Code for rare cases stands out of line, returns
 // by value and keeps nothing in local memory.  The scalar side of a group -- two quotients by the global scale, two reciprocals,
-// two E4M3 conversions -- is straight-line code, both candidates in the lanes of packed operations, for global scales inside
-// [2^-80, 2^80]; other global scales, NaN included, take the generic code per group.  One branch decides between cheap and exact
-// errors, one more takes the latter (24.5 -> 23.0 instructions an element, 65536 x 768 bf16 rowwise 46.4 -> 43.2 us in
-// four_six_rowwise_kernel, of zeros 73 -> 44).
+// two E4M3 conversions -- is straight-line code for global scales inside [2^-80, 2^80]; other global scales, NaN included, take
+// the generic code per group.  One branch decides between cheap and exact errors, one more takes the latter (24.5 -> 23.0
+// instructions an element, 65536 x 768 bf16 rowwise 46.4 -> 43.2 us in four_six_rowwise_kernel, of zeros 73 -> 44).
+//
+// Both candidates of the scalar side stand in the lanes of packed operations (kPacked) where warps have other groups to go on with:
+// fewer instructions, 4096 x 8192 bf16 with given maxima 20.3 -> 20.1 us, 20000 x 2048 with its own 27.3 -> 26.9.  Where a thread
+// has one group and little beside it, a group's chain counts, and a packed operation takes longer than a scalar one (with packs and
+// unpacks around it): scalar in four_six_kernel, the schedule-free weight of 3072 x 768 9.52 -> 9.39 us with its amax, 256 x 256
+// 5.22 -> 5.12, a tensor of 256 x 256 f32 2.01 -> 1.83, 300 x 768 f32 with given maxima 1.98 -> 1.88 (8192 x 768 5.99 -> 6.08).
 
 __device__ __forceinline__ float four_six_global_scale(float amax) {
   // utils/nvfp4/quant/kernels/four_six/helpers.rs:33-39 with scale_override = 1.0
@@ -287,6 +292,7 @@ __device__ __forceinline__ f32x2_t div_by_rcp2(f32x2_t a, f32x2_t b, f32x2_t y) 
 
 // What the groups of one global scale share.
 __device__ __noinline__ float four_six_global_scale_any(float amax) { return four_six_global_scale(amax); }
+template <bool kPacked>
 struct FourSixScale {
   float gs;       // global scale
   f32x2_t d, y;   // 6 gs + eps and 4 gs + eps, and their reciprocals
@@ -298,8 +304,14 @@ struct FourSixScale {
     gs = amax == 0.0f ? 1.0f : div_by_rcp(amax, 1536.0f, 1.0f / 1536.0f);
     const bool plain = gs >= 0x1p-80f && gs <= 0x1p80f;
     if (!plain) gs = four_six_global_scale_any(amax);
-    d = add2(mul2_rounded(pack2(gs, gs), pack2(6.0f, 4.0f)), pack2(kDenomEps, kDenomEps));
-    y = rcp_in_range2(d);
+    if (kPacked) {
+      d = add2(mul2_rounded(pack2(gs, gs), pack2(6.0f, 4.0f)), pack2(kDenomEps, kDenomEps));
+      y = rcp_in_range2(d);
+    } else {
+      const float d6 = 6.0f * gs + kDenomEps, d4 = 4.0f * gs + kDenomEps;
+      d = pack2(d6, d4);
+      y = pack2(rcp_in_range(d6), rcp_in_range(d4));
+    }
     limit = plain ? fminf(gs * 0x1p20f, 0x1p60f) : -1.0f;
   }
 };
@@ -397,12 +409,21 @@ __device__ __noinline__ FourSixChoice exact_choice_any(const Group16 g, float ga
 // v: one 16-group, ga its amax.  Returns the scale byte and writes the 8 nibble bytes into `packed`.
 // helpers.rs:42-76 and four_six.rs:309-344 of utils/nvfp4/quant/kernels.  The output nibbles are cvt(v * inv) with the
 // chosen candidate's inv, i.e. exactly that candidate's trial bytes.
-__device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float ga, const FourSixScale& sc, uint32_t opaque_zero,
+template <bool kPacked>
+__device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float ga, const FourSixScale<kPacked>& sc, uint32_t opaque_zero,
                                                    uint2& packed, float* decoded_amax = nullptr) {
   uint32_t codes;
   {
     float q6, q4;
-    unpack2(div_by_rcp2(pack2(ga, ga), sc.d, sc.y), q6, q4);
+    if (kPacked) {
+      unpack2(div_by_rcp2(pack2(ga, ga), sc.d, sc.y), q6, q4);
+    } else {
+      float d6, d4, y6, y4;
+      unpack2(sc.d, d6, d4);
+      unpack2(sc.y, y6, y4);
+      q6 = div_by_rcp(ga, d6, y6);
+      q4 = div_by_rcp(ga, d4, y4);
+    }
     uint16_t c;
     asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(c) : "f"(q4), "f"(q6));
     codes = c;
@@ -412,10 +433,17 @@ __device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float g
   asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"(static_cast<uint16_t>(codes)));
   const __half2 raw = *reinterpret_cast<const __half2*>(&h2);
   const float2 s = __half22float2(__hadd2(raw, __heq2(raw, __floats2half2_rn(0.0f, 0.0f))));
-  const f32x2_t step = mul2_rounded(pack2(s.x, s.y), pack2(sc.gs, sc.gs));
   float step6, step4, inv6, inv4;
-  unpack2(step, step6, step4);
-  unpack2(rcp_in_range2(add2(step, pack2(kDenomEps, kDenomEps))), inv6, inv4);
+  if (kPacked) {
+    const f32x2_t step = mul2_rounded(pack2(s.x, s.y), pack2(sc.gs, sc.gs));
+    unpack2(step, step6, step4);
+    unpack2(rcp_in_range2(add2(step, pack2(kDenomEps, kDenomEps))), inv6, inv4);
+  } else {
+    step6 = s.x * sc.gs;
+    step4 = s.y * sc.gs;
+    inv6 = rcp_in_range(step6 + kDenomEps);
+    inv4 = rcp_in_range(step4 + kDenomEps);
+  }
   Group16 g;
 #pragma unroll
   for (int i = 0; i < 8; ++i) g.V[i] = pack2(v[2 * i], v[2 * i + 1]);
@@ -672,11 +700,11 @@ __global__ void __launch_bounds__(256, 2)
         row_amax[kRows - 1] = max_f32(row_amax[kRows - 1], in_second[i] ? ga[i] : 0.0f);
       }
     }
-    FourSixScale sc[kRows];
+    FourSixScale<true> sc[kRows];
 #pragma unroll
     for (int h = 0; h < kRows; ++h) {  // non-negative floats order like their bit patterns
       if (kOwn) row_amax[h] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(row_amax[h])));
-      sc[h] = FourSixScale(row_amax[h]);
+      sc[h] = FourSixScale<true>(row_amax[h]);
     }
     if (kg0 == 0 && lane < kRows && row + lane < rows) {
       out_gs[row + lane] = lane ? sc[kRows - 1].gs : sc[0].gs;
@@ -688,7 +716,7 @@ __global__ void __launch_bounds__(256, 2)
     for (int i = 0; i < kGroups; ++i) {
       float v[16], d;
       words[i].widen(v);
-      FourSixScale mine = sc[0];
+      FourSixScale<true> mine = sc[0];
       if (in_second[i]) mine = sc[kRows - 1];
       uint2 nibbles;
       uint32_t b = four_six_group(v, ga[i], mine, opaque_zero, nibbles, decoded_amax ? &d : nullptr);
@@ -722,7 +750,7 @@ __global__ void __launch_bounds__(256, 4)
     tensor_amax = cta_max_of(amax, amax_count);
     if (out_amax && blockIdx.x == 0 && threadIdx.x == 0) out_amax[0] = tensor_amax;
   }
-  const FourSixScale tensor_scale(tensor_amax);
+  const FourSixScale<false> tensor_scale(tensor_amax);
   const uint32_t step = gridDim.x * 256u;
   // whole warps walk together: the scale bytes of neighbouring lanes leave in one store
   for (uint32_t g0 = blockIdx.x * 256u + (threadIdx.x & ~31u); g0 < groups; g0 += step) {
@@ -733,7 +761,7 @@ __global__ void __launch_bounds__(256, 4)
     if (in_plane && row < rows) {
       float v[16];
       src.load16(g, v);
-      const FourSixScale sc = kRowwise ? FourSixScale(amax[row]) : tensor_scale;
+      const FourSixScale<false> sc = kRowwise ? FourSixScale<false>(amax[row]) : tensor_scale;
       uint2 packed;
       float d;
       b = four_six_group(v, group_amax16(v), sc, opaque_zero, packed, decoded_amax ? &d : nullptr);
@@ -823,7 +851,7 @@ __global__ void __launch_bounds__(256, 3)
     uint32_t b = 0x38u;
     if (active) {
       const float amax = __uint_as_float(here[local_row]);
-      const FourSixScale sc(amax);
+      const FourSixScale<true> sc(amax);
       uint2 packed;
       float dec;
       b = four_six_group(v, ga, sc, opaque_zero, packed, decoded_amax ? &dec : nullptr);
@@ -900,7 +928,7 @@ __global__ void __launch_bounds__(256)
                            uint32_t padded_cols, uint64_t group_count, uint32_t opaque_zero) {
   const uint64_t g = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x;
   if (g >= group_count) return;
-  const FourSixScale sc(amax[0]);
+  const FourSixScale<false> sc(amax[0]);
   float v[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {

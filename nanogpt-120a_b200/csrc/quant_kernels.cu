@@ -1574,9 +1574,9 @@ static int launch_four_six_rows(cudaStream_t s, const Source& src, const float* 
                                 uint8_t* out_fp4, uint8_t* out_scales, int packed, float* out_gs, float* out_amax, float* decoded_amax) {
   const uint32_t per_row = kRows == 2 ? 1u : gpr / (32 * kGroups);
   const uint32_t units = kRows == 2 ? (plane_rows + 1) / 2 : plane_rows * per_row;
-  // CTAs of eight warps, as many of the latter as are resident where that gives each the same number of units, fewer otherwise
-  const uint32_t resident = 148u * 8u * 2u, per_warp = (units + resident - 1) / resident;
-  const uint32_t grid = ((units + per_warp - 1) / per_warp + 7) / 8;
+  // Every resident CTA of eight warps: an SM's units are what counts.  Fewer CTAs, each with the same number of units, put two of
+  // them on some SMs and one on the others: 2368 x 2048 bf16 6.5 -> 5.0 us, 1184 x 8192 with given maxima 9.3 -> 7.7.
+  const uint32_t grid = min((units + 7u) / 8u, 148u * 2u);
   return launch_chained(four_six_rows_kernel<Source, kOwn, kGroups, kRows>, grid, 256, 0, s, src, amax, out_fp4, out_scales, out_gs,
                         out_amax, decoded_amax, rows, plane_rows, units, gpr, FastDiv(per_row), packed, 0u);
 }
@@ -1584,9 +1584,14 @@ static int launch_four_six_rows(cudaStream_t s, const Source& src, const float* 
 template <typename Source>
 static int launch_four_six_own_rows(cudaStream_t s, const Source& src, uint32_t rows, uint32_t plane_rows, uint32_t gpr, uint8_t* out_fp4,
                                     uint8_t* out_scales, int packed, float* out_gs, float* out_amax, float* decoded_amax) {
-  // Fewer than four warps an SM leave most of it idle while a lane quantizes its groups one after the other: 1000 x 768 2.48 us by
-  // four_six_rowwise_kernel, 2.87 here; 1500 x 768 3.17 (ahead of that kernel's early set-up) and 2.87.
+  // Fewer than four warps an SM leave most of it idle while a lane quantizes its groups one after the other.  With three groups of
+  // two rows or four of one, whose chains are the longest, four_six_rowwise_kernel is the faster one as long as its CTAs are all
+  // resident (444 of five and two rows), and from 1185 to 1776 rows of 128 groups, where it needs its second turn and this kernel a
+  // second CTA on the SMs; us there and here, bf16: 1000 x 768 2.56, 2.83; 2048 x 768 2.74, 2.91; 2368 x 768 4.04, 3.50; 640 x 2048
+  // 2.69, 2.94; 1000 x 2048 4.03, 3.02; 1300 x 2048 4.07, 4.10 (f32 4.8, 5.2); 1776 x 2048 5.36, 4.17.
   if (plane_rows / (gpr == 16 || gpr == 48 ? 2u : 1u) < 148u * 4u) return -1;
+  if (gpr == 48 && plane_rows <= 444u * 5u) return -1;
+  if (gpr == 128 && (plane_rows <= 444u * 2u || (plane_rows > 148u * 8u && plane_rows <= 444u * 4u))) return -1;
 #define NVFP4_ROWS(G, R)                                                                                                    \
   return launch_four_six_rows<Source, true, G, R>(s, src, nullptr, rows, plane_rows, gpr, out_fp4, out_scales, packed, out_gs, \
                                                   out_amax, decoded_amax)
@@ -1635,13 +1640,18 @@ static int launch_four_six_source(cudaStream_t s, const Source& src, const float
   const uint32_t groups = static_cast<uint32_t>((pad_apart ? rows : plane_rows) * gpr);
   if constexpr (TakesGivenRows<Source>::value) {
     // bf16 sources; f32 ones are bound by HBM and L2 as they are (4096 x 8192 26.5 us one group at a time, 26.8 and more by
-    // rows).  With fewer than twelve warps an SM a lane's groups one after the other take longer: 500 x 4096 3.4 us in place of 3.8,
-    // 1000 x 4096 5.4 and 5.3.
-    if (rowwise && (gpr % 64 == 0 || gpr % 96 == 0) && plane_rows * (gpr / (gpr % 128 == 0 ? 128u : gpr % 96 == 0 ? 96u : 64u)) >= 148u * 12u) {
+    // rows).  A warp takes several groups of every lane at a time, so this pays where most warps have work in each turn, or there
+    // are many turns: plain and relu^2 us one group at a time and by rows, 888 x 6144 5.2, 6.4 and 6.8, 8.3; 1100 x 3072 5.0, 5.9 and
+    // 4.1, 4.9; 3000 x 4096 9.6, 11.6 and 9.5, 11.9; 8192 x 3072 18.5, 21.5 and 16.1, 19.4.  Two groups a lane gain less: 8192 x 1024
+    // 7.2, 8.3 and 7.4, 8.7; 16384 x 1024 13.3, 15.5 and 12.4, 14.6.
+    const uint64_t warps = 148u * 16u, form = gpr % 128 == 0 ? 4u : gpr % 96 == 0 ? 3u : 2u, units = plane_rows * (gpr / (32u * form));
+    const uint64_t turns = (units + warps - 1) / warps;
+    const bool by_rows = turns > (form == 2u ? 4u : 3u) || units * 10u >= turns * warps * (form > 2u && turns == 1 ? 8u : 9u);
+    if (rowwise && (gpr % 64 == 0 || gpr % 96 == 0) && by_rows) {
       const uint32_t launched_rows = static_cast<uint32_t>(pad_apart ? rows : plane_rows);
-      const auto launch = gpr % 128 == 0 ? launch_four_six_rows<Source, false, 4, 1>
-                          : gpr % 96 == 0 ? launch_four_six_rows<Source, false, 3, 1>
-                                          : launch_four_six_rows<Source, false, 2, 1>;
+      const auto launch = form == 4u   ? launch_four_six_rows<Source, false, 4, 1>
+                          : form == 3u ? launch_four_six_rows<Source, false, 3, 1>
+                                       : launch_four_six_rows<Source, false, 2, 1>;
       const int rc = launch(s, src, amax, rows, launched_rows, gpr, out_fp4, out_scales, packed, out_gs, nullptr, decoded_amax);
       return rc == 0 && pad_apart ? launch_packed_scale_pad(s, out_scales, rows, cols) : rc;
     }

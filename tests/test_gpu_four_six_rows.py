@@ -32,10 +32,12 @@ def values(rows, cols, dtype, seed):
     return torch.from_numpy(x).to(torch.bfloat16).float().numpy()
 
 
-# widths of the six forms; rows: below and at the first count that is taken (592 warps), odd, one more than whole 128-row blocks
+# widths of the six forms; rows: below and at the first count that is taken (592 warps; what four_six_rowwise_kernel does no longer
+# in one turn of its CTAs, 2220 rows of 768 and 888 of 2048), odd, one more than whole 128-row blocks, warps of several units
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("cols,rows", [(256, 1183), (256, 1185), (512, 592), (768, 1024), (768, 1185), (768, 4737), (1024, 593),
-                                       (1536, 641), (2048, 2369)])
+                                       (1536, 641), (2048, 2369), (768, 2220), (768, 2221), (2048, 888), (2048, 889), (2048, 1777),
+                                       (256, 14209)])
 @pytest.mark.parametrize("packed", [False, True])
 def test_own_rows(pkg, oracle, dev, dtype, cols, rows, packed):
     x = values(rows, cols, dtype, cols + rows)
@@ -43,7 +45,9 @@ def test_own_rows(pkg, oracle, dev, dtype, cols, rows, packed):
     check(oracle, t, x, oracle.row_amax(x))
 
 
-@pytest.mark.parametrize("cols,rows", [(2048, 1793), (3072, 887), (3072, 1281), (4096, 900), (4224, 1700), (6144, 889)])
+# two, three and four groups a lane, one unit a row and several; one turn of the warps, two, more; nearly full, and not enough
+@pytest.mark.parametrize("cols,rows", [(2048, 1793), (3072, 887), (3072, 1281), (4096, 900), (4224, 1700), (6144, 889), (1024, 2300),
+                                       (1024, 9601), (1536, 2001), (3072, 1100), (4096, 2300), (4096, 3585), (5120, 1300), (7680, 1500)])
 @pytest.mark.parametrize("relu2,packed", [(True, True), (True, False), (False, True)])
 def test_given_rows(pkg, oracle, dev, cols, rows, relu2, packed):
     q = pkg.Nvfp4QuantModule()

@@ -1919,7 +1919,11 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
   // tall tile (87 us, 49 at 128 x 128), 1024 x 2979 x K 1536 too (71 us, 52) and split 768 x 1685 x K 12736 f32 five ways (47
   // us, 31 unsplit).
   // Two outputs at 128 x 128 cost less than their first fit, at 4096 x 8192 x K 2048 alone, said (its buffers come in pairs): 8192 x
-  // 4096 x K 1024 f32 62 -> 51 us, bf16 38.7 -> 31.7, 1000 x 4096 14.2 -> 9.6, 4096 x 3072 x K 768 bf16 16.9 -> 13.3.
+  // 4096 x K 1024 f32 62 -> 51 us, bf16 38.7 -> 31.7, 1000 x 4096 14.2 -> 9.6, 4096 x 3072 x K 768 bf16 16.9 -> 13.3.  The other
+  // tiles' second outputs by the four tiles timed on 574 shapes (256 to 32768 rows, 256 to 16384 columns, K 256 to 8192, both types):
+  // the tile taken is 0.7 % slower than the fastest on average, 1.1 % with 3500 and 7000, which put 8192 x 12288 x K 4096 f32 (349 us,
+  // 289), 1024 x 12288 x K 8192 bf16 (60, 50) and 8192 x 16384 x K 3072 f32 (420, 351) on the tall tile; where it is the faster one by
+  // less, 1371 x 13768 x K 3648 bf16 (46, 50 at 128 x 192), they lose.
   struct Candidate {
     uint32_t splits;
     uint64_t cost;
@@ -1930,7 +1934,7 @@ void plan_gemm(const nvfp4_gemm_args& a, int sms, GemmPlan& pl, bool maps_refuse
     constexpr uint64_t kTileCycles[4] = {550, 700, 850, 1050}, kResidentTileCycles = 300;
     constexpr uint64_t kPairTileCycles = 710, kPairF32Epilogue = 2000, kPairSetup = 6000;
     constexpr uint64_t kEpilogue[4] = {2000, 3000, 2500, 4000}, kF32Epilogue[4] = {4000, 3000, 6000, 6000};
-    constexpr uint64_t kSecondOutput[4] = {0, 500, 3500, 7000}, kResidualTurns[4] = {0, 1000, 6000, 11000};
+    constexpr uint64_t kSecondOutput[4] = {0, 500, 3000, 9000}, kResidualTurns[4] = {0, 1000, 6000, 11000};
     constexpr uint64_t kDirectBf16[4] = {46000, 68000, 90000, 125000}, kDirectSecondBf16[4] = {26000, 42000, 57000, 92000};
     constexpr uint64_t kDirectF32[4] = {29000, 42000, 56000, 76000}, kDirectSecondF32[4] = {14000, 22000, 28000, 75000};
     constexpr uint64_t kDirectResidual[4] = {42000, 63000, 84000, 145000};

@@ -1575,7 +1575,7 @@ static int launch_four_six_rows(cudaStream_t s, const Source& src, const float* 
   const uint32_t per_row = kRows == 2 ? 1u : gpr / (32 * kGroups);
   const uint32_t units = kRows == 2 ? (plane_rows + 1) / 2 : plane_rows * per_row;
   // Every resident CTA of eight warps: an SM's units are what counts.  Fewer CTAs, each with the same number of units, put two of
-  // them on some SMs and one on the others: 2368 x 2048 bf16 6.5 -> 5.0 us, 1184 x 8192 with given maxima 9.3 -> 7.7.
+  // them on some SMs and one on the others: 2368 x 2048 bf16 6.5 -> 5.0 us, 1184 x 8192 with given maxima 9.2 -> 7.6.
   const uint32_t grid = min((units + 7u) / 8u, 148u * 2u);
   return launch_chained(four_six_rows_kernel<Source, kOwn, kGroups, kRows>, grid, 256, 0, s, src, amax, out_fp4, out_scales, out_gs,
                         out_amax, decoded_amax, rows, plane_rows, units, gpr, FastDiv(per_row), packed, 0u);
@@ -1587,8 +1587,8 @@ static int launch_four_six_own_rows(cudaStream_t s, const Source& src, uint32_t 
   // Fewer than four warps an SM leave most of it idle while a lane quantizes its groups one after the other.  With three groups of
   // two rows or four of one, whose chains are the longest, four_six_rowwise_kernel is the faster one as long as its CTAs are all
   // resident (444 of five and two rows), and from 1185 to 1776 rows of 128 groups, where it needs its second turn and this kernel a
-  // second CTA on the SMs; us there and here, bf16: 1000 x 768 2.56, 2.83; 2048 x 768 2.74, 2.91; 2368 x 768 4.04, 3.50; 640 x 2048
-  // 2.69, 2.94; 1000 x 2048 4.03, 3.02; 1300 x 2048 4.07, 4.10 (f32 4.8, 5.2); 1776 x 2048 5.36, 4.17.
+  // second CTA on the SMs; us there and here, bf16: 1000 x 768 2.61, 2.85; 2048 x 768 2.74, 2.83; 2368 x 768 4.08, 3.48; 640 x 2048
+  // 2.69, 2.91; 1000 x 2048 4.05, 3.00; 1300 x 2048 4.09, 4.07 (f32 4.64, 5.05); 1776 x 2048 5.36, 4.17.
   if (plane_rows / (gpr == 16 || gpr == 48 ? 2u : 1u) < 148u * 4u) return -1;
   if (gpr == 48 && plane_rows <= 444u * 5u) return -1;
   if (gpr == 128 && (plane_rows <= 444u * 2u || (plane_rows > 148u * 8u && plane_rows <= 444u * 4u))) return -1;
@@ -1641,9 +1641,9 @@ static int launch_four_six_source(cudaStream_t s, const Source& src, const float
   if constexpr (TakesGivenRows<Source>::value) {
     // bf16 sources; f32 ones are bound by HBM and L2 as they are (4096 x 8192 26.5 us one group at a time, 26.8 and more by
     // rows).  A warp takes several groups of every lane at a time, so this pays where most warps have work in each turn, or there
-    // are many turns: plain and relu^2 us one group at a time and by rows, 888 x 6144 5.2, 6.4 and 6.8, 8.3; 1100 x 3072 5.0, 5.9 and
-    // 4.1, 4.9; 3000 x 4096 9.6, 11.6 and 9.5, 11.9; 8192 x 3072 18.5, 21.5 and 16.1, 19.4.  Two groups a lane gain less: 8192 x 1024
-    // 7.2, 8.3 and 7.4, 8.7; 16384 x 1024 13.3, 15.5 and 12.4, 14.6.
+    // are many turns: plain and relu^2 us one group at a time and by rows, 888 x 6144 5.1, 6.1 and 5.4, 6.7; 1100 x 3072 4.3, 5.1 and
+    // 3.4, 4.3; 3000 x 4096 9.4, 11.3 and 9.3, 11.6; 8192 x 3072 17.6, 21.1 and 15.3, 18.9.  Two groups a lane gain less: 8192 x 1024
+    // 6.8, 8.2 and 7.0, 8.7; 16384 x 1024 12.3, 14.8 and 11.4, 13.9.
     const uint64_t warps = 148u * 16u, form = gpr % 128 == 0 ? 4u : gpr % 96 == 0 ? 3u : 2u, units = plane_rows * (gpr / (32u * form));
     const uint64_t turns = (units + warps - 1) / warps;
     const bool by_rows = turns > (form == 2u ? 4u : 3u) || units * 10u >= turns * warps * (form > 2u && turns == 1 ? 8u : 9u);

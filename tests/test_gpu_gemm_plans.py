@@ -45,6 +45,7 @@ def test_three_tiles_a_cta(pkg, dev, m, n, k, width, resident, cpn):
     (1000, 4096, 1024, torch.float32, 128), (1000, 4096, 1024, torch.bfloat16, 128), (2048, 4096, 1024, torch.float32, 128),
     (4096, 3072, 768, torch.bfloat16, 128),
     (4096, 8192, 2048, torch.float32, 192),   # a main loop that hides the turns of 192 columns
+    (4096, 12288, 3072, torch.float32, 192), (1024, 12288, 8192, torch.bfloat16, 256),   # not the tall tile
     (8192, 3072, 768, torch.bfloat16, 256),   # resident, two staging buffers a group
 ])
 def test_two_outputs(pkg, dev, m, n, k, dtype, width):
@@ -58,7 +59,8 @@ def test_two_outputs(pkg, dev, m, n, k, dtype, width):
     bias = torch.randn(n, generator=g, device=dev) * 0.02
     out, pre = torch.empty(m, n, device=dev, dtype=dtype), torch.empty(m, n, device=dev, dtype=dtype)
     kw = dict(bias=bias, epilogue=pkg.EPI_RELU2)
-    assert gemm.plan(x, w, out=out, aux=pre, **kw).block_n == width
+    plan = gemm.plan(x, w, out=out, aux=pre, **kw)
+    assert (plan.block_m, plan.block_n) == (128, width)
     gemm.gemm(x, w, out=out, aux=pre, **kw)
     pkg.set_gemm_tile_override(192, 256)
     try:
@@ -66,7 +68,7 @@ def test_two_outputs(pkg, dev, m, n, k, dtype, width):
         want = gemm.gemm(x, w, out=torch.empty(m, n, device=dev), aux=want_pre, **kw)
     finally:
         pkg.set_gemm_tile_override(0)
-    # f32 sums over K up to 2048 in another order, or one bf16 rounding (doubled by the square)
+    # f32 sums over K up to 8192 in another order, or one bf16 rounding (doubled by the square)
     limit = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -17
     assert float((pre.float() - want_pre).norm() / want_pre.norm()) < limit
     assert float((out.float() - want).norm() / want.norm()) < limit

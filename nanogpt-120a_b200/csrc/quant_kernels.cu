@@ -275,21 +275,6 @@ __device__ __forceinline__ float four_six_global_scale(float amax) {
   return nz(amax == 0.0f ? 1.0f : amax * 1.0f / (256.0f * 6.0f));
 }
 
-// Quotient a / b and reciprocal of two operands at once, correctly rounded in each lane (div_by_rcp, rcp_in_range).
-__device__ __forceinline__ f32x2_t neg2(f32x2_t v) { return v ^ 0x8000000080000000ull; }
-__device__ __forceinline__ f32x2_t rcp_in_range2(f32x2_t b) {
-  float lo, hi;
-  unpack2(b, lo, hi);
-  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(lo));
-  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(hi));
-  const f32x2_t y = pack2(lo, hi);
-  return fma2(y, fma2(neg2(b), y, pack2(1.0f, 1.0f)), y);
-}
-__device__ __forceinline__ f32x2_t div_by_rcp2(f32x2_t a, f32x2_t b, f32x2_t y) {
-  const f32x2_t q = mul2(a, y);
-  return fma2(fma2(neg2(b), q, a), y, q);
-}
-
 // What the groups of one global scale share.
 __device__ __noinline__ float four_six_global_scale_any(float amax) { return four_six_global_scale(amax); }
 template <bool kPacked>
@@ -454,10 +439,12 @@ __device__ __forceinline__ uint32_t four_six_group(const float (&v)[16], float g
   //                                                      | sqrt(e) - |D| |   <= 4.6 u |v| + 7 u |D|
   //   exact: q dq, the difference, square and sums:      | sqrt(err) - |D| | <= 2 u |v| + 3.5 u |D|
   // A scale byte of zero stands for the step gs in v * inv and for dq = 0: all q are 0 then, D = v, and with gs as the step
-  // the same bounds hold.  With |D| <= |v| <= 4 ga both candidates together shift sqrt(e6) - sqrt(e4) by less than 128 u ga,
-  // and ga is at most 9 steps of "six" (the largest quotient that rounds to the smallest scale byte is 1.5 times it) unless both
-  // scale bytes saturate.  Multiplied by sqrt(e6) + sqrt(e4) <= sqrt(2 (e6 + e4)) and squared: the order is certain where
-  // (e6 - e4)^2 exceeds 2 (1152 u)^2 < 2^-26 times e6 + e4.  Two candidates of one scale byte (zero groups, saturated ones) are
+  // the same bounds hold.  With |D| <= |v| <= 4 ga both candidates together shift sqrt(e6) - sqrt(e4) by less than 2 (4.6 + 7 + 2
+  // + 3.5) 4 u ga < 137 u ga, and ga is at most 9 steps of "six" (the largest quotient that rounds to the smallest scale byte is 1.5
+  // times it) unless both scale bytes saturate.  Multiplied by sqrt(e6) + sqrt(e4) <= sqrt(2 (e6 + e4)) and squared: the order is
+  // certain where (e6 - e4)^2 exceeds 2 (1233 u)^2 < 2^-26.4 times e6 + e4, and is taken for certain beyond 2^-26.  Where the byte of
+  // "six" alone is zero, the step of "four" is down to 2^-9 of it, 2^-52, and 1e-20 is below 757 u of that; but then ga is at most
+  // 6 * 2^-10 steps of "six", and (137 + 4 * 757) u ga below 19 u.  Two candidates of one scale byte (zero groups, saturated ones) are
   // the same candidate: "six", where the error is a number, and the same bytes either way.  Otherwise -- NaN, scales and values
   // outside the range of the bounds -- the exact errors decide.
   bool certain = false;
@@ -649,7 +636,7 @@ __device__ __forceinline__ float cta_max_of(const float* partials, uint32_t coun
 // whole rows, a row, or, where the rows' maxima are given (kOwn = false), a part of one.  All of them are loaded before the first
 // is quantized, the row maximum is a reduction of the warp, so that nothing ties the warps of a CTA together, and what depends
 // on the row alone -- its maximum, its scale, the place of its scale bytes -- is computed once.  Bound by issue slots like its
-// neighbours (20 instructions an element in place of 24, and four groups of a lane give the schedulers independent chains): bf16
+// neighbours (16 instructions an element in place of 24, and four groups of a lane give the schedulers independent chains): bf16
 // with own maxima 65536 x 768 46.4 -> 35.8 us, 8192 x 768 7.6 -> 5.9, 16384 x 2048 29.5 -> 20.7 (against a CTA per row block
 // with a barrier, four_six_rowwise_kernel, which takes the other widths and few rows); relu^2 with given maxima
 // 65536 x 3072 166 -> 146, 8192 x 4096 29.3 -> 25.3.  With 80 registers and three CTAs an SM 8192 x 768 took 8.1 us.
@@ -726,7 +713,6 @@ __global__ void __launch_bounds__(256, 2)
       if (!inside) b = 0x38u;  // pad rows of a packed plane hold 1.0
       if (row + (in_second[i] ? 1u : 0u) < plane_rows) scales[scale_at[i]] = static_cast<uint8_t>(b);
     }
-    if (u + warps < u) break;  // the index space ends below 2^32
   }
   if (decoded_amax) cta_atomic_max(warp_max(dec), decoded_amax);  // uniform across the CTA
 }

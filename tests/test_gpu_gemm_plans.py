@@ -6,13 +6,13 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# (rows, columns, K): tile width, resident, CTAs per column block on 148 SMs
+# (rows, columns, K): tile width, resident, CTAs per column block on 148 SMs, of a bf16 output
 @pytest.mark.parametrize("m,n,k,width,resident,cpn", [
     (8192, 2304, 768, 256, 1, 16),    # 64 row blocks on 16 CTAs
     (8100, 2304, 704, 256, 1, 16),    # ragged rows, K of three k-tiles less an atom
     (4096, 2304, 768, 128, 1, 8),
-    (7424, 2304, 768, None, 0, 0),    # 58 row blocks: 3.6 turns of 16
-    (16384, 768, 768, None, None, None),
+    (7424, 2304, 768, 192, 1, 12),    # 58 row blocks, 3.6 turns of 16: four tiles of 192 columns a CTA, not three of 256
+    (16384, 768, 768, 128, 1, 24),    # no panel of 256 columns here: it would take three CTAs of 128 row blocks, 49 a column block
 ])
 def test_three_tiles_a_cta(pkg, dev, m, n, k, width, resident, cpn):
     if torch.cuda.get_device_properties(dev).multi_processor_count != 148:
@@ -24,13 +24,12 @@ def test_three_tiles_a_cta(pkg, dev, m, n, k, width, resident, cpn):
     w = q.quantize_four_six((torch.randn(n, k, generator=g, device=dev) * 0.02).to(torch.bfloat16), rowwise=False, packed=True)
     bias = torch.randn(n, generator=g, device=dev)
     plan = gemm.plan(x, w, bias=bias, epilogue=pkg.EPI_BIAS, out=torch.empty(m, n, device=dev, dtype=torch.bfloat16))
-    if width is not None:
-        assert (plan.block_n, plan.b_resident, plan.resident_cpn) == (width, resident, cpn)
-    elif resident is not None:
-        assert plan.block_n != 256 or plan.b_resident == resident
+    assert (plan.block_m, plan.block_n, plan.b_resident, plan.resident_cpn) == (128, width, resident, cpn)
     for dtype in (torch.bfloat16, torch.float32):
-        y = gemm.gemm(x, w, bias=bias, epilogue=pkg.EPI_BIAS, out_dtype=dtype)
-        pkg.set_gemm_tile_override(128)
+        kw = dict(bias=bias, epilogue=pkg.EPI_BIAS, out=torch.empty(m, n, device=dev, dtype=dtype))
+        planned = gemm.plan(x, w, **kw).block_n
+        y = gemm.gemm(x, w, **kw)
+        pkg.set_gemm_tile_override(128 if planned != 128 else 192)
         try:
             want = gemm.gemm(x, w, bias=bias, epilogue=pkg.EPI_BIAS, out_dtype=torch.float32)
         finally:

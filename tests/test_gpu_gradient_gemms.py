@@ -1,5 +1,5 @@
 """dX and dW GEMM of a backward call beside one another: the same bits as one after the other, what follows on the stream sees both,
-small and large grids, split K, with and without a side stream, captured."""
+small and large grids, split K, with and without a side stream, captured, timed; one after the other where dW lies in dX's operands."""
 import pytest
 import torch
 from torch.profiler import ProfilerActivity, profile
@@ -95,3 +95,54 @@ def test_dw_starts_before_dx_has_ended(pkg, dev, tokens, dx_splits):
     (dx_start, dx_end), (dw_start, _) = spans
     assert dw_start < dx_start + 0.75 * (dx_end - dx_start), spans
     assert pkg.read_device_status() == 0
+
+
+@pytest.mark.parametrize("side", [False, True])
+@pytest.mark.parametrize("inside,field", [("e_h", "bytes"), ("weight_t_h", "bytes"), ("e_h", "scales_packed"), ("weight_t_h", "scales_packed")])
+def test_dweight_inside_the_operands_of_dx(pkg, dev, inside, field, side):
+    """dW may lie where dX's operands do, which its GEMM alone needs no longer: it then waits for all of dX.  Neither is split, so that
+    nothing is cleared between the two, and dX has more tiles than there are SMs."""
+    tokens, i, o = 3840, 2304, 768
+    c = Call(pkg, dev, tokens, i, o, torch.bfloat16, torch.bfloat16, side)
+    gemm = pkg.Nvfp4GemmModule()
+    dx_plan = gemm.plan(c.scratch.as_tensor("e_h"), c.scratch.as_tensor("weight_t_h"), out=c.dx)
+    tiles = -(-tokens // dx_plan.block_m) * -(-i // dx_plan.block_n)
+    assert dx_plan.k_splits == 1 and tiles > 2 * torch.cuda.get_device_properties(dev).multi_processor_count
+    assert gemm.plan(c.scratch.as_tensor("e_t_h"), c.scratch.as_tensor("input_t_h"), out=c.dw).k_splits == 1
+    want = []
+    for k in range(3):
+        c.run(k)
+        torch.cuda.synchronize()
+        want.append((c.dx.clone(), c.dw.clone()))
+    # the operand's plane in front of a buffer as large as dW (the call's extents stay what they are)
+    memory = torch.empty(o * i * 4, dtype=torch.uint8, device=dev)
+    getattr(c.scratch, inside)[field] = memory
+    c.dw = memory.view(torch.float32).view(o, i)
+    got = []
+    for k in range(6):
+        c.run(k % 3)
+        got.append((c.dx.clone(), c.dw.clone()))
+    torch.cuda.synchronize()
+    for k, (dx, dw) in enumerate(got):
+        assert torch.equal(dx, want[k % 3][0]) and torch.equal(dw, want[k % 3][1])
+    assert pkg.read_device_status() == 0
+
+
+@pytest.mark.parametrize("tokens,o", [(1000, 3072), (512, 8192)])
+def test_timed_one_after_the_other(pkg, dev, tokens, o):
+    """The events around each GEMM stand between the two."""
+    pkg.set_deterministic_reductions(True)
+    try:
+        c = Call(pkg, dev, tokens, 768, o, torch.bfloat16, torch.float32, True)
+        want = c.alone(0)
+        pkg.gemm_timing_begin(8)
+        try:
+            c.run(0)
+        finally:
+            timed = pkg.gemm_timing_end()
+        torch.cuda.synchronize()
+        assert timed[0] == 2
+        assert torch.equal(c.dx, want[0]) and torch.equal(c.dw, want[1])
+        assert pkg.read_device_status() == 0
+    finally:
+        pkg.set_deterministic_reductions(False)

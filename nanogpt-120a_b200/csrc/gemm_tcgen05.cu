@@ -137,7 +137,7 @@ struct GemmParams {
   float weight;
   uint64_t wait_timeout_ns;  // limit of every mbarrier wait
   uint32_t debug_flags;      // bit 0: CTA 0 never loads its first k-tile (exercises the bounded waits)
-  uint32_t neighbour;        // GemmNeighbour
+  uint32_t lets_next_beside;  // GemmNeighbour::kLetsNextBeside
 #ifdef NVFP4_GEMM_TRACE
   unsigned long long* trace;  // measurement builds only: [5 roles][1024] (clock << 8 | tag) records of CTA 0
 #endif
@@ -269,8 +269,9 @@ __device__ __forceinline__ void wait_for_prior_kernels() { asm volatile("griddep
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A GEMM beside its predecessor does not wait for it: that one let it start only behind its own wait, so that everything before
 // it is complete.
-__device__ __forceinline__ void wait_for_inputs(const GemmParams& p) {
-  if (p.neighbour != static_cast<uint32_t>(GemmNeighbour::kBesidePrior)) wait_for_prior_kernels();
+template <bool kBeside>
+__device__ __forceinline__ void wait_for_inputs() {
+  if (!kBeside) wait_for_prior_kernels();
 }
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
@@ -552,7 +553,9 @@ struct SubTile<__nv_bfloat16> {
 // [kBlockN x K] B panel of the current column block stays in shared memory -- one slot per
 // k-tile, its scale factors in tensor memory only -- while a CTA walks down the row blocks, so only A
 // tiles stream through the ring.  A CTA's last tile is staged over the A stages and B slots.
-template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel, bool kPair>
+// kBeside: launched with GemmNeighbour::kBesidePrior.  A form of its own, because a test at run time in the five roles' waits cost
+// every launch 2 % (24 shapes up to 9 us: 7136 x 448 x K 1344 f32 7.8 -> 8.4 us, 1000 x 1024 x K 4096 bf16 7.2 -> 7.5).
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel, bool kPair, bool kBeside>
 __global__ void __launch_bounds__(kThreads, 1)
     nvfp4_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                               const __grid_constant__ CUtensorMap tmap_out,
@@ -757,7 +760,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = false;
           break;
         }
-        wait_for_inputs(p);
+        wait_for_inputs<kBeside>();
         if (elect_one()) {
           mbar_expect_tx(bar_b_full, p.num_k_tiles * C::kBStageBytes);
           for (uint32_t kt = 0; kt < p.num_k_tiles; ++kt)
@@ -791,7 +794,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = false;
           break;
         }
-        if (issued == 0) wait_for_inputs(p);
+        if (issued == 0) wait_for_inputs<kBeside>();
         GEMM_TRACE(0, 1, lane == 0);
         // test hook: this stage is never armed nor loaded, so its consumers' waits run out
         const bool skip = (p.debug_flags & kDebugSkipFirstLoad) && blockIdx.x == 0 && issued == 0;
@@ -859,9 +862,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     // This grid is not complete before the one beside it.  One CTA waits, so that the SMs of the others go to the CTAs still to start
-    // (all of them: backward of 1000 x 3072 f32 39.4 -> 41.6 us), and its producer does: behind all roles, the test cost the
-    // streaming 128 x 256 bf16 form 36 bytes of spilled registers.
-    if (p.neighbour == static_cast<uint32_t>(GemmNeighbour::kBesidePrior) && blockIdx.x == 0) wait_for_prior_kernels();
+    // (all of them: backward of 1000 x 3072 f32 39.4 -> 41.6 us).
+    if (kBeside && blockIdx.x == 0) wait_for_prior_kernels();
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
     // The whole warp walks the loops so that tile / stage bookkeeping and the descriptors stay warp
@@ -980,7 +982,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (runs > 0 && !mbar_wait(bar_b_empty, (runs - 1) & 1u, abort_flag, kStatusMmaTimeout, p.wait_timeout_ns)) break;
         __syncwarp();
         tcgen05_fence_after();
-        wait_for_inputs(p);
+        wait_for_inputs<kBeside>();
         const uint32_t first_blk128 = n_blk * kBlockN / 128u;
         const uint8_t* src = p.sfb + static_cast<size_t>(first_blk128) * p.k_atoms * kSfTileBytes + lane * 16;
         const size_t block_bytes = static_cast<size_t>(p.k_atoms) * kSfTileBytes;
@@ -1132,7 +1134,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // issuing the stores between two barriers of its group: 65536 x 2304 and x 3072 bf16 at K = 768, 87.3 -> 83.0 us and
     // 116.9 -> 111.3 us.
     if (kTmaStore) {
-      wait_for_inputs(p);
+      wait_for_inputs<kBeside>();
       const uint32_t eg = warp - 2u;
       uint32_t buf = 0, phase = 0, tile_iter = 0, issued = 0;
       bool ok = true;
@@ -1265,8 +1267,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = true;  // warp uniform; false: some wait ran out, the rest of the list is walked without work
     const uint32_t my_bias = smem_bias + eg * kBlockN * 4;
     const float* my_bias_gen = reinterpret_cast<const float*>(smem_gen + (my_bias - smem_base));
-    wait_for_inputs(p);
-    if (gtid == 0 && eg == 0 && p.neighbour == static_cast<uint32_t>(GemmNeighbour::kLetsNextBeside)) allow_next_kernel();
+    wait_for_inputs<kBeside>();
+    if (gtid == 0 && eg == 0 && p.lets_next_beside) allow_next_kernel();
     const float gb = p.mode == NVFP4_GS_NONE ? 1.0f : load_prior(p.b_global);
     const float ga_scalar = p.mode == NVFP4_GS_TENSOR ? load_prior(p.a_global) : 1.0f;
     // the rows' global scales of a tile are fetched one tile ahead: their load latency would
@@ -1704,6 +1706,7 @@ struct GemmPlan {
   uint32_t block_m = 128, block_n = 128, num_n_blocks = 0, k_splits = 1, k_tiles_per_split = 0;
   uint32_t stages = 0, grid = 0, b_resident = 0, panel = 0, resident_cpn = 0, tma_store = 0, vec_store = 0, pair = 0;
   size_t smem_bytes = 0;
+  bool beside = false;  // GemmNeighbour::kBesidePrior
 };
 
 struct TileBytes {
@@ -1725,16 +1728,19 @@ TileBytes tile_bytes(uint32_t block_m, uint32_t block_n, uint32_t panel, bool pa
   return panel ? tile_bytes_of<128, 128, 4>() : tile_bytes_of<128, 128, 0>();
 }
 
-template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel, bool kPair = false>
+template <int kBlockM, int kBlockN, typename OutT, StorePath kStore, int kPanel, bool kPair = false, bool kBeside = false>
 int launch_schedule_variant(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo,
                          const CUtensorMap& mx, const GemmParams& p, const GemmPlan& pl) {
+  if constexpr (kStore == StorePath::kTma && !kBeside) {
+    if (pl.beside) return launch_schedule_variant<kBlockM, kBlockN, OutT, kStore, kPanel, kPair, true>(s, ma, mb, mo, mx, p, pl);
+  }
   // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
   static std::atomic<int> attr_state[kMaxDevices];  // 0 = not set, 1 = set, -(error) = failed
   const int dev = current_device();
   if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
   int st = attr_state[dev].load(std::memory_order_acquire);
   if (st == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel, kPair>,
+    const cudaError_t e = cudaFuncSetAttribute(nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel, kPair, kBeside>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
     st = e == cudaSuccess ? 1 : -static_cast<int>(e);
     attr_state[dev].store(st, std::memory_order_release);
@@ -1766,7 +1772,7 @@ int launch_schedule_variant(cudaStream_t s, const CUtensorMap& ma, const CUtenso
   cfg.attrs = attrs;
   cfg.numAttrs = kPair ? 2 : 1;
   int rc = static_cast<int>(
-      cudaLaunchKernelEx(&cfg, nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel, kPair>, ma, mb, mo, mx, p));
+      cudaLaunchKernelEx(&cfg, nvfp4_gemm_tcgen05_kernel<kBlockM, kBlockN, OutT, kStore, kPanel, kPair, kBeside>, ma, mb, mo, mx, p));
   count_launch();
   if (rc == 0) rc = static_cast<int>(cudaGetLastError());
   if (rec) cudaEventRecord(rec->stop, s);
@@ -2243,8 +2249,10 @@ int launch_gemm(cudaStream_t s, const nvfp4_gemm_args& a, bool out_is_zero, bool
     // not directly behind the other GEMM; one that lets its follower start has waited for the clearing by then
     if (neighbour == GemmNeighbour::kBesidePrior) neighbour = GemmNeighbour::kNone;
   }
+  if (neighbour == GemmNeighbour::kBesidePrior && !pl.tma_store) neighbour = GemmNeighbour::kNone;  // no such form
   if (g_timing.enabled) neighbour = GemmNeighbour::kNone;  // events between the launches
-  p.neighbour = static_cast<uint32_t>(neighbour);
+  p.lets_next_beside = neighbour == GemmNeighbour::kLetsNextBeside ? 1u : 0u;
+  pl.beside = neighbour == GemmNeighbour::kBesidePrior;
   if (launched_as) *launched_as = neighbour;
   if (a.relu2_row_amax && !row_amax_cleared) {
     cudaError_t e = cudaMemsetAsync(a.relu2_row_amax, 0, static_cast<size_t>(a.m) * sizeof(float), s);
